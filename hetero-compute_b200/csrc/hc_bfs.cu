@@ -10,8 +10,11 @@
 // HBM layout of the working set (W = ceil(N/32) words):
 //   depth, parent  int32[N]      outputs (caller's device buffer or ours)
 //   visited        uint32[W]     claimed vertices
-//   fb[3]          uint32[W]     frontier bitmaps: level L reads fb[L%3],
-//                                writes fb[(L+1)%3], zeroes fb[(L+2)%3]
+//   fb[3]          uint32[W]     frontier bitmaps of bottom-up levels: level L
+//                                reads fb[L%3], writes fb[(L+1)%3], zeroes
+//                                fb[(L+2)%3]; top-down levels keep a queue
+//                                only, and the first bottom-up level after
+//                                one builds its bitmap from the queue
 //   q[2]           int32[N]      frontier queues (top-down levels)
 //   tasks          int2[]        (vertex, chunk) pieces of long rows
 #include <algorithm>
@@ -41,6 +44,18 @@ constexpr int kHubWords = 4096;
 // memory only for neighbours whose summary bit is set (on a sparse frontier,
 // few: most rows that find no parent stop reading global memory).
 constexpr int kSumWords = 4096;
+// Thin top-down levels (at most kSoloCap vertices with at most kSoloEdges
+// edges, none of more than kSoloDeg) run on the team's first block alone, a
+// block barrier per level and the frontier in shared memory, for up to
+// kSoloLevels levels at a time while the other blocks wait at one grid
+// barrier.  Such a level is a chain of dependent L2 round trips: on the grid it
+// also pays the barrier and the global queue's counters.  The limits: one block keeps 2048
+// edges in flight, so above a few rounds of those the grid is faster; a row
+// longer than kSoloDeg would serialise on one warp.
+constexpr int kSoloCap = 1920;
+constexpr int kSoloEdges = 8192;
+constexpr int kSoloDeg = 128;
+constexpr int kSoloLevels = 1024;
 
 struct LevelCnt {
     int nf;                 // vertices in this frontier
@@ -54,6 +69,10 @@ struct BfsCtl {
     int conv;               // bitmap -> queue conversion counter
     int levels, td_levels, bu_levels;
     unsigned long long vscan, escan, reached;
+    struct {
+        int L, nf, td_levels;
+        long long edges_to_check, num_edges;
+    } solo;                  // loop state after the first block's thin levels
     struct {
         int mode, nf;
         unsigned long long t_ns;
@@ -110,13 +129,12 @@ __device__ __forceinline__ uint32_t frontier_word_sum(const uint32_t *s_fb, int 
 }
 
 // Top-down edge visitor: claim an unvisited neighbour with a CAS on its
-// parent, mark it visited and in the next frontier, queue it.
+// parent, mark it visited, queue it.
 struct TopDownVisit {
     const int64_t *index;
     const int32_t *nbr;
     int32_t *parent, *depth;
-    uint32_t *visited, *fnext, *snext;
-    int cs;
+    uint32_t *visited;
     int32_t *qnext;
     int *qlen;
     int next_depth;
@@ -127,7 +145,7 @@ struct TopDownVisit {
     };
     __device__ __forceinline__ void load(Item &it, int32_t u, int64_t e) {
         it.u = u;
-        it.v = nbr[e];
+        it.v = __ldg(nbr + e);
     }
     __device__ __forceinline__ void probe(Item &it) { it.word = __ldcg(visited + (it.v >> 5)); }
     // Stages across the round's items: all CASes in flight, then the marks,
@@ -145,22 +163,184 @@ struct TopDownVisit {
             take[j] = take[j] && old[j] == -1;
             v[j] = take[j] ? it[j].v : 0;
             if (take[j]) {
-                const uint32_t bit = 1u << (v[j] & 31);
                 depth[v[j]] = next_depth;
-                atomicOr(visited + (v[j] >> 5), bit);
-                frontier_add(fnext, snext, cs, v[j]);
-                mf += (unsigned long long)(index[v[j] + 1] - index[v[j]]);
+                atomicOr(visited + (v[j] >> 5), 1u << (v[j] & 31));
             }
         }
+#pragma unroll
+        for (int j = 0; j < kUnroll; j++)
+            if (take[j]) mf += (unsigned long long)(__ldg(index + v[j] + 1) - __ldg(index + v[j]));
         warp_append_n(take, v, qnext, qlen);
     }
+};
+
+// Shared-memory queue of the thin levels: vertex, and its row's first slot and
+// degree packed (44 + 20 bits, the degree clamped).
+struct SoloQueue {
+    int32_t u[kSoloCap];
+    unsigned long long row[kSoloCap];
+};
+constexpr unsigned long long kSoloDegMask = (1ull << 20) - 1ull;
+__device__ __forceinline__ unsigned long long solo_row(int64_t b, int64_t d) {
+    return ((unsigned long long)b << 20) | min((unsigned long long)d, kSoloDegMask);
+}
+
+// Thin top-down levels from level *L on, by one block (every thread calls it).
+// The same level as the grid's (claim by CAS on parent, mark, queue), with the
+// queue in shared memory and mirrored in the global queue, so that the grid can
+// take any level over.  Stops before a level that is too wide, that the
+// direction rule turns bottom-up, after kSoloLevels levels, or when the queue
+// is empty.  Returns with the loop state updated in every thread.
+template <bool kStats>
+__device__ __forceinline__ void solo_levels(const BfsArgs &a, BfsCtl *ctl, SoloQueue *sq, int &L, int &nf,
+                                            int &td_levels, long long &edges_to_check, long long &num_edges,
+                                            unsigned long long &my_vscan, unsigned long long &my_escan) {
+    __shared__ int s_n[3];
+    __shared__ unsigned long long s_mf[3];
+    __shared__ int s_wide[3];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    const unsigned lt = (1u << lane) - 1u;
+    const int32_t *qin = (L & 1) ? a.q1 : a.q0;
+    if (threadIdx.x < 3) {
+        s_n[threadIdx.x] = 0;
+        s_mf[threadIdx.x] = 0ull;
+        s_wide[threadIdx.x] = 0;
+    }
+    __syncthreads();
+    unsigned long long edges = 0;
+    for (int i = threadIdx.x; i < nf; i += blockDim.x) {
+        const int32_t u = __ldcg(qin + i);
+        const int64_t b = __ldg(a.index + u), d = __ldg(a.index + u + 1) - b;
+        sq[0].u[i] = u;
+        sq[0].row[i] = solo_row(b, d);
+        edges += (unsigned long long)d;
+        if (d > kSoloDeg) s_wide[0] = 1;
+    }
+    // The frontier's own edges: after a bottom-up level num_edges is not their count.
+    edges = warp_sum(edges);
+    if (lane == 0 && edges) atomicAdd(&s_mf[0], edges);
+    __syncthreads();
+    bool wide = s_wide[0] || s_mf[0] > (unsigned long long)kSoloEdges;
+    for (int step = 0; step < kSoloLevels; step++) {
+        const int ns = (step + 1) % 3;
+        if (nf == 0 || nf > kSoloCap || wide || L >= a.max_levels ||
+            (a.direction == 0 && num_edges > edges_to_check / a.alpha))
+            break;
+        const SoloQueue &cq = sq[step & 1];
+        SoloQueue &nq = sq[(step + 1) & 1];
+        int32_t *qnext = (L & 1) ? a.q0 : a.q1;
+        edges_to_check -= num_edges;
+        td_levels++;
+        if (threadIdx.x == 0) {
+            s_n[(step + 2) % 3] = 0;
+            s_mf[(step + 2) % 3] = 0ull;
+            s_wide[(step + 2) % 3] = 0;
+            if (L < kTraceLevels) {
+                ctl->trace[L].mode = 1;
+                ctl->trace[L].nf = nf;
+                ctl->trace[L].t_ns = globaltimer_ns();
+            }
+            if (kStats) {
+                my_vscan += nf;
+                my_escan += num_edges;
+            }
+        }
+        const int per = min(32, max(1, (nf + nwarps - 1) / nwarps));
+        for (int base = wib * per; base < nf; base += nwarps * per) {
+            const int i = base + lane;
+            const bool mine = lane < per && i < nf;
+            const int32_t u = mine ? cq.u[i] : -1;
+            const unsigned long long row = mine ? cq.row[i] : 0ull;
+            const long long beg = (long long)(row >> 20);
+            int total;
+            const int excl = warp_exclusive_scan((int)(row & kSoloDegMask), &total);
+            for (int k0 = 0; k0 < total; k0 += 32 * kUnroll) {
+                int32_t v[kUnroll], from[kUnroll];
+                uint32_t word[kUnroll];
+                bool take[kUnroll];
+#pragma unroll
+                for (int j = 0; j < kUnroll; j++) {
+                    const int k = k0 + 32 * j + lane;
+                    int lo = 0;
+#pragma unroll
+                    for (int st = 16; st > 0; st >>= 1) {
+                        const int c = __shfl_sync(kFull, excl, lo + st);
+                        if (c <= k) lo += st;
+                    }
+                    from[j] = __shfl_sync(kFull, u, lo);
+                    const long long bo = __shfl_sync(kFull, beg, lo);
+                    const int off = k - __shfl_sync(kFull, excl, lo);
+                    take[j] = k < total;
+                    v[j] = take[j] ? __ldg(a.nbr + bo + off) : 0;
+                }
+#pragma unroll
+                for (int j = 0; j < kUnroll; j++) word[j] = take[j] ? __ldcg(a.visited + (v[j] >> 5)) : ~0u;
+#pragma unroll
+                for (int j = 0; j < kUnroll; j++)
+                    from[j] = (word[j] >> (v[j] & 31)) & 1u ? 0 : atomicCAS(a.parent + v[j], -1, from[j]);
+#pragma unroll
+                for (int j = 0; j < kUnroll; j++) take[j] = from[j] == -1;
+                unsigned bal[kUnroll];
+                int count = 0;
+#pragma unroll
+                for (int j = 0; j < kUnroll; j++) {
+                    bal[j] = __ballot_sync(kFull, take[j]);
+                    count += __popc(bal[j]);
+                }
+                if (count == 0) continue;
+                int pos = 0;
+                if (lane == 0) pos = atomicAdd(&s_n[ns], count);
+                pos = __shfl_sync(kFull, pos, 0);
+                int64_t nb[kUnroll], nd[kUnroll];
+#pragma unroll
+                for (int j = 0; j < kUnroll; j++) {
+                    nb[j] = take[j] ? __ldg(a.index + v[j]) : 0;
+                    nd[j] = take[j] ? __ldg(a.index + v[j] + 1) : 0;
+                }
+                unsigned long long dsum = 0;
+#pragma unroll
+                for (int j = 0; j < kUnroll; j++) {
+                    if (take[j]) {
+                        const int p = pos + __popc(bal[j] & lt);
+                        a.depth[v[j]] = L + 1;
+                        atomicOr(a.visited + (v[j] >> 5), 1u << (v[j] & 31));
+                        qnext[p] = v[j];
+                        if (p < kSoloCap) {
+                            nq.u[p] = v[j];
+                            nq.row[p] = solo_row(nb[j], nd[j] - nb[j]);
+                        }
+                        dsum += (unsigned long long)(nd[j] - nb[j]);
+                        if (nd[j] - nb[j] > kSoloDeg) s_wide[ns] = 1;
+                    }
+                    pos += __popc(bal[j]);
+                }
+                dsum = warp_sum(dsum);
+                if (lane == 0) atomicAdd(&s_mf[ns], dsum);
+            }
+        }
+        __syncthreads();
+        nf = s_n[ns];
+        num_edges = (long long)s_mf[ns];
+        wide = s_wide[ns] || num_edges > kSoloEdges;
+        L++;
+    }
+}
+
+// Shared memory of one block: the hub prefix and the summary of the frontier
+// bitmap (bottom-up levels), or the two queues of the thin levels.
+union BfsShared {
+    struct {
+        uint32_t fb[kHubWords];
+        uint32_t sum[kSumWords];
+    } bu;
+    SoloQueue solo[2];
 };
 
 template <bool kStats>
 __global__ void __launch_bounds__(kBfsThreads, 2) bfs_persistent(BfsArgs a) {
     __shared__ unsigned long long s_red[32];
-    __shared__ uint32_t s_fb[kHubWords];
-    __shared__ uint32_t s_sum[kSumWords];
+    __shared__ BfsShared sh;
+    uint32_t *const s_fb = sh.bu.fb, *const s_sum = sh.bu.sum;
     BfsCtl *ctl = a.ctl;
     const int lane = threadIdx.x & 31;
     const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -170,11 +350,11 @@ __global__ void __launch_bounds__(kBfsThreads, 2) bfs_persistent(BfsArgs a) {
     const int W_act = (a.n_active + 31) >> 5;
 
     for (int i = gtid; i < a.n; i += nthreads) {
-        a.depth[i] = -1;
-        a.parent[i] = -1;
+        a.depth[i] = i == a.src ? 0 : -1;
+        a.parent[i] = i == a.src ? i : -1;
     }
     for (int i = gtid; i < W; i += nthreads) {
-        a.visited[i] = 0;
+        a.visited[i] = i == (a.src >> 5) ? 1u << (a.src & 31) : 0u;
         a.fb0[i] = 0;
         a.fb1[i] = 0;
         a.fb2[i] = 0;
@@ -185,31 +365,35 @@ __global__ void __launch_bounds__(kBfsThreads, 2) bfs_persistent(BfsArgs a) {
         a.sb2[i] = 0;
     }
     const unsigned long long t_start = globaltimer_ns();
-    if (!grid_barrier(&ctl->gs)) return;
     if (gtid == 0) {
-        const int32_t s = a.src;
-        a.depth[s] = 0;
-        a.parent[s] = s;
-        a.visited[s >> 5] = 1u << (s & 31);
-        a.fb0[s >> 5] = 1u << (s & 31);
-        a.sb0[((s >> 5) >> a.sum_shift) >> 5] = 1u << (((s >> 5) >> a.sum_shift) & 31);
-        a.q0[0] = s;
+        a.q0[0] = a.src;
         ctl->cnt[0].nf = 1;
-        ctl->cnt[0].mf = (unsigned long long)(a.index[s + 1] - a.index[s]);
+        ctl->cnt[0].mf = (unsigned long long)(a.index[a.src + 1] - a.index[a.src]);
     }
     if (!grid_barrier(&ctl->gs)) return;
 
     // Direction state (identical in every block).
     bool push = a.direction != 2;
     bool have_queue = true;
+    // Thin levels may go to one block; a level of the whole grid lies between two
+    // such turns, so that nobody still reads the state of the last one.
+    bool solo_ok = true;
+    bool bitmaps_clear = true;  // all three frontier bitmaps are zero (no bottom-up level yet)
     long long edges_to_check = a.m;
     long long num_edges = (long long)(a.index[a.src + 1] - a.index[a.src]);
-    unsigned long long my_vscan = 0, my_escan = 0, my_found = 0;
+    unsigned long long my_vscan = 0, my_escan = 0;
     int L = 0, td_levels = 0, bu_levels = 0;
+    // The level counters rotate with the levels that the whole grid runs: the
+    // thin levels of one block leave them alone, since other blocks may still
+    // be reading those of the last one.
+    int C = 0;
+    int solo_nf = -1;  // frontier size after thin levels (-1: in the counters)
 
     for (;;) {
         const int cur = L % 3, nxt = (L + 1) % 3, old = (L + 2) % 3;
-        int nf = __ldcg(&ctl->cnt[cur].nf);
+        LevelCnt *const ccur = &ctl->cnt[C % 3], *const cnxt = &ctl->cnt[(C + 1) % 3];
+        int nf = solo_nf >= 0 ? solo_nf : __ldcg(&ccur->nf);
+        solo_nf = -1;
         if (nf == 0) break;
         if (L >= a.max_levels) {
             if (gtid == 0) atomicExch(&ctl->gs.err, (int)HC_ERR_NOT_CONVERGED);
@@ -217,14 +401,13 @@ __global__ void __launch_bounds__(kBfsThreads, 2) bfs_persistent(BfsArgs a) {
         }
         if (gtid == 0) {
             if (globaltimer_ns() - t_start > c_limits.run_ns) atomicExch(&ctl->gs.err, (int)HC_ERR_TIMEOUT);
-            ctl->cnt[old].nf = 0;
-            ctl->cnt[old].tasks = 0;
-            ctl->cnt[old].mf = 0;
+            LevelCnt *const cold = &ctl->cnt[(C + 2) % 3];
+            cold->nf = 0;
+            cold->tasks = 0;
+            cold->mf = 0;
         }
         uint32_t *fcur = fb_sel(a, cur), *fnext = fb_sel(a, nxt), *fold = fb_sel(a, old);
         uint32_t *scur = sb_sel(a, cur), *snext = sb_sel(a, nxt), *sold = sb_sel(a, old);
-        for (int i = gtid; i < W_act; i += nthreads) fold[i] = 0;
-        for (int i = gtid; i < a.sum_words; i += nthreads) sold[i] = 0;
         int32_t *qcur = (L & 1) ? a.q1 : a.q0;
         int32_t *qnext = (L & 1) ? a.q0 : a.q1;
 
@@ -256,11 +439,35 @@ __global__ void __launch_bounds__(kBfsThreads, 2) bfs_persistent(BfsArgs a) {
                 nf = __ldcg(&ctl->conv);
                 have_queue = true;
             }
+            if (solo_ok && nf <= kSoloCap && num_edges <= kSoloEdges) {
+                const int L0 = L;
+                solo_ok = false;
+                if (blockIdx.x == 0) {
+                    solo_levels<kStats>(a, ctl, sh.solo, L, nf, td_levels, edges_to_check, num_edges, my_vscan,
+                                        my_escan);
+                    if (threadIdx.x == 0) {
+                        ctl->solo.L = L;
+                        ctl->solo.nf = nf;
+                        ctl->solo.td_levels = td_levels;
+                        ctl->solo.edges_to_check = edges_to_check;
+                        ctl->solo.num_edges = num_edges;
+                    }
+                }
+                if (!grid_barrier(&ctl->gs)) return;
+                L = __ldcg(&ctl->solo.L);
+                if (L != L0) {
+                    solo_nf = __ldcg(&ctl->solo.nf);
+                    td_levels = __ldcg(&ctl->solo.td_levels);
+                    edges_to_check = __ldcg(&ctl->solo.edges_to_check);
+                    num_edges = __ldcg(&ctl->solo.num_edges);
+                    continue;
+                }
+            }
             edges_to_check -= num_edges;
             td_levels++;
             const int next_depth = L + 1;
-            TopDownVisit visit{a.index, a.nbr, a.parent, a.depth, a.visited, fnext, snext, a.sum_shift, qnext,
-                               &ctl->cnt[nxt].nf, next_depth, 0ull};
+            TopDownVisit visit{a.index, a.nbr, a.parent, a.depth, a.visited, qnext, &cnxt->nf, next_depth,
+                               0ull};
             if (kStats) {
                 for (int i = gtid; i < nf; i += nthreads) {
                     const int32_t u = __ldcg(qcur + i);
@@ -268,18 +475,41 @@ __global__ void __launch_bounds__(kBfsThreads, 2) bfs_persistent(BfsArgs a) {
                 }
                 if (gtid == 0) my_vscan += nf;
             }
-            expand_small(a.index, qcur, nf, a.tasks, &ctl->cnt[cur].tasks, gwarp, nwarps, visit);
-            if (!grid_barrier(&ctl->gs)) return;
-            const int nt = __ldcg(&ctl->cnt[cur].tasks);
-            if (nt > 0) {
-                expand_tasks(a.index, a.tasks, nt, gwarp, nwarps, visit);
-            }
+            expand_small(a.index, qcur, nf, a.tasks, &ccur->tasks, gwarp, nwarps, visit);
             unsigned long long mf_blk = block_sum(visit.mf, s_red);
-            if (threadIdx.x == 0 && mf_blk) atomicAdd(&ctl->cnt[nxt].mf, mf_blk);
+            if (threadIdx.x == 0 && mf_blk) atomicAdd(&cnxt->mf, mf_blk);
             if (!grid_barrier(&ctl->gs)) return;
-            num_edges = (long long)__ldcg(&ctl->cnt[nxt].mf);
+            const int nt = __ldcg(&ccur->tasks);
+            if (nt > 0) {
+                visit.mf = 0;
+                expand_tasks(a.index, a.tasks, nt, gwarp, nwarps, visit);
+                mf_blk = block_sum(visit.mf, s_red);
+                if (threadIdx.x == 0 && mf_blk) atomicAdd(&cnxt->mf, mf_blk);
+                if (!grid_barrier(&ctl->gs)) return;
+            }
+            num_edges = (long long)__ldcg(&cnxt->mf);
             have_queue = true;
         } else {
+            if (have_queue) {
+                // Frontier came from a top-down level: set its bits.  This
+                // level's and the next one's bitmaps must be zero first.
+                if (!bitmaps_clear) {
+                    for (int i = gtid; i < W_act; i += nthreads) {
+                        fcur[i] = 0;
+                        fnext[i] = 0;
+                    }
+                    for (int i = gtid; i < a.sum_words; i += nthreads) {
+                        scur[i] = 0;
+                        snext[i] = 0;
+                    }
+                    if (!grid_barrier(&ctl->gs)) return;
+                }
+                for (int i = gtid; i < nf; i += nthreads) frontier_add(fcur, scur, a.sum_shift, __ldcg(qcur + i));
+                if (!grid_barrier(&ctl->gs)) return;
+            }
+            bitmaps_clear = false;
+            for (int i = gtid; i < W_act; i += nthreads) fold[i] = 0;
+            for (int i = gtid; i < a.sum_words; i += nthreads) sold[i] = 0;
             bu_levels++;
             const int next_depth = L + 1;
             int found_local = 0;
@@ -380,18 +610,19 @@ __global__ void __launch_bounds__(kBfsThreads, 2) bfs_persistent(BfsArgs a) {
             }
             unsigned long long f_blk = block_sum((unsigned long long)found_local, s_red);
             if (threadIdx.x == 0 && f_blk) atomicAdd((unsigned long long *)&ctl->reached, f_blk);
-            if (threadIdx.x == 0 && f_blk) atomicAdd(&ctl->cnt[nxt].nf, (int)f_blk);
+            if (threadIdx.x == 0 && f_blk) atomicAdd(&cnxt->nf, (int)f_blk);
             if (gtid == 0) ctl->conv = 0;
             if (!grid_barrier(&ctl->gs)) return;
-            const int nf_next = __ldcg(&ctl->cnt[nxt].nf);
+            const int nf_next = __ldcg(&cnxt->nf);
             if (a.direction == 0 && !(nf_next > nf || nf_next > a.n / a.beta)) {
                 push = true;
                 num_edges = 1;
             }
             have_queue = false;
         }
-        (void)my_found;
         L++;
+        C++;
+        solo_ok = true;
     }
 
     if (kStats) {

@@ -75,21 +75,25 @@ __device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long
 
 // Grid-wide barrier for cooperative (co-resident) launches.  `count` only
 // grows: every block adds one per barrier, so barrier k of a run is complete
-// when count reaches (k + 1) * gridDim.x, and a block computes that target
+// when count reaches (k + 1) * nblocks, and a block computes that target
 // from the value its own arrival returned; no block resets anything, and the
 // waiters see the last arrival itself.  The control block must be zeroed
 // before a run, and every launch of a run must use the same grid size.
-// Waiters poll `count` with an acquire load and give up after the wait
-// limit, setting *err.  Once *err is set every later barrier returns at once,
-// so a failed run drains in bounded time.  Returns false when the run must
-// stop.
+// The arrival is a release (everything the block wrote, ordered before it by
+// __syncthreads, is visible to whoever acquires it) and the poll an acquire,
+// which also drops the SM's stale L1 lines: no separate fences.  Waiters poll
+// back to back at first, since a level of a sparse frontier ends within a few
+// round trips, then sleep between polls so that a long wait leaves the L2
+// slice alone.  They give up after the wait limit, setting *err.  Once *err is
+// set every later barrier returns at once, so a failed run drains in bounded
+// time.  Returns false when the run must stop.
 struct GridSync {
     unsigned long long count;
     int err;
     int pad;
 };
 
-__device__ __forceinline__ bool grid_barrier(GridSync *gs) {
+__device__ __forceinline__ bool grid_barrier(GridSync *gs, unsigned nblocks) {
     __syncthreads();
     __shared__ int s_ok;
     if (threadIdx.x == 0) {
@@ -97,28 +101,30 @@ __device__ __forceinline__ bool grid_barrier(GridSync *gs) {
         if (*(volatile int *)&gs->err) {
             ok = 0;
         } else {
-            __threadfence();
-            const unsigned long long t = atomicAdd(&gs->count, 1ull);
-            const unsigned long long target = (t / gridDim.x + 1) * gridDim.x;
+            unsigned long long t;
+            asm volatile("atom.add.acq_rel.gpu.global.u64 %0, [%1], 1;" : "=l"(t) : "l"(&gs->count) : "memory");
+            const unsigned long long target = (t / nblocks + 1) * nblocks;
             if (t + 1 != target) {
-                unsigned long long t0 = globaltimer_ns();
-                while (ld_acquire_u64(&gs->count) < target) {
+                unsigned long long t0 = 0;
+                for (int polls = 0; ld_acquire_u64(&gs->count) < target; polls++) {
+                    if (polls < 64) continue;
+                    if (polls == 64) t0 = globaltimer_ns();
                     if (*(volatile int *)&gs->err) { ok = 0; break; }
                     if (globaltimer_ns() - t0 > c_limits.wait_ns) {
                         atomicExch(&gs->err, (int)HC_ERR_TIMEOUT);
                         ok = 0;
                         break;
                     }
-                    __nanosleep(32);
+                    __nanosleep(100);
                 }
             }
-            __threadfence();
         }
         s_ok = ok;
     }
     __syncthreads();
     return s_ok != 0;
 }
+__device__ __forceinline__ bool grid_barrier(GridSync *gs) { return grid_barrier(gs, gridDim.x); }
 
 // Warp-level helpers (full mask; the reference's ALLWARP mask at
 // src/cuda.cuh:24 evaluates to 0x80000000, which is not a full warp).

@@ -1,12 +1,16 @@
 // Load-balanced expansion of a vertex queue over its CSR rows, shared by the
 // top-down BFS and the SSSP relaxation.
 //
-// Rows of at most kSmallDeg edges are expanded warp-centrically: a warp takes
-// 32 queue entries, scans their degrees and walks the combined edge range, so
+// Short rows are expanded warp-centrically: a warp takes up to 32 queue
+// entries, scans their degrees and walks the combined edge range, so
 // neighbour loads stay coalesced within a row whatever the degree mix.  Longer
 // rows are cut into (vertex, chunk) tasks of kTaskEdges edges that every warp
-// of the grid shares after a barrier, so hub rows and small frontiers of
-// medium-degree vertices spread over the whole GPU.
+// of the grid shares after a barrier, so hub rows spread over the whole GPU.
+// A queue too short to give every warp 32 entries gives each warp fewer (at
+// least one), and a row counts as short up to kTaskEdges edges shared among
+// the warp's entries (at least kSmallDeg): a level of a thousand vertices is
+// then one round per warp and needs no second phase, instead of several
+// rounds on a few warps and tasks for the rest.
 //
 // Each lane keeps kUnroll edges in flight: all neighbour loads of a round are
 // issued, then all probes of the destination state, then the commits, which
@@ -40,16 +44,18 @@ template <class V>
 __device__ __forceinline__ void expand_small(const int64_t *__restrict__ index, const int32_t *q, int nf,
                                              int2 *tasks, int *task_count, int gwarp, int nwarps, V &vis) {
     const int lane = threadIdx.x & 31;
-    for (int base = gwarp * 32; base < nf; base += nwarps * 32) {
+    const int per = min(32, max(1, (nf + nwarps - 1) / nwarps));
+    const int short_deg = max(kSmallDeg, kTaskEdges / per);
+    for (int base = gwarp * per; base < nf; base += nwarps * per) {
         const int i = base + lane;
         int32_t u = -1;
         long long beg = 0;
         int deg = 0;
-        if (i < nf) {
+        if (lane < per && i < nf) {
             u = ld_cg(q + i);
-            beg = index[u];
-            deg = (int)(index[u + 1] - beg);
-            if (deg > kSmallDeg) {
+            beg = __ldg(index + u);
+            deg = (int)(__ldg(index + u + 1) - beg);
+            if (deg > short_deg) {
                 const int nt = (deg + kTaskEdges - 1) / kTaskEdges;
                 const int t0 = atomicAdd(task_count, nt);
                 for (int c = 0; c < nt; c++) tasks[t0 + c] = make_int2(u, c);
@@ -90,7 +96,7 @@ __device__ __forceinline__ void expand_tasks(const int64_t *__restrict__ index, 
     const int lane = threadIdx.x & 31;
     for (int t = gwarp; t < ntasks; t += nwarps) {
         const int2 tk = __ldcg(tasks + t);
-        const int64_t rb = index[tk.x], re = index[tk.x + 1];
+        const int64_t rb = __ldg(index + tk.x), re = __ldg(index + tk.x + 1);
         const int64_t beg = rb + (int64_t)tk.y * kTaskEdges;
         const int64_t end = min(re, beg + (int64_t)kTaskEdges);
         for (int64_t e0 = beg; e0 < end; e0 += 32 * kUnroll) {

@@ -120,8 +120,8 @@ struct RelaxVisit {
         int32_t v, nd, dv;
     };
     __device__ __forceinline__ void load(Item &it, int32_t u, int64_t e) {
-        it.v = nbr[e];
-        it.nd = sat_add(__ldcg(dist + u), w[e]);
+        it.v = __ldg(nbr + e);
+        it.nd = sat_add(__ldcg(dist + u), __ldg(w + e));
     }
     __device__ __forceinline__ void probe(Item &it) { it.dv = __ldcg(dist + it.v); }
     // Stages across the round's items: all atomicMins in flight, then all
@@ -148,7 +148,7 @@ struct RelaxVisit {
             near[j] = imp[j] && is_near && old[j] < next_e;
             far[j] = imp[j] && !is_near && old[j] < far_claim;
             v[j] = imp[j] ? it[j].v : 0;
-            if (near[j]) mf += (unsigned long long)(index[v[j] + 1] - index[v[j]]);
+            if (near[j]) mf += (unsigned long long)(__ldg(index + v[j] + 1) - __ldg(index + v[j]));
         }
         warp_append_n(near, v, qnext, qlen);
         if (use_far) warp_append_n(far, v, fpile, fpile_len);

@@ -1,0 +1,73 @@
+"""Thin frontiers: levels and epochs that one block runs alone, at the sizes where they start and stop."""
+import numpy as np
+import pytest
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def csr(n, u, v):
+    """Symmetric CSR of the pairs (u, v)."""
+    src, dst = np.concatenate([u, v]), np.concatenate([v, u])
+    order = np.lexsort((dst, src))
+    index = np.zeros(n + 1, np.int64)
+    np.cumsum(np.bincount(src, minlength=n), out=index[1:])
+    return index, dst[order].astype(np.int32)
+
+
+def path(n):
+    return csr(n, np.arange(n - 1), np.arange(1, n))
+
+
+def fan(width, tail):
+    """A root, `width` vertices next to it through hubs of 100 edges, and `tail` more levels of that width."""
+    hubs = (width + 99) // 100
+    first = 1 + hubs
+    lane = np.arange(width)
+    u = [np.zeros(hubs, np.int64), 1 + lane // 100]
+    v = [1 + np.arange(hubs), first + lane]
+    for t in range(tail):
+        u.append(first + t * width + lane)
+        v.append(first + (t + 1) * width + lane)
+    return csr(first + (tail + 1) * width, np.concatenate(u), np.concatenate(v))
+
+
+def star_chain(deg, links):
+    """A chain of stars: each centre has `deg` edges in all."""
+    c = np.arange(links) * deg
+    leaves = [c[i] + 1 + np.arange(deg - 2) for i in range(links)]
+    u = np.concatenate([np.repeat(c, deg - 2), c[:-1]])
+    v = np.concatenate(leaves + [c[1:]])
+    return csr(links * deg, u, v)
+
+
+GRAPHS = {
+    "path_3000": lambda: path(3000),            # more levels than one turn of the block
+    "path_2": lambda: path(2),
+    "fan_1919": lambda: fan(1919, 40),          # around the block's queue capacity
+    "fan_1920": lambda: fan(1920, 40),
+    "fan_1921": lambda: fan(1921, 40),
+    "fan_600": lambda: fan(600, 9),
+    "star_127": lambda: star_chain(127, 30),    # around the longest row it takes
+    "star_128": lambda: star_chain(128, 30),
+    "star_129": lambda: star_chain(129, 30),
+    "star_300": lambda: star_chain(300, 12),
+}
+
+
+@pytest.mark.parametrize("direction", [0, 1, 2])
+@pytest.mark.parametrize("name", sorted(GRAPHS))
+def test_bfs_thin_levels(name, direction):
+    import hc
+    index, nbr = GRAPHS[name]()
+    n = len(index) - 1
+    g = hc.Graph(index, nbr)
+    sources = [0, n - 1, n // 2]
+    for stats in (False, True):
+        depth, parent, _ = g.bfs(sources, direction=direction, stats=stats)
+        for i, s in enumerate(sources):
+            want = oracle.bfs_depth(index, nbr, s)
+            assert np.array_equal(depth[i], want)
+            assert oracle.verify_bfs_parents(index, nbr, want, parent[i], s)[0] == 0
+    g.close()
