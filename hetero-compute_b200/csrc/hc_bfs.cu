@@ -1,4 +1,5 @@
-// Direction-optimising BFS as one persistent cooperative launch per source.
+// Direction-optimising BFS: one persistent launch for all sources of a call,
+// teams of blocks running several of them at a time.
 //
 // Reference path: bfs_gpu (src/kernels/gpu/bfs.cuh:21-95) runs bottom-up
 // epochs only, one launch + blocking 4-byte D2H + cudaMemset per level; the
@@ -18,6 +19,7 @@
 //   q[2]           int32[N]      frontier queues (top-down levels)
 //   tasks          int2[]        (vertex, chunk) pieces of long rows
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <cstdlib>
@@ -65,7 +67,7 @@ struct LevelCnt {
 
 struct BfsCtl {
     GridSync gs;
-    LevelCnt cnt[3];
+    LevelCnt cnt[2][3];     // by run parity: a run's counters are set while blocks may still read the last run's
     int conv;               // bitmap -> queue conversion counter
     int levels, td_levels, bu_levels;
     unsigned long long vscan, escan, reached;
@@ -79,6 +81,20 @@ struct BfsCtl {
     } trace[kTraceLevels + 1];  // per-level record for HC_TRACE=1
 };
 
+// Results of the runs of one call, folded on the device after each run so
+// that the host need not wait for each source: the first failure (status and
+// source), the deepest run, the top-down / bottom-up level counts.
+struct BfsFold {
+    int err, err_src, levels, td_levels, bu_levels;
+    int teams_done;  // of the running launch
+};
+
+// Sources of one launch.
+constexpr int kBfsLaunchSources = 256;
+// Bytes that the workspaces of sources run at the same time may take in all;
+// past it (and when they cannot be allocated) fewer run at a time.
+constexpr size_t kBfsTeamBytes = 1ull << 30;
+
 struct BfsArgs {
     const int64_t *index;
     const int32_t *nbr;
@@ -91,7 +107,17 @@ struct BfsArgs {
     int32_t *q0, *q1;
     int2 *tasks;
     BfsCtl *ctl;
-    int32_t src;
+    BfsFold *fold, *fold_host;  // fold_host: mapped host copy, written by the launch's last team (null: none)
+    // Teams of `team` consecutive blocks run one source at a time each, team t
+    // the sources t, t + teams, ...; the pointers above are team 0's, team t's
+    // lie t * team_stride bytes (depth, parent: see out_stride) further on.
+    int team;
+    size_t team_stride;
+    // Output row of source i: depth + i * out_stride (out_stride 0: not wanted,
+    // one scratch row per team).
+    int64_t depth_stride, parent_stride;
+    int nsrc;
+    int32_t src[kBfsLaunchSources];
     int alpha, beta, direction, bu_variant, max_levels;
     // Per bottom-up level warp/thread split (the per-epoch granularity
     // selector): bottom-up level k (0 = the first) runs warp per vertex on
@@ -101,12 +127,22 @@ struct BfsArgs {
     int bu_split_levels;
 };
 
-__device__ __forceinline__ uint32_t *fb_sel(const BfsArgs &a, int i) {
-    return i == 0 ? a.fb0 : (i == 1 ? a.fb1 : a.fb2);
+// A workspace pointer of this team.
+template <class T>
+__device__ __forceinline__ T *of_team(T *p, size_t off) {
+    return reinterpret_cast<T *>(reinterpret_cast<char *>(p) + off);
 }
-__device__ __forceinline__ uint32_t *sb_sel(const BfsArgs &a, int i) {
-    return i == 0 ? a.sb0 : (i == 1 ? a.sb1 : a.sb2);
-}
+// What one run works on: the team's share of the workspace and the source's
+// outputs.  Kept in shared memory: as registers these pointers would spill the
+// levels' inner loops.
+struct BfsRun {
+    int32_t src;
+    int32_t *depth, *parent;
+    uint32_t *visited;
+    int32_t *q0, *q1;
+    int2 *tasks;
+    uint32_t *fb[3], *sb[3];
+};
 
 // Sets vertex v's bit in a frontier bitmap and, when its word was empty, the
 // word's summary bit.
@@ -191,16 +227,30 @@ __device__ __forceinline__ unsigned long long solo_row(int64_t b, int64_t d) {
 // take any level over.  Stops before a level that is too wide, that the
 // direction rule turns bottom-up, after kSoloLevels levels, or when the queue
 // is empty.  Returns with the loop state updated in every thread.
+struct SoloState {
+    int L, nf, td_levels;
+    long long edges_to_check, num_edges;
+    unsigned long long vscan, escan;
+};
+struct SoloArgs {
+    const int64_t *index;
+    const int32_t *nbr;
+    int direction, alpha, max_levels;
+};
+// Not inlined: its registers would spill the grid's levels.
 template <bool kStats>
-__device__ __forceinline__ void solo_levels(const BfsArgs &a, BfsCtl *ctl, SoloQueue *sq, int &L, int &nf,
-                                            int &td_levels, long long &edges_to_check, long long &num_edges,
-                                            unsigned long long &my_vscan, unsigned long long &my_escan) {
+__device__ __noinline__ SoloState solo_levels(SoloArgs a, const BfsRun &r, BfsCtl *ctl, SoloQueue *sq, SoloState st) {
+    int L = st.L, nf = st.nf, td_levels = st.td_levels;
+    int32_t *const parent = r.parent, *const depth = r.depth;
+    uint32_t *const visited = r.visited;
+    long long edges_to_check = st.edges_to_check, num_edges = st.num_edges;
+    unsigned long long my_vscan = st.vscan, my_escan = st.escan;
     __shared__ int s_n[3];
     __shared__ unsigned long long s_mf[3];
     __shared__ int s_wide[3];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     const unsigned lt = (1u << lane) - 1u;
-    const int32_t *qin = (L & 1) ? a.q1 : a.q0;
+    const int32_t *qin = (L & 1) ? r.q1 : r.q0;
     if (threadIdx.x < 3) {
         s_n[threadIdx.x] = 0;
         s_mf[threadIdx.x] = 0ull;
@@ -228,7 +278,7 @@ __device__ __forceinline__ void solo_levels(const BfsArgs &a, BfsCtl *ctl, SoloQ
             break;
         const SoloQueue &cq = sq[step & 1];
         SoloQueue &nq = sq[(step + 1) & 1];
-        int32_t *qnext = (L & 1) ? a.q0 : a.q1;
+        int32_t *qnext = (L & 1) ? r.q0 : r.q1;
         edges_to_check -= num_edges;
         td_levels++;
         if (threadIdx.x == 0) {
@@ -274,10 +324,10 @@ __device__ __forceinline__ void solo_levels(const BfsArgs &a, BfsCtl *ctl, SoloQ
                     v[j] = take[j] ? __ldg(a.nbr + bo + off) : 0;
                 }
 #pragma unroll
-                for (int j = 0; j < kUnroll; j++) word[j] = take[j] ? __ldcg(a.visited + (v[j] >> 5)) : ~0u;
+                for (int j = 0; j < kUnroll; j++) word[j] = take[j] ? __ldcg(visited + (v[j] >> 5)) : ~0u;
 #pragma unroll
                 for (int j = 0; j < kUnroll; j++)
-                    from[j] = (word[j] >> (v[j] & 31)) & 1u ? 0 : atomicCAS(a.parent + v[j], -1, from[j]);
+                    from[j] = (word[j] >> (v[j] & 31)) & 1u ? 0 : atomicCAS(parent + v[j], -1, from[j]);
 #pragma unroll
                 for (int j = 0; j < kUnroll; j++) take[j] = from[j] == -1;
                 unsigned bal[kUnroll];
@@ -302,8 +352,8 @@ __device__ __forceinline__ void solo_levels(const BfsArgs &a, BfsCtl *ctl, SoloQ
                 for (int j = 0; j < kUnroll; j++) {
                     if (take[j]) {
                         const int p = pos + __popc(bal[j] & lt);
-                        a.depth[v[j]] = L + 1;
-                        atomicOr(a.visited + (v[j] >> 5), 1u << (v[j] & 31));
+                        depth[v[j]] = L + 1;
+                        atomicOr(visited + (v[j] >> 5), 1u << (v[j] & 31));
                         qnext[p] = v[j];
                         if (p < kSoloCap) {
                             nq.u[p] = v[j];
@@ -324,6 +374,7 @@ __device__ __forceinline__ void solo_levels(const BfsArgs &a, BfsCtl *ctl, SoloQ
         wide = s_wide[ns] || num_edges > kSoloEdges;
         L++;
     }
+    return SoloState{L, nf, td_levels, edges_to_check, num_edges, my_vscan, my_escan};
 }
 
 // Shared memory of one block: the hub prefix and the summary of the frontier
@@ -340,37 +391,83 @@ template <bool kStats>
 __global__ void __launch_bounds__(kBfsThreads, 2) bfs_persistent(BfsArgs a) {
     __shared__ unsigned long long s_red[32];
     __shared__ BfsShared sh;
+    __shared__ int s_stop;
     uint32_t *const s_fb = sh.bu.fb, *const s_sum = sh.bu.sum;
-    BfsCtl *ctl = a.ctl;
     const int lane = threadIdx.x & 31;
-    const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
-    const int nthreads = gridDim.x * blockDim.x;
+    const int team = blockIdx.x / a.team, team_block = blockIdx.x - team * a.team;
+    const int nteams = gridDim.x / a.team;
+    BfsCtl *ctl = a.ctl + team;
+    const size_t toff = (size_t)team * a.team_stride;
+    const int gtid = team_block * blockDim.x + threadIdx.x;
+    const int nthreads = a.team * blockDim.x;
     const int gwarp = gtid >> 5, nwarps = nthreads >> 5;
     const int W = (a.n + 31) >> 5;
     const int W_act = (a.n_active + 31) >> 5;
+    // A team of one block needs no more than its own block barrier.
+    bool stop = false;  // thread 0 of a one-block team: it recorded a failure
+    auto team_sync = [&]() -> bool {
+        if (a.team > 1) return grid_barrier(&ctl->gs, (unsigned)a.team);
+        __syncthreads();
+        if (threadIdx.x == 0) s_stop = stop;
+        __syncthreads();
+        return !s_stop;
+    };
 
-    for (int i = gtid; i < a.n; i += nthreads) {
-        a.depth[i] = i == a.src ? 0 : -1;
-        a.parent[i] = i == a.src ? i : -1;
+    __shared__ BfsRun r;
+    if (threadIdx.x == 0) {
+        r.visited = of_team(a.visited, toff);
+        r.q0 = of_team(a.q0, toff);
+        r.q1 = of_team(a.q1, toff);
+        r.tasks = of_team(a.tasks, toff);
+        r.fb[0] = of_team(a.fb0, toff);
+        r.fb[1] = of_team(a.fb1, toff);
+        r.fb[2] = of_team(a.fb2, toff);
+        r.sb[0] = of_team(a.sb0, toff);
+        r.sb[1] = of_team(a.sb1, toff);
+        r.sb[2] = of_team(a.sb2, toff);
     }
-    for (int i = gtid; i < W; i += nthreads) {
-        a.visited[i] = i == (a.src >> 5) ? 1u << (a.src & 31) : 0u;
-        a.fb0[i] = 0;
-        a.fb1[i] = 0;
-        a.fb2[i] = 0;
+    unsigned long long my_vscan = 0, my_escan = 0;
+    bool failed = false;
+    int run = 0;
+
+    for (int si = team; si < a.nsrc && !failed; si += nteams, run++) {
+    __syncthreads();  // the last run's reads of r
+    if (threadIdx.x == 0) {
+        r.src = a.src[si];
+        r.depth = a.depth + (a.depth_stride ? (size_t)si * a.depth_stride : (size_t)team * a.n);
+        r.parent = a.parent + (a.parent_stride ? (size_t)si * a.parent_stride : (size_t)team * a.n);
     }
-    for (int i = gtid; i < a.sum_words; i += nthreads) {
-        a.sb0[i] = 0;
-        a.sb1[i] = 0;
-        a.sb2[i] = 0;
+    __syncthreads();
+    LevelCnt *const cnt = ctl->cnt[run & 1];
+    {
+        const int32_t src = r.src;
+        int32_t *const depth = r.depth, *const parent = r.parent;
+        for (int i = gtid; i < a.n; i += nthreads) {
+            depth[i] = i == src ? 0 : -1;
+            parent[i] = i == src ? i : -1;
+        }
+        uint32_t *const vis = r.visited, *const f0 = r.fb[0], *const f1 = r.fb[1], *const f2 = r.fb[2];
+        for (int i = gtid; i < W; i += nthreads) {
+            vis[i] = i == (src >> 5) ? 1u << (src & 31) : 0u;
+            f0[i] = 0;
+            f1[i] = 0;
+            f2[i] = 0;
+        }
+        uint32_t *const s0 = r.sb[0], *const s1 = r.sb[1], *const s2 = r.sb[2];
+        for (int i = gtid; i < a.sum_words; i += nthreads) {
+            s0[i] = 0;
+            s1[i] = 0;
+            s2[i] = 0;
+        }
     }
     const unsigned long long t_start = globaltimer_ns();
     if (gtid == 0) {
-        a.q0[0] = a.src;
-        ctl->cnt[0].nf = 1;
-        ctl->cnt[0].mf = (unsigned long long)(a.index[a.src + 1] - a.index[a.src]);
+        r.q0[0] = r.src;
+        cnt[0] = LevelCnt{1, 0, (unsigned long long)(a.index[r.src + 1] - a.index[r.src])};
+        cnt[1] = LevelCnt{0, 0, 0ull};
+        cnt[2] = LevelCnt{0, 0, 0ull};
     }
-    if (!grid_barrier(&ctl->gs)) return;
+    failed = !team_sync();
 
     // Direction state (identical in every block).
     bool push = a.direction != 2;
@@ -380,8 +477,7 @@ __global__ void __launch_bounds__(kBfsThreads, 2) bfs_persistent(BfsArgs a) {
     bool solo_ok = true;
     bool bitmaps_clear = true;  // all three frontier bitmaps are zero (no bottom-up level yet)
     long long edges_to_check = a.m;
-    long long num_edges = (long long)(a.index[a.src + 1] - a.index[a.src]);
-    unsigned long long my_vscan = 0, my_escan = 0;
+    long long num_edges = (long long)(a.index[r.src + 1] - a.index[r.src]);
     int L = 0, td_levels = 0, bu_levels = 0;
     // The level counters rotate with the levels that the whole grid runs: the
     // thin levels of one block leave them alone, since other blocks may still
@@ -389,9 +485,9 @@ __global__ void __launch_bounds__(kBfsThreads, 2) bfs_persistent(BfsArgs a) {
     int C = 0;
     int solo_nf = -1;  // frontier size after thin levels (-1: in the counters)
 
-    for (;;) {
+    while (!failed) {
         const int cur = L % 3, nxt = (L + 1) % 3, old = (L + 2) % 3;
-        LevelCnt *const ccur = &ctl->cnt[C % 3], *const cnxt = &ctl->cnt[(C + 1) % 3];
+        LevelCnt *const ccur = &cnt[C % 3], *const cnxt = &cnt[(C + 1) % 3];
         int nf = solo_nf >= 0 ? solo_nf : __ldcg(&ccur->nf);
         solo_nf = -1;
         if (nf == 0) break;
@@ -400,16 +496,19 @@ __global__ void __launch_bounds__(kBfsThreads, 2) bfs_persistent(BfsArgs a) {
             break;
         }
         if (gtid == 0) {
-            if (globaltimer_ns() - t_start > c_limits.run_ns) atomicExch(&ctl->gs.err, (int)HC_ERR_TIMEOUT);
-            LevelCnt *const cold = &ctl->cnt[(C + 2) % 3];
+            if (globaltimer_ns() - t_start > c_limits.run_ns) {
+                atomicExch(&ctl->gs.err, (int)HC_ERR_TIMEOUT);
+                stop = true;
+            }
+            LevelCnt *const cold = &cnt[(C + 2) % 3];
             cold->nf = 0;
             cold->tasks = 0;
             cold->mf = 0;
         }
-        uint32_t *fcur = fb_sel(a, cur), *fnext = fb_sel(a, nxt), *fold = fb_sel(a, old);
-        uint32_t *scur = sb_sel(a, cur), *snext = sb_sel(a, nxt), *sold = sb_sel(a, old);
-        int32_t *qcur = (L & 1) ? a.q1 : a.q0;
-        int32_t *qnext = (L & 1) ? a.q0 : a.q1;
+        uint32_t *fcur = r.fb[cur], *fnext = r.fb[nxt], *fold = r.fb[old];
+        uint32_t *scur = r.sb[cur], *snext = r.sb[nxt], *sold = r.sb[old];
+        int32_t *qcur = (L & 1) ? r.q1 : r.q0;
+        int32_t *qnext = (L & 1) ? r.q0 : r.q1;
 
         if (a.direction == 0 && push && num_edges > edges_to_check / a.alpha) push = false;
         if (gtid == 0 && L < kTraceLevels) {
@@ -435,16 +534,24 @@ __global__ void __launch_bounds__(kBfsThreads, 2) bfs_persistent(BfsArgs a) {
                         qcur[pos++] = w * 32 + b;
                     }
                 }
-                if (!grid_barrier(&ctl->gs)) return;
+                if ((failed = !team_sync())) break;
                 nf = __ldcg(&ctl->conv);
                 have_queue = true;
             }
             if (solo_ok && nf <= kSoloCap && num_edges <= kSoloEdges) {
                 const int L0 = L;
                 solo_ok = false;
-                if (blockIdx.x == 0) {
-                    solo_levels<kStats>(a, ctl, sh.solo, L, nf, td_levels, edges_to_check, num_edges, my_vscan,
-                                        my_escan);
+                if (team_block == 0) {
+                    const SoloState st = solo_levels<kStats>(
+                        SoloArgs{a.index, a.nbr, a.direction, a.alpha, a.max_levels}, r, ctl, sh.solo,
+                        SoloState{L, nf, td_levels, edges_to_check, num_edges, my_vscan, my_escan});
+                    L = st.L;
+                    nf = st.nf;
+                    td_levels = st.td_levels;
+                    edges_to_check = st.edges_to_check;
+                    num_edges = st.num_edges;
+                    my_vscan = st.vscan;
+                    my_escan = st.escan;
                     if (threadIdx.x == 0) {
                         ctl->solo.L = L;
                         ctl->solo.nf = nf;
@@ -453,7 +560,7 @@ __global__ void __launch_bounds__(kBfsThreads, 2) bfs_persistent(BfsArgs a) {
                         ctl->solo.num_edges = num_edges;
                     }
                 }
-                if (!grid_barrier(&ctl->gs)) return;
+                if ((failed = !team_sync())) break;
                 L = __ldcg(&ctl->solo.L);
                 if (L != L0) {
                     solo_nf = __ldcg(&ctl->solo.nf);
@@ -466,7 +573,7 @@ __global__ void __launch_bounds__(kBfsThreads, 2) bfs_persistent(BfsArgs a) {
             edges_to_check -= num_edges;
             td_levels++;
             const int next_depth = L + 1;
-            TopDownVisit visit{a.index, a.nbr, a.parent, a.depth, a.visited, qnext, &cnxt->nf, next_depth,
+            TopDownVisit visit{a.index, a.nbr, r.parent, r.depth, r.visited, qnext, &cnxt->nf, next_depth,
                                0ull};
             if (kStats) {
                 for (int i = gtid; i < nf; i += nthreads) {
@@ -475,17 +582,17 @@ __global__ void __launch_bounds__(kBfsThreads, 2) bfs_persistent(BfsArgs a) {
                 }
                 if (gtid == 0) my_vscan += nf;
             }
-            expand_small(a.index, qcur, nf, a.tasks, &ccur->tasks, gwarp, nwarps, visit);
+            expand_small(a.index, qcur, nf, r.tasks, &ccur->tasks, gwarp, nwarps, visit);
             unsigned long long mf_blk = block_sum(visit.mf, s_red);
             if (threadIdx.x == 0 && mf_blk) atomicAdd(&cnxt->mf, mf_blk);
-            if (!grid_barrier(&ctl->gs)) return;
+            if ((failed = !team_sync())) break;
             const int nt = __ldcg(&ccur->tasks);
             if (nt > 0) {
                 visit.mf = 0;
-                expand_tasks(a.index, a.tasks, nt, gwarp, nwarps, visit);
+                expand_tasks(a.index, r.tasks, nt, gwarp, nwarps, visit);
                 mf_blk = block_sum(visit.mf, s_red);
                 if (threadIdx.x == 0 && mf_blk) atomicAdd(&cnxt->mf, mf_blk);
-                if (!grid_barrier(&ctl->gs)) return;
+                if ((failed = !team_sync())) break;
             }
             num_edges = (long long)__ldcg(&cnxt->mf);
             have_queue = true;
@@ -502,10 +609,10 @@ __global__ void __launch_bounds__(kBfsThreads, 2) bfs_persistent(BfsArgs a) {
                         scur[i] = 0;
                         snext[i] = 0;
                     }
-                    if (!grid_barrier(&ctl->gs)) return;
+                    if ((failed = !team_sync())) break;
                 }
                 for (int i = gtid; i < nf; i += nthreads) frontier_add(fcur, scur, a.sum_shift, __ldcg(qcur + i));
-                if (!grid_barrier(&ctl->gs)) return;
+                if ((failed = !team_sync())) break;
             }
             bitmaps_clear = false;
             for (int i = gtid; i < W_act; i += nthreads) fold[i] = 0;
@@ -536,7 +643,7 @@ __global__ void __launch_bounds__(kBfsThreads, 2) bfs_persistent(BfsArgs a) {
             for (int v = gwarp; v < n_warp_al; v += nwarps) {
                 if (v >= a.n_active) break;
                 const uint32_t bit = 1u << (v & 31);
-                if (__ldcg(a.visited + (v >> 5)) & bit) continue;
+                if (__ldcg(r.visited + (v >> 5)) & bit) continue;
                 const int64_t b = a.index[v], e = a.index[v + 1];
                 int32_t par = -1;
                 int64_t probes = 0;
@@ -560,16 +667,16 @@ __global__ void __launch_bounds__(kBfsThreads, 2) bfs_persistent(BfsArgs a) {
                     my_escan += probes;
                 }
                 if (par >= 0 && lane == 0) {
-                    a.parent[v] = par;
-                    a.depth[v] = next_depth;
-                    atomicOr(a.visited + (v >> 5), bit);
+                    r.parent[v] = par;
+                    r.depth[v] = next_depth;
+                    atomicOr(r.visited + (v >> 5), bit);
                     frontier_add(fnext, snext, cs, v);
                     found_local++;
                 }
             }
             // Remaining rows: thread per vertex, warp owns one bitmap word.
             for (int w = (n_warp_al >> 5) + gwarp; w < W_act; w += nwarps) {
-                const uint32_t vis = __ldcg(a.visited + w);
+                const uint32_t vis = __ldcg(r.visited + w);
                 const int v = w * 32 + lane;
                 int32_t par = -1;
                 if (v < a.n_active && !((vis >> lane) & 1u)) {
@@ -596,13 +703,13 @@ __global__ void __launch_bounds__(kBfsThreads, 2) bfs_persistent(BfsArgs a) {
                 }
                 const unsigned bal = __ballot_sync(kFull, par >= 0);
                 if (par >= 0) {
-                    a.parent[v] = par;
-                    a.depth[v] = next_depth;
+                    r.parent[v] = par;
+                    r.depth[v] = next_depth;
                 }
                 if (lane == 0) {
                     fnext[w] = bal;
                     if (bal) {
-                        a.visited[w] = vis | bal;
+                        r.visited[w] = vis | bal;
                         atomicOr(snext + ((w >> cs) >> 5), 1u << ((w >> cs) & 31));
                     }
                     found_local += __popc(bal);
@@ -612,7 +719,7 @@ __global__ void __launch_bounds__(kBfsThreads, 2) bfs_persistent(BfsArgs a) {
             if (threadIdx.x == 0 && f_blk) atomicAdd((unsigned long long *)&ctl->reached, f_blk);
             if (threadIdx.x == 0 && f_blk) atomicAdd(&cnxt->nf, (int)f_blk);
             if (gtid == 0) ctl->conv = 0;
-            if (!grid_barrier(&ctl->gs)) return;
+            if ((failed = !team_sync())) break;
             const int nf_next = __ldcg(&cnxt->nf);
             if (a.direction == 0 && !(nf_next > nf || nf_next > a.n / a.beta)) {
                 push = true;
@@ -625,17 +732,40 @@ __global__ void __launch_bounds__(kBfsThreads, 2) bfs_persistent(BfsArgs a) {
         solo_ok = true;
     }
 
-    if (kStats) {
-        unsigned long long v = block_sum(my_vscan, s_red);
-        if (threadIdx.x == 0 && v) atomicAdd(&ctl->vscan, v);
-        unsigned long long e = block_sum(my_escan, s_red);
-        if (threadIdx.x == 0 && e) atomicAdd(&ctl->escan, e);
-    }
     if (gtid == 0) {
         ctl->levels = L;
         ctl->trace[L < kTraceLevels ? L : kTraceLevels].t_ns = globaltimer_ns();
         ctl->td_levels = td_levels;
         ctl->bu_levels = bu_levels;
+        const int err = *(volatile int *)&ctl->gs.err;
+        if (err && atomicCAS(&a.fold->err, 0, err) == 0) a.fold->err_src = r.src;
+        atomicMax(&a.fold->levels, L);
+        atomicAdd(&a.fold->td_levels, td_levels);
+        atomicAdd(&a.fold->bu_levels, bu_levels);
+    }
+    }  // next source
+
+    if (gtid == 0) {
+        __threadfence();
+        if (atomicAdd(&a.fold->teams_done, 1) == nteams - 1) {
+            __threadfence();
+            a.fold->teams_done = 0;
+            if (a.fold_host) {
+                a.fold_host->err = __ldcg(&a.fold->err);
+                a.fold_host->err_src = __ldcg(&a.fold->err_src);
+                a.fold_host->levels = __ldcg(&a.fold->levels);
+                a.fold_host->td_levels = __ldcg(&a.fold->td_levels);
+                a.fold_host->bu_levels = __ldcg(&a.fold->bu_levels);
+                __threadfence_system();
+            }
+        }
+    }
+
+    if (kStats) {
+        unsigned long long v = block_sum(my_vscan, s_red);
+        if (threadIdx.x == 0 && v) atomicAdd(&ctl->vscan, v);
+        unsigned long long e = block_sum(my_escan, s_red);
+        if (threadIdx.x == 0 && e) atomicAdd(&ctl->escan, e);
     }
 }
 
@@ -691,44 +821,60 @@ struct SuffixFill {
     }
 };
 
-// Results of the runs of one call, folded on the device after each run so
-// that the host need not wait for each source: the first failure (status and
-// source), the deepest run, the top-down / bottom-up level counts.
-struct BfsFold {
-    int err, err_src, levels, td_levels, bu_levels, pad;
-};
-
-// Folds the run just finished into *f, then clears the control block for the
-// next run (one block).
-__global__ void bfs_fold_clear(BfsCtl *ctl, BfsFold *f, int32_t src) {
-    if (threadIdx.x == 0) {
-        if (ctl->gs.err && !f->err) {
-            f->err = ctl->gs.err;
-            f->err_src = src;
-        }
-        f->levels = max(f->levels, ctl->levels);
-        f->td_levels += ctl->td_levels;
-        f->bu_levels += ctl->bu_levels;
+// Clears the fold record and what the teams' control blocks must start from.
+__global__ void bfs_clear(BfsCtl *ctl, int teams, BfsFold *f) {
+    if (threadIdx.x == 0) *f = BfsFold{0, 0, 0, 0, 0, 0};
+    for (int t = threadIdx.x; t < teams; t += blockDim.x) {
+        ctl[t].gs = GridSync{0ull, 0, 0};
+        ctl[t].conv = 0;
+        ctl[t].vscan = ctl[t].escan = ctl[t].reached = 0ull;
     }
-    __syncthreads();
-    uint32_t *w = reinterpret_cast<uint32_t *>(ctl);
-    for (int i = threadIdx.x; i < (int)(sizeof(BfsCtl) / 4); i += blockDim.x) w[i] = 0u;
+}
+
+// Blocks of bfs_persistent that are resident at a time.
+template <bool kStats>
+hc_status bfs_resident(hc_graph *g, int *blocks) {
+    static int blocks_per_sm = 0;
+    if (blocks_per_sm == 0) {
+        HC_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, bfs_persistent<kStats>, kBfsThreads, 0));
+        if (blocks_per_sm < 1) return fail(HC_ERR_CUDA, "BFS kernel cannot be resident");
+    }
+    *blocks = blocks_per_sm * g->sm_count;
+    return HC_OK;
 }
 
 template <bool kStats>
-hc_status launch_bfs(hc_graph *g, const BfsArgs &args) {
-    static int blocks_per_sm[2] = {0, 0};
-    int &bps = blocks_per_sm[kStats ? 1 : 0];
-    if (bps == 0) {
-        HC_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, bfs_persistent<kStats>, kBfsThreads, 0));
-        if (bps < 1) return fail(HC_ERR_CUDA, "BFS kernel cannot be resident");
-    }
-    dim3 grid(g->sm_count * bps), block(kBfsThreads);
-    BfsArgs a = args;
-    void *params[] = {&a};
+hc_status launch_bfs(hc_graph *g, BfsArgs &a, int teams) {
+    dim3 grid(a.team * teams), block(kBfsThreads);
     ::hc::count_launch();
+    if (a.team == 1) {  // no block waits for another
+        bfs_persistent<kStats><<<grid, block, 0, g->stream>>>(a);
+        HC_CUDA_TRY(cudaGetLastError());
+        return HC_OK;
+    }
+    void *params[] = {&a};
     HC_CUDA_TRY(cudaLaunchCooperativeKernel((void *)bfs_persistent<kStats>, grid, block, params, 0, g->stream));
     return HC_OK;
+}
+
+// Blocks per team and teams for k sources on a graph of m edges (at most `room`
+// teams), from sweeps of team
+// sizes on Kronecker and uniform graphs of 20k to 128M edges.  A team is no
+// smaller than sqrt(m) / 300 blocks: below that the sources run at a time
+// outgrow the L2 (64 sources, 128M edges: 8 teams 7.6 ms, 12 teams 10.4 ms, 1
+// team 12.9 ms; 16 sources, 8M edges: 16 teams 0.41 ms, 1 team 1.45 ms).  It is
+// no larger than sqrt(m) / 19: above that a barrier and the queue's counters
+// cost more than the blocks bring (one source, 20k edges: 8 blocks 79 us, 296
+// blocks 97 us; 8M edges: 148 blocks 108 us, 296 blocks 120 us).  Between the
+// two, as many teams as end the sources in the fewest rounds.
+void bfs_teams(const hc_graph *g, int resident, int k, int room, int *team, int *teams) {
+    const double root = std::sqrt((double)std::max<int64_t>(g->M, 1));
+    const int least = std::max(1, std::min(resident, (int)std::lround(root / 300.0)));
+    const int most = std::max(1, std::min(resident, (int)std::lround(root / 19.0)));
+    const int at_a_time = std::max(1, std::min({k, room, resident / least}));
+    const int rounds = (std::max(k, 1) + at_a_time - 1) / at_a_time;
+    *teams = (std::max(k, 1) + rounds - 1) / rounds;
+    *team = std::max(least, std::min(most, resident / *teams));
 }
 
 }  // namespace
@@ -754,7 +900,10 @@ extern "C" hc_status hc_bfs(hc_graph *g, const int32_t *sources, int32_t num_sou
     if (stats) std::memset(stats, 0, sizeof(*stats));
 
     std::vector<int32_t> src(num_sources);
-    HC_CUDA_TRY(cudaMemcpy(src.data(), sources, sizeof(int32_t) * num_sources, cudaMemcpyDefault));
+    if (is_device_pointer(sources))
+        HC_CUDA_TRY(cudaMemcpy(src.data(), sources, sizeof(int32_t) * num_sources, cudaMemcpyDefault));
+    else
+        std::copy(sources, sources + num_sources, src.begin());
     for (int32_t s : src)
         if (s < 0 || s >= g->N) return fail(HC_ERR_INVALID_ARG, "hc_bfs: source %d outside [0, %d)", s, g->N);
 
@@ -764,10 +913,47 @@ extern "C" hc_status hc_bfs(hc_graph *g, const int32_t *sources, int32_t num_sou
     int sum_shift = 0;
     while (((W + (1ll << sum_shift) - 1) >> sum_shift) > (int64_t)kSumWords * 32) sum_shift++;
     const int sum_words = (int)((((W + (1ll << sum_shift) - 1) >> sum_shift) + 31) / 32);
-    const size_t bytes = sizeof(uint32_t) * 4 * W + sizeof(int32_t) * 2 * n + sizeof(int2) * ntasks +
-                         3 * (sizeof(uint32_t) * (size_t)sum_words + 256) + 1024;
-    HC_TRY(g->ws_bfs.ensure(bytes));
-    HC_TRY(g->ws_ctl.ensure(4096));
+    // Without per-run statistics or a trace the sources of a call run in one
+    // launch, several at a time, and the host waits once, at the end (with
+    // them, it runs one at a time and reads its control block after it).
+    const bool per_run = (o.collect_stats && stats) || std::getenv("HC_TRACE");
+    const bool dev_depth = is_device_pointer(depth_out);
+    const bool dev_parent = is_device_pointer(parent_out);
+    // Host outputs: staged on the device and copied while the next sources run.
+    const bool host_depth = depth_out && !dev_depth, host_parent = parent_out && !dev_parent;
+    const size_t bytes = [&] {
+        auto up = [](size_t b) { return (b + 255) / 256 * 256; };
+        return 4 * up(4 * (size_t)W) + 3 * up(4 * (size_t)sum_words) + 2 * up(4 * (size_t)n) +
+               up(sizeof(int2) * (size_t)ntasks);
+    }();
+    int resident = 0;
+    HC_TRY(o.collect_stats ? bfs_resident<true>(g, &resident) : bfs_resident<false>(g, &resident));
+    OutPipe pipe;
+    int team = resident, teams = 1;
+    const size_t fold_bytes = 256;
+    auto reserve = [&]() -> hc_status {
+        HC_TRY(g->ws_bfs.ensure(bytes * teams));
+        HC_TRY(g->ws_ctl.ensure(std::max<size_t>(4096, fold_bytes + sizeof(BfsCtl) * (size_t)teams)));
+        if (!depth_out) HC_TRY(g->ws_out0.ensure(4 * n * (size_t)teams));
+        if (!parent_out) HC_TRY(g->ws_out1.ensure(4 * n * (size_t)teams));
+        if (host_depth || host_parent) HC_TRY(pipe.init(g, 2, 4 * n, teams));
+        return HC_OK;
+    };
+    if (!per_run) {
+        // Bytes of one source at a time: workspace, staging (both arrays, two
+        // slots), scratch rows of outputs nobody asked for.
+        const size_t each = bytes + 4 * (size_t)n * ((host_depth || host_parent ? 4 : 0) + !depth_out + !parent_out);
+        bfs_teams(g, resident, num_sources, (int)std::min<size_t>(std::max<size_t>(kBfsTeamBytes / each, 1), 1 << 20),
+                  &team, &teams);
+    }
+    hc_status reserved = reserve();
+    if (reserved == HC_ERR_OOM && teams > 1) {  // no room for several: one at a time
+        clear_error();
+        bfs_teams(g, resident, num_sources, 1, &team, &teams);
+        g->ws_bfs.release();
+        reserved = reserve();
+    }
+    HC_TRY(reserved);
     char *p = g->ws_bfs.as<char>();
     auto take = [&](size_t b) {
         char *r = p;
@@ -793,7 +979,11 @@ extern "C" hc_status hc_bfs(hc_graph *g, const int32_t *sources, int32_t num_sou
     a.q0 = (int32_t *)take(4 * n);
     a.q1 = (int32_t *)take(4 * n);
     a.tasks = (int2 *)take(sizeof(int2) * ntasks);
-    a.ctl = g->ws_ctl.as<BfsCtl>();
+    BfsFold *fold = g->ws_ctl.as<BfsFold>();
+    a.ctl = reinterpret_cast<BfsCtl *>(g->ws_ctl.as<char>() + fold_bytes);
+    a.fold = fold;
+    a.team = team;
+    a.team_stride = bytes;
     a.alpha = o.alpha;
     a.beta = o.beta;
     a.direction = o.direction;
@@ -806,16 +996,8 @@ extern "C" hc_status hc_bfs(hc_graph *g, const int32_t *sources, int32_t num_sou
             a.bu_split[k] = std::max(0, std::min(g->tune.bfs_bu_split[k], g->n_active));
     }
 
-    const bool dev_depth = is_device_pointer(depth_out);
-    const bool dev_parent = is_device_pointer(parent_out);
-    if (!depth_out) HC_TRY(g->ws_out0.ensure(4 * n));
-    if (!parent_out) HC_TRY(g->ws_out1.ensure(4 * n));
-    // Host outputs: staged on the device and copied while the next source runs.
-    const bool host_depth = depth_out && !dev_depth, host_parent = parent_out && !dev_parent;
-    OutPipe pipe;
     SuffixFill fill;  // declared after the pipe: its threads are joined first on any return
     if (host_depth || host_parent) {
-        HC_TRY(pipe.init(g, 2, 4 * n));
         const int64_t n_copy = g->degree_sorted ? (int64_t)g->n_active : n;
         if (n_copy < n) {
             pipe.copy_bytes = sizeof(int32_t) * (size_t)n_copy;
@@ -824,49 +1006,70 @@ extern "C" hc_status hc_bfs(hc_graph *g, const int32_t *sources, int32_t num_sou
     }
 
     double total_ms = 0;
-    // Without per-run statistics or a trace the runs go back to back: each
-    // run's result is folded on the device and the host waits once, at the
-    // end (with them, it reads each run's control block after it).
-    const bool per_run = (o.collect_stats && stats) || std::getenv("HC_TRACE");
-    static_assert(sizeof(BfsCtl) + 64 <= 2048, "BfsCtl overlaps the fold record");
-    BfsFold *fold = reinterpret_cast<BfsFold *>(reinterpret_cast<char *>(a.ctl) + 2560);
     if (!per_run) {
-        HC_TRY(ctl_zero(g, fold, sizeof(BfsFold)));
-        HC_TRY(ctl_zero(g, a.ctl, sizeof(BfsCtl)));
+        BfsFold *h_fold = nullptr;
+        HC_TRY(ctl_slot(g, 0, (void **)&h_fold, (void **)&a.fold_host));
+        { bfs_clear<<<1, 256, 0, g->stream>>>(a.ctl, teams, fold); ::hc::count_launch(); }
+        HC_CUDA_TRY(cudaGetLastError());
         HC_CUDA_TRY(cudaEventRecord(g->ev_start, g->stream));
+        // Host outputs are copied a launch at a time, so a launch runs one source per team.
+        const bool staged = host_depth || host_parent;
+        const int per_launch = staged ? teams : kBfsLaunchSources;
+        a.depth_stride = depth_out ? n : 0;
+        a.parent_stride = parent_out ? n : 0;
+        for (int32_t i = 0, l = 0; i < num_sources; i += per_launch, l++) {
+            a.nsrc = std::min(per_launch, num_sources - i);
+            std::copy(src.begin() + i, src.begin() + i + a.nsrc, a.src);
+            int32_t *stage[2] = {nullptr, nullptr};
+            if (staged) HC_TRY(pipe.acquire(l, stage));
+            a.depth = dev_depth ? depth_out + (size_t)i * n : host_depth ? stage[0] : g->ws_out0.as<int32_t>();
+            a.parent = dev_parent ? parent_out + (size_t)i * n : host_parent ? stage[1] : g->ws_out1.as<int32_t>();
+            HC_TRY(launch_bfs<false>(g, a, std::min(teams, a.nsrc)));
+            if (staged) {
+                void *dst[2] = {host_depth ? (void *)(depth_out + (size_t)i * n) : nullptr,
+                                host_parent ? (void *)(parent_out + (size_t)i * n) : nullptr};
+                HC_TRY(pipe.release(l, dst, a.nsrc));
+            }
+        }
+        HC_CUDA_TRY(cudaEventRecord(g->ev_stop, g->stream));
+        HC_CUDA_TRY(cudaStreamSynchronize(g->stream));
+        if (num_sources > 0) {
+            BfsFold f;
+            std::memcpy(&f, h_fold, sizeof(f));
+            if (f.err) return fail((hc_status)f.err, "hc_bfs: device run from source %d ended with status %d",
+                                   f.err_src, f.err);
+            if (stats) {
+                stats->levels = f.levels;
+                stats->td_levels = f.td_levels;
+                stats->bu_levels = f.bu_levels;
+            }
+        }
+        float ms = 0;
+        HC_CUDA_TRY(cudaEventElapsedTime(&ms, g->ev_start, g->ev_stop));
+        total_ms = ms;
     }
-    for (int32_t i = 0; i < num_sources; i++) {
-        a.src = src[i];
+    for (int32_t i = 0; per_run && i < num_sources; i++) {
+        a.nsrc = 1;
+        a.src[0] = src[i];
         int32_t *stage[2] = {nullptr, nullptr};
         if (host_depth || host_parent) HC_TRY(pipe.acquire(i, stage));
         a.depth = dev_depth ? depth_out + (size_t)i * n : host_depth ? stage[0] : g->ws_out0.as<int32_t>();
         a.parent = dev_parent ? parent_out + (size_t)i * n : host_parent ? stage[1] : g->ws_out1.as<int32_t>();
-        if (!per_run) {
-            HC_TRY(launch_bfs<false>(g, a));
-            if (host_depth || host_parent) {
-                void *dst[2] = {host_depth ? (void *)(depth_out + (size_t)i * n) : nullptr,
-                                host_parent ? (void *)(parent_out + (size_t)i * n) : nullptr};
-                HC_TRY(pipe.release(i, dst));
-            }
-            { bfs_fold_clear<<<1, 256, 0, g->stream>>>(a.ctl, fold, a.src); ::hc::count_launch(); }
-            HC_CUDA_TRY(cudaGetLastError());
-            continue;
-        }
-        HC_TRY(ctl_zero(g, a.ctl, sizeof(BfsCtl)));
+        { bfs_clear<<<1, 256, 0, g->stream>>>(a.ctl, 1, fold); ::hc::count_launch(); }
         HC_CUDA_TRY(cudaEventRecord(g->ev_start, g->stream));
-        HC_TRY(o.collect_stats ? launch_bfs<true>(g, a) : launch_bfs<false>(g, a));
+        HC_TRY(o.collect_stats ? launch_bfs<true>(g, a, 1) : launch_bfs<false>(g, a, 1));
         HC_CUDA_TRY(cudaEventRecord(g->ev_stop, g->stream));
         if (host_depth || host_parent) {
             void *dst[2] = {host_depth ? (void *)(depth_out + (size_t)i * n) : nullptr,
                             host_parent ? (void *)(parent_out + (size_t)i * n) : nullptr};
-            HC_TRY(pipe.release(i, dst));
+            HC_TRY(pipe.release(i, dst, 1));
         }
-        static_assert(sizeof(BfsCtl) <= kCtlSlotBytes, "BfsCtl exceeds a control-read slot");
+        static_assert(sizeof(BfsCtl) + 256 + 64 <= 2560 && sizeof(BfsCtl) <= kCtlSlotBytes, "BfsCtl exceeds a control-read slot");
         BfsCtl c;
         const void *h_ctl = nullptr, *h_cnt = nullptr;
         HC_TRY(ctl_read(g, a.ctl, sizeof(c), 0, &h_ctl));
         if (o.collect_stats && stats) {
-            unsigned long long *cnt = (unsigned long long *)((char *)a.ctl + 2048);
+            unsigned long long *cnt = (unsigned long long *)(g->ws_ctl.as<char>() + 3072);
             HC_TRY(ctl_zero(g, cnt, 8));
             { count_reached<<<g->sm_count * 4, 256, 0, g->stream>>>(a.depth, g->N, cnt); ::hc::count_launch(); }
             HC_TRY(ctl_read(g, cnt, 8, 1, &h_cnt));
@@ -896,24 +1099,6 @@ extern "C" hc_status hc_bfs(hc_graph *g, const int32_t *sources, int32_t num_sou
             for (int l = 0; l < nl; l++)
                 std::fprintf(stderr, "[hc bfs]   L%-3d %s nf=%-9d %8.1f us\n", l, c.trace[l].mode == 1 ? "TD" : "BU",
                              c.trace[l].nf, (c.trace[l + 1].t_ns - c.trace[l].t_ns) * 1e-3);
-        }
-    }
-    if (!per_run) {
-        HC_CUDA_TRY(cudaEventRecord(g->ev_stop, g->stream));
-        const void *h_fold = nullptr;
-        HC_TRY(ctl_read(g, fold, sizeof(BfsFold), 0, &h_fold));
-        HC_CUDA_TRY(cudaStreamSynchronize(g->stream));
-        BfsFold f;
-        std::memcpy(&f, h_fold, sizeof(f));
-        if (f.err) return fail((hc_status)f.err, "hc_bfs: device run from source %d ended with status %d",
-                               f.err_src, f.err);
-        float ms = 0;
-        HC_CUDA_TRY(cudaEventElapsedTime(&ms, g->ev_start, g->ev_stop));
-        total_ms = ms;
-        if (stats) {
-            stats->levels = f.levels;
-            stats->td_levels = f.td_levels;
-            stats->bu_levels = f.bu_levels;
         }
     }
     if (host_depth || host_parent) HC_TRY(pipe.finish());
@@ -954,7 +1139,7 @@ constexpr size_t kNaTasks = (size_t)(kNoAllocMaxEdges / kTaskEdges + kNoAllocMax
 // Frontier summaries: one bit per bitmap word (kNaWords <= 32 * kSumWords).
 constexpr size_t kNaSumWords = (kNaWords + 31) / 32;
 static_assert(kNaWords <= (size_t)kSumWords * 32, "summary of the fixed-size bitmaps needs a shift");
-constexpr size_t kNoAllocBytes = na_align(sizeof(BfsCtl)) + na_align(sizeof(int)) + 4 * na_align(4 * kNaWords) +
+constexpr size_t kNoAllocBytes = na_align(sizeof(BfsCtl)) + na_align(sizeof(BfsFold)) + na_align(sizeof(int)) + 4 * na_align(4 * kNaWords) +
                                  3 * na_align(4 * kNaSumWords) + 2 * na_align(4 * (size_t)kNoAllocMaxNodes) +
                                  na_align(sizeof(int2) * kNaTasks);
 
@@ -1029,6 +1214,7 @@ extern "C" hc_status hc_bfs_noalloc(const int64_t *index, const int32_t *neighbo
     };
     BfsArgs a{};
     a.ctl = reinterpret_cast<BfsCtl *>(take(sizeof(BfsCtl)));
+    a.fold = reinterpret_cast<BfsFold *>(take(sizeof(BfsFold)));
     int *check_flag = reinterpret_cast<int *>(take(sizeof(int)));
     a.visited = reinterpret_cast<uint32_t *>(take(4 * kNaWords));
     a.fb0 = reinterpret_cast<uint32_t *>(take(4 * kNaWords));
@@ -1050,7 +1236,9 @@ extern "C" hc_status hc_bfs_noalloc(const int64_t *index, const int32_t *neighbo
     a.m = num_edges;
     a.depth = depth_out;
     a.parent = parent_out;
-    a.src = source;
+    a.nsrc = 1;
+    a.src[0] = source;
+    a.team = sms * bps;
     a.alpha = 15;
     a.beta = 18;
     a.direction = 0;
@@ -1069,6 +1257,7 @@ extern "C" hc_status hc_bfs_noalloc(const int64_t *index, const int32_t *neighbo
     // The array keeps the previous call's contents; the control block must
     // start at zero (the kernel initialises everything else it reads).
     HC_CUDA_TRY(cudaMemsetAsync(a.ctl, 0, sizeof(BfsCtl), s));
+    HC_CUDA_TRY(cudaMemsetAsync(a.fold, 0, sizeof(BfsFold), s));
     void *params[] = {&a};
     ::hc::count_launch();
     HC_CUDA_TRY(cudaLaunchCooperativeKernel((void *)bfs_persistent<false>, dim3(sms * bps), dim3(kBfsThreads), params,

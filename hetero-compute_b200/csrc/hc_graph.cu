@@ -50,6 +50,13 @@ bool reclaim(hc_graph *g, unsigned keep, const DevBuf *self) {
         drop(g->wf32);
     }
     if (!(keep & kKeepBatch)) drop(g->ws_batch);
+    // Workspaces of several sources at a time (hc_bfs itself opens no scope).
+    drop(g->ws_bfs);
+    if (!(keep & kKeepSssp)) {
+        drop(g->ws_sssp);
+        for (auto &slot : g->ws_stage)
+            for (auto &b : slot) drop(b);
+    }
     return freed;
 }
 }  // namespace
@@ -120,7 +127,7 @@ hc_status copy_out(void *dst_any, const void *src_dev, size_t bytes, cudaStream_
     return HC_OK;
 }
 
-hc_status OutPipe::init(hc_graph *graph, int arrays, size_t each) {
+hc_status OutPipe::init(hc_graph *graph, int arrays, size_t each, int rows) {
     g = graph;
     narr = arrays;
     bytes = each;
@@ -133,7 +140,7 @@ hc_status OutPipe::init(hc_graph *graph, int arrays, size_t each) {
             HC_CUDA_TRY(cudaEventCreateWithFlags(&g->ev_done[s], cudaEventDisableTiming));
             HC_CUDA_TRY(cudaEventRecord(g->ev_done[s], g->copy_stream));  // nothing to wait for yet
         }
-        for (int j = 0; j < arrays; j++) HC_TRY(g->ws_stage[s][j].ensure(each));
+        for (int j = 0; j < arrays; j++) HC_TRY(g->ws_stage[s][j].ensure(each * (size_t)rows));
     }
     return HC_OK;
 }
@@ -146,11 +153,12 @@ hc_status OutPipe::acquire(int i, int32_t **bufs) {
     return HC_OK;
 }
 
-hc_status OutPipe::release(int i, void *const *dst) {
+hc_status OutPipe::release(int i, void *const *dst, int rows) {
     const int s = i & 1;
     HC_CUDA_TRY(cudaEventRecord(g->ev_ready[s], g->stream));
     pending = true;
     pend_slot = s;
+    pend_rows = rows;
     for (int j = 0; j < narr; j++) pend_dst[j] = dst[j];
     return HC_OK;
 }
@@ -161,9 +169,9 @@ hc_status OutPipe::flush() {
     const int s = pend_slot;
     HC_CUDA_TRY(cudaStreamWaitEvent(g->copy_stream, g->ev_ready[s], 0));
     for (int j = 0; j < narr; j++)
-        if (pend_dst[j])
-            HC_CUDA_TRY(cudaMemcpyAsync(pend_dst[j], g->ws_stage[s][j].ptr, copy_bytes, cudaMemcpyDefault,
-                                        g->copy_stream));
+        if (pend_dst[j] && pend_rows > 0)
+            HC_CUDA_TRY(cudaMemcpy2DAsync(pend_dst[j], bytes, g->ws_stage[s][j].ptr, bytes, copy_bytes, pend_rows,
+                                          cudaMemcpyDefault, g->copy_stream));
     HC_CUDA_TRY(cudaEventRecord(g->ev_done[s], g->copy_stream));
     return HC_OK;
 }
@@ -190,16 +198,25 @@ hc_status ctl_zero(hc_graph *g, void *dev, size_t bytes) {
     return HC_OK;
 }
 
-hc_status ctl_read(hc_graph *g, const void *dev, size_t bytes, int slot, const void **host) {
-    if (bytes > kCtlSlotBytes || slot < 0 || slot >= kCtlSlots) return fail(HC_ERR_INVALID_ARG, "ctl_read: bad slot");
+hc_status ctl_slot(hc_graph *g, int slot, void **host, void **dev) {
+    if (slot < 0 || slot >= kCtlSlots) return fail(HC_ERR_INVALID_ARG, "ctl_slot: bad slot");
     if (!g->ctl_host) {
         HC_CUDA_TRY(cudaHostAlloc(&g->ctl_host, kCtlSlotBytes * kCtlSlots, cudaHostAllocMapped));
         HC_CUDA_TRY(cudaHostGetDevicePointer(&g->ctl_host_dev, g->ctl_host, 0));
     }
-    uint32_t *d = reinterpret_cast<uint32_t *>(static_cast<char *>(g->ctl_host_dev) + (size_t)slot * kCtlSlotBytes);
+    *host = static_cast<char *>(g->ctl_host) + (size_t)slot * kCtlSlotBytes;
+    *dev = static_cast<char *>(g->ctl_host_dev) + (size_t)slot * kCtlSlotBytes;
+    return HC_OK;
+}
+
+hc_status ctl_read(hc_graph *g, const void *dev, size_t bytes, int slot, const void **host) {
+    if (bytes > kCtlSlotBytes) return fail(HC_ERR_INVALID_ARG, "ctl_read: bad slot");
+    void *h = nullptr, *hd = nullptr;
+    HC_TRY(ctl_slot(g, slot, &h, &hd));
+    uint32_t *d = static_cast<uint32_t *>(hd);
     { words_to_host<<<1, 256, 0, g->stream>>>(d, reinterpret_cast<const uint32_t *>(dev), (int)((bytes + 3) / 4)); count_launch(); }
     HC_CUDA_TRY(cudaGetLastError());
-    *host = static_cast<const char *>(g->ctl_host) + (size_t)slot * kCtlSlotBytes;
+    *host = h;
     return HC_OK;
 }
 

@@ -127,19 +127,21 @@ hc_status ensure_pr_derived(hc_graph *g, bool weighted);
 struct OutPipe {
     hc_graph *g = nullptr;
     int narr = 0;
-    size_t bytes = 0;
-    size_t copy_bytes = 0;  // bytes of each array copied out (init: all; a caller may shorten it)
+    int pend_rows = 1;
+    size_t bytes = 0;       // of one row
+    size_t copy_bytes = 0;  // bytes of each row copied out (init: all; a caller may shorten it)
     bool pending = false;
     int pend_slot = 0;
     void *pend_dst[2] = {nullptr, nullptr};
-    // Staging and events for `arrays` outputs of `bytes` each.
-    hc_status init(hc_graph *graph, int arrays, size_t each);
+    // Staging and events for `arrays` outputs of up to `rows` rows of `each` bytes.
+    hc_status init(hc_graph *graph, int arrays, size_t each, int rows = 1);
     // Staging buffers of source i (after the wait for the slot's last copy).
     hc_status acquire(int i, int32_t **bufs);
     // Source i's results are complete on the compute stream once what is
     // queued there has run; copy them to dst[] (null entries are skipped).
     // The copy is issued by the next acquire or by finish.
-    hc_status release(int i, void *const *dst);
+    // `rows` consecutive rows of each array.
+    hc_status release(int i, void *const *dst, int rows = 1);
     hc_status flush();
     hc_status finish();
 };
@@ -180,12 +182,15 @@ constexpr size_t kCtlSlotBytes = 4096;
 constexpr int kCtlSlots = 4;
 hc_status ctl_zero(hc_graph *g, void *dev, size_t bytes);
 hc_status ctl_read(hc_graph *g, const void *dev, size_t bytes, int slot, const void **host);
+// Slot `slot` itself: its host address, and the device address of the same
+// memory for a kernel that writes its result there.
+hc_status ctl_slot(hc_graph *g, int slot, void **host, void **dev);
 // Device memory pressure.  Derived arrays that can be built again (the
 // pull sweeps' pair array, the reference-order schedule, the weighted
-// PageRank arrays) and the batched workspace are released, when an
-// allocation fails, unless the running call needs them; the allocation is
+// PageRank arrays), the batched workspace and the BFS and SSSP workspaces and
+// staging are released, when an allocation fails, unless the running call needs them; the allocation is
 // then tried once more.  A call states what it needs for its lifetime.
-enum : unsigned { kKeepAdj = 1u, kKeepPrOrd = 2u, kKeepPrWeighted = 4u, kKeepBatch = 8u };
+enum : unsigned { kKeepAdj = 1u, kKeepPrOrd = 2u, kKeepPrWeighted = 4u, kKeepBatch = 8u, kKeepSssp = 16u };
 struct ReclaimScope {
     ReclaimScope(hc_graph *g, unsigned keep);
     ~ReclaimScope();

@@ -71,3 +71,30 @@ def test_bfs_thin_levels(name, direction):
             assert np.array_equal(depth[i], want)
             assert oracle.verify_bfs_parents(index, nbr, want, parent[i], s)[0] == 0
     g.close()
+
+
+@pytest.mark.parametrize("scale,count", [(6, 1), (6, 300), (10, 7), (13, 65), (17, 18)])
+@pytest.mark.parametrize("host", [False, True])
+def test_bfs_sources_at_a_time(scale, count, host):
+    """Sources run several at a time, in one launch or (more than one launch takes, host outputs) several."""
+    import torch
+
+    import hc
+    host_g = hc.gen_kronecker(scale, 16, 3)
+    n = host_g.num_nodes
+    g = hc.Graph.from_host(host_g)
+    picks = np.random.default_rng(scale).integers(0, n, count).astype(np.int32)  # isolated and repeated ones too
+    if host:
+        depth, parent, _ = g.bfs(picks)
+        only = g.bfs(picks, want_depth=False)[1]
+    else:
+        out = [torch.full((count, n), 7, dtype=torch.int32, device="cuda") for _ in range(3)]
+        depth, parent, _ = g.bfs(picks, out[0], out[1])
+        only = g.bfs(picks, None, out[2], want_depth=False)[1].cpu().numpy()
+        depth, parent = depth.cpu().numpy(), parent.cpu().numpy()
+    for i in sorted({0, count // 2, count - 1, *range(0, count, 17)}):
+        want = oracle.bfs_depth(host_g.index, host_g.neighbors, picks[i])
+        assert np.array_equal(depth[i], want)
+        for p in (parent[i], only[i]):
+            assert oracle.verify_bfs_parents(host_g.index, host_g.neighbors, want, p, picks[i])[0] == 0
+    g.close()
