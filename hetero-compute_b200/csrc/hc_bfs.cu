@@ -51,11 +51,13 @@ constexpr int kSumWords = 4096;
 // block barrier per level and the frontier in shared memory, for up to
 // kSoloLevels levels at a time while the other blocks wait at one grid
 // barrier.  Such a level is a chain of dependent L2 round trips: on the grid it
-// also pays the barrier and the global queue's counters.  The limits: one block keeps 2048
-// edges in flight, so above a few rounds of those the grid is faster; a row
-// longer than kSoloDeg would serialise on one warp.
+// also pays the barrier and the global queue's counters (a 100-vertex level of a
+// grid graph: 2.9 us here, 7 us there).  The limits: one block keeps 2048 edges
+// in flight, and above one round of those the grid is faster (1023 x 1025
+// grid: limit 1024 9.6 ms, 2048 9.1 ms, 4096 10.0 ms, 8192 13.5 ms, no thin
+// levels 16 ms); a row longer than kSoloDeg would serialise on one warp.
 constexpr int kSoloCap = 1920;
-constexpr int kSoloEdges = 8192;
+constexpr int kSoloEdges = 2048;
 constexpr int kSoloDeg = 128;
 constexpr int kSoloLevels = 1024;
 
@@ -246,31 +248,32 @@ __device__ __noinline__ SoloState solo_levels(SoloArgs a, const BfsRun &r, BfsCt
     long long edges_to_check = st.edges_to_check, num_edges = st.num_edges;
     unsigned long long my_vscan = st.vscan, my_escan = st.escan;
     __shared__ int s_n[3];
-    __shared__ unsigned long long s_mf[3];
+    __shared__ unsigned long long s_sum;
+    __shared__ unsigned s_mf[3];  // exact while no row is long (see the end)
     __shared__ int s_wide[3];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     const unsigned lt = (1u << lane) - 1u;
     const int32_t *qin = (L & 1) ? r.q1 : r.q0;
     if (threadIdx.x < 3) {
         s_n[threadIdx.x] = 0;
-        s_mf[threadIdx.x] = 0ull;
+        s_mf[threadIdx.x] = 0u;
         s_wide[threadIdx.x] = 0;
     }
     __syncthreads();
-    unsigned long long edges = 0;
+    unsigned edges = 0;
     for (int i = threadIdx.x; i < nf; i += blockDim.x) {
         const int32_t u = __ldcg(qin + i);
         const int64_t b = __ldg(a.index + u), d = __ldg(a.index + u + 1) - b;
         sq[0].u[i] = u;
         sq[0].row[i] = solo_row(b, d);
-        edges += (unsigned long long)d;
+        edges += (unsigned)min(d, (int64_t)kSoloEdges);
         if (d > kSoloDeg) s_wide[0] = 1;
     }
     // The frontier's own edges: after a bottom-up level num_edges is not their count.
-    edges = warp_sum(edges);
+    edges = __reduce_add_sync(kFull, edges);
     if (lane == 0 && edges) atomicAdd(&s_mf[0], edges);
     __syncthreads();
-    bool wide = s_wide[0] || s_mf[0] > (unsigned long long)kSoloEdges;
+    bool wide = s_wide[0] || s_mf[0] > (unsigned)kSoloEdges;
     for (int step = 0; step < kSoloLevels; step++) {
         const int ns = (step + 1) % 3;
         if (nf == 0 || nf > kSoloCap || wide || L >= a.max_levels ||
@@ -283,7 +286,7 @@ __device__ __noinline__ SoloState solo_levels(SoloArgs a, const BfsRun &r, BfsCt
         td_levels++;
         if (threadIdx.x == 0) {
             s_n[(step + 2) % 3] = 0;
-            s_mf[(step + 2) % 3] = 0ull;
+            s_mf[(step + 2) % 3] = 0u;
             s_wide[(step + 2) % 3] = 0;
             if (L < kTraceLevels) {
                 ctl->trace[L].mode = 1;
@@ -347,7 +350,7 @@ __device__ __noinline__ SoloState solo_levels(SoloArgs a, const BfsRun &r, BfsCt
                     nb[j] = take[j] ? __ldg(a.index + v[j]) : 0;
                     nd[j] = take[j] ? __ldg(a.index + v[j] + 1) : 0;
                 }
-                unsigned long long dsum = 0;
+                unsigned dsum = 0;
 #pragma unroll
                 for (int j = 0; j < kUnroll; j++) {
                     if (take[j]) {
@@ -359,12 +362,12 @@ __device__ __noinline__ SoloState solo_levels(SoloArgs a, const BfsRun &r, BfsCt
                             nq.u[p] = v[j];
                             nq.row[p] = solo_row(nb[j], nd[j] - nb[j]);
                         }
-                        dsum += (unsigned long long)(nd[j] - nb[j]);
+                        dsum += (unsigned)min(nd[j] - nb[j], (int64_t)kSoloEdges);
                         if (nd[j] - nb[j] > kSoloDeg) s_wide[ns] = 1;
                     }
                     pos += __popc(bal[j]);
                 }
-                dsum = warp_sum(dsum);
+                dsum = __reduce_add_sync(kFull, dsum);
                 if (lane == 0) atomicAdd(&s_mf[ns], dsum);
             }
         }
@@ -373,6 +376,22 @@ __device__ __noinline__ SoloState solo_levels(SoloArgs a, const BfsRun &r, BfsCt
         num_edges = (long long)s_mf[ns];
         wide = s_wide[ns] || num_edges > kSoloEdges;
         L++;
+    }
+    if (wide && L != st.L) {
+        // The sum of a frontier with long rows, exactly: the direction rule reads it.
+        __syncthreads();
+        if (threadIdx.x == 0) s_sum = 0ull;
+        __syncthreads();
+        const int32_t *q = (L & 1) ? r.q1 : r.q0;
+        unsigned long long sum = 0;
+        for (int i = threadIdx.x; i < nf; i += blockDim.x) {
+            const int32_t u = __ldcg(q + i);
+            sum += (unsigned long long)(__ldg(a.index + u + 1) - __ldg(a.index + u));
+        }
+        sum = warp_sum(sum);
+        if (lane == 0 && sum) atomicAdd(&s_sum, sum);
+        __syncthreads();
+        num_edges = (long long)s_sum;
     }
     return SoloState{L, nf, td_levels, edges_to_check, num_edges, my_vscan, my_escan};
 }

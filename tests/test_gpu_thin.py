@@ -98,3 +98,71 @@ def test_bfs_sources_at_a_time(scale, count, host):
         for p in (parent[i], only[i]):
             assert oracle.verify_bfs_parents(host_g.index, host_g.neighbors, want, p, picks[i])[0] == 0
     g.close()
+
+
+def weights(index, nbr, top):
+    """Symmetric integer weights in [0, top]: a hash of the unordered pair."""
+    row = np.repeat(np.arange(len(index) - 1, dtype=np.int64), np.diff(index))
+    lo, hi = np.minimum(row, nbr), np.maximum(row, nbr)
+    h = (lo * 2654435761 + hi * 40503 + 12345) & 0x7FFFFFFF
+    return ((h >> 7) % (top + 1)).astype(np.int32)
+
+
+def shuffled(index, nbr, seed):
+    """The same graph under a random relabelling: rows of all lengths side by side."""
+    n = len(index) - 1
+    perm = np.random.default_rng(seed).permutation(n)
+    row = np.repeat(np.arange(n), np.diff(index))
+    u, v = perm[row], perm[nbr]
+    keep = u < v
+    return csr(n, u[keep], v[keep])
+
+
+@pytest.mark.parametrize("top", [1, 255, 70000])
+@pytest.mark.parametrize("name", sorted(GRAPHS) + ["mixed"])
+def test_sssp_thin_epochs(name, top):
+    import hc
+    if name == "mixed":  # unsorted: long rows inside groups of short ones
+        k = hc.gen_kronecker(12, 16, 5)
+        index, nbr = shuffled(k.index, k.neighbors, 1)
+    else:
+        index, nbr = GRAPHS[name]()
+    w = weights(index, nbr, top)
+    n = len(index) - 1
+    g = hc.Graph(index, nbr, w)
+    sources = [0, n - 1, n // 2]
+    want = [oracle.sssp_dijkstra(index, nbr, w, s) for s in sources]
+    for kw in ({}, {"delta": -1}, {"delta": 1 + top // 8, "pull_alpha": -1}, {"pull_alpha": 1 << 20}, {"stats": True}):
+        dist, parent, _ = g.sssp(sources, want_parent=True, **kw)
+        for i, s in enumerate(sources):
+            assert np.array_equal(dist[i], want[i]), (kw, s)
+            v = np.flatnonzero((dist[i] != hc.INF_DIST) & (np.arange(n) != s))
+            assert (parent[i][v] >= 0).all() and (parent[i][dist[i] == hc.INF_DIST] == -1).all()
+            assert (dist[i][parent[i][v]] <= dist[i][v]).all()
+    g.close()
+
+
+@pytest.mark.parametrize("scale,count", [(6, 1), (6, 300), (10, 7), (13, 65), (16, 18)])
+@pytest.mark.parametrize("out", ["host", "device", "parents"])
+def test_sssp_sources_at_a_time(scale, count, out):
+    import torch
+
+    import hc
+    h = hc.gen_kronecker(scale, 16, 3, wtype=hc.W_I32)
+    n = h.num_nodes
+    g = hc.Graph.from_host(h)
+    picks = np.random.default_rng(scale).integers(0, n, count).astype(np.int32)  # isolated and repeated ones too
+    if out == "host":
+        dist = g.sssp(picks)[0]
+    else:
+        dist = torch.full((count, n), 7, dtype=torch.int32, device="cuda")
+        parent = torch.full((count, n), 7, dtype=torch.int32, device="cuda") if out == "parents" else None
+        g.sssp(picks, dist, parent)
+        dist = dist.cpu().numpy()
+    for i in sorted({0, count // 2, count - 1, *range(0, count, 17)}):
+        assert np.array_equal(dist[i], oracle.sssp_dijkstra(h.index, h.neighbors, h.weights, picks[i]))
+        if out == "parents":
+            p = parent[i].cpu().numpy()
+            v = np.flatnonzero((dist[i] != hc.INF_DIST) & (np.arange(n) != picks[i]))
+            assert p[picks[i]] == picks[i] and (p[v] >= 0).all() and (dist[i][p[v]] < dist[i][v]).all()
+    g.close()
