@@ -69,12 +69,13 @@ struct EpochCnt {
     int nq;                 // vertices in this near queue
     int tasks;              // long-row tasks queued while expanding it
     unsigned long long mf;  // sum of their degrees
+    int32_t low;            // at most the smallest distance in it
 };
 
 // Loop state of a run that one block hands to the others after thin epochs.
 struct SoloState {
     int E, phase, fgen, nq;
-    int32_t T;
+    int32_t T, low;
     unsigned long long mf, vproc, erelax;
 };
 
@@ -89,6 +90,7 @@ struct SsspCtl {
     // (three slots, by pull): the next epoch's push-or-pull test, without
     // building its queue.
     unsigned long long pull_mf[3];
+    int32_t pull_low[3];  // the smallest distance it wrote
     SoloState solo;
     int epochs, phases, pulls, pad;
     unsigned long long vproc, erelax;
@@ -166,6 +168,7 @@ struct RelaxVisit {
     bool use_far;
     unsigned long long relaxed;
     unsigned long long mf;  // degree sum of this thread's near appends
+    int32_t low;            // smallest near candidate below its target's distance (this thread)
     struct Item {
         int32_t v, nd, dv;
     };
@@ -185,7 +188,10 @@ struct RelaxVisit {
         for (int j = 0; j < kUnroll; j++) {
             relaxed += act[j];
             imp[j] = act[j] && it[j].nd < it[j].dv;
-            if (imp[j]) atomicMin(dist + it[j].v, it[j].nd);
+            if (imp[j]) {
+                atomicMin(dist + it[j].v, it[j].nd);
+                low = min(low, it[j].nd);
+            }
             old[j] = imp[j] ? (it[j].nd < T ? atomicMax(stamp + it[j].v, next_e) : atomicMax(fstamp + it[j].v, far_claim))
                             : 0;
         }
@@ -210,27 +216,30 @@ struct RelaxVisit {
 __device__ __forceinline__ int wbucket(int32_t w, int ws) { return w >> ws; }
 __device__ __forceinline__ int32_t wbucket_floor(int bk, int ws) { return bk << ws; }
 
-// dist[u] + w for a pair whose weight is below `bound`, else INT32_MAX
-// without touching dist: a candidate is at least its weight, so a pair with
-// w >= bound cannot lower a row whose best so far is `bound`.
+// dist[u] + w for a pair whose weight is below `gap`, else INT32_MAX without
+// touching dist.  The gap of a row is the best distance it has so far, less
+// `low`: a distance that has not been relaxed along its edges yet is at least
+// `low` (the smallest one in the queue, and candidates only add to it), and the
+// smaller ones were relaxed when they were set, so a pair with w >= gap cannot
+// lower the row.
 // The gather goes through L1 (.ca): most edges point at a few thousand hub
 // rows, whose distances then stay on the SM.  A value cached earlier in the
 // same sweep can be stale, but distances only fall, so it is an upper bound,
 // and the row that lowered it is marked changed and relaxed again next epoch;
 // kernel boundaries and the grid barrier's fence invalidate L1 between epochs.
-__device__ __forceinline__ int32_t pull_cand(const int32_t *dist, int2 p, int32_t bound) {
-    return p.y < bound ? sat_add(__ldca(dist + p.x), p.y) : kInfDist;
+__device__ __forceinline__ int32_t pull_cand(const int32_t *dist, int2 p, int32_t gap) {
+    return p.y < gap ? sat_add(__ldca(dist + p.x), p.y) : kInfDist;
 }
 
 // The warp walks the pairs [b, e) of one row, 128 at a time, with a running
-// bound (the row's distance d0, then the best candidate): pairs at or above it
-// gather nothing, and the walk stops at the first window whose leading bucket
-// floor reaches it.  The leading weight of the next window is read one window
+// bound (the row's distance d0, then the best candidate): pairs at or above its
+// gap to `low` gather nothing, and the walk stops at the first window whose
+// leading bucket floor reaches it.  The leading weight of the next window is read one window
 // ahead, so that the stop test comes before the window's loads; `test_first`
 // tests the first window too (a range that starts among the row's heavier
 // pairs).  Returns the bound; *next receives the slot it stopped at.
 __device__ __forceinline__ int32_t pull_walk(const SsspArgs &a, const int32_t *dist, int64_t b, int64_t e, int32_t d0,
-                                             bool test_first, int64_t *next) {
+                                             int32_t low, bool test_first, int64_t *next) {
     const int lane = threadIdx.x & 31;
     const int32_t *wcol = reinterpret_cast<const int32_t *>(a.adj) + 1;
     int32_t wnext = test_first ? __ldg(wcol + 2 * b) : 0;
@@ -238,7 +247,7 @@ __device__ __forceinline__ int32_t pull_walk(const SsspArgs &a, const int32_t *d
     int64_t i0 = b;
     for (; i0 < e; i0 += 128) {
         // Pair i0 carries the smallest bucket of the rest of the range.
-        if ((i0 > b || test_first) && wbucket_floor(wbucket(wnext, a.ws), a.ws) >= bound) break;
+        if ((i0 > b || test_first) && wbucket_floor(wbucket(wnext, a.ws), a.ws) >= bound - low) break;
         int2 q[4];
 #pragma unroll
         for (int j = 0; j < 4; j++) {
@@ -248,7 +257,7 @@ __device__ __forceinline__ int32_t pull_walk(const SsspArgs &a, const int32_t *d
         if (i0 + 128 < e) wnext = __ldg(wcol + 2 * (i0 + 128));
         int32_t m = kInfDist;
 #pragma unroll
-        for (int j = 0; j < 4; j++) m = min(m, pull_cand(dist, q[j], bound));
+        for (int j = 0; j < 4; j++) m = min(m, pull_cand(dist, q[j], bound - low));
         bound = min(bound, __reduce_min_sync(kFull, m));
     }
     *next = min(i0, e);
@@ -261,14 +270,15 @@ __device__ __forceinline__ int32_t pull_walk(const SsspArgs &a, const int32_t *d
 // each and lower dist by atomicMin.  In a stream group (32 rows, one warp, the
 // only writer of its rows and of their word of the bitmap) a lane walks its own
 // row, four pairs at a time, and stops where the bucket floor reaches its
-// bound: on weights uniform in [1, 255] with distances near 40 that is a fifth
-// of the row, so the sweep reads and searches that much less than a warp that
-// streams the whole group.  Rows longer than kLaneRow would hold their warp
-// up and are walked by the whole of it.  Lowered vertices are marked in `changed`.
+// gap: on weights uniform in [1, 255] that is a small part of the row, so the
+// sweep reads and searches that much less than a warp that streams the whole
+// group.  Rows longer than kLaneRow would hold their warp up and are walked by
+// the whole of it.  Lowered vertices are marked in `changed`.
 constexpr int kLaneRow = 128;
 template <bool kStats>
 __device__ __forceinline__ void pull_sweep(const SsspArgs &a, int32_t *dist, uint32_t *changed, int gwarp, int nwarps,
-                                           unsigned long long &my_e, int32_t T, unsigned long long &my_mf) {
+                                           unsigned long long &my_e, int32_t T, int32_t low,
+                                           unsigned long long &my_mf, int32_t &my_low) {
     const int lane = threadIdx.x & 31;
     const PrPlanDev &p = a.plan;
     const int total = p.n_tasks + p.n_long + p.n_stream;
@@ -291,9 +301,11 @@ __device__ __forceinline__ void pull_sweep(const SsspArgs &a, int32_t *dist, uin
             }
             const int32_t d0 = __shfl_sync(kFull, __ldcg(dist + r), 0);
             int64_t next;
-            const int32_t bound = pull_walk(a, dist, b, e, d0, test_first, &next);
+            if (d0 <= low) continue;  // final
+            const int32_t bound = pull_walk(a, dist, b, e, d0, low, test_first, &next);
             if (lane == 0) {
                 if (bound < d0 && bound < __ldcg(dist + r) && bound < atomicMin(dist + r, bound)) {
+                    my_low = min(my_low, bound);
                     const uint32_t bit = 1u << (r & 31);
                     if (!(atomicOr(changed + (r >> 5), bit) & bit) && bound < T)
                         my_mf += (unsigned long long)(__ldg(a.index + r + 1) - __ldg(a.index + r));
@@ -311,31 +323,32 @@ __device__ __forceinline__ void pull_sweep(const SsspArgs &a, int32_t *dist, uin
                 d0 = __ldcg(dist + r);
             }
             int32_t bound = d0;
-            const bool whole = e - b > kLaneRow;
-            int64_t i = whole ? e : b;
+            const bool whole = e - b > kLaneRow && d0 > low;
+            int64_t i = whole || d0 <= low ? e : b;
             while (i < e) {
                 int2 q[4];
 #pragma unroll
                 for (int j = 0; j < 4; j++) q[j] = i + j < e ? __ldg(a.adj + i + j) : make_int2(0, kInfDist);
-                if (wbucket_floor(wbucket(q[0].y, a.ws), a.ws) >= bound) break;
+                if (wbucket_floor(wbucket(q[0].y, a.ws), a.ws) >= bound - low) break;
                 int32_t m[4];
 #pragma unroll
-                for (int j = 0; j < 4; j++) m[j] = pull_cand(dist, q[j], bound);
+                for (int j = 0; j < 4; j++) m[j] = pull_cand(dist, q[j], bound - low);
                 bound = min(bound, min(min(m[0], m[1]), min(m[2], m[3])));
                 i += 4;
             }
-            if (kStats && !whole) my_e += (unsigned long long)(min(i, e) - b);
+            if (kStats && !whole && d0 > low) my_e += (unsigned long long)(min(i, e) - b);
             for (unsigned left = __ballot_sync(kFull, whole); left; left &= left - 1u) {
                 const int src = __ffs(left) - 1;
                 const int64_t wb = __shfl_sync(kFull, b, src), we = __shfl_sync(kFull, e, src);
                 int64_t next;
-                const int32_t got = pull_walk(a, dist, wb, we, __shfl_sync(kFull, d0, src), false, &next);
+                const int32_t got = pull_walk(a, dist, wb, we, __shfl_sync(kFull, d0, src), low, false, &next);
                 if (lane == src) bound = got;
                 if (kStats && lane == 0) my_e += (unsigned long long)(next - wb);
             }
             const bool ch = bound < d0;
             if (ch) {
                 dist[r] = bound;
+                my_low = min(my_low, bound);
                 if (bound < T) my_mf += (unsigned long long)(e - b);
             }
             const unsigned bal = __ballot_sync(kFull, ch);
@@ -582,20 +595,31 @@ __device__ __noinline__ SoloState solo_epochs(SoloArgs a, const SsspRun &r, Sssp
         k++;
     }
     __syncthreads();
-    if (wide && st.nq > 0) {
-        // The sum of a queue with long rows, exactly: the pull test reads it.
-        if (threadIdx.x == 0) s_sum = 0ull;
+    if (st.nq > 0) {
+        // The queue's degree sum (exact with long rows too) and its smallest
+        // distance: a pull reads them.
+        if (threadIdx.x == 0) {
+            s_sum = 0ull;
+            s_min = kInfDist;
+        }
         __syncthreads();
+        int32_t low = kInfDist;
         const int32_t *q = (st.E & 1) ? r.q1 : r.q0;
         unsigned long long sum = 0;
         for (int i = threadIdx.x; i < st.nq; i += blockDim.x) {
             const int32_t u = __ldcg(q + i);
             sum += (unsigned long long)(__ldg(a.index + u + 1) - __ldg(a.index + u));
+            low = min(low, __ldcg(dist + u));
         }
         sum = warp_sum(sum);
-        if (lane == 0 && sum) atomicAdd(&s_sum, sum);
+        low = __reduce_min_sync(kFull, low);
+        if (lane == 0) {
+            if (sum) atomicAdd(&s_sum, sum);
+            atomicMin(&s_min, low);
+        }
         __syncthreads();
         st.mf = s_sum;
+        st.low = s_min;
     }
     if (threadIdx.x < 2) far_len[threadIdx.x] = s_far[threadIdx.x];
     return st;
@@ -606,6 +630,12 @@ union SsspShared {
     SoloQueue solo[2];                          // thin epochs
     uint32_t fold[kSsspThreads / 32][2][32];    // per warp: near / far masks of its 32 words
 };
+
+// Lowers *p to the smallest x of the warp (every lane calls it).
+__device__ __forceinline__ void note_low(int32_t *p, int32_t x) {
+    x = __reduce_min_sync(kFull, x);
+    if ((threadIdx.x & 31) == 0 && x < kInfDist && x < __ldcg(p)) atomicMin(p, x);
+}
 
 template <bool kStats>
 __global__ void __launch_bounds__(kSsspThreads, 2) sssp_persistent(SsspArgs a) {
@@ -677,12 +707,13 @@ __global__ void __launch_bounds__(kSsspThreads, 2) sssp_persistent(SsspArgs a) {
         const unsigned long long t_start = globaltimer_ns();
         if (gtid == 0) {
             r.q0[0] = r.src;
-            cnt[0] = EpochCnt{1, 0, (unsigned long long)(a.index[r.src + 1] - a.index[r.src])};
-            cnt[1] = EpochCnt{0, 0, 0ull};
-            cnt[2] = EpochCnt{0, 0, 0ull};
+            cnt[0] = EpochCnt{1, 0, (unsigned long long)(a.index[r.src + 1] - a.index[r.src]), 0};
+            cnt[1] = EpochCnt{0, 0, 0ull, kInfDist};
+            cnt[2] = EpochCnt{0, 0, 0ull, kInfDist};
             far_len[0] = far_len[1] = 0;
             *min_far = kInfDist;
             ctl->pull_mf[0] = ctl->pull_mf[1] = ctl->pull_mf[2] = 0ull;
+            ctl->pull_low[0] = ctl->pull_low[1] = ctl->pull_low[2] = kInfDist;
         }
         failed = !team_sync();
 
@@ -704,9 +735,11 @@ __global__ void __launch_bounds__(kSsspThreads, 2) sssp_persistent(SsspArgs a) {
                 cold->nq = 0;
                 cold->tasks = 0;
                 cold->mf = 0;
+                cold->low = kInfDist;
             }
             int nq = from_solo ? __ldcg(&ctl->solo.nq) : __ldcg(&ccur->nq);
             unsigned long long mfc = from_solo ? __ldcg(&ctl->solo.mf) : __ldcg(&ccur->mf);
+            int32_t low = from_solo ? __ldcg(&ctl->solo.low) : __ldcg(&ccur->low);
             from_solo = false;
             int fl = 0;
             if (nq == 0) {
@@ -720,7 +753,7 @@ __global__ void __launch_bounds__(kSsspThreads, 2) sssp_persistent(SsspArgs a) {
                 if (team_block == 0) {
                     const SoloState st = solo_epochs<kStats>(
                         SoloArgs{a.index, a.nbr, a.w, a.m, a.delta, a.pull_alpha, a.max_epochs, pulls > 0}, r, ctl,
-                        far_len, sh.solo, SoloState{E, phase, fgen, nq, T, mfc, 0ull, 0ull});
+                        far_len, sh.solo, SoloState{E, phase, fgen, nq, T, low, mfc, 0ull, 0ull});
                     if (threadIdx.x == 0) {
                         ctl->solo = st;
                         if (kStats) {
@@ -845,6 +878,7 @@ __global__ void __launch_bounds__(kSsspThreads, 2) sssp_persistent(SsspArgs a) {
                 fgen++;
                 nq = __ldcg(&ccur->nq);
                 mfc = __ldcg(&ccur->mf);
+                low = mfar;
                 if (nq == 0) continue;
             }
             if (E >= a.max_epochs) {
@@ -867,17 +901,19 @@ __global__ void __launch_bounds__(kSsspThreads, 2) sssp_persistent(SsspArgs a) {
             if (kStats && gtid == 0) my_v += nq;
             if (!pull) {
                 RelaxVisit relax{a.index, a.nbr, a.w, r.dist, r.stamp, r.fstamp, qnext, &cnxt->nq, fpile,
-                                 fpile_len, T, next_e, fgen, use_far, 0ull, 0ull};
+                                 fpile_len, T, next_e, fgen, use_far, 0ull, 0ull, kInfDist};
                 expand_small(a.index, qcur, nq, r.tasks, &ccur->tasks, gwarp, nwarps, relax);
                 unsigned long long mfb = block_sum(relax.mf, s_red);
                 if (threadIdx.x == 0 && mfb) atomicAdd(&cnxt->mf, mfb);
                 relax.mf = 0;
+                note_low(&cnxt->low, relax.low);
                 if ((failed = !team_sync())) break;
                 const int nt = __ldcg(&ccur->tasks);
                 if (nt > 0) {
                     expand_tasks(a.index, r.tasks, nt, gwarp, nwarps, relax);
                     mfb = block_sum(relax.mf, s_red);
                     if (threadIdx.x == 0 && mfb) atomicAdd(&cnxt->mf, mfb);
+                    note_low(&cnxt->low, relax.low);
                     if ((failed = !team_sync())) break;
                 }
                 if (kStats) my_e += relax.relaxed;
@@ -895,13 +931,17 @@ __global__ void __launch_bounds__(kSsspThreads, 2) sssp_persistent(SsspArgs a) {
                 if (gtid == 0) {
                     *fpile_len = 0;
                     ctl->pull_mf[(pulls + 1) % 3] = 0ull;  // last read two sweeps ago
+                    ctl->pull_low[(pulls + 1) % 3] = kInfDist;
                 }
                 unsigned long long my_mf = 0;
-                pull_sweep<kStats>(a, r.dist, r.changed, gwarp, nwarps, my_e, T, my_mf);
+                int32_t my_low = kInfDist;
+                pull_sweep<kStats>(a, r.dist, r.changed, gwarp, nwarps, my_e, T, low, my_mf, my_low);
+                note_low(&ctl->pull_low[pulls % 3], my_low);
                 const unsigned long long mfb = block_sum(my_mf, s_red);
                 if (threadIdx.x == 0 && mfb) atomicAdd(&ctl->pull_mf[pulls % 3], mfb);
                 if ((failed = !team_sync())) break;
                 const unsigned long long pull_mf = __ldcg(&ctl->pull_mf[pulls % 3]);
+                low = __ldcg(&ctl->pull_low[pulls % 3]);
                 pulls++;
                 fgen++;  // the rows it lowered rejoin the pile under a new claim
                 if (!((double)pull_mf * (double)a.pull_alpha > (double)a.m) || E + 1 >= a.max_epochs) break;
@@ -1010,6 +1050,7 @@ __global__ void __launch_bounds__(kSsspThreads, 2) sssp_persistent(SsspArgs a) {
                 }
                 mf_next = block_sum(mf_next, s_red);
                 if (threadIdx.x == 0 && mf_next) atomicAdd(&cnxt->mf, mf_next);
+                if (gtid == 0) atomicMin(&cnxt->low, low);  // every queued row is one that the sweep lowered
             }
             if ((failed = !team_sync())) break;
             E++;
