@@ -29,6 +29,19 @@ struct PrPlanDev {
     const HubInfo *hubs;
     int n_stream, n_long, n_tasks, n_hub;
 };
+
+// Row plan of the multi-column PageRank sweeps:
+//   tasks   chunks of rows longer than one chunk (hub index, chunk)
+//   longs   rows of more than kSpmmLong edges, a warp each
+//   the rest, kSpmmRows consecutive rows to a warp
+constexpr int kSpmmLong = 64;
+constexpr int kSpmmRows = 8;
+struct SpmmPlanDev {
+    const int32_t *longs;
+    const int2 *tasks;
+    const HubInfo *hubs;
+    int n_long, n_tasks, n_hub, chunk;
+};
 }  // namespace hc
 
 // Layout in HBM (one allocation per array, 256-byte aligned by cudaMalloc):
@@ -66,6 +79,9 @@ struct hc_graph {
     hc::PrPlanDev pr_view{};   // host copy of its pointers and counts
     int32_t pr_partial_slots = 0;
     hc::DevBuf pr_plan_huge_rows;
+    hc::DevBuf spmm_plan;          // multi-column row plan (device arrays)
+    hc::SpmmPlanDev spmm_view{};
+    int32_t spmm_partial_slots = 0;
     // level schedule of the reference-order PageRank sweep (hc_pr_ordered.cu):
     // order[N] | level_off[levels + 1] | level_long[levels] | deg as fp32 [N];
     // levels -1 = not built

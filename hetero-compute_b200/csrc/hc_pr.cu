@@ -348,30 +348,38 @@ __global__ void __launch_bounds__(kPrThreads) pr_edge_grad(PrPlanDev plan, const
 }
 
 // ---------------------------------------------------------------- SpMM form
-// K columns per vertex, vertex-major [N][K]; warp per row, lane c handles
-// columns c, c+32, ...; hub rows are chunked like the single-column plan.
+// K columns per vertex, vertex-major [N][S], S = K rounded up to four (the
+// added columns hold zeros).  Every gather is a float4: kLanes lanes hold one
+// neighbour's row segment (kVec float4 each), so a warp has 32 / kLanes
+// neighbours per load and kFlight loads in flight.  A hub chunk or long row is
+// spread over the whole warp; shorter rows take 32 / kLanes at a time, one per
+// kLanes lanes.  (One neighbour per round trip left a warp waiting on L2 for its
+// whole row: Kronecker scale 18, 48 columns, 541 us a sweep; the gathers are 1.46
+// GB through L2.)
 struct SpmmArgs {
     const int64_t *index;
     const int32_t *nbr;
     const float *ew;
-    const float *gin;        // [N][K], already divided by deg (unweighted)
+    const float *gin;        // [N][S], already divided by deg (unweighted)
     const float *xin;
-    const float *basev;      // [N][K] dense base, or null with seeds
+    const float *basev;      // [N][S] dense base, or null with seeds
     const int32_t *seed_off; // sparse teleport: column c has seeds seed_idx[seed_off[c]..seed_off[c+1])
     const int32_t *seed_idx;
     float d;
     const float *ps;         // per-row gather scale
     float *xout, *gout;
-    float *partials;         // [chunks][K]
+    float *partials;         // [chunks][S]
     unsigned *hub_count;
-    double *col_l1;          // [K] accumulators for this sweep
+    double *col_l1;          // [S] accumulators for this sweep
     const int32_t *col_map;  // packed column -> seed-list column (null: identity)
-    int K;                   // columns in the packed layout
+    int K, S;                // columns in the packed layout, and its row stride
     int32_t n_active;
 };
+__host__ __device__ constexpr int spmm_stride(int K) { return (K + 3) / 4 * 4; }
 
 __device__ __forceinline__ float spmm_base(const SpmmArgs &a, int32_t r, int c, float one_minus_d) {
-    if (a.basev) return a.basev[(size_t)r * a.K + c];
+    if (a.basev) return a.basev[(size_t)r * a.S + c];
+    if (c >= a.K) return 0.f;
     // Uniform over the seed set of column c.
     const int cc = a.col_map ? a.col_map[c] : c;
     const int32_t b = a.seed_off[cc], e = a.seed_off[cc + 1];
@@ -380,61 +388,119 @@ __device__ __forceinline__ float spmm_base(const SpmmArgs &a, int32_t r, int c, 
     return 0.f;
 }
 
-template <int kCols>
-__global__ void __launch_bounds__(kPrThreads) spmm_sweep(SpmmArgs a, PrPlanDev plan, const uint8_t *is_seed) {
-    const int lane = threadIdx.x & 31;
+__device__ __forceinline__ void add4(float4 &x, const float4 &y) {
+    x.x += y.x;
+    x.y += y.y;
+    x.z += y.z;
+    x.w += y.w;
+}
+__device__ __forceinline__ void fma4(float4 &x, float w, const float4 &y) {
+    x.x += w * y.x;
+    x.y += w * y.y;
+    x.z += w * y.z;
+    x.w += w * y.w;
+}
+
+// Adds w * gin[nbr] over the edges i = b, b + step, ... below e to this lane's columns.
+template <int kVec, int kLanes, bool kEW>
+__device__ __forceinline__ void spmm_range(const SpmmArgs &a, int64_t b, int64_t e, int step, int q0,
+                                           float4 (&acc)[kVec]) {
+    constexpr int kFlight = kVec > 1 ? 4 : 8;
+    for (int64_t i0 = b; i0 < e; i0 += (int64_t)step * kFlight) {
+        float4 v[kFlight][kVec];
+        float w[kFlight];
+        int32_t u[kFlight];
+#pragma unroll
+        for (int f = 0; f < kFlight; f++) {
+            const int64_t i = i0 + (int64_t)f * step;
+            u[f] = i < e ? __ldg(a.nbr + i) : -1;
+            w[f] = kEW && i < e ? __ldg(a.ew + i) : 0.f;
+        }
+#pragma unroll
+        for (int f = 0; f < kFlight; f++)
+#pragma unroll
+            for (int j = 0; j < kVec; j++) {
+                const int c = q0 + 4 * kLanes * j;
+                v[f][j] = u[f] >= 0 && c < a.S ? __ldg(reinterpret_cast<const float4 *>(a.gin + (size_t)u[f] * a.S + c))
+                                               : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+        for (int f = 0; f < kFlight; f++)
+#pragma unroll
+            for (int j = 0; j < kVec; j++) {
+                if (kEW) fma4(acc[j], w[f], v[f][j]);
+                else add4(acc[j], v[f][j]);
+            }
+    }
+}
+
+template <int kVec, int kLanes, bool kEW>
+__global__ void __launch_bounds__(kPrThreads) spmm_sweep(SpmmArgs a, SpmmPlanDev plan, const uint8_t *is_seed) {
+    constexpr int kSub = 32 / kLanes;  // rows (or neighbours of one row) at a time
+    __shared__ float s_l1[kPrThreads / 32][4 * kLanes * kVec];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const int sub = lane / kLanes, q0 = 4 * (lane % kLanes);
     const int gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
-    const int K = a.K;
     const float omd = 1.0f - a.d;
-    float l1[kCols];
+    float4 l1[kVec];
 #pragma unroll
-    for (int j = 0; j < kCols; j++) l1[j] = 0.f;
-    // Every row with edges is its own item here (long rows and stream rows
-    // alike); hub rows are chunked.
-    const int n_rows = a.n_active;
-    const int total = plan.n_tasks + n_rows;
-    auto finish = [&](int32_t r, float *acc) {
-        const float pscale = a.ps ? a.ps[r] : 1.0f;
+    for (int j = 0; j < kVec; j++) l1[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto clear = [](float4 (&x)[kVec]) {
+#pragma unroll
+        for (int j = 0; j < kVec; j++) x[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    // The subs' sums of one row, in every sub.
+    auto combine = [](float4 (&x)[kVec]) {
+#pragma unroll
+        for (int o = kLanes; o < 32; o <<= 1)
+#pragma unroll
+            for (int j = 0; j < kVec; j++) {
+                float4 y;
+                y.x = __shfl_xor_sync(kFull, x[j].x, o);
+                y.y = __shfl_xor_sync(kFull, x[j].y, o);
+                y.z = __shfl_xor_sync(kFull, x[j].z, o);
+                y.w = __shfl_xor_sync(kFull, x[j].w, o);
+                add4(x[j], y);
+            }
+    };
+    auto finish = [&](int32_t r, const float4 (&acc)[kVec]) {
+        const float ps = a.ps ? a.ps[r] : 1.0f;
         const bool seed = is_seed ? is_seed[r] != 0 : true;
 #pragma unroll
-        for (int j = 0; j < kCols; j++) {
-            const int c = lane + 32 * j;
-            if (c < K) {
-                const size_t o = (size_t)r * K + c;
-                const float base = seed ? spmm_base(a, r, c, omd) : 0.f;
-                const float nv = base + a.d * acc[j];
-                const float ov = a.xin[o];
-                a.xout[o] = nv;
-                if (a.gout != a.xout) a.gout[o] = nv * pscale;
-                l1[j] += fabsf(nv - ov);
+        for (int j = 0; j < kVec; j++) {
+            const int c = q0 + 4 * kLanes * j;
+            if (c < a.S) {
+                const size_t o = (size_t)r * a.S + c;
+                const float4 ov = *reinterpret_cast<const float4 *>(a.xin + o);
+                float4 nv = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (seed) nv = make_float4(spmm_base(a, r, c, omd), spmm_base(a, r, c + 1, omd),
+                                           spmm_base(a, r, c + 2, omd), spmm_base(a, r, c + 3, omd));
+                fma4(nv, a.d, acc[j]);
+                *reinterpret_cast<float4 *>(a.xout + o) = nv;
+                if (a.gout != a.xout)
+                    *reinterpret_cast<float4 *>(a.gout + o) = make_float4(nv.x * ps, nv.y * ps, nv.z * ps, nv.w * ps);
+                add4(l1[j], make_float4(fabsf(nv.x - ov.x), fabsf(nv.y - ov.y), fabsf(nv.z - ov.z), fabsf(nv.w - ov.w)));
             }
         }
     };
+    const int total = plan.n_tasks + plan.n_long + (a.n_active + kSpmmRows - 1) / kSpmmRows;
     for (int item = gwarp; item < total; item += nwarps) {
-        float acc[kCols];
-#pragma unroll
-        for (int j = 0; j < kCols; j++) acc[j] = 0.f;
+        float4 acc[kVec];
+        clear(acc);
         if (item < plan.n_tasks) {
             const int2 tk = plan.tasks[item];
             const HubInfo h = plan.hubs[tk.x];
-            const int64_t rb = a.index[h.row], re = a.index[h.row + 1];
-            const int64_t b = rb + (int64_t)tk.y * kHubChunk;
-            const int64_t e = min(re, b + (int64_t)kHubChunk);
-            for (int64_t i = b; i < e; i++) {
-                const int32_t u = a.nbr[i];
-                const float wv = a.ew ? a.ew[i] : 1.0f;
-                const float *gu = a.gin + (size_t)u * K;
+            const int64_t rb = __ldg(a.index + h.row), re = __ldg(a.index + h.row + 1);
+            const int64_t b = rb + (int64_t)tk.y * plan.chunk;
+            spmm_range<kVec, kLanes, kEW>(a, b + sub, min(re, b + (int64_t)plan.chunk), kSub, q0, acc);
+            combine(acc);
+            if (sub == 0) {
 #pragma unroll
-                for (int j = 0; j < kCols; j++) {
-                    const int c = lane + 32 * j;
-                    if (c < K) acc[j] += wv * __ldg(gu + c);
+                for (int j = 0; j < kVec; j++) {
+                    const int c = q0 + 4 * kLanes * j;
+                    if (c < a.S) *reinterpret_cast<float4 *>(a.partials + (size_t)(h.first + tk.y) * a.S + c) = acc[j];
                 }
-            }
-#pragma unroll
-            for (int j = 0; j < kCols; j++) {
-                const int c = lane + 32 * j;
-                if (c < K) a.partials[(size_t)(h.first + tk.y) * K + c] = acc[j];
             }
             __syncwarp();
             int last = 0;
@@ -443,41 +509,55 @@ __global__ void __launch_bounds__(kPrThreads) spmm_sweep(SpmmArgs a, PrPlanDev p
                 last = atomicAdd(a.hub_count + tk.x, 1u) == (unsigned)(h.nchunks - 1);
             }
             last = __shfl_sync(kFull, last, 0);
-            if (last) {
-                __threadfence();
+            if (!last) continue;
+            __threadfence();
+            clear(acc);
+#pragma unroll 4
+            for (int ch = sub; ch < h.nchunks; ch += kSub) {
 #pragma unroll
-                for (int j = 0; j < kCols; j++) acc[j] = 0.f;
-                for (int ch = 0; ch < h.nchunks; ch++) {
-#pragma unroll
-                    for (int j = 0; j < kCols; j++) {
-                        const int c = lane + 32 * j;
-                        if (c < K) acc[j] += __ldcg(a.partials + (size_t)(h.first + ch) * K + c);
-                    }
+                for (int j = 0; j < kVec; j++) {
+                    const int c = q0 + 4 * kLanes * j;
+                    if (c < a.S)
+                        add4(acc[j], __ldcg(reinterpret_cast<const float4 *>(a.partials + (size_t)(h.first + ch) * a.S + c)));
                 }
-                if (lane == 0) a.hub_count[tk.x] = 0;
-                finish(h.row, acc);
             }
+            combine(acc);
+            if (lane == 0) a.hub_count[tk.x] = 0;
+            if (sub == 0) finish(h.row, acc);
+        } else if (item < plan.n_tasks + plan.n_long) {
+            const int32_t r = plan.longs[item - plan.n_tasks];
+            spmm_range<kVec, kLanes, kEW>(a, __ldg(a.index + r) + sub, __ldg(a.index + r + 1), kSub, q0, acc);
+            combine(acc);
+            if (sub == 0) finish(r, acc);
         } else {
-            const int32_t r = item - plan.n_tasks;
-            const int64_t b = a.index[r], e = a.index[r + 1];
-            if (e - b > kHubEdges) continue;  // handled as chunks
-            for (int64_t i = b; i < e; i++) {
-                const int32_t u = a.nbr[i];
-                const float wv = a.ew ? a.ew[i] : 1.0f;
-                const float *gu = a.gin + (size_t)u * K;
-#pragma unroll
-                for (int j = 0; j < kCols; j++) {
-                    const int c = lane + 32 * j;
-                    if (c < K) acc[j] += wv * __ldg(gu + c);
+            const int32_t r0 = (item - plan.n_tasks - plan.n_long) * kSpmmRows;
+            const int nr = min(kSpmmRows, a.n_active - r0);
+            const int64_t start = __ldg(a.index + r0 + min(lane, nr));
+            const int64_t deg = __shfl_down_sync(kFull, start, 1) - start;
+            if (!__any_sync(kFull, lane < nr && deg <= kSpmmLong)) continue;
+#pragma unroll 1
+            for (int k0 = 0; k0 < nr; k0 += kSub) {
+                const int k = k0 + sub;
+                const int64_t b = __shfl_sync(kFull, start, min(k, 31)), e = __shfl_sync(kFull, start, min(k + 1, 31));
+                if (k < nr && e - b <= kSpmmLong) {
+                    clear(acc);
+                    spmm_range<kVec, kLanes, kEW>(a, b, e, 1, q0, acc);
+                    finish(r0 + k, acc);
                 }
             }
-            finish(r, acc);
         }
     }
+    // Column sums: the subs', then the block's warps', then one atomic per column.
+    combine(l1);
+    if (sub == 0) {
 #pragma unroll
-    for (int j = 0; j < kCols; j++) {
-        const int c = lane + 32 * j;
-        if (c < K && l1[j] != 0.f) atomicAdd(a.col_l1 + c, (double)l1[j]);
+        for (int j = 0; j < kVec; j++) *reinterpret_cast<float4 *>(&s_l1[wib][q0 + 4 * kLanes * j]) = l1[j];
+    }
+    __syncthreads();
+    for (int c = threadIdx.x; c < a.K; c += blockDim.x) {
+        double t = 0.0;
+        for (int w = 0; w < kPrThreads / 32; w++) t += (double)s_l1[w][c];
+        if (t != 0.0) atomicAdd(a.col_l1 + c, t);
     }
 }
 
@@ -486,14 +566,15 @@ __global__ void __launch_bounds__(kPrThreads) spmm_sweep(SpmmArgs a, PrPlanDev p
 __global__ void spmm_init(int32_t n, int K, const float *basev, const int32_t *seed_off, const int32_t *seed_idx,
                           const uint8_t *is_seed, float d, const float *ps, float *x, float *g, float *x2, float *g2,
                           int32_t n_active) {
-    const size_t total = (size_t)n * K;
+    const int S = spmm_stride(K);
+    const size_t total = (size_t)n * S;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const int32_t v = (int32_t)(i / K);
-        const int c = (int)(i % K);
+        const int32_t v = (int32_t)(i / S);
+        const int c = (int)(i % S);
         float base = 0.f;
         if (basev) {
             base = basev[i];
-        } else if (is_seed[v]) {
+        } else if (c < K && is_seed[v]) {
             const int32_t b = seed_off[c], e = seed_off[c + 1];
             for (int32_t j = b; j < e; j++)
                 if (seed_idx[j] == v) base = (1.0f - d) / (float)(e - b);
@@ -507,23 +588,30 @@ __global__ void spmm_init(int32_t n, int K, const float *basev, const int32_t *s
     }
 }
 
-// Repacks the live columns of x ([n][kw]) into xo ([n][nkw], gather copy go =
-// xo * ps when go is set); a column with newpos < 0 has converged and goes to
-// its place col_map[c] in out ([n][K0]).  Rows stay contiguous on both sides.
+// Repacks the live columns of x (kw columns) into xo (nkw columns, gather copy
+// go = xo * ps when go is set), both at their padded strides; a column with
+// newpos < 0 has converged and goes to its place col_map[c] in out ([n][K0]).
+// Padding columns stay zero.
 __global__ void spmm_repack(int32_t n, int kw, const float *x, const int32_t *newpos, const int32_t *col_map,
                             int K0, float *out, int nkw, float *xo, float *go, const float *ps) {
     const size_t total = (size_t)n * kw;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         const int32_t v = (int32_t)(i / kw);
         const int c = (int)(i % kw);
-        const float val = x[i];
+        const float val = x[(size_t)v * spmm_stride(kw) + c];
         const int np = newpos[c];
+        const int so = spmm_stride(nkw);
         if (np < 0) {
             out[(size_t)v * K0 + col_map[c]] = val;
         } else {
-            xo[(size_t)v * nkw + np] = val;
-            if (go) go[(size_t)v * nkw + np] = ps ? val * ps[v] : val;
+            xo[(size_t)v * so + np] = val;
+            if (go) go[(size_t)v * so + np] = ps ? val * ps[v] : val;
         }
+        if (c == 0)
+            for (int z = nkw; z < so; z++) {
+                xo[(size_t)v * so + z] = 0.f;
+                if (go) go[(size_t)v * so + z] = 0.f;
+            }
     }
 }
 
@@ -531,7 +619,7 @@ __global__ void spmm_repack(int32_t n, int kw, const float *x, const int32_t *ne
 __global__ void spmm_take_column(int32_t n, int kw, int c, const float *x, const float *ps, float *x0, float *x1,
                                  float *g0, float *g1) {
     for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-        const float val = x[(size_t)v * kw + c];
+        const float val = x[(size_t)v * spmm_stride(kw) + c];
         x0[v] = val;
         x1[v] = val;
         if (g0) {
@@ -634,7 +722,73 @@ hc_status ensure_plan(hc_graph *g) {
     return HC_OK;
 }
 
+// The multi-column sweeps' row plan, built on the first such call.  A chunk is M
+// / 65536 edges rounded down to a power of two, in [512, 2048]: a chunk is a
+// serial chain of its warp, and its partial sums take a row of columns each.
+hc_status ensure_spmm_plan(hc_graph *g) {
+    if (g->spmm_plan.ptr) return HC_OK;
+    const int32_t na = g->n_active;
+    std::vector<int64_t> idx((size_t)na + 1);
+    HC_CUDA_TRY(cudaMemcpy(idx.data(), g->index.as<int64_t>(), sizeof(int64_t) * ((size_t)na + 1),
+                           cudaMemcpyDeviceToHost));
+    int64_t chunk = 512;
+    while (chunk < 2048 && chunk * 2 * 65536 <= g->M) chunk *= 2;
+    std::vector<int32_t> longs;
+    std::vector<int2> tasks;
+    std::vector<HubInfo> hubs;
+    int32_t slots = 0;
+    for (int32_t r = 0; r < na; r++) {
+        const int64_t d = idx[r + 1] - idx[r];
+        if (d > chunk) {
+            HubInfo h{r, slots, (int32_t)((d + chunk - 1) / chunk), 0};
+            for (int c = 0; c < h.nchunks; c++) tasks.push_back(make_int2((int)hubs.size(), c));
+            slots += h.nchunks;
+            hubs.push_back(h);
+        } else if (d > kSpmmLong) {
+            longs.push_back(r);
+        }
+    }
+    auto up = [](size_t b) { return (b + 255) / 256 * 256; };
+    const size_t b_long = up(longs.size() * 4), b_tasks = up(tasks.size() * sizeof(int2));
+    HC_TRY(g->spmm_plan.ensure(b_long + b_tasks + up(hubs.size() * sizeof(HubInfo)) + 256));
+    char *p = g->spmm_plan.as<char>();
+    SpmmPlanDev v{};
+    v.longs = (const int32_t *)p;
+    v.tasks = (const int2 *)(p + b_long);
+    v.hubs = (const HubInfo *)(p + b_long + b_tasks);
+    if (!longs.empty()) HC_CUDA_TRY(cudaMemcpy(p, longs.data(), longs.size() * 4, cudaMemcpyHostToDevice));
+    if (!tasks.empty()) {
+        HC_CUDA_TRY(cudaMemcpy(p + b_long, tasks.data(), tasks.size() * sizeof(int2), cudaMemcpyHostToDevice));
+        HC_CUDA_TRY(cudaMemcpy(p + b_long + b_tasks, hubs.data(), hubs.size() * sizeof(HubInfo), cudaMemcpyHostToDevice));
+    }
+    v.n_long = (int)longs.size();
+    v.n_tasks = (int)tasks.size();
+    v.n_hub = (int)hubs.size();
+    v.chunk = (int)chunk;
+    g->spmm_view = v;
+    g->spmm_partial_slots = slots;
+    return HC_OK;
+}
+
 namespace {
+
+template <bool kEW>
+void launch_spmm_cols(hc_graph *g, const SpmmArgs &a, const uint8_t *is_seed) {
+    const int grid = g->sm_count * 8;
+    const SpmmPlanDev &plan = g->spmm_view;
+    if (a.S <= 8) spmm_sweep<1, 2, kEW><<<grid, kPrThreads, 0, g->stream>>>(a, plan, is_seed);
+    else if (a.S <= 16) spmm_sweep<1, 4, kEW><<<grid, kPrThreads, 0, g->stream>>>(a, plan, is_seed);
+    else if (a.S <= 32) spmm_sweep<1, 8, kEW><<<grid, kPrThreads, 0, g->stream>>>(a, plan, is_seed);
+    else if (a.S <= 64) spmm_sweep<1, 16, kEW><<<grid, kPrThreads, 0, g->stream>>>(a, plan, is_seed);
+    else if (a.S <= 128) spmm_sweep<1, 32, kEW><<<grid, kPrThreads, 0, g->stream>>>(a, plan, is_seed);
+    else spmm_sweep<2, 32, kEW><<<grid, kPrThreads, 0, g->stream>>>(a, plan, is_seed);
+    ::hc::count_launch();
+}
+
+void launch_spmm(hc_graph *g, const SpmmArgs &a, const uint8_t *is_seed) {
+    if (a.ew) launch_spmm_cols<true>(g, a, is_seed);
+    else launch_spmm_cols<false>(g, a, is_seed);
+}
 
 PrPlanDev plan_view(hc_graph *g, int *partial_slots) {
     *partial_slots = g->pr_partial_slots;
@@ -966,9 +1120,13 @@ extern "C" hc_status hc_pr_forward(hc_graph *g, const float *teleport, int32_t n
     if (ncols > 1) {
         // Dense multi-column form.
         const int K = ncols;
-        const size_t nk = (size_t)n * K;
-        const size_t bytes = 5 * nk * sizeof(float) + (size_t)(partial_slots + 1) * K * sizeof(float) +
-                             (size_t)(plan.n_hub + 1) * 4 + (size_t)K * 8 + 4096;
+        if (K > 256) return fail(HC_ERR_UNSUPPORTED, "hc_pr_forward: at most 256 columns per call");
+        HC_TRY(ensure_spmm_plan(g));
+        const int S = spmm_stride(K);
+        const size_t nk = (size_t)n * S;
+        const size_t slots = (size_t)g->spmm_partial_slots + 1;
+        const size_t bytes = 5 * nk * sizeof(float) + slots * S * sizeof(float) +
+                             (size_t)(g->spmm_view.n_hub + 1) * 4 + (size_t)S * 8 + 4096;
         HC_TRY(g->ws_pr.ensure(bytes));
         char *p = g->ws_pr.as<char>();
         auto take = [&](size_t b) {
@@ -979,12 +1137,18 @@ extern "C" hc_status hc_pr_forward(hc_graph *g, const float *teleport, int32_t n
         float *basev = (float *)take(nk * 4);
         float *x[2] = {(float *)take(nk * 4), (float *)take(nk * 4)};
         float *gv[2] = {(float *)take(nk * 4), (float *)take(nk * 4)};
-        float *partials = (float *)take((size_t)(partial_slots + 1) * K * 4);
-        unsigned *hub_count = (unsigned *)take((size_t)(plan.n_hub + 1) * 4);
-        double *col_l1 = (double *)take((size_t)K * 8);
-        HC_TRY(copy_in(basev, teleport, nk * 4, g->stream));
+        float *partials = (float *)take(slots * S * 4);
+        unsigned *hub_count = (unsigned *)take((size_t)(g->spmm_view.n_hub + 1) * 4);
+        double *col_l1 = (double *)take((size_t)S * 8);
+        if (S == K) {
+            HC_TRY(copy_in(basev, teleport, nk * 4, g->stream));
+        } else {
+            HC_CUDA_TRY(cudaMemsetAsync(basev, 0, nk * 4, g->stream));
+            HC_CUDA_TRY(cudaMemcpy2DAsync(basev, (size_t)S * 4, teleport, (size_t)K * 4, (size_t)K * 4, n,
+                                          cudaMemcpyDefault, g->stream));
+        }
         { scale_vec<<<g->sm_count * 8, 256, 0, g->stream>>>(basev, 1.0f - o.damping, basev, nk); ::hc::count_launch(); }
-        HC_CUDA_TRY(cudaMemsetAsync(hub_count, 0, (size_t)(plan.n_hub + 1) * 4, g->stream));
+        HC_CUDA_TRY(cudaMemsetAsync(hub_count, 0, (size_t)(g->spmm_view.n_hub + 1) * 4, g->stream));
         const float *ps = weighted ? nullptr : g->inv_deg.as<float>();
         { spmm_init<<<g->sm_count * 8, 256, 0, g->stream>>>(g->N, K, basev, nullptr, nullptr, nullptr, o.damping, ps,
                                                           x[0], gv[0], x[1], gv[1], g->n_active); ::hc::count_launch(); }
@@ -1000,6 +1164,7 @@ extern "C" hc_status hc_pr_forward(hc_graph *g, const float *teleport, int32_t n
         a.hub_count = hub_count;
         a.col_l1 = col_l1;
         a.K = K;
+        a.S = S;
         a.n_active = g->n_active;
         HC_CUDA_TRY(cudaEventRecord(g->ev_start, g->stream));
         int it = 0;
@@ -1011,13 +1176,7 @@ extern "C" hc_status hc_pr_forward(hc_graph *g, const float *teleport, int32_t n
             a.xout = x[(it + 1) & 1];
             a.gout = weighted ? a.xout : gv[(it + 1) & 1];
             HC_CUDA_TRY(cudaMemsetAsync(col_l1, 0, (size_t)K * 8, g->stream));
-            const int cols = (K + 31) / 32;
-            const int grid = g->sm_count * 8;
-            if (cols <= 1) { spmm_sweep<1><<<grid, kPrThreads, 0, g->stream>>>(a, plan, nullptr); ::hc::count_launch(); }
-            else if (cols <= 2) { spmm_sweep<2><<<grid, kPrThreads, 0, g->stream>>>(a, plan, nullptr); ::hc::count_launch(); }
-            else if (cols <= 4) { spmm_sweep<4><<<grid, kPrThreads, 0, g->stream>>>(a, plan, nullptr); ::hc::count_launch(); }
-            else if (cols <= 8) { spmm_sweep<8><<<grid, kPrThreads, 0, g->stream>>>(a, plan, nullptr); ::hc::count_launch(); }
-            else return fail(HC_ERR_UNSUPPORTED, "hc_pr_forward: at most 256 columns per call");
+            launch_spmm(g, a, nullptr);
             HC_CUDA_TRY(cudaGetLastError());
             HC_CUDA_TRY(cudaMemcpyAsync(hl1.data(), col_l1, (size_t)K * 8, cudaMemcpyDeviceToHost, g->stream));
             HC_CUDA_TRY(cudaStreamSynchronize(g->stream));
@@ -1026,7 +1185,8 @@ extern "C" hc_status hc_pr_forward(hc_graph *g, const float *teleport, int32_t n
             conv = o.tol_l1 > 0.f && mx < (double)o.tol_l1;
         }
         HC_CUDA_TRY(cudaEventRecord(g->ev_stop, g->stream));
-        HC_TRY(copy_out(scores_out, x[it & 1], nk * 4, g->stream));
+        HC_CUDA_TRY(cudaMemcpy2DAsync(scores_out, (size_t)K * 4, x[it & 1], (size_t)S * 4, (size_t)K * 4, n,
+                                      cudaMemcpyDefault, g->stream));
         HC_CUDA_TRY(cudaStreamSynchronize(g->stream));
         float ms = 0;
         HC_CUDA_TRY(cudaEventElapsedTime(&ms, g->ev_start, g->ev_stop));
@@ -1263,9 +1423,13 @@ extern "C" hc_status hc_ppr_batched(hc_graph *g, const int32_t *seed_offsets, co
         if (s < 0 || s >= g->N) return fail(HC_ERR_INVALID_ARG, "hc_ppr_batched: seed %d out of range", s);
     const int K = ncols;
     const int64_t n = g->N;
-    const size_t nk = (size_t)n * K;
-    const size_t bytes = 4 * nk * sizeof(float) + (size_t)(partial_slots + 1) * K * 4 + (size_t)(plan.n_hub + 1) * 4 +
-                         (size_t)K * 8 + (size_t)n + (size_t)(nseeds + ncols + 1) * 4 + 5 * (size_t)n * 4 + 16384;
+    HC_TRY(ensure_spmm_plan(g));
+    const int S = spmm_stride(K);
+    const size_t nk = (size_t)n * K, ns = (size_t)n * S;
+    // One column's partial sums and counters (the tail's sweeps) fit these too.
+    const size_t slots = std::max((size_t)g->spmm_partial_slots * S, (size_t)partial_slots) + S;
+    const size_t counters = (size_t)std::max(g->spmm_view.n_hub, plan.n_hub) + 1;
+    const size_t bytes = 4 * ns * sizeof(float) + slots * 4 + counters * 4 + (size_t)S * 8 + (size_t)n + (size_t)(nseeds + ncols + 1) * 4 + 5 * (size_t)n * 4 + 16384;
     HC_TRY(g->ws_pr.ensure(bytes));
     char *p = g->ws_pr.as<char>();
     auto take = [&](size_t b) {
@@ -1273,11 +1437,11 @@ extern "C" hc_status hc_ppr_batched(hc_graph *g, const int32_t *seed_offsets, co
         p += (b + 255) / 256 * 256;
         return r;
     };
-    float *x[2] = {(float *)take(nk * 4), (float *)take(nk * 4)};
-    float *gv[2] = {(float *)take(nk * 4), (float *)take(nk * 4)};
-    float *partials = (float *)take((size_t)(partial_slots + 1) * K * 4);
-    unsigned *hub_count = (unsigned *)take((size_t)(plan.n_hub + 1) * 4);
-    double *col_l1 = (double *)take((size_t)K * 8);
+    float *x[2] = {(float *)take(ns * 4), (float *)take(ns * 4)};
+    float *gv[2] = {(float *)take(ns * 4), (float *)take(ns * 4)};
+    float *partials = (float *)take(slots * 4);
+    unsigned *hub_count = (unsigned *)take(counters * 4);
+    double *col_l1 = (double *)take((size_t)S * 8);
     uint8_t *is_seed = (uint8_t *)take((size_t)n);
     int32_t *d_off = (int32_t *)take((size_t)(ncols + 1) * 4);
     int32_t *d_seeds = (int32_t *)take((size_t)nseeds * 4);
@@ -1287,7 +1451,7 @@ extern "C" hc_status hc_ppr_batched(hc_graph *g, const int32_t *seed_offsets, co
     HC_CUDA_TRY(cudaMemcpyAsync(d_off, off.data(), (ncols + 1) * 4, cudaMemcpyHostToDevice, g->stream));
     HC_CUDA_TRY(cudaMemcpyAsync(d_seeds, sd.data(), (size_t)nseeds * 4, cudaMemcpyHostToDevice, g->stream));
     HC_CUDA_TRY(cudaMemsetAsync(is_seed, 0, (size_t)n, g->stream));
-    HC_CUDA_TRY(cudaMemsetAsync(hub_count, 0, (size_t)(plan.n_hub + 1) * 4, g->stream));
+    HC_CUDA_TRY(cudaMemsetAsync(hub_count, 0, counters * 4, g->stream));
     { mark_seeds<<<64, 256, 0, g->stream>>>(d_seeds, nseeds, is_seed); ::hc::count_launch(); }
     const float *ps = weighted ? nullptr : g->inv_deg.as<float>();
     { spmm_init<<<g->sm_count * 8, 256, 0, g->stream>>>(g->N, K, nullptr, d_off, d_seeds, is_seed, o.damping, ps,
@@ -1336,8 +1500,10 @@ extern "C" hc_status hc_ppr_batched(hc_graph *g, const int32_t *seed_offsets, co
         // Rows without edges (past n_active) are never written by a sweep:
         // give the buffer the next sweep writes their values in the new layout.
         if (nkw > 0 && g->n_active < g->N)
-            HC_CUDA_TRY(cudaMemcpyAsync(x[cur] + (size_t)g->n_active * nkw, x[cur ^ 1] + (size_t)g->n_active * nkw,
-                                        (size_t)(g->N - g->n_active) * nkw * 4, cudaMemcpyDeviceToDevice, g->stream));
+            HC_CUDA_TRY(cudaMemcpyAsync(x[cur] + (size_t)g->n_active * spmm_stride(nkw),
+                                        x[cur ^ 1] + (size_t)g->n_active * spmm_stride(nkw),
+                                        (size_t)(g->N - g->n_active) * spmm_stride(nkw) * 4, cudaMemcpyDeviceToDevice,
+                                        g->stream));
         return HC_OK;
     };
     // The single-column solver's run_solve records g's events: this call
@@ -1363,17 +1529,13 @@ extern "C" hc_status hc_ppr_batched(hc_graph *g, const int32_t *seed_offsets, co
     constexpr int kSingleCols = 4;
     for (; it < o.max_iters && kw > (K > kSingleCols ? kSingleCols : 0); it++) {
         a.K = kw;
+        a.S = spmm_stride(kw);
         a.gin = weighted ? x[cur] : gv[cur];
         a.xin = x[cur];
         a.xout = x[cur ^ 1];
         a.gout = weighted ? a.xout : gv[cur ^ 1];
         HC_CUDA_TRY(cudaMemsetAsync(col_l1, 0, (size_t)kw * 8, g->stream));
-        const int cols = (kw + 31) / 32;
-        const int grid = g->sm_count * 8;
-        if (cols <= 1) { spmm_sweep<1><<<grid, kPrThreads, 0, g->stream>>>(a, plan, is_seed); ::hc::count_launch(); }
-        else if (cols <= 2) { spmm_sweep<2><<<grid, kPrThreads, 0, g->stream>>>(a, plan, is_seed); ::hc::count_launch(); }
-        else if (cols <= 4) { spmm_sweep<4><<<grid, kPrThreads, 0, g->stream>>>(a, plan, is_seed); ::hc::count_launch(); }
-        else { spmm_sweep<8><<<grid, kPrThreads, 0, g->stream>>>(a, plan, is_seed); ::hc::count_launch(); }
+        launch_spmm(g, a, is_seed);
         HC_CUDA_TRY(cudaGetLastError());
         bytes_model += 8.0 * (n + 1) + 4.0 * g->M * (weighted ? 2 : 1) + 12.0 * (double)n * kw;
         cur ^= 1;

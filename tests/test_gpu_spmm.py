@@ -1,0 +1,71 @@
+"""Multi-column PageRank at the widths and row lengths where its sweep changes form."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+DAMPING, TOL = 0.85, 1e-6
+# The stop leaves at most TOL * d / (1 - d) in any entry; fp32 sums of at most 2000 terms of total <= 1 add 2000 * 2^-24.
+BOUND = TOL * DAMPING / (1 - DAMPING) + 2000 * 2.0 ** -24
+
+
+def stars(degrees):
+    """Star centres of these degrees on a common ring of leaves, leaves linked in a path: every row length side by side."""
+    leaves = max(degrees)
+    u, v = [], []
+    for i, d in enumerate(degrees):
+        u.append(np.full(d, leaves + i))
+        v.append((np.arange(d) + 7 * i) % leaves)
+    u.append(np.arange(leaves - 1))
+    v.append(np.arange(1, leaves))
+    u, v = np.concatenate(u), np.concatenate(v)
+    n = leaves + len(degrees)
+    src, dst = np.concatenate([u, v]), np.concatenate([v, u])
+    order = np.lexsort((dst, src))
+    index = np.zeros(n + 1, np.int64)
+    np.cumsum(np.bincount(src, minlength=n), out=index[1:])
+    return index, dst[order].astype(np.int32)
+
+
+def fixed_point(index, nbr, w, t):
+    """x = (1-d) t + d A x in 64 bits, A[v,u] = w(u->v) / sum of u's weights (symmetric weights)."""
+    n = len(index) - 1
+    row = np.repeat(np.arange(n), np.diff(index))
+    s = np.bincount(row, weights=w, minlength=n)
+    vals = (w / s[nbr])[:, None]
+    x = t.copy()
+    for _ in range(400):
+        y = np.zeros_like(x)
+        np.add.at(y, row, vals * x[nbr])
+        x = (1 - DAMPING) * t + DAMPING * y
+    return x
+
+
+@pytest.mark.parametrize("weighted", [False, True])
+@pytest.mark.parametrize("k", [2, 4, 5, 8, 9, 16, 17, 31, 33, 64, 65, 129, 256])
+def test_columns(k, weighted):
+    import hc
+    index, nbr = stars([1, 63, 64, 65, 127, 511, 512, 513, 1025, 1537])
+    n = len(index) - 1
+    row = np.repeat(np.arange(n), np.diff(index))
+    w = (1 + (row + nbr) % 7).astype(np.float32) if weighted else None
+    g = hc.Graph(index, nbr, w)
+    rng = np.random.default_rng(k)
+    # Dense teleports of two distinct columns, repeated: a column's place must not matter.
+    two = rng.random((n, 2)).astype(np.float32)
+    two /= two.sum(0)
+    t = np.ascontiguousarray(two[:, np.arange(k) % 2])
+    x, st = g.pagerank(t, tol_l1=TOL, max_iters=300, weighted=weighted)
+    want = fixed_point(index, nbr, np.ones(len(nbr)) if w is None else w.astype(np.float64), two.astype(np.float64))
+    assert st.converged and np.abs(x - want[:, np.arange(k) % 2]).max() <= BOUND
+    # Seeds: two per column.
+    seeds = np.stack([np.arange(k) % n, (np.arange(k) * 37 + 5) % n], 1).astype(np.int32)
+    seeds[seeds[:, 0] == seeds[:, 1], 1] += 1
+    x, st = g.ppr_batched(np.arange(k + 1) * 2, seeds.ravel(), tol_l1=TOL, max_iters=300, weighted=weighted)
+    cols = sorted({0, 1, k // 2, k - 1})
+    t = np.zeros((n, len(cols)))
+    for i, c in enumerate(cols):
+        t[seeds[c], i] = 0.5
+    want = fixed_point(index, nbr, np.ones(len(nbr)) if w is None else w.astype(np.float64), t)
+    assert st.converged and np.abs(x[:, cols] - want).max() <= BOUND
+    g.close()
