@@ -73,6 +73,12 @@ __device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long
     return v;
 }
 
+__device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long long *p) {
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+
 // Grid-wide barrier for cooperative (co-resident) launches.  `count` only
 // grows: every block adds one per barrier, so barrier k of a run is complete
 // when count reaches (k + 1) * nblocks, and a block computes that target
@@ -80,11 +86,11 @@ __device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long
 // waiters see the last arrival itself.  The control block must be zeroed
 // before a run, and every launch of a run must use the same grid size.
 // The arrival is a release (everything the block wrote, ordered before it by
-// __syncthreads, is visible to whoever acquires it) and the poll an acquire,
-// which also drops the SM's stale L1 lines: no separate fences.  Waiters poll
-// back to back at first, since a level of a sparse frontier ends within a few
-// round trips, then sleep between polls so that a long wait leaves the L2
-// slice alone.  They give up after the wait limit, setting *err.  Once *err is
+// __syncthreads, is visible to whoever acquires it); the polls are relaxed and
+// one acquire follows the last: an acquire drops the SM's L1 lines, which the
+// SM's other blocks may still be gathering from.  Waiters poll back to back at
+// first, since a level of a sparse frontier ends within a few round trips, then
+// sleep between polls so that a long wait leaves the L2 slice alone.  They give up after the wait limit, setting *err.  Once *err is
 // set every later barrier returns at once, so a failed run drains in bounded
 // time.  Returns false when the run must stop.
 struct GridSync {
@@ -106,7 +112,7 @@ __device__ __forceinline__ bool grid_barrier(GridSync *gs, unsigned nblocks) {
             const unsigned long long target = (t / nblocks + 1) * nblocks;
             if (t + 1 != target) {
                 unsigned long long t0 = 0;
-                for (int polls = 0; ld_acquire_u64(&gs->count) < target; polls++) {
+                for (int polls = 0; ld_relaxed_u64(&gs->count) < target; polls++) {
                     if (polls < 64) continue;
                     if (polls == 64) t0 = globaltimer_ns();
                     if (*(volatile int *)&gs->err) { ok = 0; break; }
@@ -117,6 +123,7 @@ __device__ __forceinline__ bool grid_barrier(GridSync *gs, unsigned nblocks) {
                     }
                     __nanosleep(100);
                 }
+                (void)ld_acquire_u64(&gs->count);
             }
         }
         s_ok = ok;

@@ -4,14 +4,20 @@
 #include "hc_device.cuh"
 
 namespace hc {
-// Row plan shared by the PageRank sweeps and the SSSP pull sweep, built once
-// per graph from the offsets of the rows with edges:
-//   stream groups  32 consecutive rows with <= kStreamEdges edges in total
-//   long rows      <= kHubEdges edges, one warp per row
-//   hub rows       > kHubEdges edges, cut into kHubChunk-edge tasks
-constexpr int kStreamEdges = 2048;
-constexpr int kHubEdges = 4096;
-constexpr int kHubChunk = 2048;
+// Row plan of the PageRank sweeps, and another of the SSSP pull sweep, built
+// once per graph from the offsets of the rows with edges:
+//   stream groups  32 consecutive rows, one warp
+//   long rows      one warp per row
+//   hub rows       more than two chunks of edges, cut into tasks of one chunk
+// A long row, a task or a PageRank stream group is a serial chain of its warp's
+// 128-edge steps (about a microsecond each), so on a small graph, whose sweep is
+// no more than a few of those, they are short; on a large one they are long, as
+// a task ends with a fence and a counter and a warp per short row wastes lanes.
+//   chunk          M / 4096 edges rounded down to a power of two, in [256, 2048]
+//   stream group   at most M / 8192 edges, rounded likewise, in [256, 2048]
+//                  (the SSSP pull, a lane per row, always 2048)
+constexpr int kMinChunk = 256;
+constexpr int kMaxChunk = 2048;
 // Batched SSSP keeps 16-bit distances when no weight exceeds this.
 constexpr int32_t kMsspNarrowMaxW = 0x0FFF;
 
@@ -28,6 +34,7 @@ struct PrPlanDev {
     const int2 *tasks;      // (hub index, chunk)
     const HubInfo *hubs;
     int n_stream, n_long, n_tasks, n_hub;
+    int chunk;              // edges per hub task
 };
 
 // Row plan of the multi-column PageRank sweeps:
@@ -78,6 +85,8 @@ struct hc_graph {
     hc::DevBuf pr_plan;        // row plan (device arrays)
     hc::PrPlanDev pr_view{};   // host copy of its pointers and counts
     int32_t pr_partial_slots = 0;
+    hc::DevBuf sssp_plan;      // the SSSP pull's row plan
+    hc::PrPlanDev sssp_view{};
     hc::DevBuf pr_plan_huge_rows;
     hc::DevBuf spmm_plan;          // multi-column row plan (device arrays)
     hc::SpmmPlanDev spmm_view{};
@@ -182,8 +191,10 @@ hc_status edge_symmetry(hc_graph *g, const uint32_t *wbits, bool *structure, boo
 // The edge weights as fp32 for weighted PageRank: the weight array itself
 // (fp32 graphs) or its converted copy (int32 graphs, built by ensure_pr_derived).
 const float *pr_weights(const hc_graph *g);
-// Builds the row plan if missing (g->pr_view, g->pr_partial_slots).
+// Builds the PageRank row plan (g->pr_view, g->pr_partial_slots) or the SSSP
+// pull's (g->sssp_view) if missing.
 hc_status ensure_plan(hc_graph *g);
+hc_status ensure_sssp_plan(hc_graph *g);
 // Computes w_negative, w_max, w_mean and w_symmetric once (int32 weights).
 hc_status ensure_weight_stats(hc_graph *g);
 // Per-run control traffic kept off the copy engines.  A host-output call

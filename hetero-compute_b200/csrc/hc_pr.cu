@@ -7,17 +7,18 @@
 // vector that already carries the 1/deg factor (4-byte neighbour stream +
 // 4-byte gather), with the L1 / per-vertex residual reduced in the same pass.
 //
-// Work plan (built once per graph from the row offsets):
-//   stream groups  32 consecutive rows with <= kStreamEdges edges in total;
-//                  one warp streams the whole edge range coalesced and reduces
-//                  it segment by segment (CSR-stream, Greathouse & Daga 2014)
+// Work plan (built once per graph from the row offsets, see hc_graph.cuh):
+//   stream groups  32 consecutive rows of few edges in total; one warp streams
+//                  the whole edge range coalesced and reduces it segment by
+//                  segment (CSR-stream, Greathouse & Daga 2014)
 //   long rows      one warp per row, 128-bit neighbour loads
-//   hub rows       > kHubEdges edges, cut into kHubChunk-edge chunks; each
-//                  chunk's warp writes a partial, the last one to finish sums
-//                  the partials in chunk order (deterministic) and finalises
+//   hub rows       cut into chunks; each chunk's warp writes a partial, the last
+//                  one to finish sums the partials in chunk order
+//                  (deterministic) and finalises
 // Vertices without edges keep (1-d) t_v, written once before the iterations.
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <vector>
 
 #include "hc_graph.cuh"
@@ -26,15 +27,26 @@ namespace hc {
 namespace {
 
 constexpr int kPrThreads = 256;
+constexpr int kPrBlocks = 6;  // per SM: the gathers want warps more than registers
 constexpr int kMaxIterSlots = 4096;
 
+// Grid barrier and per-iteration sums of one solve: a slot per iteration, all
+// zero at the start, so that no block resets a sum another still reads (past
+// kMaxIterSlots iterations they come round, cleared two iterations ahead).
+struct IterSlot {
+    double l1;       // Jacobi: sum |change|; conjugate gradients: p . q
+    double rz, z1;   // conjugate gradients: r . z, sum |z|
+    int changed, pad;
+};
 struct IterState {
-    double l1[kMaxIterSlots];
-    int changed[kMaxIterSlots];
-    unsigned blocks_done;
-    int done;
-    int iters;
-    int pad;
+    GridSync gs;
+    int done, blocks_done;   // sweeps launched one by one
+    IterSlot slot[kMaxIterSlots];
+};
+// What a solve reports, in mapped host memory.
+struct SolveOut {
+    int err, iters, done, changed;
+    double l1;
 };
 
 // One pull sweep: out[v] = base_v + d * rs_v * sum_{e in row v} ew_e * gin[nbr_e].
@@ -42,74 +54,80 @@ struct SweepArgs {
     const int64_t *index;
     const int32_t *nbr;
     const float *ew;        // per-slot edge weight (kEW)
-    const float *gin;       // gathered vector
-    const float *xin;       // previous iterate (residual)
     const float *basev;     // per-vertex base (kBaseVec), already scaled by (1-d)
     float base_scalar;
     float d;
     const float *rs;        // per-row scale (kRS)
     const float *ps;        // gather-out scale (kPS)
-    float *xout;
-    float *gout;            // gather vector for the next sweep (kPS) -- else == xout
+    float *x[2], *g[2];     // iterates and their gather vectors (g == x without kPS)
     float *partials;
     unsigned *hub_count;
     IterState *st;
-    int it;
-    float omega;            // Chebyshev weight of this iteration (1: plain Jacobi)
+    SolveOut *out;
+    float *final_x;         // the result is copied here too (null: not)
+    float cheb_rho;         // > 0: Chebyshev weights (0: plain Jacobi)
     float tol_l1, eps;
     int max_iters;
-    int32_t n_active;
+    int32_t n, n_active;
+};
+// The vectors of one sweep.  They are written by other blocks of the same
+// launch, so they are read through L1 by coherent loads; the grid barrier's
+// acquire drops what L1 holds of the last sweep's.
+struct SweepIter {
+    const float *gin;       // gathered vector
+    const float *xin;       // previous iterate (residual)
+    float *xout;
+    float *gout;            // gather vector for the next sweep (kPS) -- else == xout
+    float omega;            // Chebyshev weight of this iteration (1: plain Jacobi)
 };
 
 template <bool kEW, bool kRS, bool kPS, bool kBaseVec, bool kCG = false>
-__device__ __forceinline__ void finish_row(const SweepArgs &a, int32_t r, float sum, float &l1, int &chg) {
+__device__ __forceinline__ void finish_row(const SweepArgs &a, const SweepIter &v, int32_t r, float sum, float &l1, int &chg) {
     if constexpr (kCG) {
         // Conjugate-gradient product (gin = p): xout = (S p)_r, and
         // p_r q_r with q = s p - d S p summed where the residual goes.
-        const float pr = a.gin[r];
+        const float pr = v.gin[r];
         const float rsr = a.rs[r];
         const float sr = rsr > 0.f ? 1.0f / rsr : 0.f;
-        a.xout[r] = sum;
+        v.xout[r] = sum;
         l1 += pr * (sr * pr - a.d * sum);
         return;
     }
     const float base = kBaseVec ? a.basev[r] : a.base_scalar;
     const float scale = kRS ? a.rs[r] : 1.0f;
     float nv = base + a.d * (scale * sum);
-    const float ov = a.xin[r];
+    const float ov = v.xin[r];
     // The residual |J(x_k) - x_k| of the fixed-point equation: the change of
     // a plain Jacobi sweep, and the stopping rule of both iterations.
     const float dl = fabsf(nv - ov);
     // Chebyshev semi-iteration: x_{k+1} = omega (J(x_k) - x_{k-1}) + x_{k-1};
     // x_{k-1} is what the output buffer still holds.
-    if (a.omega != 1.0f) {
-        const float prev = a.xout[r];
-        nv = a.omega * (nv - prev) + prev;
+    if (v.omega != 1.0f) {
+        const float prev = v.xout[r];
+        nv = v.omega * (nv - prev) + prev;
     }
-    a.xout[r] = nv;
-    if (kPS) a.gout[r] = nv * a.ps[r];
+    v.xout[r] = nv;
+    if (kPS) v.gout[r] = nv * a.ps[r];
     l1 += dl;
     chg += dl > a.eps;
 }
 
 template <bool kEW>
-__device__ __forceinline__ float edge_val(const SweepArgs &a, int64_t e) {
-    const float g = __ldg(a.gin + a.nbr[e]);
-    return kEW ? g * a.ew[e] : g;
+__device__ __forceinline__ float edge_val(const SweepArgs &a, const SweepIter &v, int64_t e) {
+    const float g = __ldca(v.gin + __ldg(a.nbr + e));
+    return kEW ? g * __ldg(a.ew + e) : g;
 }
 
+// One sweep over every row with edges, by the whole grid; l1 and chg receive
+// this thread's share of the residual.
 template <bool kEW, bool kRS, bool kPS, bool kBaseVec, bool kCG = false>
-__global__ void __launch_bounds__(kPrThreads) pr_sweep(SweepArgs a, PrPlanDev plan) {
-    __shared__ float s_acc[kPrThreads / 32][32];
-    __shared__ double s_l1[32];
-    __shared__ int s_chg[32];
-    __shared__ int s_last;
-    if (*(volatile int *)&a.st->done) return;
+__device__ __forceinline__ void sweep_rows(const SweepArgs &a, const PrPlanDev &plan, const SweepIter &it,
+                                           float (*s_acc)[32], float &l1, int &chg) {
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
-    float l1 = 0.f;
-    int chg = 0;
+    l1 = 0.f;
+    chg = 0;
     const int total_items = plan.n_tasks + plan.n_long + plan.n_stream;
 
     for (int item = gwarp; item < total_items; item += nwarps) {
@@ -118,18 +136,18 @@ __global__ void __launch_bounds__(kPrThreads) pr_sweep(SweepArgs a, PrPlanDev pl
             const int2 tk = plan.tasks[item];
             const HubInfo h = plan.hubs[tk.x];
             const int64_t rb = a.index[h.row], re = a.index[h.row + 1];
-            const int64_t b = rb + (int64_t)tk.y * kHubChunk;
-            const int64_t e = min(re, b + (int64_t)kHubChunk);
+            const int64_t b = rb + (int64_t)tk.y * plan.chunk;
+            const int64_t e = min(re, b + (int64_t)plan.chunk);
             // Four independent partial sums keep four gathers in flight.
             float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
             int64_t i = b + lane;
             for (; i + 96 < e; i += 128) {
-                s0 += edge_val<kEW>(a, i);
-                s1 += edge_val<kEW>(a, i + 32);
-                s2 += edge_val<kEW>(a, i + 64);
-                s3 += edge_val<kEW>(a, i + 96);
+                s0 += edge_val<kEW>(a, it, i);
+                s1 += edge_val<kEW>(a, it, i + 32);
+                s2 += edge_val<kEW>(a, it, i + 64);
+                s3 += edge_val<kEW>(a, it, i + 96);
             }
-            for (; i < e; i += 32) s0 += edge_val<kEW>(a, i);
+            for (; i < e; i += 32) s0 += edge_val<kEW>(a, it, i);
             float s = warp_sum((s0 + s1) + (s2 + s3));
             int last = 0;
             if (lane == 0) {
@@ -145,7 +163,7 @@ __global__ void __launch_bounds__(kPrThreads) pr_sweep(SweepArgs a, PrPlanDev pl
                 t = warp_sum(t);
                 if (lane == 0) {
                     a.hub_count[tk.x] = 0;
-                    finish_row<kEW, kRS, kPS, kBaseVec, kCG>(a, h.row, t, l1, chg);
+                    finish_row<kEW, kRS, kPS, kBaseVec, kCG>(a, it, h.row, t, l1, chg);
                 }
             }
         } else if (item < plan.n_tasks + plan.n_long) {
@@ -154,21 +172,21 @@ __global__ void __launch_bounds__(kPrThreads) pr_sweep(SweepArgs a, PrPlanDev pl
             float s = 0.f;
             // Scalar head up to a 16-byte boundary, then 128-bit neighbour loads.
             const int64_t ab = min(e, (b + 3) & ~(int64_t)3);
-            if (b + lane < ab) s += edge_val<kEW>(a, b + lane);
+            if (b + lane < ab) s += edge_val<kEW>(a, it, b + lane);
             for (int64_t i = ab + 4 * lane; i + 3 < e; i += 128) {
-                const int4 v4 = *reinterpret_cast<const int4 *>(a.nbr + i);
+                const int4 v4 = __ldg(reinterpret_cast<const int4 *>(a.nbr + i));
                 if (kEW) {
-                    const float4 w4 = *reinterpret_cast<const float4 *>(a.ew + i);
-                    s += __ldg(a.gin + v4.x) * w4.x + __ldg(a.gin + v4.y) * w4.y +
-                         __ldg(a.gin + v4.z) * w4.z + __ldg(a.gin + v4.w) * w4.w;
+                    const float4 w4 = __ldg(reinterpret_cast<const float4 *>(a.ew + i));
+                    s += __ldca(it.gin + v4.x) * w4.x + __ldca(it.gin + v4.y) * w4.y +
+                         __ldca(it.gin + v4.z) * w4.z + __ldca(it.gin + v4.w) * w4.w;
                 } else {
-                    s += (__ldg(a.gin + v4.x) + __ldg(a.gin + v4.y)) + (__ldg(a.gin + v4.z) + __ldg(a.gin + v4.w));
+                    s += (__ldca(it.gin + v4.x) + __ldca(it.gin + v4.y)) + (__ldca(it.gin + v4.z) + __ldca(it.gin + v4.w));
                 }
             }
             const int64_t tail = ab + ((e - ab) & ~(int64_t)3);
-            if (tail + lane < e) s += edge_val<kEW>(a, tail + lane);
+            if (tail + lane < e) s += edge_val<kEW>(a, it, tail + lane);
             s = warp_sum(s);
-            if (lane == 0) finish_row<kEW, kRS, kPS, kBaseVec, kCG>(a, r, s, l1, chg);
+            if (lane == 0) finish_row<kEW, kRS, kPS, kBaseVec, kCG>(a, it, r, s, l1, chg);
         } else {
             // Stream group: rows r0 .. r0+31 (clipped to n_active).
             const int32_t r0 = plan.stream[item - plan.n_tasks - plan.n_long] * 32;
@@ -187,7 +205,7 @@ __global__ void __launch_bounds__(kPrThreads) pr_sweep(SweepArgs a, PrPlanDev pl
 #pragma unroll
                 for (int j = 0; j < 4; j++) {
                     const int k = k0 + 32 * j + lane;
-                    vals[j] = k < gend ? edge_val<kEW>(a, s0 + k) : 0.f;
+                    vals[j] = k < gend ? edge_val<kEW>(a, it, s0 + k) : 0.f;
                 }
 #pragma unroll
                 for (int j = 0; j < 4; j++) {
@@ -215,47 +233,113 @@ __global__ void __launch_bounds__(kPrThreads) pr_sweep(SweepArgs a, PrPlanDev pl
                     __syncwarp();
                 }
             }
-            if (r < a.n_active) finish_row<kEW, kRS, kPS, kBaseVec, kCG>(a, r, s_acc[wib][lane], l1, chg);
+            if (r < a.n_active) finish_row<kEW, kRS, kPS, kBaseVec, kCG>(a, it, r, s_acc[wib][lane], l1, chg);
             __syncwarp();
         }
     }
 
-    // Residual reduction; the last block to finish decides convergence.
-    double dl1 = warp_sum((double)l1);
-    int dchg = warp_sum(chg);
-    if (lane == 0) {
-        s_l1[wib] = dl1;
-        s_chg[wib] = dchg;
+}
+
+// Adds the block's sums of l1 and chg to the iteration's slot (every thread calls it).
+__device__ __forceinline__ void add_residual(IterSlot *slot, float l1, int chg) {
+    __shared__ double s_l1[kPrThreads / 32];
+    __shared__ int s_chg[kPrThreads / 32];
+    const double dl1 = warp_sum((double)l1);
+    const int dchg = __reduce_add_sync(kFull, chg);
+    if ((threadIdx.x & 31) == 0) {
+        s_l1[threadIdx.x >> 5] = dl1;
+        s_chg[threadIdx.x >> 5] = dchg;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
         double t = 0;
         int c = 0;
-        for (int i = 0; i < (int)(blockDim.x >> 5); i++) {
+        for (int i = 0; i < kPrThreads / 32; i++) {
             t += s_l1[i];
             c += s_chg[i];
         }
-        const int slot = a.it % kMaxIterSlots;
-        if (t != 0.0) atomicAdd(&a.st->l1[slot], t);
-        if (c) atomicAdd(&a.st->changed[slot], c);
-        __threadfence();
-        s_last = atomicAdd(&a.st->blocks_done, 1u) == gridDim.x - 1;
+        if (t != 0.0) atomicAdd(&slot->l1, t);
+        if (c) atomicAdd(&slot->changed, c);
     }
-    __syncthreads();
-    if (s_last && threadIdx.x == 0) {
-        __threadfence();
-        const int slot = a.it % kMaxIterSlots;
-        const double tl1 = *(volatile double *)&a.st->l1[slot];
-        const int tch = *(volatile int *)&a.st->changed[slot];
+}
+
+// Sweeps until converged, in one cooperative launch: a grid barrier between
+// sweeps, and every block evaluates the stopping rule from the iteration's
+// sums.  (A launch per sweep and a host check per four took 340 us for any
+// small graph; here a sweep of one costs its own few microseconds.)
+// cheb_rho > 0: Chebyshev semi-iteration for a Jacobi operator whose spectrum
+// lies in [-cheb_rho, cheb_rho] (a reversible walk scaled by d): weights
+// omega_1 = 1, omega_2 = 1 / (1 - rho^2 / 2), omega_{k+1} = 1 / (1 - rho^2
+// omega_k / 4) (Golub and Varga, 1961).
+template <bool kEW, bool kRS, bool kPS, bool kBaseVec>
+__global__ void __launch_bounds__(kPrThreads, kPrBlocks) pr_solve(SweepArgs a, PrPlanDev plan) {
+    __shared__ float s_acc[kPrThreads / 32][32];
+    const double rho2 = (double)a.cheb_rho * a.cheb_rho;
+    double omega = 1.0;
+    int it = 0, done = 0;
+    bool ok = true;
+    while (it < a.max_iters && !done) {
+        if (a.cheb_rho > 0.f)
+            omega = it == 0 ? 1.0 : it == 1 ? 1.0 / (1.0 - rho2 / 2.0) : 1.0 / (1.0 - rho2 * omega / 4.0);
+        const int cur = it & 1;
+        const SweepIter v{kPS ? a.g[cur] : a.x[cur], a.x[cur], a.x[cur ^ 1], kPS ? a.g[cur ^ 1] : a.x[cur ^ 1],
+                          (float)omega};
+        float l1;
+        int chg;
+        sweep_rows<kEW, kRS, kPS, kBaseVec>(a, plan, v, s_acc, l1, chg);
+        IterSlot *const slot = &a.st->slot[it % kMaxIterSlots];
+        add_residual(slot, l1, chg);
+        if (it + 2 >= kMaxIterSlots && blockIdx.x == 0 && threadIdx.x == 0)
+            a.st->slot[(it + 2) % kMaxIterSlots] = IterSlot{0.0, 0.0, 0.0, 0, 0};
+        if (!(ok = grid_barrier(&a.st->gs))) break;
         // eps >= 3e38 marks the per-vertex rule as unused.
-        const bool conv = (a.tol_l1 > 0.f && tl1 < (double)a.tol_l1) || (a.eps < 3e38f && tch == 0);
-        a.st->iters = a.it + 1;
-        a.st->blocks_done = 0;
-        // Clear the slot the next sweep will use.
-        const int ns = (a.it + 1) % kMaxIterSlots;
-        a.st->l1[ns] = 0.0;
-        a.st->changed[ns] = 0;
-        if (conv || a.it + 1 >= a.max_iters) a.st->done = conv ? 1 : 2;
+        if ((a.tol_l1 > 0.f && __ldcg(&slot->l1) < (double)a.tol_l1) || (a.eps < 3e38f && __ldcg(&slot->changed) == 0))
+            done = 1;
+        it++;
+    }
+    if (ok && a.final_x) {
+        const float *x = a.x[it & 1];
+        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += gridDim.x * blockDim.x) a.final_x[i] = x[i];
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        a.out->err = *(volatile int *)&a.st->gs.err;
+        a.out->iters = it;
+        a.out->done = done ? 1 : 2;
+        a.out->l1 = it > 0 ? __ldcg(&a.st->slot[(it - 1) % kMaxIterSlots].l1) : 0.0;
+        a.out->changed = it > 0 ? __ldcg(&a.st->slot[(it - 1) % kMaxIterSlots].changed) : 0;
+        __threadfence_system();
+    }
+}
+
+// One sweep as its own launch (see launched_sweeps): the last block to finish
+// decides convergence, and sweeps queued after it return at once.
+template <bool kEW, bool kRS, bool kPS, bool kBaseVec>
+__global__ void __launch_bounds__(kPrThreads) pr_step(SweepArgs a, PrPlanDev plan, SweepIter v, int it) {
+    __shared__ float s_acc[kPrThreads / 32][32];
+    if (*(volatile int *)&a.st->done) return;
+    float l1;
+    int chg;
+    sweep_rows<kEW, kRS, kPS, kBaseVec>(a, plan, v, s_acc, l1, chg);
+    IterSlot *const slot = &a.st->slot[it % kMaxIterSlots];
+    add_residual(slot, l1, chg);
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(&a.st->blocks_done, 1) == (int)gridDim.x - 1) {
+            __threadfence();
+            const double tl1 = __ldcg(&slot->l1);
+            const int tch = __ldcg(&slot->changed);
+            a.st->blocks_done = 0;
+            a.st->slot[(it + 1) % kMaxIterSlots] = IterSlot{0.0, 0.0, 0.0, 0, 0};
+            const bool conv = (a.tol_l1 > 0.f && tl1 < (double)a.tol_l1) || (a.eps < 3e38f && tch == 0);
+            if (conv || it + 1 >= a.max_iters) {
+                a.st->done = 1;
+                a.out->iters = it + 1;
+                a.out->l1 = tl1;
+                a.out->changed = tch;
+                a.out->done = conv ? 1 : 2;
+                __threadfence_system();
+            }
+        }
     }
 }
 
@@ -312,8 +396,8 @@ __global__ void __launch_bounds__(kPrThreads) pr_edge_grad(PrPlanDev plan, const
                 const int2 tk = plan.tasks[item];
                 u = plan.hubs[tk.x].row;
                 const int64_t rb = index[u], re = index[u + 1];
-                b = rb + (int64_t)tk.y * kHubChunk;
-                e = min(re, b + (int64_t)kHubChunk);
+                b = rb + (int64_t)tk.y * plan.chunk;
+                e = min(re, b + (int64_t)plan.chunk);
             } else {
                 u = plan.longrows[item - plan.n_tasks];
                 b = index[u];
@@ -664,8 +748,16 @@ __global__ void spmm_residual(const double *col_l1, int K, float tol, int *done_
 
 // ------------------------------------------------------------------- plan
 
-hc_status ensure_plan(hc_graph *g) {
-    if (g->pr_plan.ptr) return HC_OK;
+namespace {
+// m / per rounded down to a power of two, in [kMinChunk, kMaxChunk].
+int64_t plan_size(int64_t m, int64_t per) {
+    int64_t x = kMinChunk;
+    while (x < kMaxChunk && x * 2 * per <= m) x *= 2;
+    return x;
+}
+
+hc_status build_plan(hc_graph *g, int64_t stream_edges, int64_t chunk, DevBuf *buf, PrPlanDev *view,
+                     int32_t *slots) {
     const int32_t na = g->n_active;
     std::vector<int64_t> idx((size_t)na + 1);
     HC_CUDA_TRY(cudaMemcpy(idx.data(), g->index.as<int64_t>(), sizeof(int64_t) * ((size_t)na + 1),
@@ -678,14 +770,14 @@ hc_status ensure_plan(hc_graph *g) {
     for (int32_t gid = 0; gid < ngroups; gid++) {
         const int32_t r0 = gid * 32, r1 = std::min(r0 + 32, na);
         const int64_t tot = idx[r1] - idx[r0];
-        if (tot <= kStreamEdges) {
+        if (tot <= stream_edges) {
             stream.push_back(gid);
             continue;
         }
         for (int32_t r = r0; r < r1; r++) {
             const int64_t d = idx[r + 1] - idx[r];
-            if (d > kHubEdges) {
-                HubInfo h{r, partial_slots, (int32_t)((d + kHubChunk - 1) / kHubChunk), 0};
+            if (d > 2 * chunk) {
+                HubInfo h{r, partial_slots, (int32_t)((d + chunk - 1) / chunk), 0};
                 for (int c = 0; c < h.nchunks; c++) tasks.push_back(make_int2((int)hubs.size(), c));
                 partial_slots += h.nchunks;
                 hubs.push_back(h);
@@ -694,18 +786,17 @@ hc_status ensure_plan(hc_graph *g) {
             }
         }
     }
-    const size_t b_hdr = 256;
-    const size_t b_stream = (stream.size() * 4 + 255) / 256 * 256;
-    const size_t b_long = (longrows.size() * 4 + 255) / 256 * 256;
-    const size_t b_tasks = (tasks.size() * sizeof(int2) + 255) / 256 * 256;
-    const size_t b_hubs = (hubs.size() * sizeof(HubInfo) + 255) / 256 * 256;
-    HC_TRY(g->pr_plan.ensure(b_hdr + b_stream + b_long + b_tasks + b_hubs + 256));
-    char *p = g->pr_plan.as<char>() + b_hdr;
+    auto up = [](size_t b) { return (b + 255) / 256 * 256; };
+    const size_t b_stream = up(stream.size() * 4), b_long = up(longrows.size() * 4);
+    const size_t b_tasks = up(tasks.size() * sizeof(int2)), b_hubs = up(hubs.size() * sizeof(HubInfo));
+    HC_TRY(buf->ensure(b_stream + b_long + b_tasks + b_hubs + 256));
+    char *p = buf->as<char>();
     PrPlanDev v{};
     v.n_stream = (int)stream.size();
     v.n_long = (int)longrows.size();
     v.n_tasks = (int)tasks.size();
     v.n_hub = (int)hubs.size();
+    v.chunk = (int)chunk;
     v.stream = (const int32_t *)p;
     if (!stream.empty()) HC_CUDA_TRY(cudaMemcpy(p, stream.data(), stream.size() * 4, cudaMemcpyHostToDevice));
     p += b_stream;
@@ -717,9 +808,21 @@ hc_status ensure_plan(hc_graph *g) {
     p += b_tasks;
     v.hubs = (const HubInfo *)p;
     if (!hubs.empty()) HC_CUDA_TRY(cudaMemcpy(p, hubs.data(), hubs.size() * sizeof(HubInfo), cudaMemcpyHostToDevice));
-    g->pr_view = v;
-    g->pr_partial_slots = partial_slots;
+    *view = v;
+    *slots = partial_slots;
     return HC_OK;
+}
+}  // namespace
+
+hc_status ensure_plan(hc_graph *g) {
+    if (g->pr_plan.ptr) return HC_OK;
+    return build_plan(g, plan_size(g->M, 8192), plan_size(g->M, 4096), &g->pr_plan, &g->pr_view, &g->pr_partial_slots);
+}
+
+hc_status ensure_sssp_plan(hc_graph *g) {
+    if (g->sssp_plan.ptr) return HC_OK;
+    int32_t slots = 0;  // the pull keeps no partial sums
+    return build_plan(g, kMaxChunk, plan_size(g->M, 4096), &g->sssp_plan, &g->sssp_view, &slots);
 }
 
 // The multi-column sweeps' row plan, built on the first such call.  A chunk is M
@@ -795,41 +898,87 @@ PrPlanDev plan_view(hc_graph *g, int *partial_slots) {
     return g->pr_view;
 }
 
-template <bool kEW, bool kRS, bool kPS, bool kBaseVec, bool kCG = false>
-hc_status launch_sweep(hc_graph *g, const SweepArgs &a, const PrPlanDev &plan) {
-    static int bps = 0;
-    if (bps == 0) {
-        HC_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, pr_sweep<kEW, kRS, kPS, kBaseVec, kCG>,
-                                                                  kPrThreads, 0));
-        bps = std::max(bps, 1);
+// A cooperative launch of `fn` over the row plan's items: no more blocks than a
+// warp each needs (a barrier costs by the block), all that fit otherwise.
+hc_status launch_solve(hc_graph *g, const void *fn, int *blocks_per_sm, SweepArgs &a, const PrPlanDev &plan,
+                       int64_t vector_items, void *extra) {
+    if (*blocks_per_sm == 0) {
+        int b = 0;
+        HC_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fn, kPrThreads, 0));
+        if (b < 1) return fail(HC_ERR_CUDA, "PageRank kernel cannot be resident");
+        *blocks_per_sm = b;
     }
-    { pr_sweep<kEW, kRS, kPS, kBaseVec, kCG><<<g->sm_count * bps, kPrThreads, 0, g->stream>>>(a, plan); ::hc::count_launch(); }
-    HC_CUDA_TRY(cudaGetLastError());
+    const int64_t warps = std::max<int64_t>((int64_t)plan.n_tasks + plan.n_long + plan.n_stream, vector_items / 32);
+    const int64_t want = std::max<int64_t>(1, (warps + kPrThreads / 32 - 1) / (kPrThreads / 32));
+    const int grid = (int)std::min<int64_t>(want, (int64_t)*blocks_per_sm * g->sm_count);
+    PrPlanDev p = plan;
+    void *params[] = {&a, &p, extra};
+    ::hc::count_launch();
+    HC_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kPrThreads), params, 0, g->stream));
     return HC_OK;
 }
 
-using SweepFn = hc_status (*)(hc_graph *, const SweepArgs &, const PrPlanDev &);
+// Whether a solve's sweeps are launched one by one: on a graph of at least 2^24
+// edges without hub rows, whose sweeps miss L1 throughout (uniform, 33M edges: 1.19
+// ms so, 1.33 ms in one launch; at 8M edges both 0.48 ms).  With hubs one launch is
+// the faster at every size (Kronecker scale 22: 2.99 and 2.87 ms, scale 20: 0.94 and
+// 0.85 ms, scale 12: 0.35 and 0.09 ms).
+bool launched_sweeps(const hc_graph *g, const PrPlanDev &plan) { return plan.n_tasks == 0 && g->M >= (1ll << 24); }
 
-SweepFn pick_sweep(bool ew, bool rs, bool ps, bool basev) {
+using SolveFn = hc_status (*)(hc_graph *, SweepArgs &, const PrPlanDev &, volatile SolveOut *);
+
+// The Chebyshev weight of sweep `it` (the recurrence of pr_solve).
+double next_omega(double omega, int it, float rho) {
+    if (rho <= 0.f) return 1.0;
+    const double rho2 = (double)rho * rho;
+    return it == 0 ? 1.0 : it == 1 ? 1.0 / (1.0 - rho2 / 2.0) : 1.0 / (1.0 - rho2 * omega / 4.0);
+}
+
+template <bool kEW, bool kRS, bool kPS, bool kBaseVec>
+hc_status launch_pr_solve(hc_graph *g, SweepArgs &a, const PrPlanDev &plan, volatile SolveOut *out) {
+    if (launched_sweeps(g, plan)) {
+        static int step_bps = 0;
+        if (step_bps == 0) {
+            HC_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&step_bps, pr_step<kEW, kRS, kPS, kBaseVec>,
+                                                                      kPrThreads, 0));
+            step_bps = std::max(step_bps, 1);
+        }
+        // Launches are queued in rounds, the host looking once per round.
+        constexpr int kRound = 4;
+        double omega = 1.0;
+        for (int it = 0; it < a.max_iters && !out->done;) {
+            for (int k = 0; k < kRound && it < a.max_iters; k++, it++) {
+                omega = next_omega(omega, it, a.cheb_rho);
+                const int cur = it & 1;
+                const SweepIter v{kPS ? a.g[cur] : a.x[cur], a.x[cur], a.x[cur ^ 1], kPS ? a.g[cur ^ 1] : a.x[cur ^ 1],
+                                  (float)omega};
+                { pr_step<kEW, kRS, kPS, kBaseVec><<<g->sm_count * step_bps, kPrThreads, 0, g->stream>>>(a, plan, v, it); ::hc::count_launch(); }
+            }
+            HC_CUDA_TRY(cudaGetLastError());
+            HC_CUDA_TRY(cudaStreamSynchronize(g->stream));
+        }
+        if (a.final_x)
+            HC_CUDA_TRY(cudaMemcpyAsync(a.final_x, a.x[out->iters & 1], (size_t)a.n * 4, cudaMemcpyDeviceToDevice,
+                                        g->stream));
+        return HC_OK;
+    }
+    static int bps = 0;
+    return launch_solve(g, (const void *)pr_solve<kEW, kRS, kPS, kBaseVec>, &bps, a, plan, 0, nullptr);
+}
+
+SolveFn pick_solve(bool ew, bool rs, bool ps, bool basev) {
     const int key = (ew ? 8 : 0) | (rs ? 4 : 0) | (ps ? 2 : 0) | (basev ? 1 : 0);
     switch (key) {
-        case 0: return launch_sweep<false, false, false, false>;
-        case 1: return launch_sweep<false, false, false, true>;
-        case 2: return launch_sweep<false, false, true, false>;
-        case 3: return launch_sweep<false, false, true, true>;
-        case 4: return launch_sweep<false, true, false, false>;
-        case 5: return launch_sweep<false, true, false, true>;
-        case 8: return launch_sweep<true, false, false, false>;
-        case 9: return launch_sweep<true, false, false, true>;
-        case 12: return launch_sweep<true, true, false, false>;
-        case 13: return launch_sweep<true, true, false, true>;
+        case 2: return launch_pr_solve<false, false, true, false>;
+        case 3: return launch_pr_solve<false, false, true, true>;
+        case 5: return launch_pr_solve<false, true, false, true>;
+        case 8: return launch_pr_solve<true, false, false, false>;
+        case 9: return launch_pr_solve<true, false, false, true>;
+        case 13: return launch_pr_solve<true, true, false, true>;
         default: return nullptr;
     }
 }
 
-// Runs sweeps until the device marks the state done.  Launches are queued in
-// rounds of kRound and the host checks the done flag once per round; sweeps
-// queued after convergence return immediately.
 struct SolveResult {
     int iters;
     int done;
@@ -838,56 +987,41 @@ struct SolveResult {
     float ms;
 };
 
-// Sweeps until converged.  cheb_rho > 0: Chebyshev semi-iteration for a
-// Jacobi operator whose spectrum lies in [-cheb_rho, cheb_rho] (a reversible
-// walk scaled by d): weights omega_1 = 1, omega_2 = 1 / (1 - rho^2 / 2),
-// omega_{k+1} = 1 / (1 - rho^2 omega_k / 4) (Golub and Varga, 1961).
-hc_status run_solve(hc_graph *g, SweepArgs a, const PrPlanDev &plan, SweepFn fn, float *x[2], float *gv[2],
-                    bool separate_g, SolveResult *res, float cheb_rho = 0.f) {
-    IterState *st = reinterpret_cast<IterState *>(g->ws_ctl.ptr);
-    HC_CUDA_TRY(cudaMemsetAsync(st, 0, sizeof(IterState), g->stream));
+// The solve's state for max_iters iterations, zeroed, and its report's mapped slot.
+hc_status solve_begin(hc_graph *g, SweepArgs &a, SolveOut **out) {
+    HC_TRY(g->ws_ctl.ensure(sizeof(IterState) + 4096));
+    a.st = reinterpret_cast<IterState *>(g->ws_ctl.ptr);
+    const size_t slots = std::min<size_t>((size_t)a.max_iters + 1, kMaxIterSlots);
+    HC_CUDA_TRY(cudaMemsetAsync(a.st, 0, offsetof(IterState, slot) + sizeof(IterSlot) * slots, g->stream));
+    HC_TRY(ctl_slot(g, 0, (void **)out, (void **)&a.out));
+    **out = SolveOut{0, 0, 0, 0, 0.0};
     HC_CUDA_TRY(cudaEventRecord(g->ev_start, g->stream));
-    constexpr int kRound = 4;
-    int host_done = 0;
-    struct Tail {
-        int done, iters;
-    };
-    HC_TRY(g->pinned.ensure(64));
-    volatile Tail *pt = g->pinned.as<Tail>();
-    const double rho2 = (double)cheb_rho * cheb_rho;
-    double omega = 1.0;
-    for (int it = 0; it < a.max_iters && !host_done;) {
-        for (int k = 0; k < kRound && it < a.max_iters; k++, it++) {
-            a.it = it;
-            if (cheb_rho > 0.f) omega = it == 0 ? 1.0 : it == 1 ? 1.0 / (1.0 - rho2 / 2.0) : 1.0 / (1.0 - rho2 * omega / 4.0);
-            a.omega = (float)omega;
-            a.gin = separate_g ? gv[it & 1] : x[it & 1];
-            a.xin = x[it & 1];
-            a.xout = x[(it + 1) & 1];
-            a.gout = separate_g ? gv[(it + 1) & 1] : a.xout;
-            HC_TRY(fn(g, a, plan));
-        }
-        HC_CUDA_TRY(cudaMemcpyAsync((void *)pt, &st->done, sizeof(Tail), cudaMemcpyDeviceToHost, g->stream));
-        HC_CUDA_TRY(cudaStreamSynchronize(g->stream));
-        host_done = pt->done;
-    }
+    return HC_OK;
+}
+hc_status solve_end(hc_graph *g, const SolveOut *out, SolveResult *res) {
     HC_CUDA_TRY(cudaEventRecord(g->ev_stop, g->stream));
     HC_CUDA_TRY(cudaStreamSynchronize(g->stream));
-    Tail t;
-    HC_CUDA_TRY(cudaMemcpy(&t, &st->done, sizeof(Tail), cudaMemcpyDeviceToHost));
-    res->iters = t.iters;
-    res->done = t.done;
-    const int slot = (t.iters - 1) % kMaxIterSlots;
-    double l1 = 0;
-    int chg = 0;
-    if (t.iters > 0) {
-        HC_CUDA_TRY(cudaMemcpy(&l1, &st->l1[slot], sizeof(double), cudaMemcpyDeviceToHost));
-        HC_CUDA_TRY(cudaMemcpy(&chg, &st->changed[slot], sizeof(int), cudaMemcpyDeviceToHost));
-    }
-    res->l1 = l1;
-    res->changed = chg;
+    if (out->err) return fail((hc_status)out->err, "PageRank: device run ended with status %d", out->err);
+    res->iters = out->iters;
+    res->done = out->done;
+    res->l1 = out->l1;
+    res->changed = out->changed;
     HC_CUDA_TRY(cudaEventElapsedTime(&res->ms, g->ev_start, g->ev_stop));
     return HC_OK;
+}
+
+hc_status run_solve(hc_graph *g, SweepArgs a, const PrPlanDev &plan, SolveFn fn, float *x[2], float *gv[2],
+                    SolveResult *res, float cheb_rho = 0.f, float *final_x = nullptr) {
+    for (int k = 0; k < 2; k++) {
+        a.x[k] = x[k];
+        a.g[k] = gv ? gv[k] : x[k];
+    }
+    a.cheb_rho = cheb_rho;
+    a.final_x = final_x;
+    SolveOut *out = nullptr;
+    HC_TRY(solve_begin(g, a, &out));
+    HC_TRY(fn(g, a, plan, out));
+    return solve_end(g, out, res);
 }
 
 // ------------------------------------------------- adjoint by conjugate gradients
@@ -899,12 +1033,10 @@ hc_status run_solve(hc_graph *g, SweepArgs a, const PrPlanDev &plan, SweepFn fn,
 // residual c + d A^T lambda - lambda, so the stopping rule is the same as the
 // sweeps'.  Rows without weight (s = 0) keep lambda = c.  Vectors are fp32,
 // dot products fp64; alpha, beta and the stop decision stay on the device.
-struct CgState {
-    double acc0, acc1;       // block partial sums of the running kernel
-    double rz, alpha, beta, z1;
-    double tol;
-    unsigned blocks;
-    int iters, max_iters, converged;
+struct CgArgs {
+    const float *c;
+    float *lam, *r, *p, *sp;
+    float rel_tol;  // stop at |z|_1 < rel_tol * |c|_1
 };
 
 __device__ __forceinline__ float row_weight(const float *rs, int32_t v) {
@@ -912,174 +1044,132 @@ __device__ __forceinline__ float row_weight(const float *rs, int32_t v) {
     return r > 0.f ? 1.0f / r : 0.f;
 }
 
-// Accumulates (a0, a1) over the grid; the last block to finish returns true
-// in thread 0 with the totals in *t0, *t1 and the accumulators cleared.
-__device__ __forceinline__ bool grid_sum2(CgState *cg, double a0, double a1, double *t0, double *t1) {
+// Adds the block's sums of rz and z1 to the iteration's slot (every thread calls it).
+__device__ __forceinline__ void add_dots(IterSlot *slot, double rz, double z1) {
     __shared__ double s0[32], s1[32];
-    __shared__ int s_last;
-    a0 = block_sum(a0, s0);
-    a1 = block_sum(a1, s1);
+    rz = block_sum(rz, s0);
+    z1 = block_sum(z1, s1);
     if (threadIdx.x == 0) {
-        if (a0 != 0.0) atomicAdd(&cg->acc0, a0);
-        if (a1 != 0.0) atomicAdd(&cg->acc1, a1);
-        __threadfence();
-        s_last = atomicAdd(&cg->blocks, 1u) == gridDim.x - 1;
+        if (rz != 0.0) atomicAdd(&slot->rz, rz);
+        if (z1 != 0.0) atomicAdd(&slot->z1, z1);
     }
-    __syncthreads();
-    if (!s_last || threadIdx.x != 0) return false;
-    __threadfence();
-    *t0 = *(volatile double *)&cg->acc0;
-    *t1 = *(volatile double *)&cg->acc1;
-    cg->acc0 = 0.0;
-    cg->acc1 = 0.0;
-    cg->blocks = 0;
-    return true;
 }
 
-// r = s (c - lambda) + d S lambda, z = r / s, p = z; rz = r.z, stop if |z|_1 < tol.
-__global__ void cg_start(int32_t n, const float *c, float *lam, const float *slam, const float *rs, float d, float *r,
-                         float *p, CgState *cg, IterState *st) {
-    double rz = 0.0, z1 = 0.0;
-    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-        const float sv = row_weight(rs, v);
-        if (sv == 0.f) {
-            lam[v] = c[v];
-            r[v] = 0.f;
-            p[v] = 0.f;
-            continue;
+// The whole solve in one cooperative launch, a grid barrier after each sweep and
+// each vector pass (three an iteration).
+template <bool kEW>
+__global__ void __launch_bounds__(kPrThreads, kPrBlocks) pr_cg(SweepArgs a, PrPlanDev plan, CgArgs q) {
+    __shared__ float s_acc[kPrThreads / 32][32];
+    __shared__ double s_c[32];
+    const int gtid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
+    GridSync *const gs = &a.st->gs;
+    float l1;
+    int chg;
+    int iters = 0, converged = 0;
+    double rz = 0.0, z1 = 0.0, c1 = 0.0, tol = 0.0;
+    // S x by the pull sweep with each row's own weights; its residual is p . q.
+    sweep_rows<kEW, false, false, false, true>(a, plan, SweepIter{q.lam, q.lam, q.sp, q.sp, 1.f}, s_acc, l1, chg);
+    bool ok = grid_barrier(gs);
+    if (ok) {
+        // r = s (c - lambda) + d S lambda, z = r / s, p = z.
+        for (int v = gtid; v < a.n; v += nthreads) {
+            const float sv = row_weight(a.rs, v);
+            c1 += fabs((double)q.c[v]);
+            if (sv == 0.f) {
+                q.lam[v] = q.c[v];
+                q.r[v] = 0.f;
+                q.p[v] = 0.f;
+                continue;
+            }
+            const float rv = sv * (q.c[v] - q.lam[v]) + a.d * q.sp[v];
+            const float zv = rv * a.rs[v];
+            q.r[v] = rv;
+            q.p[v] = zv;
+            rz += (double)rv * zv;
+            z1 += fabs((double)zv);
         }
-        const float rv = sv * (c[v] - lam[v]) + d * slam[v];
-        const float zv = rv * rs[v];
-        r[v] = rv;
-        p[v] = zv;
-        rz += (double)rv * zv;
-        z1 += fabs((double)zv);
+        add_dots(&a.st->slot[0], rz, z1);
+        __syncthreads();
+        c1 = block_sum(c1, s_c);
+        if (threadIdx.x == 0 && c1 != 0.0) atomicAdd(&a.st->slot[0].l1, c1);
+        ok = grid_barrier(gs);
     }
-    double trz, tz1;
-    if (grid_sum2(cg, rz, z1, &trz, &tz1)) {
-        cg->rz = trz;
-        cg->z1 = tz1;
-        if (tz1 < cg->tol || trz <= 0.0) {
-            cg->converged = 1;
-            st->done = 1;
+    if (ok) {
+        rz = __ldcg(&a.st->slot[0].rz);
+        z1 = __ldcg(&a.st->slot[0].z1);
+        tol = (double)(float)(q.rel_tol * __ldcg(&a.st->slot[0].l1));
+        converged = z1 < tol || rz <= 0.0;
+    }
+    for (int it = 1; ok && !converged && it <= a.max_iters; it++) {
+        IterSlot *const slot = &a.st->slot[it];
+        sweep_rows<kEW, false, false, false, true>(a, plan, SweepIter{q.p, q.p, q.sp, q.sp, 1.f}, s_acc, l1, chg);
+        add_residual(slot, l1, 0);
+        if (!(ok = grid_barrier(gs))) break;
+        const double pq = __ldcg(&slot->l1);
+        if (!(pq > 0.0)) break;  // p = 0 (already exact) or a breakdown: stop
+        // lambda += alpha p, r -= alpha q.
+        const float alpha = (float)(rz / pq);
+        double nrz = 0.0, nz1 = 0.0;
+        for (int v = gtid; v < a.n; v += nthreads) {
+            const float pv = q.p[v];
+            const float qv = row_weight(a.rs, v) * pv - a.d * q.sp[v];
+            q.lam[v] += alpha * pv;
+            const float rv = q.r[v] - alpha * qv;
+            q.r[v] = rv;
+            const float zv = rv * a.rs[v];
+            nrz += (double)rv * zv;
+            nz1 += fabs((double)zv);
         }
+        add_dots(slot, nrz, nz1);
+        if (!(ok = grid_barrier(gs))) break;
+        nrz = __ldcg(&slot->rz);
+        z1 = __ldcg(&slot->z1);
+        const float beta = (float)(rz > 0.0 ? nrz / rz : 0.0);
+        rz = nrz;
+        iters++;
+        converged = z1 < tol;
+        if (converged || it == a.max_iters) break;
+        // p = z + beta p (the same thread's entries as above).
+        for (int v = gtid; v < a.n; v += nthreads) q.p[v] = q.r[v] * a.rs[v] + beta * q.p[v];
+        ok = grid_barrier(gs);
+    }
+    if (gtid == 0) {
+        a.out->err = *(volatile int *)&gs->err;
+        a.out->iters = iters;
+        a.out->done = converged;
+        a.out->l1 = z1;
+        a.out->changed = 0;
+        __threadfence_system();
     }
 }
 
-// alpha = rz / (p . q), p . q from the sweep's residual slot; lambda += alpha
-// p, r -= alpha q; beta = r.z / rz; stop on |z|_1 < tol or the cap.
-__global__ void cg_update(int32_t n, const float *p, const float *sp, const float *rs, float d, float *lam, float *r,
-                          CgState *cg, IterState *st, int slot) {
-    if (*(volatile int *)&st->done) return;
-    const double pq = *(volatile double *)&st->l1[slot];
-    if (!(pq > 0.0)) {  // p = 0 (already exact) or a breakdown: stop
-        if (blockIdx.x == 0 && threadIdx.x == 0) st->done = 1;
-        return;
-    }
-    const float alpha = (float)(cg->rz / pq);
-    double rz = 0.0, z1 = 0.0;
-    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-        const float pv = p[v];
-        const float q = row_weight(rs, v) * pv - d * sp[v];
-        lam[v] += alpha * pv;
-        const float rv = r[v] - alpha * q;
-        r[v] = rv;
-        const float zv = rv * rs[v];
-        rz += (double)rv * zv;
-        z1 += fabs((double)zv);
-    }
-    double trz, tz1;
-    if (grid_sum2(cg, rz, z1, &trz, &tz1)) {
-        cg->beta = cg->rz > 0.0 ? trz / cg->rz : 0.0;
-        cg->rz = trz;
-        cg->z1 = tz1;
-        cg->iters++;
-        if (tz1 < cg->tol) cg->converged = 1;
-        if (cg->converged || cg->iters >= cg->max_iters) st->done = 1;
-    }
-}
-
-// p = z + beta p.
-__global__ void cg_direction(int32_t n, const float *r, const float *rs, float *p, const CgState *cg,
-                             const IterState *st) {
-    if (*(volatile const int *)&st->done) return;
-    const float beta = (float)cg->beta;
-    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
-        p[v] = r[v] * rs[v] + beta * p[v];
+template <bool kEW>
+hc_status launch_cg(hc_graph *g, SweepArgs &a, const PrPlanDev &plan, CgArgs &q) {
+    static int bps = 0;
+    return launch_solve(g, (const void *)pr_cg<kEW>, &bps, a, plan, a.n, &q);
 }
 
 // Solves the adjoint into lam (which holds the start) with the row plan's
 // sweep for S x.  `work` holds 3 vectors of n floats.
-hc_status run_cg(hc_graph *g, const PrPlanDev &plan, bool weighted, const float *c, float *lam, float d, double tol,
+hc_status run_cg(hc_graph *g, const PrPlanDev &plan, bool weighted, const float *c, float *lam, float d, float rel_tol,
                  int max_iters, float *work, float *partials, unsigned *hub_count, SolveResult *res) {
     const int64_t n = g->N;
-    float *r = work, *pv = work + n, *sp = work + 2 * n;
-    IterState *st = reinterpret_cast<IterState *>(g->ws_ctl.ptr);
-    CgState *cg = reinterpret_cast<CgState *>(g->ws_ctl.as<char>() + (sizeof(IterState) + 255) / 256 * 256);
-    const float *rs = weighted ? g->inv_wsum.as<float>() : g->inv_deg.as<float>();
-    HC_CUDA_TRY(cudaMemsetAsync(st, 0, sizeof(IterState), g->stream));
-    CgState h{};
-    h.tol = tol;
-    h.max_iters = max_iters;
-    HC_CUDA_TRY(cudaMemcpyAsync(cg, &h, sizeof(h), cudaMemcpyHostToDevice, g->stream));
-    // y = S x through the pull sweep (own-row weights, no stopping rule of
-    // its own: it returns at once once st->done is set); in the iterations
-    // its epilogue also sums p . q (kCG).
+    CgArgs q{c, lam, work, work + n, work + 2 * n, rel_tol};
     SweepArgs a{};
     a.index = g->index.as<int64_t>();
     a.nbr = g->nbr.as<int32_t>();
     a.ew = weighted ? pr_weights(g) : nullptr;
-    a.base_scalar = 0.f;
-    a.d = 1.0f;
-    a.rs = rs;
-    a.omega = 1.0f;
+    a.d = d;
+    a.rs = weighted ? g->inv_wsum.as<float>() : g->inv_deg.as<float>();
     a.partials = partials;
     a.hub_count = hub_count;
-    a.st = st;
-    a.tol_l1 = 0.f;
-    a.eps = 3.4e38f;
     a.max_iters = max_iters;
+    a.n = g->N;
     a.n_active = g->n_active;
-    SweepFn sweep = pick_sweep(weighted, false, false, false);
-    SweepFn cg_sweep = weighted ? launch_sweep<true, false, false, false, true> : launch_sweep<false, false, false, false, true>;
-    const int grid = g->sm_count * 4;
-    HC_CUDA_TRY(cudaEventRecord(g->ev_start, g->stream));
-    a.it = 0;
-    a.gin = lam;
-    a.xin = sp;
-    a.xout = sp;
-    a.gout = sp;
-    HC_TRY(sweep(g, a, plan));
-    { cg_start<<<grid, 256, 0, g->stream>>>((int32_t)n, c, lam, sp, rs, d, r, pv, cg, st); ::hc::count_launch(); }
-    HC_CUDA_TRY(cudaGetLastError());
-    constexpr int kRound = 4;
-    HC_TRY(g->pinned.ensure(64));
-    volatile int *hdone = g->pinned.as<int>();
-    int it = 0;
-    for (bool done = false; !done && it < max_iters;) {
-        for (int k = 0; k < kRound && it < max_iters; k++, it++) {
-            a.it = it + 1;
-            a.gin = pv;
-            a.d = d;
-            HC_TRY(cg_sweep(g, a, plan));
-            const int slot = a.it % kMaxIterSlots;
-            { cg_update<<<grid, 256, 0, g->stream>>>((int32_t)n, pv, sp, rs, d, lam, r, cg, st, slot); ::hc::count_launch(); }
-            { cg_direction<<<grid, 256, 0, g->stream>>>((int32_t)n, r, rs, pv, cg, st); ::hc::count_launch(); }
-            HC_CUDA_TRY(cudaGetLastError());
-        }
-        HC_CUDA_TRY(cudaMemcpyAsync((void *)hdone, &st->done, sizeof(int), cudaMemcpyDeviceToHost, g->stream));
-        HC_CUDA_TRY(cudaStreamSynchronize(g->stream));
-        done = *hdone != 0;
-    }
-    HC_CUDA_TRY(cudaEventRecord(g->ev_stop, g->stream));
-    HC_CUDA_TRY(cudaStreamSynchronize(g->stream));
-    HC_CUDA_TRY(cudaMemcpy(&h, cg, sizeof(h), cudaMemcpyDeviceToHost));
-    res->iters = h.iters;
-    res->done = h.converged;
-    res->l1 = h.z1;
-    res->changed = 0;
-    HC_CUDA_TRY(cudaEventElapsedTime(&res->ms, g->ev_start, g->ev_stop));
-    return HC_OK;
+    SolveOut *out = nullptr;
+    HC_TRY(solve_begin(g, a, &out));
+    HC_TRY(weighted ? launch_cg<true>(g, a, plan, q) : launch_cg<false>(g, a, plan, q));
+    return solve_end(g, out, res);
 }
 
 void fill_opts(const hc_pr_opts *opts, hc_pr_opts *o) {
@@ -1246,18 +1336,23 @@ extern "C" hc_status hc_pr_forward(hc_graph *g, const float *teleport, int32_t n
     a.ps = ps;
     a.partials = partials;
     a.hub_count = hub_count;
-    a.st = reinterpret_cast<IterState *>(g->ws_ctl.ptr);
     a.tol_l1 = o.tol_l1;
     a.eps = o.eps_vertex > 0.f ? o.eps_vertex : 3.4e38f;
     a.max_iters = o.max_iters;
+    a.n = g->N;
     a.n_active = g->n_active;
-    SweepFn fn = pick_sweep(weighted, false, !weighted, basevec);
+    SolveFn fn = pick_solve(weighted, false, !weighted, basevec);
     if (!fn) return fail(HC_ERR_UNSUPPORTED, "hc_pr_forward: no sweep for this option set");
     if (o.eps_vertex <= 0.f) a.eps = 3.4e38f;
     SolveResult r;
-    HC_TRY(run_solve(g, a, plan, fn, x, gv, !weighted, &r, cheb ? o.damping : 0.f));
-    HC_TRY(copy_out(scores_out, x[r.iters & 1], n * 4, g->stream));
-    HC_CUDA_TRY(cudaStreamSynchronize(g->stream));
+    // Device scores are written by the solve itself.
+    const bool dev_out = is_device_pointer(scores_out);
+    HC_TRY(run_solve(g, a, plan, fn, x, weighted ? nullptr : gv, &r, cheb ? o.damping : 0.f,
+                     dev_out ? scores_out : nullptr));
+    if (!dev_out) {
+        HC_TRY(copy_out(scores_out, x[r.iters & 1], n * 4, g->stream));
+        HC_CUDA_TRY(cudaStreamSynchronize(g->stream));
+    }
     if (stats) {
         stats->iterations = r.iters;
         stats->converged = r.done == 1;
@@ -1285,7 +1380,6 @@ extern "C" hc_status hc_pr_backward(hc_graph *g, const float *scores, const floa
     int partial_slots = 0;
     PrPlanDev plan = plan_view(g, &partial_slots);
     const int64_t n = g->N;
-    HC_TRY(g->ws_ctl.ensure(sizeof(IterState) + sizeof(CgState) + 4096));
     // cvec, lam[2], xs, spare and the three vectors of the CG solve.
     const size_t bytes = 8 * (size_t)n * 4 + (size_t)(partial_slots + 1) * 4 + (size_t)(plan.n_hub + 1) * 4 + 8192;
     HC_TRY(g->ws_pr.ensure(bytes));
@@ -1324,22 +1418,11 @@ extern "C" hc_status hc_pr_backward(hc_graph *g, const float *scores, const floa
     a.ps = nullptr;
     a.partials = partials;
     a.hub_count = hub_count;
-    a.st = reinterpret_cast<IterState *>(g->ws_ctl.ptr);
-    // The adjoint's L1 rule is relative to sum |dL/dx| (lambda scales with it).
-    {
-        HC_TRY(g->pinned.ensure(64));
-        double *hacc = g->pinned.as<double>();
-        double *dacc = reinterpret_cast<double *>(spare);  // scratch until the solve ends
-        HC_CUDA_TRY(cudaMemsetAsync(dacc, 0, sizeof(double), g->stream));
-        { sum_abs<<<g->sm_count * 4, 256, 0, g->stream>>>(cvec, g->N, dacc); ::hc::count_launch(); }
-        HC_CUDA_TRY(cudaMemcpyAsync(hacc, dacc, sizeof(double), cudaMemcpyDeviceToHost, g->stream));
-        HC_CUDA_TRY(cudaStreamSynchronize(g->stream));
-        a.tol_l1 = (float)(o.tol_l1 * *hacc);
-    }
     a.eps = o.eps_vertex > 0.f ? o.eps_vertex : 3.4e38f;
     a.max_iters = o.max_iters;
+    a.n = g->N;
     a.n_active = g->n_active;
-    SweepFn fn = pick_sweep(weighted, true, false, true);
+    SolveFn fn = pick_solve(weighted, true, false, true);
     // lambda = c + d A^T lambda.  For a reversible walk (symmetric weights)
     // A^T = D^-1 S is similar to a symmetric matrix with spectrum in [-1, 1]:
     // conjugate gradients on (D - d S) lambda = D c (accel 0 / 1), or Chebyshev
@@ -1351,12 +1434,20 @@ extern "C" hc_status hc_pr_backward(hc_graph *g, const float *scores, const floa
     float *lfin;
     if (sym && o.accel != 2) {
         HC_CUDA_TRY(cudaMemsetAsync(cg_work + 2 * n, 0, n * 4, g->stream));  // S p rows without edges stay 0
-        HC_TRY(run_cg(g, plan, weighted, cvec, lam[0], o.damping, (double)a.tol_l1, o.max_iters, cg_work, partials,
+        HC_TRY(run_cg(g, plan, weighted, cvec, lam[0], o.damping, o.tol_l1, o.max_iters, cg_work, partials,
                       hub_count, &r));
         lfin = lam[0];
     } else {
-        float *gdummy[2] = {spare, spare};
-        HC_TRY(run_solve(g, a, plan, fn, lam, gdummy, false, &r, sym ? o.damping : 0.f));
+        // The L1 rule is relative to sum |dL/dx| (lambda scales with it).
+        HC_TRY(g->pinned.ensure(64));
+        double *hacc = g->pinned.as<double>();
+        double *dacc = reinterpret_cast<double *>(spare);  // scratch until the solve ends
+        HC_CUDA_TRY(cudaMemsetAsync(dacc, 0, sizeof(double), g->stream));
+        { sum_abs<<<g->sm_count * 4, 256, 0, g->stream>>>(cvec, g->N, dacc); ::hc::count_launch(); }
+        HC_CUDA_TRY(cudaMemcpyAsync(hacc, dacc, sizeof(double), cudaMemcpyDeviceToHost, g->stream));
+        HC_CUDA_TRY(cudaStreamSynchronize(g->stream));
+        a.tol_l1 = (float)(o.tol_l1 * *hacc);
+        HC_TRY(run_solve(g, a, plan, fn, lam, nullptr, &r, sym ? o.damping : 0.f));
         lfin = lam[r.iters & 1];
     }
     HC_CUDA_TRY(cudaEventRecord(g->ev_start, g->stream));
@@ -1577,14 +1668,12 @@ extern "C" hc_status hc_ppr_batched(hc_graph *g, const int32_t *seed_offsets, co
         sa.ps = ps;
         sa.partials = partials;
         sa.hub_count = hub_count;
-        sa.st = reinterpret_cast<IterState *>(g->ws_ctl.ptr);
         sa.tol_l1 = o.tol_l1;
         sa.eps = 3.4e38f;
         sa.max_iters = o.max_iters - it;
+        sa.n = g->N;
         sa.n_active = g->n_active;
-        SweepFn fn = pick_sweep(weighted, false, !weighted, true);
-        HC_TRY(g->ws_ctl.ensure(sizeof(IterState) + 4096));
-        sa.st = reinterpret_cast<IterState *>(g->ws_ctl.ptr);
+        SolveFn fn = pick_solve(weighted, false, !weighted, true);
         bool all_conv = true;
         for (int c = 0; c < kw; c++) {
             const int oc = hmap[c];
@@ -1598,7 +1687,7 @@ extern "C" hc_status hc_ppr_batched(hc_graph *g, const int32_t *seed_offsets, co
             }
             HC_CUDA_TRY(cudaGetLastError());
             SolveResult r;
-            HC_TRY(run_solve(g, sa, plan, fn, col_x, col_g, !weighted, &r));
+            HC_TRY(run_solve(g, sa, plan, fn, col_x, weighted ? nullptr : col_g, &r));
             { spmm_put_column<<<g->sm_count * 4, 256, 0, g->stream>>>(g->N, col_x[r.iters & 1], K, oc, out); ::hc::count_launch(); }
             HC_CUDA_TRY(cudaGetLastError());
             tail_iters = std::max(tail_iters, r.iters);

@@ -69,3 +69,27 @@ def test_columns(k, weighted):
     want = fixed_point(index, nbr, np.ones(len(nbr)) if w is None else w.astype(np.float64), t)
     assert st.converged and np.abs(x[:, cols] - want).max() <= BOUND
     g.close()
+
+
+@pytest.mark.parametrize("kind,scale", [("uniform", 20), ("kronecker", 18), ("kronecker", 8), ("uniform", 6)])
+def test_single_column_against_two(kind, scale):
+    """The single-column solve (one launch, or a launch per sweep on a large graph without hubs) against the
+    multi-column sweeps: each stops within TOL * d / (1 - d) of the fixed point in L1, and fp32 rounding adds at
+    most 100 sweeps of 2^-23 of the total."""
+    import torch
+
+    import hc
+    g = hc.Graph.generate(hc.GEN_UNIFORM if kind == "uniform" else hc.GEN_KRONECKER, scale, 16, 1)
+    n = g.num_nodes
+    t = torch.full((n, 2), 1.0 / n, device="cuda")
+    two = torch.empty((n, 2), device="cuda")
+    g.pagerank(t, two, tol_l1=TOL, max_iters=100)
+    for accel in (0, 1):
+        one = torch.empty(n, device="cuda")
+        _, st = g.pagerank(None, one, tol_l1=TOL, max_iters=100, accel=accel)
+        host, _ = g.pagerank(None, tol_l1=TOL, max_iters=100, accel=accel)
+        assert st.converged and np.abs(one.cpu().numpy() - host).sum() <= 1e-4 * TOL + 100 * 2.0 ** -23
+        assert (one - two[:, 0]).abs().double().sum().item() <= 2 * TOL * DAMPING / (1 - DAMPING) + 100 * 2.0 ** -23
+    capped, st = g.pagerank(None, tol_l1=TOL, max_iters=2)
+    assert st.iterations == 2 and not st.converged
+    g.close()
