@@ -486,7 +486,7 @@ hc_status ensure_pr_derived(hc_graph *g, bool weighted) {
 
 int64_t hc_graph::bytes_held() const {
     const hc::DevBuf *bufs[] = {&index, &nbr, &wgt, &inv_deg, &inv_wsum, &wtn, &wf32, &pr_plan,
-                                &pr_plan_huge_rows, &spmm_plan, &sssp_plan, &pr_ord, &ws_bfs, &ws_sssp, &ws_pr, &ws_batch,
+                                &pr_plan_huge_rows, &spmm_plan, &base_plan, &pr_ord, &ws_bfs, &ws_sssp, &ws_pr, &ws_batch,
                                 &ws_out0, &ws_out1, &ws_ctl, &ws_plan_ms, &ws_plan_mssp, &ws_src, &sssp_adj};
     int64_t t = 0;
     for (auto *b : bufs) t += (int64_t)b->bytes;
@@ -643,7 +643,7 @@ hc_status hc_graph_destroy(hc_graph *g) {
     if (g->own_stream) cudaStreamSynchronize(g->own_stream);
     if (g->stream && g->stream != g->own_stream) cudaStreamSynchronize(g->stream);
     DevBuf *bufs[] = {&g->index, &g->nbr, &g->wgt, &g->inv_deg, &g->inv_wsum, &g->wtn, &g->wf32, &g->pr_plan,
-                      &g->pr_plan_huge_rows, &g->spmm_plan, &g->sssp_plan, &g->ws_bfs, &g->ws_sssp, &g->ws_pr, &g->ws_batch,
+                      &g->pr_plan_huge_rows, &g->spmm_plan, &g->base_plan, &g->ws_bfs, &g->ws_sssp, &g->ws_pr, &g->ws_batch,
                       &g->ws_out0, &g->ws_out1, &g->ws_ctl, &g->ws_plan_ms, &g->ws_plan_mssp, &g->ws_src,
                       &g->sssp_adj, &g->pr_ord};
     for (auto *b : bufs) b->release();

@@ -4,8 +4,8 @@
 #include "hc_device.cuh"
 
 namespace hc {
-// Row plan of the PageRank sweeps, and another of the SSSP pull sweep, built
-// once per graph from the offsets of the rows with edges:
+// Row plans of the PageRank sweeps and the SSSP pull sweep, built once per graph
+// from the offsets of the rows with edges:
 //   stream groups  32 consecutive rows, one warp
 //   long rows      one warp per row
 //   hub rows       more than two chunks of edges, cut into tasks of one chunk
@@ -15,7 +15,10 @@ namespace hc {
 // a task ends with a fence and a counter and a warp per short row wastes lanes.
 //   chunk          M / 4096 edges rounded down to a power of two, in [256, 2048]
 //   stream group   at most M / 8192 edges, rounded likewise, in [256, 2048]
-//                  (the SSSP pull, a lane per row, always 2048)
+// The SSSP pull (a lane per row) and the adjoint's conjugate gradients use the
+// plan of 2048 edges at every size.  The gradient of a weight is a difference of
+// two nearly equal numbers, so another order of the sums in the solve would show
+// in its last digits.
 constexpr int kMinChunk = 256;
 constexpr int kMaxChunk = 2048;
 // Batched SSSP keeps 16-bit distances when no weight exceeds this.
@@ -85,8 +88,9 @@ struct hc_graph {
     hc::DevBuf pr_plan;        // row plan (device arrays)
     hc::PrPlanDev pr_view{};   // host copy of its pointers and counts
     int32_t pr_partial_slots = 0;
-    hc::DevBuf sssp_plan;      // the SSSP pull's row plan
-    hc::PrPlanDev sssp_view{};
+    hc::DevBuf base_plan;      // the plan of 2048 edges (SSSP pull, adjoint)
+    hc::PrPlanDev base_view{};
+    int32_t base_partial_slots = 0;
     hc::DevBuf pr_plan_huge_rows;
     hc::DevBuf spmm_plan;          // multi-column row plan (device arrays)
     hc::SpmmPlanDev spmm_view{};
@@ -191,10 +195,10 @@ hc_status edge_symmetry(hc_graph *g, const uint32_t *wbits, bool *structure, boo
 // The edge weights as fp32 for weighted PageRank: the weight array itself
 // (fp32 graphs) or its converted copy (int32 graphs, built by ensure_pr_derived).
 const float *pr_weights(const hc_graph *g);
-// Builds the PageRank row plan (g->pr_view, g->pr_partial_slots) or the SSSP
-// pull's (g->sssp_view) if missing.
+// Builds the PageRank row plan (g->pr_view, g->pr_partial_slots) or the plan of
+// 2048 edges (g->base_view, g->base_partial_slots) if missing.
 hc_status ensure_plan(hc_graph *g);
-hc_status ensure_sssp_plan(hc_graph *g);
+hc_status ensure_base_plan(hc_graph *g);
 // Computes w_negative, w_max, w_mean and w_symmetric once (int32 weights).
 hc_status ensure_weight_stats(hc_graph *g);
 // Per-run control traffic kept off the copy engines.  A host-output call

@@ -819,10 +819,9 @@ hc_status ensure_plan(hc_graph *g) {
     return build_plan(g, plan_size(g->M, 8192), plan_size(g->M, 4096), &g->pr_plan, &g->pr_view, &g->pr_partial_slots);
 }
 
-hc_status ensure_sssp_plan(hc_graph *g) {
-    if (g->sssp_plan.ptr) return HC_OK;
-    int32_t slots = 0;  // the pull keeps no partial sums
-    return build_plan(g, kMaxChunk, plan_size(g->M, 4096), &g->sssp_plan, &g->sssp_view, &slots);
+hc_status ensure_base_plan(hc_graph *g) {
+    if (g->base_plan.ptr) return HC_OK;
+    return build_plan(g, kMaxChunk, kMaxChunk, &g->base_plan, &g->base_view, &g->base_partial_slots);
 }
 
 // The multi-column sweeps' row plan, built on the first such call.  A chunk is M
@@ -899,18 +898,19 @@ PrPlanDev plan_view(hc_graph *g, int *partial_slots) {
 }
 
 // A cooperative launch of `fn` over the row plan's items: no more blocks than a
-// warp each needs (a barrier costs by the block), all that fit otherwise.
-hc_status launch_solve(hc_graph *g, const void *fn, int *blocks_per_sm, SweepArgs &a, const PrPlanDev &plan,
-                       int64_t vector_items, void *extra) {
+// warp each needs (a barrier costs by the block), or all that fit (`all`).
+hc_status launch_solve(hc_graph *g, const void *fn, int *blocks_per_sm, SweepArgs &a, const PrPlanDev &plan, bool all,
+                       void *extra) {
     if (*blocks_per_sm == 0) {
         int b = 0;
         HC_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fn, kPrThreads, 0));
         if (b < 1) return fail(HC_ERR_CUDA, "PageRank kernel cannot be resident");
         *blocks_per_sm = b;
     }
-    const int64_t warps = std::max<int64_t>((int64_t)plan.n_tasks + plan.n_long + plan.n_stream, vector_items / 32);
+    const int64_t warps = (int64_t)plan.n_tasks + plan.n_long + plan.n_stream;
     const int64_t want = std::max<int64_t>(1, (warps + kPrThreads / 32 - 1) / (kPrThreads / 32));
-    const int grid = (int)std::min<int64_t>(want, (int64_t)*blocks_per_sm * g->sm_count);
+    const int64_t fit = (int64_t)*blocks_per_sm * g->sm_count;
+    const int grid = (int)(all ? fit : std::min(want, fit));
     PrPlanDev p = plan;
     void *params[] = {&a, &p, extra};
     ::hc::count_launch();
@@ -963,7 +963,7 @@ hc_status launch_pr_solve(hc_graph *g, SweepArgs &a, const PrPlanDev &plan, vola
         return HC_OK;
     }
     static int bps = 0;
-    return launch_solve(g, (const void *)pr_solve<kEW, kRS, kPS, kBaseVec>, &bps, a, plan, 0, nullptr);
+    return launch_solve(g, (const void *)pr_solve<kEW, kRS, kPS, kBaseVec>, &bps, a, plan, false, nullptr);
 }
 
 SolveFn pick_solve(bool ew, bool rs, bool ps, bool basev) {
@@ -1146,7 +1146,9 @@ __global__ void __launch_bounds__(kPrThreads, kPrBlocks) pr_cg(SweepArgs a, PrPl
 template <bool kEW>
 hc_status launch_cg(hc_graph *g, SweepArgs &a, const PrPlanDev &plan, CgArgs &q) {
     static int bps = 0;
-    return launch_solve(g, (const void *)pr_cg<kEW>, &bps, a, plan, a.n, &q);
+    // Each thread sums its rows' share of p . q, so the grid is part of the
+    // rounding: one size for every graph (see the row plans).
+    return launch_solve(g, (const void *)pr_cg<kEW>, &bps, a, plan, true, &q);
 }
 
 // Solves the adjoint into lam (which holds the start) with the row plan's
@@ -1376,9 +1378,9 @@ extern "C" hc_status hc_pr_backward(hc_graph *g, const float *scores, const floa
     if (stats) std::memset(stats, 0, sizeof(*stats));
     const bool weighted = o.weighted != 0;
     HC_TRY(ensure_pr_derived(g, weighted));
-    HC_TRY(ensure_plan(g));
-    int partial_slots = 0;
-    PrPlanDev plan = plan_view(g, &partial_slots);
+    HC_TRY(ensure_base_plan(g));
+    const int partial_slots = g->base_partial_slots;
+    const PrPlanDev plan = g->base_view;
     const int64_t n = g->N;
     // cvec, lam[2], xs, spare and the three vectors of the CG solve.
     const size_t bytes = 8 * (size_t)n * 4 + (size_t)(partial_slots + 1) * 4 + (size_t)(plan.n_hub + 1) * 4 + 8192;

@@ -1352,7 +1352,7 @@ extern "C" hc_status hc_sssp(hc_graph *g, const int32_t *sources, int32_t num_so
     // Weights must be non-negative; the mean weight sets the default delta.
     HC_TRY(ensure_weight_stats(g));
     if (g->w_negative) return fail(HC_ERR_INVALID_ARG, "hc_sssp: negative edge weight");
-    HC_TRY(ensure_sssp_plan(g));
+    HC_TRY(ensure_base_plan(g));
 
     const int64_t n = g->N;
     const int64_t W = (n + 31) / 32;
@@ -1418,7 +1418,7 @@ extern "C" hc_status hc_sssp(hc_graph *g, const int32_t *sources, int32_t num_so
     a.fold = fold;
     a.team = team;
     a.team_stride = bytes;
-    a.plan = g->sssp_view;
+    a.plan = g->base_view;
     a.max_epochs = o.max_epochs > 0 ? o.max_epochs : 0x7fffffff;
     // The pull sweep reads w(u->v) from v's row: only valid when weights are symmetric.
     // Zero fields: the handle's tuned values, else the defaults.
