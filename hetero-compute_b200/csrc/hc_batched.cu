@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(kMsThreads) msbfs_hub(const int64_t *index, co
 // tasks of kMsPushChunk edges; each edge ORs the source's frontier words, minus
 // the target's seen words, into an accumulator x[v] and queues v once per
 // level; a finalize pass applies x to seen / next / depth and clears it.
-constexpr int kMsPushChunk = 2048;
+constexpr int kMsPushChunk = 128;  // a chunk is its warp's serial chain of 32-edge steps
 
 __global__ void msbfs_push_tasks(const int64_t *index, const uint32_t *act, int32_t n_active, int2 *tasks,
                                  MsCtl *ctl) {

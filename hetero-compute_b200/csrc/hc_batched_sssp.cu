@@ -11,7 +11,7 @@
 // dropped last epoch) and a queue of active vertices drive the epochs: every
 // edge out of the queue is relaxed for the active lanes, a warp keeping four
 // edges in flight (row loads, then atomic minimums, then the activity updates
-// of the four targets).  Rows longer than kLongRow are cut into chunks
+// of the four targets).  Rows longer than kPushChunk are cut into chunks
 // processed by a second launch.  While the queue covers a large part of the
 // graph (and weights are symmetric) an epoch is a pull instead: a warp per row
 // takes the minimum over its active neighbours and writes the row once, so
@@ -31,7 +31,13 @@
 namespace hc {
 namespace {
 
-constexpr int kLongRow = 2048;
+// Longer rows are cut into chunks of this many edges, a warp each: a warp has at
+// most four edges in flight, so a chunk is a serial chain of its length (a push
+// of 384k edges took 1.8 ms when rows of up to 2048 edges went to one warp).
+// Pushes cut finer: their step is a row load and an atomic round trip, and
+// their chunks share nothing but the queue; a pull's chunks merge by atomics.
+constexpr int kPushChunk = 128;
+constexpr int kPullChunk = 512;
 // An epoch is a pull when the edges out of its queue, times kPullAlpha, exceed
 // M: a pull reads every row of the distance matrix once, a push only the rows
 // its queue's edges reach.
@@ -78,6 +84,13 @@ struct WideDist {
     __device__ static W cand(W du, W w) { return sum(du, w); }
     __device__ static bool lowers(W nd, W d) { return nd < d; }
     __device__ static void atomic_lower(W *p, W nd, W) { atomicMin(p, nd); }
+    // Lowers the marked words of a row to their candidates du[s] + w (seen: d[s]).
+    template <int SPL>
+    __device__ static void lower_row(W *p, const bool (&low)[SPL], const W (&du)[SPL], W w, const W (&)[SPL]) {
+#pragma unroll
+        for (int s = 0; s < SPL; s++)
+            if (low[s]) atomicMin(p + s, cand(du[s], w));
+    }
     __device__ static W lower_of(W a, W b) { return min(a, b); }
     __device__ static void note(W &, W) {}
 };
@@ -102,6 +115,19 @@ struct NarrowDist {
             if (prev == old) return;
             old = prev;
         }
+    }
+    // Lowers the marked words of a row to their candidates du[s] + w (seen: d[s]):
+    // the first swap of every word is in flight before any is looked at, and
+    // the few that found another value go on by themselves.
+    template <int SPL>
+    __device__ static void lower_row(W *p, const bool (&low)[SPL], const W (&du)[SPL], W w, const W (&d)[SPL]) {
+        W prev[SPL];
+#pragma unroll
+        for (int s = 0; s < SPL; s++)
+            prev[s] = low[s] ? atomicCAS(p + s, d[s], __vminu2(d[s], cand(du[s], w))) : d[s];
+#pragma unroll
+        for (int s = 0; s < SPL; s++)
+            if (prev[s] != d[s]) atomic_lower(p + s, cand(du[s], w), prev[s]);
     }
     __device__ static W lower_of(W a, W b) { return __vminu2(a, b); }
     // Running per-halfword maximum of the finite values written.
@@ -272,22 +298,22 @@ __device__ __forceinline__ void relax_range(const int64_t *index, const int32_t 
                     for (int s = 0; s < SPL; s++) d[k][s] = D::kInfWord;
                 }
             }
-            // The update is a fire-and-forget atomic minimum; the target is
-            // marked active whenever the loaded value was larger, which covers
-            // every real improvement (values only fall between the load and
-            // the atomic) at the price of an occasional redundant rescan.
+            // The target is marked active whenever the loaded value was larger,
+            // which covers every real improvement (values only fall between the
+            // load and the atomic) at the price of an occasional redundant
+            // rescan.
 #pragma unroll
             for (int k = 0; k < F; k++) {
                 imp[k] = false;
+                bool low[SPL];
 #pragma unroll
                 for (int s = 0; s < SPL; s++) {
                     const W nd = D::cand(du[s], wt[k]);
-                    if (ok[k] && D::lowers(nd, d[k][s])) {
-                        D::atomic_lower(dist + (size_t)v[k] * KW + lane * SPL + s, nd, d[k][s]);
-                        D::note(wmax, D::lower_of(nd, d[k][s]));  // only the halves that fell
-                        imp[k] = true;
-                    }
+                    low[s] = ok[k] && D::lowers(nd, d[k][s]);
+                    if (low[s]) D::note(wmax, D::lower_of(nd, d[k][s]));  // only the halves that fell
+                    imp[k] |= low[s];
                 }
+                if (imp[k]) D::template lower_row<SPL>(dist + (size_t)v[k] * KW + lane * SPL, low, du, wt[k], d[k]);
             }
             unsigned mybal = 0u;  // lane k < F: target k's new activity bits
             int32_t myv = 0;
@@ -335,9 +361,9 @@ __global__ void __launch_bounds__(256) mssp_epoch(const int64_t *index, const in
         const int32_t u = qcur[qi];
         const uint32_t m = act_cur[u];
         const int64_t b = index[u], e = index[u + 1];
-        if (e - b > kLongRow) {
+        if (e - b > kPushChunk) {
             if (lane == 0) {
-                const int nc = (int)((e - b + kLongRow - 1) / kLongRow);
+                const int nc = (int)((e - b + kPushChunk - 1) / kPushChunk);
                 const int t0 = atomicAdd(ntasks, nc);
                 for (int c = 0; c < nc; c++) tasks[t0 + c] = make_int2(u, c);
             }
@@ -373,8 +399,8 @@ __global__ void __launch_bounds__(256) mssp_tasks(const int64_t *index, const in
         const int32_t u = tk.x;
         const uint32_t m = act_cur[u];
         const int64_t rb = index[u], re = index[u + 1];
-        const int64_t b = rb + (int64_t)tk.y * kLongRow;
-        const int64_t e = (re < b + kLongRow) ? re : b + kLongRow;
+        const int64_t b = rb + (int64_t)tk.y * kPushChunk;
+        const int64_t e = (re < b + kPushChunk) ? re : b + kPushChunk;
         typename D::W du[SPL];
         load_words<SPL>(dist + (size_t)u * 32 * SPL + lane * SPL, du);
         relax_range<D, SPL>(index, nbr, w, dist, m, du, b, e, act_next, qnext, qnext_len, rel, qe, wmax);
@@ -388,8 +414,8 @@ __global__ void __launch_bounds__(256) mssp_tasks(const int64_t *index, const in
 
 // Pull epoch, used while the queue covers a large part of the graph (weights
 // symmetric, so w(u->v) is read from v's row).  Items [row_begin, row_end)
-// are rows of at most kLongRow edges, one warp each, the only writer of that
-// row; the items after them are kLongRow-edge chunks of the longer rows, which
+// are rows of at most kPullChunk edges, one warp each, the only writer of that
+// row; the items after them are kPullChunk-edge chunks of the longer rows, which
 // merge with atomic minimums.  A warp takes the minimum over the neighbours
 // whose activity mask has its lane's bit, four neighbours in flight, and
 // writes the row and its activity mask once.
@@ -425,14 +451,14 @@ __global__ void __launch_bounds__(256) mssp_pull(const int64_t *index, const int
             v = row_begin + (int32_t)it;
             b = index[v];
             e = index[v + 1];
-            if (e == b || e - b > kLongRow) continue;
+            if (e == b || e - b > kPullChunk) continue;
             chunk = false;
         } else {
             const int2 tk = tasks[it - n_rows];
             v = tk.x;
             const int64_t re = index[v + 1];
-            b = index[v] + (int64_t)tk.y * kLongRow;
-            e = (re < b + kLongRow) ? re : b + kLongRow;
+            b = index[v] + (int64_t)tk.y * kPullChunk;
+            e = (re < b + kPullChunk) ? re : b + kPullChunk;
             chunk = true;
         }
         W *row = dist + (size_t)v * KW + lane * SPL;
@@ -537,12 +563,12 @@ __global__ void mssp_compact(const int64_t *index, const uint32_t *act, int32_t 
     if (lane == 0 && qe) atomicAdd(&ctl->qedges[c ^ 1], qe);
 }
 
-// (row, chunk) tasks for the rows longer than kLongRow.
+// (row, chunk) tasks for the rows longer than kPullChunk.
 __global__ void mssp_plan(const int64_t *index, int32_t n, int2 *tasks, int *ntasks) {
     for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
         const int64_t deg = index[v + 1] - index[v];
-        if (deg <= kLongRow) continue;
-        const int nc = (int)((deg + kLongRow - 1) / kLongRow);
+        if (deg <= kPullChunk) continue;
+        const int nc = (int)((deg + kPullChunk - 1) / kPullChunk);
         const int t0 = atomicAdd(ntasks, nc);
         for (int c = 0; c < nc; c++) tasks[t0 + c] = make_int2((int32_t)v, c);
     }
@@ -550,7 +576,7 @@ __global__ void mssp_plan(const int64_t *index, int32_t n, int2 *tasks, int *nta
 
 hc_status ensure_pull_plan(hc_graph *g) {
     if (g->mssp_tasks >= 0) return HC_OK;
-    const int64_t max_tasks = 2 * (g->M / kLongRow) + 1;
+    const int64_t max_tasks = 2 * (g->M / kPullChunk) + 1;
     HC_TRY(g->ws_plan_mssp.ensure(sizeof(int2) * max_tasks + 256));
     int *cnt = reinterpret_cast<int *>(g->ws_plan_mssp.as<char>() + sizeof(int2) * max_tasks);
     HC_CUDA_TRY(cudaMemsetAsync(cnt, 0, 4, g->stream));
@@ -705,7 +731,7 @@ hc_status run_group(hc_graph *g, const int32_t *h_src, int k, int32_t *dst, int 
     constexpr int KW = 32 * SPL;
     constexpr int K = KW * D::kPer;
     const int64_t n = g->N;
-    const int64_t max_tasks = 2 * (g->M / kLongRow) + n / kLongRow + 64;
+    const int64_t max_tasks = 2 * (g->M / kPushChunk) + 64;  // sum over rows longer than a chunk
     HC_TRY(g->ws_batch.ensure((size_t)n * KW * 4 + (size_t)n * 4 * 4 + sizeof(int2) * max_tasks + 8192));
     char *p = g->ws_batch.as<char>();
     auto take = [&](size_t bytes) {
