@@ -21,6 +21,7 @@
 // group.
 #include <algorithm>
 #include <chrono>
+#include <climits>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -93,6 +94,13 @@ struct WideDist {
     }
     __device__ static W lower_of(W a, W b) { return min(a, b); }
     __device__ static void note(W &, W) {}
+    // The value x where it is below d, else unreachable.
+    __device__ static W fell(W x, W d) { return x < d ? x : kInfWord; }
+    __device__ static int32_t half(W x, int) { return x; }
+    __device__ static W pack(const int32_t *p) { return __ldca(p); }
+    static constexpr int32_t kInfHalf = kInfDist;
+    // The largest best - low over the word's distances (0 where low is larger).
+    __device__ static int32_t gap(W best, W low) { return max(best - low, 0); }
 };
 
 struct NarrowDist {
@@ -130,6 +138,17 @@ struct NarrowDist {
             if (prev[s] != d[s]) atomic_lower(p + s, cand(du[s], w), prev[s]);
     }
     __device__ static W lower_of(W a, W b) { return __vminu2(a, b); }
+    __device__ static W fell(W x, W d) { return x | ~__vcmpltu2(x, d); }
+    __device__ static int32_t half(W x, int h) { return (int32_t)((x >> (16 * h)) & 0xFFFFu); }
+    __device__ static W pack(const int32_t *p) {
+        const int2 x = __ldca(reinterpret_cast<const int2 *>(p));
+        return (W)x.x | ((W)x.y << 16);
+    }
+    static constexpr int32_t kInfHalf = (int32_t)kInf16;
+    __device__ static int32_t gap(W best, W low) {
+        const W g = __vsubus2(best, low);
+        return (int32_t)max(g & 0xFFFFu, g >> 16);
+    }
     // Running per-halfword maximum of the finite values written.
     __device__ static void note(W &mx, W x) { mx = __vmaxu2(mx, x & __vcmpltu2(x, kInfWord)); }
 };
@@ -171,6 +190,38 @@ __device__ __forceinline__ void note_flush(MsspCtl *ctl, typename D::W mx) {
     }
 }
 
+// Smallest distance that each source wrote in an epoch, an int32 per source so
+// that a minimum needs no compare-and-swap.  Every thread of the block calls
+// this at the end of a kernel with its warp's minima in `my`: they meet in
+// shared memory, and one warp passes on those below the current value.
+template <class D, int SPL>
+__device__ __forceinline__ void low_flush(int32_t *lows, const typename D::W (&my)[SPL]) {
+    __shared__ typename D::W s_low[8][32 * SPL];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+#pragma unroll
+    for (int s = 0; s < SPL; s++) s_low[wib][lane + 32 * s] = my[s];
+    __syncthreads();
+    for (int i = threadIdx.x; i < 32 * SPL; i += blockDim.x) {
+        typename D::W m = s_low[0][i];
+#pragma unroll
+        for (int w = 1; w < 8; w++) m = D::lower_of(m, s_low[w][i]);
+        int32_t *p = lows + ((i & 31) * SPL + (i >> 5)) * D::kPer;
+#pragma unroll
+        for (int h = 0; h < D::kPer; h++) {
+            const int32_t x = D::half(m, h);
+            if (x < __ldcg(p + h)) atomicMin(p + h, x);
+        }
+    }
+}
+
+// A lane's SPL words of those minima.
+template <class D, int SPL>
+__device__ __forceinline__ void load_lows(const int32_t *lows, typename D::W (&low)[SPL]) {
+    const int32_t *p = lows + (threadIdx.x & 31) * SPL * D::kPer;
+#pragma unroll
+    for (int s = 0; s < SPL; s++) low[s] = D::pack(p + s * D::kPer);
+}
+
 // A lane's SPL distance words of one vertex.  kL1: through L1 (neighbour
 // rows, which many warps of an SM read: most edges point at a few thousand hub
 // rows); a value cached earlier in the same launch may be stale, but
@@ -207,7 +258,12 @@ __device__ __forceinline__ void load_words(const W *p, W (&d)[SPL]) {
 }
 
 template <class D, int SPL>
-__global__ void mssp_init(int32_t n, typename D::W *dist, uint32_t *act0, uint32_t *act1) {
+__global__ void mssp_init(int32_t n, typename D::W *dist, uint32_t *act0, uint32_t *act1, int32_t *lows0, int32_t *lows1) {
+    if (blockIdx.x == 0)
+        for (int i = threadIdx.x; i < 32 * SPL * D::kPer; i += blockDim.x) {
+            lows0[i] = 0;  // the seeds
+            lows1[i] = D::kInfHalf;
+        }
     const size_t total = (size_t)n * 32 * SPL;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x)
         dist[i] = D::kInfWord;
@@ -264,7 +320,7 @@ __device__ __forceinline__ void relax_range(const int64_t *index, const int32_t 
                                             typename D::W *dist, uint32_t m, const typename D::W (&du)[SPL],
                                             int64_t e0, int64_t e1, uint32_t *act_next, int32_t *qnext, int *qlen,
                                             unsigned long long &relaxed, unsigned long long &qe,
-                                            typename D::W &wmax) {
+                                            typename D::W &wmax, typename D::W (&mylow)[SPL]) {
     using W = typename D::W;
     constexpr int KW = 32 * SPL;
     const int lane = threadIdx.x & 31;
@@ -310,7 +366,10 @@ __device__ __forceinline__ void relax_range(const int64_t *index, const int32_t 
                 for (int s = 0; s < SPL; s++) {
                     const W nd = D::cand(du[s], wt[k]);
                     low[s] = ok[k] && D::lowers(nd, d[k][s]);
-                    if (low[s]) D::note(wmax, D::lower_of(nd, d[k][s]));  // only the halves that fell
+                    if (low[s]) {
+                        D::note(wmax, D::lower_of(nd, d[k][s]));  // only the halves that fell
+                        mylow[s] = D::lower_of(mylow[s], D::fell(nd, d[k][s]));
+                    }
                     imp[k] |= low[s];
                 }
                 if (imp[k]) D::template lower_row<SPL>(dist + (size_t)v[k] * KW + lane * SPL, low, du, wt[k], d[k]);
@@ -347,7 +406,7 @@ template <class D, int SPL>
 __global__ void __launch_bounds__(256) mssp_epoch(const int64_t *index, const int32_t *nbr, const int32_t *w,
                                                   typename D::W *dist, const int32_t *qcur, const uint32_t *act_cur,
                                                   uint32_t *act_next, int32_t *qnext, int2 *tasks, MsspCtl *ctl, int c,
-                                                  unsigned long long *relaxed) {
+                                                  unsigned long long *relaxed, int32_t *lows_next) {
     const int nq = ctl_queue(ctl, c);
     if (nq == 0 || ctl_pull(ctl, c)) return;
     int *qnext_len = &ctl->qlen[c ^ 1];
@@ -356,7 +415,9 @@ __global__ void __launch_bounds__(256) mssp_epoch(const int64_t *index, const in
     const int gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
     unsigned long long rel = 0, qe = 0;
-    typename D::W wmax = 0;
+    typename D::W wmax = 0, mylow[SPL];
+#pragma unroll
+    for (int s = 0; s < SPL; s++) mylow[s] = D::kInfWord;
     for (int qi = gwarp; qi < nq; qi += nwarps) {
         const int32_t u = qcur[qi];
         const uint32_t m = act_cur[u];
@@ -371,9 +432,10 @@ __global__ void __launch_bounds__(256) mssp_epoch(const int64_t *index, const in
         }
         typename D::W du[SPL];
         load_words<SPL>(dist + (size_t)u * 32 * SPL + lane * SPL, du);
-        relax_range<D, SPL>(index, nbr, w, dist, m, du, b, e, act_next, qnext, qnext_len, rel, qe, wmax);
+        relax_range<D, SPL>(index, nbr, w, dist, m, du, b, e, act_next, qnext, qnext_len, rel, qe, wmax, mylow);
     }
     note_flush<D>(ctl, wmax);
+    low_flush<D, SPL>(lows_next, mylow);
     rel = warp_sum(rel);
     qe = warp_sum(qe);
     if (lane == 0 && rel) atomicAdd(relaxed, rel);
@@ -384,7 +446,7 @@ template <class D, int SPL>
 __global__ void __launch_bounds__(256) mssp_tasks(const int64_t *index, const int32_t *nbr, const int32_t *w,
                                                   typename D::W *dist, const int2 *tasks, const uint32_t *act_cur,
                                                   uint32_t *act_next, int32_t *qnext, MsspCtl *ctl, int c,
-                                                  unsigned long long *relaxed) {
+                                                  unsigned long long *relaxed, int32_t *lows_next) {
     const int nq = ctl_queue(ctl, c);
     if (nq == 0 || ctl_pull(ctl, c)) return;
     int *qnext_len = &ctl->qlen[c ^ 1];
@@ -393,7 +455,9 @@ __global__ void __launch_bounds__(256) mssp_tasks(const int64_t *index, const in
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
     const int nt = ctl->ntasks;
     unsigned long long rel = 0, qe = 0;
-    typename D::W wmax = 0;
+    typename D::W wmax = 0, mylow[SPL];
+#pragma unroll
+    for (int s = 0; s < SPL; s++) mylow[s] = D::kInfWord;
     for (int t = gwarp; t < nt; t += nwarps) {
         const int2 tk = tasks[t];
         const int32_t u = tk.x;
@@ -403,9 +467,10 @@ __global__ void __launch_bounds__(256) mssp_tasks(const int64_t *index, const in
         const int64_t e = (re < b + kPushChunk) ? re : b + kPushChunk;
         typename D::W du[SPL];
         load_words<SPL>(dist + (size_t)u * 32 * SPL + lane * SPL, du);
-        relax_range<D, SPL>(index, nbr, w, dist, m, du, b, e, act_next, qnext, qnext_len, rel, qe, wmax);
+        relax_range<D, SPL>(index, nbr, w, dist, m, du, b, e, act_next, qnext, qnext_len, rel, qe, wmax, mylow);
     }
     note_flush<D>(ctl, wmax);
+    low_flush<D, SPL>(lows_next, mylow);
     rel = warp_sum(rel);
     qe = warp_sum(qe);
     if (lane == 0 && rel) atomicAdd(relaxed, rel);
@@ -419,6 +484,10 @@ __global__ void __launch_bounds__(256) mssp_tasks(const int64_t *index, const in
 // merge with atomic minimums.  A warp takes the minimum over the neighbours
 // whose activity mask has its lane's bit, four neighbours in flight, and
 // writes the row and its activity mask once.
+// A distance that has not been relaxed along its edges yet was written in the
+// last epoch or is written in this one, so it is at least the smallest one that
+// its source wrote in the last epoch (`lows`); an edge as heavy as the row's
+// widest gap to those, over its sources, can lower nothing and is passed over.
 //
 // An epoch runs in two launches on degree-sorted graphs: the hub prefix (the
 // rows holding half the edges, and the long-row chunks) first, then the other
@@ -431,7 +500,8 @@ __global__ void __launch_bounds__(256) mssp_pull(const int64_t *index, const int
                                                  typename D::W *dist, int32_t row_begin, int32_t row_end,
                                                  const int2 *tasks, int ntasks, const uint32_t *act_cur,
                                                  uint32_t *act_next, int fresh, MsspCtl *ctl, int c,
-                                                 unsigned long long *relaxed) {
+                                                 unsigned long long *relaxed, const int32_t *lows,
+                                                 int32_t *lows_next) {
     using W = typename D::W;
     const int nq = ctl_queue(ctl, c);
     if (nq == 0 || !ctl_pull(ctl, c)) return;
@@ -440,7 +510,9 @@ __global__ void __launch_bounds__(256) mssp_pull(const int64_t *index, const int
     const int gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
     unsigned long long rel = 0;
-    W wmax = 0;
+    W wmax = 0, mylow[SPL];
+#pragma unroll
+    for (int s = 0; s < SPL; s++) mylow[s] = D::kInfWord;
     const int32_t n_rows = row_end - row_begin;
     const int64_t total = (int64_t)n_rows + ntasks;
     for (int64_t it = gwarp; it < total; it += nwarps) {
@@ -466,13 +538,26 @@ __global__ void __launch_bounds__(256) mssp_pull(const int64_t *index, const int
         load_words<SPL>(row, dv);
 #pragma unroll
         for (int s = 0; s < SPL; s++) best[s] = dv[s];
+        // Edges are loaded one step ahead, so that neither the row's distances
+        // nor the gap delays them.
+        int32_t next_u = b + lane < e ? __ldg(nbr + b + lane) : 0, next_w = b + lane < e ? __ldg(w + b + lane) : INT32_MAX;
         for (int64_t base = b; base < e; base += 32) {
-            const int64_t my = base + lane;
-            int32_t uu = 0, ww = 0;
+            const int32_t uu = next_u, ww = next_w;
+            const int64_t ahead = base + 32 + lane;
+            next_u = ahead < e ? __ldg(nbr + ahead) : 0;
+            next_w = ahead < e ? __ldg(w + ahead) : INT32_MAX;
+            // The widest gap of the row's sources to what they can still receive.
+            int32_t gap = 0;
+            {
+                W low[SPL];
+                load_lows<D, SPL>(lows, low);
+#pragma unroll
+                for (int s = 0; s < SPL; s++) gap = max(gap, D::gap(best[s], low[s]));
+                gap = __reduce_max_sync(kFull, gap);
+            }
+            if (gap == 0) break;
             uint32_t aa = 0;
-            if (my < e) {
-                uu = nbr[my];
-                ww = w[my];
+            if (ww < gap) {  // INT32_MAX past the range's end: no gap is larger
                 aa = __ldcg(act_cur + uu);
                 // A hub row (below row_begin) may have changed earlier in this epoch.
                 if (fresh && uu < row_begin) aa |= __ldcg(act_next + uu);
@@ -517,7 +602,10 @@ __global__ void __launch_bounds__(256) mssp_pull(const int64_t *index, const int
         const unsigned bal = __ballot_sync(kFull, imp);
         if (!bal) continue;
 #pragma unroll
-        for (int s = 0; s < SPL; s++) D::note(wmax, best[s]);
+        for (int s = 0; s < SPL; s++) {
+            D::note(wmax, best[s]);
+            mylow[s] = D::lower_of(mylow[s], D::fell(best[s], dv[s]));
+        }
         if (chunk) {
 #pragma unroll
             for (int s = 0; s < SPL; s++)
@@ -532,6 +620,7 @@ __global__ void __launch_bounds__(256) mssp_pull(const int64_t *index, const int
         }
     }
     note_flush<D>(ctl, wmax);
+    low_flush<D, SPL>(lows_next, mylow);
     rel = warp_sum(rel);
     if (lane == 0 && rel) atomicAdd(relaxed, rel);
 }
@@ -609,11 +698,13 @@ __global__ void mssp_clear(const int32_t *q, uint32_t *act, const MsspCtl *ctl, 
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nq; i += gridDim.x * blockDim.x) act[q[i]] = 0;
 }
 
-// Closes epoch parity c: counts it, resets its counters for reuse, and decides
+// Closes epoch parity c (one block): clears the minima it read, counts it, resets its counters for reuse, and decides
 // whether another epoch runs (queue non-empty, under the epoch cap and the
 // time bound, and for narrow words inside the 16-bit range); inside a graph
 // it sets the while node's condition.
-__global__ void mssp_end(MsspCtl *ctl, int c, cudaGraphConditionalHandle cond, int use_cond) {
+__global__ void mssp_end(MsspCtl *ctl, int c, int32_t *lows, int count, int32_t inf,
+                         cudaGraphConditionalHandle cond, int use_cond) {
+    for (int i = threadIdx.x; i < count; i += blockDim.x) lows[i] = inf;  // the next epoch's to write
     if (blockIdx.x != 0 || threadIdx.x != 0) return;
     bool go = false;
     if (!ctl->stop && ctl->qlen[c] > 0) {
@@ -688,6 +779,7 @@ __global__ void mssp_transpose(const typename D::W *dist, int32_t n, int nsrc, i
 template <class D>
 struct MsspBufs {
     typename D::W *dist;
+    int32_t *lows[2];  // smallest distance each source wrote: epoch parity c reads lows[c], writes lows[c ^ 1]
     uint32_t *act[2];
     int32_t *q[2];
     int2 *tasks;
@@ -705,19 +797,20 @@ void launch_epoch(const hc_graph *g, cudaStream_t st, const MsspBufs<D> &b, int 
     const int64_t *index = g->index.as<int64_t>();
     const int32_t *nbr = g->nbr.as<int32_t>(), *w = g->wgt.as<int32_t>();
     mssp_epoch<D, SPL><<<grid, 256, 0, st>>>(index, nbr, w, b.dist, b.q[c], b.act[c], b.act[c ^ 1], b.q[c ^ 1],
-                                             b.tasks, b.ctl, c, relaxed);
+                                             b.tasks, b.ctl, c, relaxed, b.lows[c ^ 1]);
     mssp_tasks<D, SPL><<<grid, 256, 0, st>>>(index, nbr, w, b.dist, b.tasks, b.act[c], b.act[c ^ 1], b.q[c ^ 1],
-                                             b.ctl, c, relaxed);
+                                             b.ctl, c, relaxed, b.lows[c ^ 1]);
     const int32_t hub = g->mssp_hub_rows > 0 ? g->mssp_hub_rows : g->n_active;
     mssp_pull<D, SPL><<<grid, 256, 0, st>>>(index, nbr, w, b.dist, 0, hub, g->ws_plan_mssp.as<int2>(),
                                             g->mssp_tasks < 0 ? 0 : g->mssp_tasks, b.act[c], b.act[c ^ 1], 0, b.ctl,
-                                            c, relaxed);
+                                            c, relaxed, b.lows[c], b.lows[c ^ 1]);
     if (hub < g->n_active)
         mssp_pull<D, SPL><<<grid, 256, 0, st>>>(index, nbr, w, b.dist, hub, g->n_active, nullptr, 0, b.act[c],
-                                                b.act[c ^ 1], 1, b.ctl, c, relaxed);
+                                                b.act[c ^ 1], 1, b.ctl, c, relaxed, b.lows[c], b.lows[c ^ 1]);
     mssp_clear<<<grid, 256, 0, st>>>(b.q[c], b.act[c], b.ctl, c);
     mssp_compact<<<grid, 256, 0, st>>>(index, b.act[c ^ 1], g->N, b.q[c ^ 1], b.ctl, c);
-    mssp_end<<<1, 32, 0, st>>>(b.ctl, c, cond, use_cond);
+    mssp_end<<<1, 128, 0, st>>>(b.ctl, c, b.lows[c], 32 * SPL * D::kPer, D::kInfHalf, cond,
+                                use_cond);
 }
 constexpr int kEpochLaunches = 7;
 
@@ -732,7 +825,8 @@ hc_status run_group(hc_graph *g, const int32_t *h_src, int k, int32_t *dst, int 
     constexpr int K = KW * D::kPer;
     const int64_t n = g->N;
     const int64_t max_tasks = 2 * (g->M / kPushChunk) + 64;  // sum over rows longer than a chunk
-    HC_TRY(g->ws_batch.ensure((size_t)n * KW * 4 + (size_t)n * 4 * 4 + sizeof(int2) * max_tasks + 8192));
+    HC_TRY(g->ws_batch.ensure((size_t)n * KW * 4 + (size_t)n * 4 * 4 + sizeof(int2) * max_tasks +
+                              2 * (size_t)K * 4 + 8192));
     char *p = g->ws_batch.as<char>();
     auto take = [&](size_t bytes) {
         char *r = p;
@@ -747,12 +841,14 @@ hc_status run_group(hc_graph *g, const int32_t *h_src, int k, int32_t *dst, int 
     b.q[1] = (int32_t *)take((size_t)n * 4);
     b.tasks = (int2 *)take(sizeof(int2) * max_tasks);
     b.ctl = (MsspCtl *)take(sizeof(MsspCtl));
+    b.lows[0] = (int32_t *)take((size_t)K * 4);
+    b.lows[1] = (int32_t *)take((size_t)K * 4);
     b.src = (int32_t *)take(sizeof(int32_t) * K);
     const int grid = g->sm_count * 8;
     HC_TRY(g->pinned.ensure(2 * sizeof(MsspCtl) + 64));
     MsspCtl *hctl = g->pinned.as<MsspCtl>();
     HC_CUDA_TRY(cudaMemcpyAsync(b.src, h_src, sizeof(int32_t) * k, cudaMemcpyHostToDevice, g->stream));
-    { mssp_init<D, SPL><<<grid, 256, 0, g->stream>>>(g->N, b.dist, b.act[0], b.act[1]); ::hc::count_launch(); }
+    { mssp_init<D, SPL><<<grid, 256, 0, g->stream>>>(g->N, b.dist, b.act[0], b.act[1], b.lows[0], b.lows[1]); ::hc::count_launch(); }
     {
         mssp_seed<D, SPL><<<1, 32, 0, g->stream>>>(k, b.src, g->index.as<int64_t>(), b.dist, b.act[0], b.q[0], b.ctl,
                                                    pull_alpha, (long long)g->M, max_epochs, g->w_max);

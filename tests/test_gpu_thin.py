@@ -166,3 +166,30 @@ def test_sssp_sources_at_a_time(scale, count, out):
             v = np.flatnonzero((dist[i] != hc.INF_DIST) & (np.arange(n) != picks[i]))
             assert p[picks[i]] == picks[i] and (p[v] >= 0).all() and (dist[i][p[v]] < dist[i][v]).all()
     g.close()
+
+
+@pytest.mark.parametrize("bits", [0, 32])
+@pytest.mark.parametrize("top", [1, 255, 3000])
+@pytest.mark.parametrize("name", ["path_3000", "fan_600", "star_129", "star_300", "mixed"])
+def test_sssp_batched_gaps(name, top, bits):
+    """Batched pulls pass over edges heavier than a row's widest gap: zero weights, heavy ones, unreached rows."""
+    import hc
+    if name == "mixed":
+        k = hc.gen_kronecker(11, 16, 5)
+        index, nbr = shuffled(k.index, k.neighbors, 1)
+    else:
+        index, nbr = GRAPHS[name]()
+    w = weights(index, nbr, top)
+    n = len(index) - 1
+    g = hc.Graph(index, nbr, w)
+    sources = np.random.default_rng(top).integers(0, n, 70).astype(np.int32)
+    for alpha in (0, -1, 1 << 20):  # default switch, pushes only, pulls wherever edges are queued
+        for use_graph in (hc.GRAPH_AUTO, hc.GRAPH_ON, hc.GRAPH_OFF):
+            dist, _ = g.sssp_batched(sources, switch_alpha=alpha, dist_bits=bits, use_graph=use_graph)
+            for i in (0, 33, 69):
+                assert np.array_equal(dist[i], oracle.sssp_dijkstra(index, nbr, w, sources[i])), (alpha, use_graph)
+    for use_graph in (hc.GRAPH_AUTO, hc.GRAPH_ON, hc.GRAPH_OFF):
+        depth, _ = g.bfs_batched(sources, use_graph=use_graph)
+        for i in (0, 33, 69):
+            assert np.array_equal(depth[i], oracle.bfs_depth(index, nbr, sources[i])), use_graph
+    g.close()
