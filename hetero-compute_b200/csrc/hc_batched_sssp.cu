@@ -37,8 +37,16 @@ namespace {
 // of 384k edges took 1.8 ms when rows of up to 2048 edges went to one warp).
 // Pushes cut finer: their step is a row load and an atomic round trip, and
 // their chunks share nothing but the queue; a pull's chunks merge by atomics.
+// On a small graph, whose epoch is little more than its longest chain, they are
+// cut finer: M / 4096 edges rounded down to a power of two, in [64, 512] (scale
+// 12, 64 sources: 1.20 -> 1.12 ms a call).
 constexpr int kPushChunk = 128;
 constexpr int kPullChunk = 512;
+inline int pull_chunk(int64_t m) {
+    int c = 64;
+    while (c < kPullChunk && (int64_t)c * 2 * 4096 <= m) c *= 2;
+    return c;
+}
 // An epoch is a pull when the edges out of its queue, times kPullAlpha, exceed
 // M: a pull reads every row of the distance matrix once, a push only the rows
 // its queue's edges reach.
@@ -479,8 +487,8 @@ __global__ void __launch_bounds__(256) mssp_tasks(const int64_t *index, const in
 
 // Pull epoch, used while the queue covers a large part of the graph (weights
 // symmetric, so w(u->v) is read from v's row).  Items [row_begin, row_end)
-// are rows of at most kPullChunk edges, one warp each, the only writer of that
-// row; the items after them are kPullChunk-edge chunks of the longer rows, which
+// are rows of at most one chunk of edges, one warp each, the only writer of that
+// row; the items after them are chunks of the longer rows, which
 // merge with atomic minimums.  A warp takes the minimum over the neighbours
 // whose activity mask has its lane's bit, four neighbours in flight, and
 // writes the row and its activity mask once.
@@ -498,7 +506,7 @@ __global__ void __launch_bounds__(256) mssp_tasks(const int64_t *index, const in
 template <class D, int SPL>
 __global__ void __launch_bounds__(256) mssp_pull(const int64_t *index, const int32_t *nbr, const int32_t *w,
                                                  typename D::W *dist, int32_t row_begin, int32_t row_end,
-                                                 const int2 *tasks, int ntasks, const uint32_t *act_cur,
+                                                 const int2 *tasks, int ntasks, int pull_chunk, const uint32_t *act_cur,
                                                  uint32_t *act_next, int fresh, MsspCtl *ctl, int c,
                                                  unsigned long long *relaxed, const int32_t *lows,
                                                  int32_t *lows_next) {
@@ -523,14 +531,14 @@ __global__ void __launch_bounds__(256) mssp_pull(const int64_t *index, const int
             v = row_begin + (int32_t)it;
             b = index[v];
             e = index[v + 1];
-            if (e == b || e - b > kPullChunk) continue;
+            if (e == b || e - b > pull_chunk) continue;
             chunk = false;
         } else {
             const int2 tk = tasks[it - n_rows];
             v = tk.x;
             const int64_t re = index[v + 1];
-            b = index[v] + (int64_t)tk.y * kPullChunk;
-            e = (re < b + kPullChunk) ? re : b + kPullChunk;
+            b = index[v] + (int64_t)tk.y * pull_chunk;
+            e = (re < b + pull_chunk) ? re : b + pull_chunk;
             chunk = true;
         }
         W *row = dist + (size_t)v * KW + lane * SPL;
@@ -652,12 +660,12 @@ __global__ void mssp_compact(const int64_t *index, const uint32_t *act, int32_t 
     if (lane == 0 && qe) atomicAdd(&ctl->qedges[c ^ 1], qe);
 }
 
-// (row, chunk) tasks for the rows longer than kPullChunk.
-__global__ void mssp_plan(const int64_t *index, int32_t n, int2 *tasks, int *ntasks) {
+// (row, chunk) tasks for the rows longer than one chunk.
+__global__ void mssp_plan(const int64_t *index, int32_t n, int2 *tasks, int *ntasks, int chunk) {
     for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
         const int64_t deg = index[v + 1] - index[v];
-        if (deg <= kPullChunk) continue;
-        const int nc = (int)((deg + kPullChunk - 1) / kPullChunk);
+        if (deg <= chunk) continue;
+        const int nc = (int)((deg + chunk - 1) / chunk);
         const int t0 = atomicAdd(ntasks, nc);
         for (int c = 0; c < nc; c++) tasks[t0 + c] = make_int2((int32_t)v, c);
     }
@@ -665,11 +673,12 @@ __global__ void mssp_plan(const int64_t *index, int32_t n, int2 *tasks, int *nta
 
 hc_status ensure_pull_plan(hc_graph *g) {
     if (g->mssp_tasks >= 0) return HC_OK;
-    const int64_t max_tasks = 2 * (g->M / kPullChunk) + 1;
+    const int chunk = pull_chunk(g->M);
+    const int64_t max_tasks = 2 * (g->M / chunk) + 1;
     HC_TRY(g->ws_plan_mssp.ensure(sizeof(int2) * max_tasks + 256));
     int *cnt = reinterpret_cast<int *>(g->ws_plan_mssp.as<char>() + sizeof(int2) * max_tasks);
     HC_CUDA_TRY(cudaMemsetAsync(cnt, 0, 4, g->stream));
-    { mssp_plan<<<g->sm_count * 8, 256, 0, g->stream>>>(g->index.as<int64_t>(), g->N, g->ws_plan_mssp.as<int2>(), cnt); ::hc::count_launch(); }
+    { mssp_plan<<<g->sm_count * 8, 256, 0, g->stream>>>(g->index.as<int64_t>(), g->N, g->ws_plan_mssp.as<int2>(), cnt, chunk); ::hc::count_launch(); }
     HC_CUDA_TRY(cudaGetLastError());
     int h = 0;
     HC_CUDA_TRY(cudaMemcpyAsync(&h, cnt, 4, cudaMemcpyDeviceToHost, g->stream));
@@ -802,10 +811,10 @@ void launch_epoch(const hc_graph *g, cudaStream_t st, const MsspBufs<D> &b, int 
                                              b.ctl, c, relaxed, b.lows[c ^ 1]);
     const int32_t hub = g->mssp_hub_rows > 0 ? g->mssp_hub_rows : g->n_active;
     mssp_pull<D, SPL><<<grid, 256, 0, st>>>(index, nbr, w, b.dist, 0, hub, g->ws_plan_mssp.as<int2>(),
-                                            g->mssp_tasks < 0 ? 0 : g->mssp_tasks, b.act[c], b.act[c ^ 1], 0, b.ctl,
+                                            g->mssp_tasks < 0 ? 0 : g->mssp_tasks, pull_chunk(g->M), b.act[c], b.act[c ^ 1], 0, b.ctl,
                                             c, relaxed, b.lows[c], b.lows[c ^ 1]);
     if (hub < g->n_active)
-        mssp_pull<D, SPL><<<grid, 256, 0, st>>>(index, nbr, w, b.dist, hub, g->n_active, nullptr, 0, b.act[c],
+        mssp_pull<D, SPL><<<grid, 256, 0, st>>>(index, nbr, w, b.dist, hub, g->n_active, nullptr, 0, pull_chunk(g->M), b.act[c],
                                                 b.act[c ^ 1], 1, b.ctl, c, relaxed, b.lows[c], b.lows[c ^ 1]);
     mssp_clear<<<grid, 256, 0, st>>>(b.q[c], b.act[c], b.ctl, c);
     mssp_compact<<<grid, 256, 0, st>>>(index, b.act[c ^ 1], g->N, b.q[c ^ 1], b.ctl, c);
@@ -819,7 +828,7 @@ constexpr int kEpochLaunches = 7;
 // dst then holds no valid result.
 template <class D, int SPL>
 hc_status run_group(hc_graph *g, const int32_t *h_src, int k, int32_t *dst, int max_epochs, int pull_alpha,
-                    bool use_graph, WhileGraph &eg, int *epochs_out, unsigned long long *relaxed, bool *fits) {
+                    int use_graph, WhileGraph &eg, int *epochs_out, unsigned long long *relaxed, bool *fits) {
     using W = typename D::W;
     constexpr int KW = 32 * SPL;
     constexpr int K = KW * D::kPer;
@@ -856,9 +865,26 @@ hc_status run_group(hc_graph *g, const int32_t *h_src, int k, int32_t *dst, int 
     }
     HC_CUDA_TRY(cudaGetLastError());
     const bool trace = std::getenv("HC_TRACE") != nullptr;
-    if (use_graph && !trace) {
+    // As the batched BFS's loop: plain launches in rounds first, a graph when
+    // kLaunchEpochs epochs have not ended it.
+    constexpr int kLaunchRound = 4, kLaunchEpochs = 40;
+    bool ended = false;
+    if (use_graph != HC_GRAPH_ON && use_graph != HC_GRAPH_OFF && !trace && !eg.exec) {
+        for (int ep = 0; !ended && ep < kLaunchEpochs; ep += kLaunchRound) {
+            for (int k = 0; k < kLaunchRound; k++) launch_epoch<D, SPL>(g, g->stream, b, k & 1, relaxed, 0, 0);
+            ::hc::count_launch(kLaunchRound * kEpochLaunches);
+            HC_CUDA_TRY(cudaGetLastError());
+            HC_CUDA_TRY(cudaMemcpyAsync(hctl, b.ctl, sizeof(MsspCtl), cudaMemcpyDeviceToHost, g->stream));
+            HC_CUDA_TRY(cudaStreamSynchronize(g->stream));
+            // An epoch that ends with an empty queue leaves both queues empty.
+            ended = hctl->stop || (hctl->qlen[0] == 0 && hctl->qlen[1] == 0);
+        }
+    }
+    if (ended) {
+    } else if (use_graph != HC_GRAPH_OFF && !trace) {
         // The graph's body is two epochs (parity 0 then 1); kernels of an
         // epoch whose queue is empty return at once.
+        const int before = use_graph == HC_GRAPH_ON || eg.exec ? 0 : hctl->epochs;
         if (!eg.exec) {
             auto body = [&](cudaStream_t cs, cudaGraphConditionalHandle cond) {
                 launch_epoch<D, SPL>(g, cs, b, 0, relaxed, cond, 1);
@@ -869,7 +895,7 @@ hc_status run_group(hc_graph *g, const int32_t *h_src, int k, int32_t *dst, int 
         HC_CUDA_TRY(cudaGraphLaunch(eg.exec, g->stream));
         HC_CUDA_TRY(cudaMemcpyAsync(hctl, b.ctl, sizeof(MsspCtl), cudaMemcpyDeviceToHost, g->stream));
         HC_CUDA_TRY(cudaStreamSynchronize(g->stream));
-        ::hc::count_launch(2 * kEpochLaunches * ((hctl->epochs + 1) / 2));
+        ::hc::count_launch(2 * kEpochLaunches * ((hctl->epochs - before + 1) / 2));
     } else {
         for (int ep = 0;; ep++) {
             const auto t0 = std::chrono::steady_clock::now();
@@ -926,7 +952,7 @@ hc_status run_group(hc_graph *g, const int32_t *h_src, int k, int32_t *dst, int 
 // sources).
 template <class D>
 hc_status run_group_spl(int spl, hc_graph *g, const int32_t *h_src, int k, int32_t *dst, int max_epochs,
-                        int pull_alpha, bool use_graph, WhileGraph &eg, int *ep, unsigned long long *relaxed,
+                        int pull_alpha, int use_graph, WhileGraph &eg, int *ep, unsigned long long *relaxed,
                         bool *fits) {
     switch (spl) {
         case 1: return run_group<D, 1>(g, h_src, k, dst, max_epochs, pull_alpha, use_graph, eg, ep, relaxed, fits);
@@ -998,8 +1024,7 @@ extern "C" hc_status hc_sssp_batched(hc_graph *g, const int32_t *sources, int32_
     HC_CUDA_TRY(cudaMemsetAsync(relaxed, 0, 8, g->stream));
     HC_CUDA_TRY(cudaEventRecord(g->ev_start, g->stream));
     int epochs_max = 0, groups = 0, wide_groups = 0, reruns = 0;
-    // The epoch loop runs as a CUDA graph unless use_graph asks otherwise.
-    const bool use_graph = o.use_graph != HC_GRAPH_OFF;
+    const int use_graph = o.use_graph;
     // Built by the first group of each kind, reused by the others.  Once a
     // group has been rerun with 32-bit words, the rest of the call stays
     // 32-bit (their workspace differs), at most 256 sources per group.
