@@ -1033,6 +1033,12 @@ hc_status run_solve(hc_graph *g, SweepArgs a, const PrPlanDev &plan, SolveFn fn,
 // residual c + d A^T lambda - lambda, so the stopping rule is the same as the
 // sweeps'.  Rows without weight (s = 0) keep lambda = c.  Vectors are fp32,
 // dot products fp64; alpha, beta and the stop decision stay on the device.
+// From this many edges on an iteration's phases are launches of their own: the
+// vector passes then run with as many threads as suit them and the sweep without
+// the loop around it (adjoint solve, Kronecker scale 20: 2.66 ms so, 3.09 ms in one
+// launch; scale 18: 1.18 and 1.00 ms).
+constexpr int64_t kCgLaunchEdges = 1ll << 23;
+
 struct CgArgs {
     const float *c;
     float *lam, *r, *p, *sp;
@@ -1055,6 +1061,50 @@ __device__ __forceinline__ void add_dots(IterSlot *slot, double rz, double z1) {
     }
 }
 
+// This thread's share of the vector passes.
+// r = s (c - lambda) + d S lambda, z = r / s, p = z.
+__device__ __forceinline__ void cg_start_rows(const SweepArgs &a, const CgArgs &q, int gtid, int nthreads, double &rz,
+                                              double &z1, double &c1) {
+    for (int v = gtid; v < a.n; v += nthreads) {
+        const float sv = row_weight(a.rs, v);
+        c1 += fabs((double)q.c[v]);
+        if (sv == 0.f) {
+            q.lam[v] = q.c[v];
+            q.r[v] = 0.f;
+            q.p[v] = 0.f;
+            continue;
+        }
+        const float rv = sv * (q.c[v] - q.lam[v]) + a.d * q.sp[v];
+        const float zv = rv * a.rs[v];
+        q.r[v] = rv;
+        q.p[v] = zv;
+        rz += (double)rv * zv;
+        z1 += fabs((double)zv);
+    }
+}
+// lambda += alpha p, r -= alpha q.
+__device__ __forceinline__ void cg_update_rows(const SweepArgs &a, const CgArgs &q, int gtid, int nthreads, float alpha,
+                                               double &rz, double &z1) {
+    for (int v = gtid; v < a.n; v += nthreads) {
+        const float pv = q.p[v];
+        const float qv = row_weight(a.rs, v) * pv - a.d * q.sp[v];
+        q.lam[v] += alpha * pv;
+        const float rv = q.r[v] - alpha * qv;
+        q.r[v] = rv;
+        const float zv = rv * a.rs[v];
+        rz += (double)rv * zv;
+        z1 += fabs((double)zv);
+    }
+}
+// p = z + beta p.
+__device__ __forceinline__ void cg_direction_rows(const SweepArgs &a, const CgArgs &q, int gtid, int nthreads,
+                                                  float beta) {
+    for (int v = gtid; v < a.n; v += nthreads) q.p[v] = q.r[v] * a.rs[v] + beta * q.p[v];
+}
+__device__ __forceinline__ double cg_tol(const SweepArgs &a, const CgArgs &q) {
+    return (double)(float)(q.rel_tol * __ldcg(&a.st->slot[0].l1));
+}
+
 // The whole solve in one cooperative launch, a grid barrier after each sweep and
 // each vector pass (three an iteration).
 template <bool kEW>
@@ -1071,23 +1121,7 @@ __global__ void __launch_bounds__(kPrThreads, kPrBlocks) pr_cg(SweepArgs a, PrPl
     sweep_rows<kEW, false, false, false, true>(a, plan, SweepIter{q.lam, q.lam, q.sp, q.sp, 1.f}, s_acc, l1, chg);
     bool ok = grid_barrier(gs);
     if (ok) {
-        // r = s (c - lambda) + d S lambda, z = r / s, p = z.
-        for (int v = gtid; v < a.n; v += nthreads) {
-            const float sv = row_weight(a.rs, v);
-            c1 += fabs((double)q.c[v]);
-            if (sv == 0.f) {
-                q.lam[v] = q.c[v];
-                q.r[v] = 0.f;
-                q.p[v] = 0.f;
-                continue;
-            }
-            const float rv = sv * (q.c[v] - q.lam[v]) + a.d * q.sp[v];
-            const float zv = rv * a.rs[v];
-            q.r[v] = rv;
-            q.p[v] = zv;
-            rz += (double)rv * zv;
-            z1 += fabs((double)zv);
-        }
+        cg_start_rows(a, q, gtid, nthreads, rz, z1, c1);
         add_dots(&a.st->slot[0], rz, z1);
         __syncthreads();
         c1 = block_sum(c1, s_c);
@@ -1097,7 +1131,7 @@ __global__ void __launch_bounds__(kPrThreads, kPrBlocks) pr_cg(SweepArgs a, PrPl
     if (ok) {
         rz = __ldcg(&a.st->slot[0].rz);
         z1 = __ldcg(&a.st->slot[0].z1);
-        tol = (double)(float)(q.rel_tol * __ldcg(&a.st->slot[0].l1));
+        tol = cg_tol(a, q);
         converged = z1 < tol || rz <= 0.0;
     }
     for (int it = 1; ok && !converged && it <= a.max_iters; it++) {
@@ -1107,19 +1141,8 @@ __global__ void __launch_bounds__(kPrThreads, kPrBlocks) pr_cg(SweepArgs a, PrPl
         if (!(ok = grid_barrier(gs))) break;
         const double pq = __ldcg(&slot->l1);
         if (!(pq > 0.0)) break;  // p = 0 (already exact) or a breakdown: stop
-        // lambda += alpha p, r -= alpha q.
-        const float alpha = (float)(rz / pq);
         double nrz = 0.0, nz1 = 0.0;
-        for (int v = gtid; v < a.n; v += nthreads) {
-            const float pv = q.p[v];
-            const float qv = row_weight(a.rs, v) * pv - a.d * q.sp[v];
-            q.lam[v] += alpha * pv;
-            const float rv = q.r[v] - alpha * qv;
-            q.r[v] = rv;
-            const float zv = rv * a.rs[v];
-            nrz += (double)rv * zv;
-            nz1 += fabs((double)zv);
-        }
+        cg_update_rows(a, q, gtid, nthreads, (float)(rz / pq), nrz, nz1);
         add_dots(slot, nrz, nz1);
         if (!(ok = grid_barrier(gs))) break;
         nrz = __ldcg(&slot->rz);
@@ -1129,8 +1152,7 @@ __global__ void __launch_bounds__(kPrThreads, kPrBlocks) pr_cg(SweepArgs a, PrPl
         iters++;
         converged = z1 < tol;
         if (converged || it == a.max_iters) break;
-        // p = z + beta p (the same thread's entries as above).
-        for (int v = gtid; v < a.n; v += nthreads) q.p[v] = q.r[v] * a.rs[v] + beta * q.p[v];
+        cg_direction_rows(a, q, gtid, nthreads, beta);  // the same thread's entries as above
         ok = grid_barrier(gs);
     }
     if (gtid == 0) {
@@ -1143,8 +1165,87 @@ __global__ void __launch_bounds__(kPrThreads, kPrBlocks) pr_cg(SweepArgs a, PrPl
     }
 }
 
+// The same phases as launches of their own (see run_cg).  Iteration it's sums are
+// in slot it; launches queued after the end return at once.
 template <bool kEW>
-hc_status launch_cg(hc_graph *g, SweepArgs &a, const PrPlanDev &plan, CgArgs &q) {
+__global__ void __launch_bounds__(kPrThreads, kPrBlocks) cg_sweep(SweepArgs a, PrPlanDev plan, CgArgs q, int it) {
+    __shared__ float s_acc[kPrThreads / 32][32];
+    if (*(volatile int *)&a.st->done) return;
+    float l1;
+    int chg;
+    const float *x = it == 0 ? q.lam : q.p;
+    sweep_rows<kEW, false, false, false, true>(a, plan, SweepIter{x, x, q.sp, q.sp, 1.f}, s_acc, l1, chg);
+    if (it > 0) add_residual(&a.st->slot[it], l1, 0);
+}
+__device__ __forceinline__ void cg_report(const SweepArgs &a, int iters, bool converged, double z1) {
+    a.st->done = 1;
+    a.out->iters = iters;
+    a.out->l1 = z1;
+    a.out->changed = 0;
+    a.out->done = converged ? 1 : 2;
+    __threadfence_system();
+}
+__global__ void cg_start(SweepArgs a, CgArgs q) {
+    __shared__ double s_c[32];
+    double rz = 0.0, z1 = 0.0, c1 = 0.0;
+    cg_start_rows(a, q, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, rz, z1, c1);
+    add_dots(&a.st->slot[0], rz, z1);
+    __syncthreads();
+    c1 = block_sum(c1, s_c);
+    if (threadIdx.x == 0 && c1 != 0.0) atomicAdd(&a.st->slot[0].l1, c1);
+}
+__global__ void cg_update(SweepArgs a, CgArgs q, int it) {
+    if (*(volatile int *)&a.st->done) return;
+    const double rz = __ldcg(&a.st->slot[it - 1].rz), pq = __ldcg(&a.st->slot[it].l1);
+    if (!(pq > 0.0)) return;  // cg_direction stops
+    double nrz = 0.0, nz1 = 0.0;
+    cg_update_rows(a, q, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, (float)(rz / pq), nrz, nz1);
+    add_dots(&a.st->slot[it], nrz, nz1);
+}
+// it 0: only the test after the start.
+__global__ void cg_direction(SweepArgs a, CgArgs q, int it) {
+    if (*(volatile int *)&a.st->done) return;
+    const bool first = blockIdx.x == 0 && threadIdx.x == 0;
+    const double nrz = __ldcg(&a.st->slot[it].rz), z1 = __ldcg(&a.st->slot[it].z1), tol = cg_tol(a, q);
+    if (it == 0) {
+        if (first && (z1 < tol || nrz <= 0.0)) cg_report(a, 0, true, z1);
+        return;
+    }
+    if (!(__ldcg(&a.st->slot[it].l1) > 0.0)) {  // p = 0 (already exact) or a breakdown
+        if (first) cg_report(a, it - 1, false, __ldcg(&a.st->slot[it - 1].z1));
+        return;
+    }
+    if (z1 < tol || it >= a.max_iters) {
+        if (first) cg_report(a, it, z1 < tol, z1);
+        return;
+    }
+    const double rz = __ldcg(&a.st->slot[it - 1].rz);
+    cg_direction_rows(a, q, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x,
+                      (float)(rz > 0.0 ? nrz / rz : 0.0));
+}
+
+template <bool kEW>
+hc_status launch_cg(hc_graph *g, SweepArgs &a, const PrPlanDev &plan, CgArgs &q, volatile SolveOut *out) {
+    if (g->M >= kCgLaunchEdges) {
+        const int grid = g->sm_count * 4, sweep_grid = g->sm_count * kPrBlocks;
+        auto sweep = [&](int it) { cg_sweep<kEW><<<sweep_grid, kPrThreads, 0, g->stream>>>(a, plan, q, it); ::hc::count_launch(); };
+        auto direction = [&](int it) { cg_direction<<<grid, kPrThreads, 0, g->stream>>>(a, q, it); ::hc::count_launch(); };
+        sweep(0);
+        { cg_start<<<grid, kPrThreads, 0, g->stream>>>(a, q); ::hc::count_launch(); }
+        direction(0);
+        // Launches are queued in rounds, the host looking once per round.
+        constexpr int kRound = 4;
+        for (int it = 1; it <= a.max_iters && !out->done;) {
+            for (int k = 0; k < kRound && it <= a.max_iters; k++, it++) {
+                sweep(it);
+                { cg_update<<<grid, kPrThreads, 0, g->stream>>>(a, q, it); ::hc::count_launch(); }
+                direction(it);
+            }
+            HC_CUDA_TRY(cudaGetLastError());
+            HC_CUDA_TRY(cudaStreamSynchronize(g->stream));
+        }
+        return HC_OK;
+    }
     static int bps = 0;
     // Each thread sums its rows' share of p . q, so the grid is part of the
     // rounding: one size for every graph (see the row plans).
@@ -1170,8 +1271,10 @@ hc_status run_cg(hc_graph *g, const PrPlanDev &plan, bool weighted, const float 
     a.n_active = g->n_active;
     SolveOut *out = nullptr;
     HC_TRY(solve_begin(g, a, &out));
-    HC_TRY(weighted ? launch_cg<true>(g, a, plan, q) : launch_cg<false>(g, a, plan, q));
-    return solve_end(g, out, res);
+    HC_TRY(weighted ? launch_cg<true>(g, a, plan, q, out) : launch_cg<false>(g, a, plan, q, out));
+    HC_TRY(solve_end(g, out, res));
+    res->done = res->done == 1;
+    return HC_OK;
 }
 
 void fill_opts(const hc_pr_opts *opts, hc_pr_opts *o) {

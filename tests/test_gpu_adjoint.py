@@ -166,3 +166,27 @@ def test_asymmetric_weights_fall_back_to_jacobi():
     dt, dw, _ = g.pagerank_backward(x, c.astype(np.float32), weighted=True, tol_l1=1e-9, max_iters=500)
     assert np.abs(dt - dt64).max() < 1e-5 * np.abs(dt64).max()
     assert np.abs(dw - dw64).max() < 1e-4 * np.abs(dw64).max()
+
+
+@pytest.mark.parametrize("scale", [17, 19])
+def test_adjoint_launch_forms(scale):
+    """The conjugate gradients in one launch (below 2^23 edges) and as launches: x is linear in the teleport, so
+    c . x = (dL/dt) . t up to both solves' stops (relative 1e-6) and fp32 rounding."""
+    import torch
+
+    import hc
+    g = hc.Graph.generate(hc.GEN_KRONECKER, scale, 16, 1, hc.W_F32)
+    n = g.num_nodes
+    assert (g.num_edges >= 1 << 23) == (scale == 19)
+    c = torch.from_numpy(np.random.default_rng(scale).standard_normal(n).astype(np.float32)).cuda()
+    x, dt = torch.empty(n, device="cuda"), torch.empty(n, device="cuda")
+    o = dict(tol_l1=1e-6, max_iters=200, weighted=True)
+    g.pagerank(None, x, **o)
+    _, _, st = g.pagerank_backward(x, c, dteleport=dt, want_dw=False, **o)
+    assert st.converged and 5 <= st.iterations <= 60
+    lhs, rhs = float((c.double() * x.double()).sum()), float(dt.double().sum() / n)
+    assert abs(lhs - rhs) <= 1e-4 * float((c.double() * x.double()).abs().sum())
+    again = torch.empty(n, device="cuda")
+    _, _, st = g.pagerank_backward(x, c, dteleport=again, want_dw=False, tol_l1=1e-6, max_iters=3, weighted=True)
+    assert st.iterations == 3 and not st.converged
+    g.close()
