@@ -325,7 +325,7 @@ def run_suite(a):
 
 def profile_case(a):
     """One source of BFS and SSSP, then one PageRank solve: the launches an ncu
-    capture of bfs_persistent / sssp_persistent / sssp_pull_kernel / pr_sweep
+    capture of bfs_persistent / sssp_persistent / pr_solve
     selects.  With --suite batched: one 512-source batched BFS, one 512-source
     batched SSSP group on 16-bit distances and one 256-source group on int32
     distances (device outputs).  Under a profiler that replays each captured
@@ -852,8 +852,8 @@ def main():
         except Exception:
             traffic = None
     roof = {"bound": "hbm", "kernel": {"bfs": "bfs_persistent",
-                                       "sssp": "sssp_persistent + sssp_pull_kernel",
-                                       "pagerank": "pr_sweep"}[dom],
+                                       "sssp": "sssp_persistent",
+                                       "pagerank": "pr_solve"}[dom],
             "achieved": achieved, "peak": hbm, "unit": "GB/s",
             "frac": achieved / hbm if achieved else None, "peak_kind": peak_kind, "traffic": traffic,
             "traffic_unit": "DRAM bytes per source (per solve for pagerank), one ncu capture "

@@ -86,13 +86,54 @@ __global__ void msbfs_seed(int nsrc, const int32_t *src, uint64_t *seen, uint64_
     }
 }
 
+// A vertex's K64 words by the widest accesses they allow: 32 bytes (rows of 4 and
+// 8 words are 32-byte aligned), 16 or 8.  The lanes of a warp gather unrelated
+// rows, so every access is a cycle of the L1 per lane, and eight-byte loads made
+// those the bound of a dense level (scale 20, 512 sources: a level of 31M edges
+// 0.89 ms).  kRead: not written by this kernel.
+template <int K64, bool kRead = true>
+__device__ __forceinline__ void load_row64(const uint64_t *p, uint64_t (&w)[K64]) {
+    if constexpr (K64 >= 4) {
+#pragma unroll
+        for (int j = 0; j < K64; j += 4) {
+            if constexpr (kRead)
+                asm("ld.global.nc.v4.u64 {%0, %1, %2, %3}, [%4];"
+                    : "=l"(w[j]), "=l"(w[j + 1]), "=l"(w[j + 2]), "=l"(w[j + 3]) : "l"(p + j));
+            else
+                asm volatile("ld.global.v4.u64 {%0, %1, %2, %3}, [%4];"
+                             : "=l"(w[j]), "=l"(w[j + 1]), "=l"(w[j + 2]), "=l"(w[j + 3]) : "l"(p + j) : "memory");
+        }
+    } else if constexpr (K64 == 2) {
+        const ulonglong2 x = kRead ? __ldg(reinterpret_cast<const ulonglong2 *>(p))
+                                   : *reinterpret_cast<const ulonglong2 *>(p);
+        w[0] = x.x;
+        w[1] = x.y;
+    } else {
+        w[0] = kRead ? __ldg(p) : *p;
+    }
+}
+template <int K64>
+__device__ __forceinline__ void store_row64(uint64_t *p, const uint64_t (&w)[K64]) {
+    if constexpr (K64 >= 4) {
+#pragma unroll
+        for (int j = 0; j < K64; j += 4)
+            asm volatile("st.global.v4.u64 [%0], {%1, %2, %3, %4};" ::"l"(p + j), "l"(w[j]), "l"(w[j + 1]),
+                         "l"(w[j + 2]), "l"(w[j + 3]) : "memory");
+    } else if constexpr (K64 == 2) {
+        *reinterpret_cast<ulonglong2 *>(p) = make_ulonglong2(w[0], w[1]);
+    } else {
+        *p = w[0];
+    }
+}
+
 // front words of source-active vertices are gathered only where act has the bit.
 template <int K64>
 __device__ __forceinline__ void or_front(const uint64_t *front, const uint32_t *act, int32_t u, uint64_t (&acc)[K64]) {
     if ((__ldg(act + (u >> 5)) >> (u & 31)) & 1u) {
-        const uint64_t *f = front + (size_t)u * K64;
+        uint64_t f[K64];
+        load_row64<K64>(front + (size_t)u * K64, f);
 #pragma unroll
-        for (int j = 0; j < K64; j++) acc[j] |= __ldg(f + j);
+        for (int j = 0; j < K64; j++) acc[j] |= f[j];
     }
 }
 
@@ -154,22 +195,19 @@ __global__ void __launch_bounds__(kMsThreads) msbfs_pull(const int64_t *index, c
         uint64_t nw[K64];
         bool any = false, full = true;
         if (work) {
-            uint64_t *sv = seen + (size_t)v * K64;
+            uint64_t s[K64];
+            load_row64<K64, false>(seen + (size_t)v * K64, s);
 #pragma unroll
             for (int j = 0; j < K64; j++) {
                 const uint64_t fm = full_mask<K64>(j, nsrc);
-                const uint64_t s = sv[j];
-                nw[j] = acc[j] & ~s & fm;
+                nw[j] = acc[j] & ~s[j] & fm;
                 any |= nw[j] != 0;
-                full &= ((s | nw[j]) & fm) == fm;
+                s[j] |= nw[j];
+                full &= (s[j] & fm) == fm;
             }
             if (any) {
-                uint64_t *fv = next + (size_t)v * K64;
-#pragma unroll
-                for (int j = 0; j < K64; j++) {
-                    sv[j] |= nw[j];
-                    fv[j] = nw[j];
-                }
+                store_row64<K64>(seen + (size_t)v * K64, s);
+                store_row64<K64>(next + (size_t)v * K64, nw);
             }
         } else {
 #pragma unroll
@@ -310,8 +348,7 @@ __global__ void __launch_bounds__(kMsThreads) msbfs_push(const int64_t *index, c
         const int2 tk = tasks[t];
         const int32_t u = tk.x;
         uint64_t fu[K64];
-#pragma unroll
-        for (int j = 0; j < K64; j++) fu[j] = __ldg(front + (size_t)u * K64 + j);
+        load_row64<K64>(front + (size_t)u * K64, fu);
         const int64_t rb = index[u], re = index[u + 1];
         const int64_t b = rb + (int64_t)tk.y * kMsPushChunk, e = min(re, b + (int64_t)kMsPushChunk);
         for (int64_t i0 = b; i0 < e; i0 += 32) {
@@ -320,11 +357,12 @@ __global__ void __launch_bounds__(kMsThreads) msbfs_push(const int64_t *index, c
             int32_t v = 0;
             if (i < e) {
                 v = nbr[i];
-                const uint64_t *sv = seen + (size_t)v * K64;
+                uint64_t s[K64];
+                load_row64<K64>(seen + (size_t)v * K64, s);
                 bool any = false;
 #pragma unroll
                 for (int j = 0; j < K64; j++) {
-                    const uint64_t nw = fu[j] & ~__ldcg(sv + j);
+                    const uint64_t nw = fu[j] & ~s[j];
                     if (nw) {
                         atomicOr((unsigned long long *)&xacc[(size_t)v * K64 + j], nw);
                         any = true;

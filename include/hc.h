@@ -176,7 +176,10 @@ typedef struct hc_bfs_stats {
     double ms;            /* device time, summed over sources */
 } hc_bfs_stats;
 
-/* BFS from each source in turn (one persistent launch per source).
+/* BFS from each source.  One persistent launch takes up to 256 sources and runs
+ * several at a time, each by a team of the GPU's blocks with a workspace of its
+ * own (at most 1 GB in all, and one at a time when that cannot be allocated or
+ * when statistics are collected).
  * depth_out / parent_out: [num_sources][num_nodes] int32, -1 = unreached;
  * parent[src] = src.  Either may be NULL.  Replaces bfs_gpu
  * (src/kernels/gpu/bfs.cuh:21-95), which is bottom-up only and returns
@@ -229,7 +232,8 @@ typedef struct hc_sssp_stats {
     double ms;
 } hc_sssp_stats;
 
-/* Single-source shortest paths over int32 weights (graph wtype HC_W_I32).
+/* Single-source shortest paths over int32 weights (graph wtype HC_W_I32), several
+ * sources at a time as hc_bfs (workspaces of at most 2 GB in all).
  * dist_out: [num_sources][num_nodes] int32, INT32_MAX = unreachable.
  * Distances are int32 and every candidate dist + w is clamped at INT32_MAX:
  * when a path of num_active - 1 edges of the largest weight could reach the
@@ -327,7 +331,7 @@ hc_status hc_ppr_batched(hc_graph *g, const int32_t *seed_offsets, const int32_t
 /* --------------------------------------------------------------- batched */
 
 /* hc_batch_opts.use_graph */
-#define HC_GRAPH_AUTO 0   /* the library's choice (a graph where the loop has one) */
+#define HC_GRAPH_AUTO 0   /* the library's choice: launches in rounds, a graph once the loop is long */
 #define HC_GRAPH_ON 1     /* run the epoch loop as a CUDA graph (while node) */
 #define HC_GRAPH_OFF 2    /* host loop: one launch sequence and one sync per epoch */
 
@@ -395,7 +399,7 @@ typedef struct hc_tuning {
      * (hc_equal_edge_ranges), 32-aligned. */
     int32_t bfs_bu_split[HC_BFS_SPLIT_LEVELS];
     int32_t bfs_bu_split_levels;
-    /* Blocks per SM of the persistent SSSP kernel (its push epochs): fewer
+    /* Blocks per SM of the persistent SSSP kernel: fewer
      * blocks make each grid barrier cheaper, more give large frontiers more
      * warps.  0 = as many as fit (2). */
     int32_t sssp_blocks_per_sm;
