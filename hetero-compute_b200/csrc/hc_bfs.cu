@@ -406,8 +406,15 @@ union BfsShared {
     SoloQueue solo[2];
 };
 
-template <bool kStats>
-__global__ void __launch_bounds__(kBfsThreads, 2) bfs_persistent(BfsArgs a) {
+// kBlocks resident blocks per SM: two, or three for many sources at a time.  The
+// levels wait on dependent loads (issue slots 32 % used, DRAM 14 %), and with
+// enough teams to fill them a third block's warps are worth the spills they cost
+// (64 sources, Kronecker scale 22: 7.2 -> 6.0 ms, scale 16: 216 -> 205 us; but one
+// source at scale 22 253 -> 261 us, 64 at scale 10 90 -> 98 us).
+constexpr int kBfsWideSources = 4;
+constexpr int64_t kBfsWideEdges = 1ll << 20;
+template <bool kStats, int kBlocks>
+__global__ void __launch_bounds__(kBfsThreads, kBlocks) bfs_persistent(BfsArgs a) {
     __shared__ unsigned long long s_red[32];
     __shared__ BfsShared sh;
     __shared__ int s_stop;
@@ -851,28 +858,29 @@ __global__ void bfs_clear(BfsCtl *ctl, int teams, BfsFold *f) {
 }
 
 // Blocks of bfs_persistent that are resident at a time.
-template <bool kStats>
+template <bool kStats, int kBlocks>
 hc_status bfs_resident(hc_graph *g, int *blocks) {
     static int blocks_per_sm = 0;
     if (blocks_per_sm == 0) {
-        HC_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, bfs_persistent<kStats>, kBfsThreads, 0));
+        HC_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, bfs_persistent<kStats, kBlocks>,
+                                                                  kBfsThreads, 0));
         if (blocks_per_sm < 1) return fail(HC_ERR_CUDA, "BFS kernel cannot be resident");
     }
     *blocks = blocks_per_sm * g->sm_count;
     return HC_OK;
 }
 
-template <bool kStats>
+template <bool kStats, int kBlocks>
 hc_status launch_bfs(hc_graph *g, BfsArgs &a, int teams) {
     dim3 grid(a.team * teams), block(kBfsThreads);
     ::hc::count_launch();
     if (a.team == 1) {  // no block waits for another
-        bfs_persistent<kStats><<<grid, block, 0, g->stream>>>(a);
+        bfs_persistent<kStats, kBlocks><<<grid, block, 0, g->stream>>>(a);
         HC_CUDA_TRY(cudaGetLastError());
         return HC_OK;
     }
     void *params[] = {&a};
-    HC_CUDA_TRY(cudaLaunchCooperativeKernel((void *)bfs_persistent<kStats>, grid, block, params, 0, g->stream));
+    HC_CUDA_TRY(cudaLaunchCooperativeKernel((void *)bfs_persistent<kStats, kBlocks>, grid, block, params, 0, g->stream));
     return HC_OK;
 }
 
@@ -890,7 +898,7 @@ void bfs_teams(const hc_graph *g, int resident, int k, int room, int *team, int 
     const double root = std::sqrt((double)std::max<int64_t>(g->M, 1));
     const int least = std::max(1, std::min(resident, (int)std::lround(root / 300.0)));
     const int most = std::max(1, std::min(resident, (int)std::lround(root / 19.0)));
-    const int at_a_time = std::max(1, std::min({k, room, resident / least}));
+    const int at_a_time = std::max(1, std::min({k, room, resident / least, kBfsLaunchSources}));
     const int rounds = (std::max(k, 1) + at_a_time - 1) / at_a_time;
     *teams = (std::max(k, 1) + rounds - 1) / rounds;
     *team = std::max(least, std::min(most, resident / *teams));
@@ -946,7 +954,10 @@ extern "C" hc_status hc_bfs(hc_graph *g, const int32_t *sources, int32_t num_sou
                up(sizeof(int2) * (size_t)ntasks);
     }();
     int resident = 0;
-    HC_TRY(o.collect_stats ? bfs_resident<true>(g, &resident) : bfs_resident<false>(g, &resident));
+    const bool wide = !per_run && num_sources >= kBfsWideSources && g->M >= kBfsWideEdges;
+    HC_TRY((o.collect_stats ? bfs_resident<true, 2>(g, &resident)
+            : wide          ? bfs_resident<false, 3>(g, &resident)
+                            : bfs_resident<false, 2>(g, &resident)));
     OutPipe pipe;
     int team = resident, teams = 1;
     const size_t fold_bytes = 256;
@@ -1043,7 +1054,8 @@ extern "C" hc_status hc_bfs(hc_graph *g, const int32_t *sources, int32_t num_sou
             if (staged) HC_TRY(pipe.acquire(l, stage));
             a.depth = dev_depth ? depth_out + (size_t)i * n : host_depth ? stage[0] : g->ws_out0.as<int32_t>();
             a.parent = dev_parent ? parent_out + (size_t)i * n : host_parent ? stage[1] : g->ws_out1.as<int32_t>();
-            HC_TRY(launch_bfs<false>(g, a, std::min(teams, a.nsrc)));
+            HC_TRY((wide ? launch_bfs<false, 3>(g, a, std::min(teams, a.nsrc))
+                         : launch_bfs<false, 2>(g, a, std::min(teams, a.nsrc))));
             if (staged) {
                 void *dst[2] = {host_depth ? (void *)(depth_out + (size_t)i * n) : nullptr,
                                 host_parent ? (void *)(parent_out + (size_t)i * n) : nullptr};
@@ -1076,7 +1088,7 @@ extern "C" hc_status hc_bfs(hc_graph *g, const int32_t *sources, int32_t num_sou
         a.parent = dev_parent ? parent_out + (size_t)i * n : host_parent ? stage[1] : g->ws_out1.as<int32_t>();
         { bfs_clear<<<1, 256, 0, g->stream>>>(a.ctl, 1, fold); ::hc::count_launch(); }
         HC_CUDA_TRY(cudaEventRecord(g->ev_start, g->stream));
-        HC_TRY(o.collect_stats ? launch_bfs<true>(g, a, 1) : launch_bfs<false>(g, a, 1));
+        HC_TRY((o.collect_stats ? launch_bfs<true, 2>(g, a, 1) : launch_bfs<false, 2>(g, a, 1)));
         HC_CUDA_TRY(cudaEventRecord(g->ev_stop, g->stream));
         if (host_depth || host_parent) {
             void *dst[2] = {host_depth ? (void *)(depth_out + (size_t)i * n) : nullptr,
@@ -1222,7 +1234,7 @@ extern "C" hc_status hc_bfs_noalloc(const int64_t *index, const int32_t *neighbo
     HC_TRY(noalloc_scratch(dev, &base));
     int sms = 0, bps = 0;
     HC_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    HC_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, bfs_persistent<false>, kBfsThreads, 0));
+    HC_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, (bfs_persistent<false, 2>), kBfsThreads, 0));
     if (bps < 1) return fail(HC_ERR_CUDA, "hc_bfs_noalloc: BFS kernel cannot be resident");
 
     unsigned char *p = base;
@@ -1279,7 +1291,7 @@ extern "C" hc_status hc_bfs_noalloc(const int64_t *index, const int32_t *neighbo
     HC_CUDA_TRY(cudaMemsetAsync(a.fold, 0, sizeof(BfsFold), s));
     void *params[] = {&a};
     ::hc::count_launch();
-    HC_CUDA_TRY(cudaLaunchCooperativeKernel((void *)bfs_persistent<false>, dim3(sms * bps), dim3(kBfsThreads), params,
+    HC_CUDA_TRY(cudaLaunchCooperativeKernel((void *)bfs_persistent<false, 2>, dim3(sms * bps), dim3(kBfsThreads), params,
                                             0, s));
     int err = 0;
     HC_CUDA_TRY(cudaMemcpyAsync(&err, &a.ctl->gs.err, sizeof(int), cudaMemcpyDeviceToHost, s));

@@ -637,8 +637,15 @@ __device__ __forceinline__ void note_low(int32_t *p, int32_t x) {
     if ((threadIdx.x & 31) == 0 && x < kInfDist && x < __ldcg(p)) atomicMin(p, x);
 }
 
-template <bool kStats>
-__global__ void __launch_bounds__(kSsspThreads, 2) sssp_persistent(SsspArgs a) {
+// kBlocks resident blocks per SM: two, or three for many sources at a time on a
+// graph with hub rows, whose pulls wait on gathers (issue slots 32 % used, DRAM 20
+// %) and gain more from a third block's warps than its spills cost (16 sources,
+// Kronecker scale 22: 12.2 -> 10.7 ms, scale 20: 3.57 -> 3.28 ms; without hubs,
+// where the pushes' atomics are the work, 16 sources, uniform 2^18: 2.48 -> 2.98).
+constexpr int kSsspWideSources = 4;
+constexpr int64_t kSsspWideEdges = 1ll << 20;
+template <bool kStats, int kBlocks>
+__global__ void __launch_bounds__(kSsspThreads, kBlocks) sssp_persistent(SsspArgs a) {
     __shared__ unsigned long long s_red[32];
     __shared__ int s_min[32];
     __shared__ SsspShared sh;
@@ -1227,11 +1234,11 @@ __global__ void sssp_clear(SsspCtl *ctl, int teams, SsspFold *f) {
 }
 
 // Blocks of sssp_persistent that are resident at a time (fewer when the handle's tuning says so).
-template <bool kStats>
+template <bool kStats, int kBlocks>
 hc_status sssp_resident(hc_graph *g, int *blocks) {
     static int blocks_per_sm = 0;
     if (blocks_per_sm == 0) {
-        HC_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, sssp_persistent<kStats>,
+        HC_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, sssp_persistent<kStats, kBlocks>,
                                                                   kSsspThreads, 0));
         if (blocks_per_sm < 1) return fail(HC_ERR_CUDA, "SSSP kernel cannot be resident");
     }
@@ -1241,17 +1248,17 @@ hc_status sssp_resident(hc_graph *g, int *blocks) {
     return HC_OK;
 }
 
-template <bool kStats>
+template <bool kStats, int kBlocks>
 hc_status launch_sssp(hc_graph *g, SsspArgs &a, int teams) {
     dim3 grid(a.team * teams), block(kSsspThreads);
     ::hc::count_launch();
     if (a.team == 1) {  // no block waits for another
-        sssp_persistent<kStats><<<grid, block, 0, g->stream>>>(a);
+        sssp_persistent<kStats, kBlocks><<<grid, block, 0, g->stream>>>(a);
         HC_CUDA_TRY(cudaGetLastError());
         return HC_OK;
     }
     void *params[] = {&a};
-    HC_CUDA_TRY(cudaLaunchCooperativeKernel((void *)sssp_persistent<kStats>, grid, block, params, 0, g->stream));
+    HC_CUDA_TRY(cudaLaunchCooperativeKernel((void *)sssp_persistent<kStats, kBlocks>, grid, block, params, 0, g->stream));
     return HC_OK;
 }
 
@@ -1267,7 +1274,7 @@ void sssp_teams(const hc_graph *g, int resident, int k, int room, int *team, int
     const double root = std::sqrt((double)std::max<int64_t>(g->M, 1));
     const int least = std::max(1, std::min(resident, (int)std::lround(root / 300.0)));
     const int most = std::max(1, std::min(resident, (int)std::lround(root / 9.0)));
-    const int at_a_time = std::max(1, std::min({k, room, resident / least}));
+    const int at_a_time = std::max(1, std::min({k, room, resident / least, kSsspLaunchSources}));
     const int rounds = (std::max(k, 1) + at_a_time - 1) / at_a_time;
     *teams = (std::max(k, 1) + rounds - 1) / rounds;
     *team = std::max(least, std::min(most, resident / *teams));
@@ -1368,7 +1375,11 @@ extern "C" hc_status hc_sssp(hc_graph *g, const int32_t *sources, int32_t num_so
     // Parents and the range check read the distances after a launch: without
     // an output for them, one scratch row per source of a launch is kept.
     int resident = 0;
-    HC_TRY(o.collect_stats ? sssp_resident<true>(g, &resident) : sssp_resident<false>(g, &resident));
+    const bool wide = !per_run && num_sources >= kSsspWideSources && g->M >= kSsspWideEdges &&
+                      g->base_view.n_tasks > 0;
+    HC_TRY((o.collect_stats ? sssp_resident<true, 2>(g, &resident)
+            : wide          ? sssp_resident<false, 3>(g, &resident)
+                            : sssp_resident<false, 2>(g, &resident)));
     OutPipe pipe;
     int team = resident, teams = 1;
     const size_t fold_bytes = 256;
@@ -1469,8 +1480,10 @@ extern "C" hc_status hc_sssp(hc_graph *g, const int32_t *sources, int32_t num_so
             { sssp_clear<<<1, 256, 0, g->stream>>>(a.ctl, 1, fold); ::hc::count_launch(); }
             HC_CUDA_TRY(cudaEventRecord(g->ev_start, g->stream));
         }
-        HC_TRY(o.collect_stats ? launch_sssp<true>(g, a, std::min(teams, a.nsrc))
-                               : launch_sssp<false>(g, a, std::min(teams, a.nsrc)));
+        const int use = std::min(teams, a.nsrc);
+        HC_TRY((o.collect_stats ? launch_sssp<true, 2>(g, a, use)
+                : wide          ? launch_sssp<false, 3>(g, a, use)
+                                : launch_sssp<false, 2>(g, a, use)));
         if (per_run) HC_CUDA_TRY(cudaEventRecord(g->ev_stop, g->stream));
         for (int32_t j = 0; j < a.nsrc; j++) {
             const int32_t *row = a.dist + (size_t)j * n;
