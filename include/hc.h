@@ -401,7 +401,7 @@ typedef struct hc_tuning {
     int32_t bfs_bu_split_levels;
     /* Blocks per SM of the persistent SSSP kernel: fewer
      * blocks make each grid barrier cheaper, more give large frontiers more
-     * warps.  0 = as many as fit (2). */
+     * warps.  0 = as many as fit (2; 3 with many sources on a large graph). */
     int32_t sssp_blocks_per_sm;
 } hc_tuning;
 
