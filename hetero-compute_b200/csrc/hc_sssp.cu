@@ -84,7 +84,10 @@ struct SsspCtl {
     // By run parity: a run's counters are set while blocks may still read the
     // last run's.
     EpochCnt cnt[2][3];
-    int far_len[2][2];
+    // Lengths of the two far piles, in two pairs of which one is current: a
+    // turn of thin epochs reads that pair and writes the other (see far_len in
+    // sssp_persistent).
+    int far_len[2][2][2];
     int min_far[2];
     // Degree sum of the rows a pull sweep lowered below the near threshold
     // (three slots, by pull): the next epoch's push-or-pull test, without
@@ -381,11 +384,13 @@ struct SoloArgs {
 // it): the same relaxations, claims and buckets as the grid's, with the near
 // queue in shared memory and mirrored in the global queue, so that the grid can
 // take any epoch over.  Stops before an epoch that is too wide or a pull, before
-// a phase change over too long a pile, after kSoloEpochs, or at the end.
+// a phase change over too long a pile, after kSoloEpochs, or at the end.  The far
+// piles' lengths are read from far_len and left in far_next: the other blocks may
+// still be reading far_len while this one runs.
 // Not inlined: its registers would spill the grid's epochs.
 template <bool kStats>
-__device__ __noinline__ SoloState solo_epochs(SoloArgs a, const SsspRun &r, SsspCtl *ctl, int *far_len, SoloQueue *sq,
-                                              SoloState st) {
+__device__ __noinline__ SoloState solo_epochs(SoloArgs a, const SsspRun &r, SsspCtl *ctl, const int *far_len,
+                                              int *far_next, SoloQueue *sq, SoloState st) {
     __shared__ int s_n[3], s_wide[3], s_far[2], s_min;
     __shared__ unsigned s_mf[3];  // exact while no row is long (see the end)
     __shared__ unsigned long long s_sum;
@@ -621,7 +626,7 @@ __device__ __noinline__ SoloState solo_epochs(SoloArgs a, const SsspRun &r, Sssp
         st.mf = s_sum;
         st.low = s_min;
     }
-    if (threadIdx.x < 2) far_len[threadIdx.x] = s_far[threadIdx.x];
+    if (threadIdx.x < 2) far_next[threadIdx.x] = s_far[threadIdx.x];
     return st;
 }
 
@@ -698,7 +703,16 @@ __global__ void __launch_bounds__(kSsspThreads, kBlocks) sssp_persistent(SsspArg
         __syncthreads();
         const int par = run & 1;
         EpochCnt *const cnt = ctl->cnt[par];
-        int *const far_len = ctl->far_len[par];
+        // The current pair of pile lengths.  At the top of an epoch with an empty
+        // near queue every thread reads far_len, and the first block may enter the
+        // thin epochs before the last thread has: nothing orders that read before
+        // what the thin epochs store.  So they store the new lengths into the other
+        // pair, which nobody reads before the team barrier after the turn, where
+        // every block changes over, whether the turn did anything or not.  The next
+        // turn, which writes this pair, comes after a whole-team epoch (solo_ok) and
+        // so after a barrier that every reader of this pair has reached.
+        int pair = 0;
+        int *far_len = ctl->far_len[par][0];
         int *const min_far = &ctl->min_far[par];
         {
             int32_t *const dist = r.dist, *const stamp = r.stamp, *const fstamp = r.fstamp;
@@ -760,7 +774,7 @@ __global__ void __launch_bounds__(kSsspThreads, kBlocks) sssp_persistent(SsspArg
                 if (team_block == 0) {
                     const SoloState st = solo_epochs<kStats>(
                         SoloArgs{a.index, a.nbr, a.w, a.m, a.delta, a.pull_alpha, a.max_epochs, pulls > 0}, r, ctl,
-                        far_len, sh.solo, SoloState{E, phase, fgen, nq, T, low, mfc, 0ull, 0ull});
+                        far_len, ctl->far_len[par][pair ^ 1], sh.solo, SoloState{E, phase, fgen, nq, T, low, mfc, 0ull, 0ull});
                     if (threadIdx.x == 0) {
                         ctl->solo = st;
                         if (kStats) {
@@ -770,6 +784,8 @@ __global__ void __launch_bounds__(kSsspThreads, kBlocks) sssp_persistent(SsspArg
                     }
                 }
                 if ((failed = !team_sync())) break;
+                pair ^= 1;
+                far_len = ctl->far_len[par][pair];
                 const int E1 = __ldcg(&ctl->solo.E), phase1 = __ldcg(&ctl->solo.phase);
                 const bool moved = E1 != E || phase1 != phase || (nq == 0 && __ldcg(far_len + (phase & 1)) == 0);
                 if (moved) {

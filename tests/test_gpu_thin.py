@@ -193,3 +193,23 @@ def test_sssp_batched_gaps(name, top, bits):
         for i in (0, 33, 69):
             assert np.array_equal(depth[i], oracle.bfs_depth(index, nbr, sources[i])), use_graph
     g.close()
+
+
+@pytest.mark.parametrize("name,delta", [("kron16", 1), ("kron16", 3), ("kron18", 2), ("grid", 1), ("grid", 40)])
+def test_sssp_pile_handover(name, delta):
+    """Teams of many blocks and small buckets: whole-team epochs end again and again with an empty near queue and
+    a short pile, which one block takes over and hands back.  Every source, run several times."""
+    import hc
+    if name == "grid":
+        h = hc.gen_grid(211, 190, 3, wtype=hc.W_I32)
+    else:
+        h = hc.gen_kronecker(int(name[4:]), 16, 3, wtype=hc.W_I32)
+    g = hc.Graph.from_host(h)
+    sources = hc.pick_sources(h, 6)
+    want = np.stack([oracle.sssp_dijkstra(h.index, h.neighbors, h.weights, s) for s in sources])
+    for alpha in (-1, 0):  # pushes only (phases to the end), and with pulls
+        for count in (1, 2, 6):  # one team of every block, several teams
+            for _ in range(4):
+                dist, _, _ = g.sssp(sources[:count], delta=delta, pull_alpha=alpha)
+                assert np.array_equal(dist, want[:count]), (alpha, count)
+    g.close()
