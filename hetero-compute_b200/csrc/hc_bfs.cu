@@ -933,6 +933,7 @@ extern "C" hc_status hc_bfs(hc_graph *g, const int32_t *sources, int32_t num_sou
         std::copy(sources, sources + num_sources, src.begin());
     for (int32_t s : src)
         if (s < 0 || s >= g->N) return fail(HC_ERR_INVALID_ARG, "hc_bfs: source %d outside [0, %d)", s, g->N);
+    HC_TRY(after_default_stream(g));
 
     const int64_t n = g->N;
     const int64_t W = (n + 31) / 32;

@@ -127,6 +127,13 @@ hc_status copy_out(void *dst_any, const void *src_dev, size_t bytes, cudaStream_
     return HC_OK;
 }
 
+hc_status after_default_stream(hc_graph *g) {
+    if (!g->ev_default) HC_CUDA_TRY(cudaEventCreateWithFlags(&g->ev_default, cudaEventDisableTiming));
+    HC_CUDA_TRY(cudaEventRecord(g->ev_default, cudaStreamLegacy));
+    HC_CUDA_TRY(cudaStreamWaitEvent(g->stream, g->ev_default, 0));
+    return HC_OK;
+}
+
 hc_status OutPipe::init(hc_graph *graph, int arrays, size_t each, int rows) {
     g = graph;
     narr = arrays;
@@ -656,6 +663,7 @@ hc_status hc_graph_destroy(hc_graph *g) {
     if (g->copy_stream) cudaStreamDestroy(g->copy_stream);
     g->pinned.release();
     if (g->ctl_host) cudaFreeHost(g->ctl_host);
+    if (g->ev_default) cudaEventDestroy(g->ev_default);
     if (g->ev_start) cudaEventDestroy(g->ev_start);
     if (g->ev_stop) cudaEventDestroy(g->ev_stop);
     if (g->own_stream) cudaStreamDestroy(g->own_stream);

@@ -68,6 +68,7 @@ struct hc_graph {
     cudaStream_t own_stream = nullptr;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev_start = nullptr, ev_stop = nullptr;
+    cudaEvent_t ev_default = nullptr;  // after_default_stream
 
     int32_t N = 0;
     int64_t M = 0;
@@ -146,6 +147,11 @@ struct hc_graph {
 namespace hc {
 // Make the handle's device current; returns HC_ERR_CUDA on failure.
 hc_status activate(hc_graph *g);
+// Orders the handle's stream after what the caller has queued on the legacy
+// default stream so far.  The handle's own stream does not wait for it by
+// itself, and a caller's output may be memory that a kernel queued there still
+// uses (a tensor that an allocator handed on in the order of that stream).
+hc_status after_default_stream(hc_graph *g);
 // Builds inv_deg (and, for weighted graphs, inv_wsum / wtn) if missing.
 hc_status ensure_pr_derived(hc_graph *g, bool weighted);
 // Per-source outputs bound for host memory, double-buffered: source i writes

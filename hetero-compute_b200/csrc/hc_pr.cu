@@ -1304,6 +1304,7 @@ extern "C" hc_status hc_pr_forward(hc_graph *g, const float *teleport, int32_t n
     fill_opts(opts, &o);
     if (o.max_iters > kMaxIterSlots - 1) o.max_iters = kMaxIterSlots - 1;
     if (stats) std::memset(stats, 0, sizeof(*stats));
+    HC_TRY(after_default_stream(g));
     const bool weighted = o.weighted != 0;
     HC_TRY(ensure_pr_derived(g, weighted));
     HC_TRY(ensure_plan(g));
@@ -1479,6 +1480,7 @@ extern "C" hc_status hc_pr_backward(hc_graph *g, const float *scores, const floa
     fill_opts(opts, &o);
     if (o.max_iters > kMaxIterSlots - 1) o.max_iters = kMaxIterSlots - 1;
     if (stats) std::memset(stats, 0, sizeof(*stats));
+    HC_TRY(after_default_stream(g));
     const bool weighted = o.weighted != 0;
     HC_TRY(ensure_pr_derived(g, weighted));
     HC_TRY(ensure_base_plan(g));

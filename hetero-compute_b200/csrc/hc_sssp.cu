@@ -1371,6 +1371,7 @@ extern "C" hc_status hc_sssp(hc_graph *g, const int32_t *sources, int32_t num_so
         std::copy(sources, sources + num_sources, src.begin());
     for (int32_t s : src)
         if (s < 0 || s >= g->N) return fail(HC_ERR_INVALID_ARG, "hc_sssp: source %d outside [0, %d)", s, g->N);
+    HC_TRY(after_default_stream(g));
 
     // Weights must be non-negative; the mean weight sets the default delta.
     HC_TRY(ensure_weight_stats(g));

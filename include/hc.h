@@ -149,7 +149,10 @@ hc_status hc_graph_get_csr(hc_graph *g, int64_t *index, int32_t *neighbors, void
  * each degree-1 candidate, from the device). */
 hc_status hc_graph_pick_sources(hc_graph *g, int32_t count, int32_t *out);
 /* Work of this handle goes to `stream` (a cudaStream_t); NULL restores the
- * handle's own stream. */
+ * handle's own stream.  hc_bfs, hc_sssp, hc_pr_forward, hc_pr_backward and the
+ * batched calls touch the caller's arrays after everything queued on the legacy
+ * default stream before the call; work on other streams is the caller's to
+ * order.  Calls return when their outputs are complete. */
 hc_status hc_graph_set_stream(hc_graph *g, void *stream);
 hc_status hc_graph_get_info(const hc_graph *g, hc_graph_info *info);
 
