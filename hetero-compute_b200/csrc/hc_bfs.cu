@@ -295,7 +295,7 @@ __device__ __noinline__ SoloState solo_levels(SoloArgs a, const BfsRun &r, BfsCt
             }
             if (kStats) {
                 my_vscan += nf;
-                my_escan += num_edges;
+                my_escan += s_mf[step % 3];  // num_edges is 1 after a bottom-up level
             }
         }
         const int per = min(32, max(1, (nf + nwarps - 1) / nwarps));

@@ -213,3 +213,54 @@ def test_sssp_pile_handover(name, delta):
                 dist, _, _ = g.sssp(sources[:count], delta=delta, pull_alpha=alpha)
                 assert np.array_equal(dist, want[:count]), (alpha, count)
     g.close()
+
+
+def scanned(index, nbr, n_active, src, alpha=15, beta=18):
+    """(vertices, edges) that a run of the direction rule scans: every frontier edge in top-down levels, and in
+    bottom-up ones each unvisited row up to its first neighbour in the frontier."""
+    n = len(index) - 1
+    deg = np.diff(index)
+    depth = oracle.bfs_depth(index, nbr, src)
+    push, to_check, edges = True, int(index[-1]), int(deg[src])
+    vertices = probes = 0
+    for level in range(depth.max() + 1):
+        front = np.flatnonzero(depth == level)
+        if push and edges > to_check // alpha:
+            push = False
+        if push:
+            to_check -= edges
+            vertices += len(front)
+            probes += int(deg[front].sum())
+            edges = int(deg[depth == level + 1].sum())
+        else:
+            open_ = np.flatnonzero((depth[:n_active] > level) | (depth[:n_active] < 0))
+            vertices += len(open_)
+            for v in open_:
+                hit = np.flatnonzero(depth[nbr[index[v]:index[v + 1]]] == level)
+                probes += int(hit[0]) + 1 if len(hit) else int(deg[v])
+            grown = int((depth == level + 1).sum())
+            if not (grown > len(front) or grown > n // beta):
+                push, edges = True, 1
+    return vertices, probes
+
+
+@pytest.mark.parametrize("tail", [0, 1, 3, 40])
+@pytest.mark.parametrize("width", [1, 20, 700])
+def test_bfs_scanned_edges(width, tail):
+    """Statistics of runs whose bottom-up levels are followed by thin top-down ones: a Kronecker core with a strip
+    of `tail` levels, `width` vertices each, hanging on its vertices of highest degree."""
+    import hc
+    k = hc.gen_kronecker(11, 16, 3)
+    core = k.num_nodes
+    row = np.repeat(np.arange(core), k.degrees())
+    u, v = [row[row < k.neighbors]], [k.neighbors[row < k.neighbors]]
+    for t in range(tail):
+        lane = np.arange(width)
+        u.append(lane if t == 0 else core + (t - 1) * width + lane)
+        v.append(core + t * width + lane)
+    index, nbr = csr(core + tail * width, np.concatenate(u), np.concatenate(v))
+    g = hc.Graph(index, nbr)
+    for src in (1, int(hc.pick_sources(k, 3)[2]), len(index) - 2):
+        _, _, st = g.bfs([src], stats=True)
+        assert (st.vertices_scanned, st.edges_scanned) == scanned(index, nbr, g.info().num_active, src), src
+    g.close()
