@@ -201,11 +201,22 @@ __device__ __forceinline__ void note_flush(MsspCtl *ctl, typename D::W mx) {
 // Smallest distance that each source wrote in an epoch, an int32 per source so
 // that a minimum needs no compare-and-swap.  Every thread of the block calls
 // this at the end of a kernel with its warp's minima in `my`: they meet in
-// shared memory, and one warp passes on those below the current value.
+// shared memory and go to one of kLowParts rows by block, which mssp_end folds.
+// A block that wrote nothing leaves at once.  On a small graph, whose epochs are a
+// few microseconds, every block's look at one row of minima was half of them
+// (uniform, 2^12 vertices, degree 8, 250 sources: one row 1390 us a call, so 1120
+// us, no minima and no gaps 1100 us; Kronecker scale 16, 150 sources: no gaps 6.4
+// ms, so 1.9 ms).
+constexpr int kLowParts = 16;
 template <class D, int SPL>
-__device__ __forceinline__ void low_flush(int32_t *lows, const typename D::W (&my)[SPL]) {
+__device__ __forceinline__ void low_flush(int32_t *parts, const typename D::W (&my)[SPL]) {
     __shared__ typename D::W s_low[8][32 * SPL];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    bool any = false;
+#pragma unroll
+    for (int s = 0; s < SPL; s++) any |= my[s] != D::kInfWord;
+    if (!__syncthreads_or(any)) return;
+    int32_t *const lows = parts + (size_t)(blockIdx.x % kLowParts) * (32 * SPL * D::kPer);
 #pragma unroll
     for (int s = 0; s < SPL; s++) s_low[wib][lane + 32 * s] = my[s];
     __syncthreads();
@@ -217,7 +228,7 @@ __device__ __forceinline__ void low_flush(int32_t *lows, const typename D::W (&m
 #pragma unroll
         for (int h = 0; h < D::kPer; h++) {
             const int32_t x = D::half(m, h);
-            if (x < __ldcg(p + h)) atomicMin(p + h, x);
+            if (x < D::kInfHalf) atomicMin(p + h, x);
         }
     }
 }
@@ -266,11 +277,11 @@ __device__ __forceinline__ void load_words(const W *p, W (&d)[SPL]) {
 }
 
 template <class D, int SPL>
-__global__ void mssp_init(int32_t n, typename D::W *dist, uint32_t *act0, uint32_t *act1, int32_t *lows0, int32_t *lows1) {
+__global__ void mssp_init(int32_t n, typename D::W *dist, uint32_t *act0, uint32_t *act1, int32_t *lows, int32_t *parts) {
     if (blockIdx.x == 0)
-        for (int i = threadIdx.x; i < 32 * SPL * D::kPer; i += blockDim.x) {
-            lows0[i] = 0;  // the seeds
-            lows1[i] = D::kInfHalf;
+        for (int i = threadIdx.x; i < 32 * SPL * D::kPer * kLowParts; i += blockDim.x) {
+            if (i < 32 * SPL * D::kPer) lows[i] = 0;  // the seeds
+            parts[i] = D::kInfHalf;
         }
     const size_t total = (size_t)n * 32 * SPL;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x)
@@ -414,7 +425,7 @@ template <class D, int SPL>
 __global__ void __launch_bounds__(256) mssp_epoch(const int64_t *index, const int32_t *nbr, const int32_t *w,
                                                   typename D::W *dist, const int32_t *qcur, const uint32_t *act_cur,
                                                   uint32_t *act_next, int32_t *qnext, int2 *tasks, MsspCtl *ctl, int c,
-                                                  unsigned long long *relaxed, int32_t *lows_next) {
+                                                  unsigned long long *relaxed, int32_t *low_parts) {
     const int nq = ctl_queue(ctl, c);
     if (nq == 0 || ctl_pull(ctl, c)) return;
     int *qnext_len = &ctl->qlen[c ^ 1];
@@ -443,7 +454,7 @@ __global__ void __launch_bounds__(256) mssp_epoch(const int64_t *index, const in
         relax_range<D, SPL>(index, nbr, w, dist, m, du, b, e, act_next, qnext, qnext_len, rel, qe, wmax, mylow);
     }
     note_flush<D>(ctl, wmax);
-    low_flush<D, SPL>(lows_next, mylow);
+    low_flush<D, SPL>(low_parts, mylow);
     rel = warp_sum(rel);
     qe = warp_sum(qe);
     if (lane == 0 && rel) atomicAdd(relaxed, rel);
@@ -454,7 +465,7 @@ template <class D, int SPL>
 __global__ void __launch_bounds__(256) mssp_tasks(const int64_t *index, const int32_t *nbr, const int32_t *w,
                                                   typename D::W *dist, const int2 *tasks, const uint32_t *act_cur,
                                                   uint32_t *act_next, int32_t *qnext, MsspCtl *ctl, int c,
-                                                  unsigned long long *relaxed, int32_t *lows_next) {
+                                                  unsigned long long *relaxed, int32_t *low_parts) {
     const int nq = ctl_queue(ctl, c);
     if (nq == 0 || ctl_pull(ctl, c)) return;
     int *qnext_len = &ctl->qlen[c ^ 1];
@@ -478,7 +489,7 @@ __global__ void __launch_bounds__(256) mssp_tasks(const int64_t *index, const in
         relax_range<D, SPL>(index, nbr, w, dist, m, du, b, e, act_next, qnext, qnext_len, rel, qe, wmax, mylow);
     }
     note_flush<D>(ctl, wmax);
-    low_flush<D, SPL>(lows_next, mylow);
+    low_flush<D, SPL>(low_parts, mylow);
     rel = warp_sum(rel);
     qe = warp_sum(qe);
     if (lane == 0 && rel) atomicAdd(relaxed, rel);
@@ -509,7 +520,7 @@ __global__ void __launch_bounds__(256) mssp_pull(const int64_t *index, const int
                                                  const int2 *tasks, int ntasks, int pull_chunk, const uint32_t *act_cur,
                                                  uint32_t *act_next, int fresh, MsspCtl *ctl, int c,
                                                  unsigned long long *relaxed, const int32_t *lows,
-                                                 int32_t *lows_next) {
+                                                 int32_t *low_parts) {
     using W = typename D::W;
     const int nq = ctl_queue(ctl, c);
     if (nq == 0 || !ctl_pull(ctl, c)) return;
@@ -628,7 +639,7 @@ __global__ void __launch_bounds__(256) mssp_pull(const int64_t *index, const int
         }
     }
     note_flush<D>(ctl, wmax);
-    low_flush<D, SPL>(lows_next, mylow);
+    low_flush<D, SPL>(low_parts, mylow);
     rel = warp_sum(rel);
     if (lane == 0 && rel) atomicAdd(relaxed, rel);
 }
@@ -707,14 +718,25 @@ __global__ void mssp_clear(const int32_t *q, uint32_t *act, const MsspCtl *ctl, 
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nq; i += gridDim.x * blockDim.x) act[q[i]] = 0;
 }
 
-// Closes epoch parity c (one block): clears the minima it read, counts it, resets its counters for reuse, and decides
+// Closes epoch parity c (one block): all warps but the first fold the minima it
+// wrote into those that the next one reads; thread 0 counts it, resets its counters for reuse, and decides
 // whether another epoch runs (queue non-empty, under the epoch cap and the
 // time bound, and for narrow words inside the 16-bit range); inside a graph
 // it sets the while node's condition.
-__global__ void mssp_end(MsspCtl *ctl, int c, int32_t *lows, int count, int32_t inf,
+__global__ void mssp_end(MsspCtl *ctl, int c, int32_t *lows, int32_t *parts, int count, int32_t inf,
                          cudaGraphConditionalHandle cond, int use_cond) {
-    for (int i = threadIdx.x; i < count; i += blockDim.x) lows[i] = inf;  // the next epoch's to write
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
+    if (threadIdx.x >= 32) {
+        for (int i = threadIdx.x - 32; i < count; i += blockDim.x - 32) {
+            int32_t m = inf;
+#pragma unroll
+            for (int k = 0; k < kLowParts; k++) m = min(m, parts[k * count + i]);
+            lows[i] = m;
+#pragma unroll
+            for (int k = 0; k < kLowParts; k++) parts[k * count + i] = inf;
+        }
+        return;
+    }
+    if (threadIdx.x != 0) return;
     bool go = false;
     if (!ctl->stop && ctl->qlen[c] > 0) {
         ctl->epochs++;
@@ -788,7 +810,8 @@ __global__ void mssp_transpose(const typename D::W *dist, int32_t n, int nsrc, i
 template <class D>
 struct MsspBufs {
     typename D::W *dist;
-    int32_t *lows[2];  // smallest distance each source wrote: epoch parity c reads lows[c], writes lows[c ^ 1]
+    int32_t *lows;       // smallest distance each source wrote in the last epoch
+    int32_t *low_parts;  // ... in this one: kLowParts rows
     uint32_t *act[2];
     int32_t *q[2];
     int2 *tasks;
@@ -806,20 +829,19 @@ void launch_epoch(const hc_graph *g, cudaStream_t st, const MsspBufs<D> &b, int 
     const int64_t *index = g->index.as<int64_t>();
     const int32_t *nbr = g->nbr.as<int32_t>(), *w = g->wgt.as<int32_t>();
     mssp_epoch<D, SPL><<<grid, 256, 0, st>>>(index, nbr, w, b.dist, b.q[c], b.act[c], b.act[c ^ 1], b.q[c ^ 1],
-                                             b.tasks, b.ctl, c, relaxed, b.lows[c ^ 1]);
+                                             b.tasks, b.ctl, c, relaxed, b.low_parts);
     mssp_tasks<D, SPL><<<grid, 256, 0, st>>>(index, nbr, w, b.dist, b.tasks, b.act[c], b.act[c ^ 1], b.q[c ^ 1],
-                                             b.ctl, c, relaxed, b.lows[c ^ 1]);
+                                             b.ctl, c, relaxed, b.low_parts);
     const int32_t hub = g->mssp_hub_rows > 0 ? g->mssp_hub_rows : g->n_active;
     mssp_pull<D, SPL><<<grid, 256, 0, st>>>(index, nbr, w, b.dist, 0, hub, g->ws_plan_mssp.as<int2>(),
                                             g->mssp_tasks < 0 ? 0 : g->mssp_tasks, pull_chunk(g->M), b.act[c], b.act[c ^ 1], 0, b.ctl,
-                                            c, relaxed, b.lows[c], b.lows[c ^ 1]);
+                                            c, relaxed, b.lows, b.low_parts);
     if (hub < g->n_active)
         mssp_pull<D, SPL><<<grid, 256, 0, st>>>(index, nbr, w, b.dist, hub, g->n_active, nullptr, 0, pull_chunk(g->M), b.act[c],
-                                                b.act[c ^ 1], 1, b.ctl, c, relaxed, b.lows[c], b.lows[c ^ 1]);
+                                                b.act[c ^ 1], 1, b.ctl, c, relaxed, b.lows, b.low_parts);
     mssp_clear<<<grid, 256, 0, st>>>(b.q[c], b.act[c], b.ctl, c);
     mssp_compact<<<grid, 256, 0, st>>>(index, b.act[c ^ 1], g->N, b.q[c ^ 1], b.ctl, c);
-    mssp_end<<<1, 128, 0, st>>>(b.ctl, c, b.lows[c], 32 * SPL * D::kPer, D::kInfHalf, cond,
-                                use_cond);
+    mssp_end<<<1, 288, 0, st>>>(b.ctl, c, b.lows, b.low_parts, 32 * SPL * D::kPer, D::kInfHalf, cond, use_cond);
 }
 constexpr int kEpochLaunches = 7;
 
@@ -835,7 +857,7 @@ hc_status run_group(hc_graph *g, const int32_t *h_src, int k, int32_t *dst, int 
     const int64_t n = g->N;
     const int64_t max_tasks = 2 * (g->M / kPushChunk) + 64;  // sum over rows longer than a chunk
     HC_TRY(g->ws_batch.ensure((size_t)n * KW * 4 + (size_t)n * 4 * 4 + sizeof(int2) * max_tasks +
-                              2 * (size_t)K * 4 + 8192));
+                              (1 + kLowParts) * (size_t)K * 4 + 8192));
     char *p = g->ws_batch.as<char>();
     auto take = [&](size_t bytes) {
         char *r = p;
@@ -850,14 +872,14 @@ hc_status run_group(hc_graph *g, const int32_t *h_src, int k, int32_t *dst, int 
     b.q[1] = (int32_t *)take((size_t)n * 4);
     b.tasks = (int2 *)take(sizeof(int2) * max_tasks);
     b.ctl = (MsspCtl *)take(sizeof(MsspCtl));
-    b.lows[0] = (int32_t *)take((size_t)K * 4);
-    b.lows[1] = (int32_t *)take((size_t)K * 4);
+    b.lows = (int32_t *)take((size_t)K * 4);
+    b.low_parts = (int32_t *)take((size_t)K * 4 * kLowParts);
     b.src = (int32_t *)take(sizeof(int32_t) * K);
     const int grid = g->sm_count * 8;
     HC_TRY(g->pinned.ensure(2 * sizeof(MsspCtl) + 64));
     MsspCtl *hctl = g->pinned.as<MsspCtl>();
     HC_CUDA_TRY(cudaMemcpyAsync(b.src, h_src, sizeof(int32_t) * k, cudaMemcpyHostToDevice, g->stream));
-    { mssp_init<D, SPL><<<grid, 256, 0, g->stream>>>(g->N, b.dist, b.act[0], b.act[1], b.lows[0], b.lows[1]); ::hc::count_launch(); }
+    { mssp_init<D, SPL><<<grid, 256, 0, g->stream>>>(g->N, b.dist, b.act[0], b.act[1], b.lows, b.low_parts); ::hc::count_launch(); }
     {
         mssp_seed<D, SPL><<<1, 32, 0, g->stream>>>(k, b.src, g->index.as<int64_t>(), b.dist, b.act[0], b.q[0], b.ctl,
                                                    pull_alpha, (long long)g->M, max_epochs, g->w_max);
