@@ -36,17 +36,19 @@ constexpr int kMaxIterSlots = 4096;
 struct IterSlot {
     double l1;       // Jacobi: sum |change|; conjugate gradients: p . q
     double rz, z1;   // conjugate gradients: r . z, sum |z|
-    int changed, pad;
+    int changed;
+    int pause;       // the launch ends after this iteration (see pr_solve)
 };
 struct IterState {
     GridSync gs;
     int done, blocks_done;   // sweeps launched one by one
     IterSlot slot[kMaxIterSlots];
 };
-// What a solve reports, in mapped host memory.
+// What a solve reports, in mapped host memory.  done: 1 converged, 2 stopped, 0
+// paused at the run limit: another launch goes on from iteration `iters`.
 struct SolveOut {
     int err, iters, done, changed;
-    double l1;
+    double l1, omega;
 };
 
 // One pull sweep: out[v] = base_v + d * rs_v * sum_{e in row v} ew_e * gin[nbr_e].
@@ -68,6 +70,8 @@ struct SweepArgs {
     float cheb_rho;         // > 0: Chebyshev weights (0: plain Jacobi)
     float tol_l1, eps;
     int max_iters;
+    int first_iter;         // where this launch goes on, and the Chebyshev weight it left off with
+    double first_omega;
     int32_t n, n_active;
 };
 // The vectors of one sweep.  They are written by other blocks of the same
@@ -271,14 +275,17 @@ __device__ __forceinline__ void add_residual(IterSlot *slot, float l1, int chg) 
 // lies in [-cheb_rho, cheb_rho] (a reversible walk scaled by d): weights
 // omega_1 = 1, omega_2 = 1 / (1 - rho^2 / 2), omega_{k+1} = 1 / (1 - rho^2
 // omega_k / 4) (Golub and Varga, 1961).
+// A launch that has run for the run limit ends after its iteration, and the host
+// launches the rest (run_solve): a solve may take longer, one launch may not.
 template <bool kEW, bool kRS, bool kPS, bool kBaseVec>
 __global__ void __launch_bounds__(kPrThreads, kPrBlocks) pr_solve(SweepArgs a, PrPlanDev plan) {
     __shared__ float s_acc[kPrThreads / 32][32];
     const double rho2 = (double)a.cheb_rho * a.cheb_rho;
-    double omega = 1.0;
-    int it = 0, done = 0;
-    bool ok = true;
-    while (it < a.max_iters && !done) {
+    const unsigned long long t_start = globaltimer_ns();
+    double omega = a.first_omega;
+    int it = a.first_iter, done = 0;
+    bool ok = true, paused = false;
+    while (it < a.max_iters && !done && !paused) {
         if (a.cheb_rho > 0.f)
             omega = it == 0 ? 1.0 : it == 1 ? 1.0 / (1.0 - rho2 / 2.0) : 1.0 / (1.0 - rho2 * omega / 4.0);
         const int cur = it & 1;
@@ -289,22 +296,27 @@ __global__ void __launch_bounds__(kPrThreads, kPrBlocks) pr_solve(SweepArgs a, P
         sweep_rows<kEW, kRS, kPS, kBaseVec>(a, plan, v, s_acc, l1, chg);
         IterSlot *const slot = &a.st->slot[it % kMaxIterSlots];
         add_residual(slot, l1, chg);
-        if (it + 2 >= kMaxIterSlots && blockIdx.x == 0 && threadIdx.x == 0)
-            a.st->slot[(it + 2) % kMaxIterSlots] = IterSlot{0.0, 0.0, 0.0, 0, 0};
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            if (it + 2 >= kMaxIterSlots) a.st->slot[(it + 2) % kMaxIterSlots] = IterSlot{0.0, 0.0, 0.0, 0, 0};
+            if (globaltimer_ns() - t_start > c_limits.run_ns) slot->pause = 1;
+        }
         if (!(ok = grid_barrier(&a.st->gs))) break;
         // eps >= 3e38 marks the per-vertex rule as unused.
         if ((a.tol_l1 > 0.f && __ldcg(&slot->l1) < (double)a.tol_l1) || (a.eps < 3e38f && __ldcg(&slot->changed) == 0))
             done = 1;
+        paused = __ldcg(&slot->pause) != 0;
         it++;
     }
-    if (ok && a.final_x) {
+    paused = paused && !done && it < a.max_iters;
+    if (ok && !paused && a.final_x) {
         const float *x = a.x[it & 1];
         for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += gridDim.x * blockDim.x) a.final_x[i] = x[i];
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         a.out->err = *(volatile int *)&a.st->gs.err;
         a.out->iters = it;
-        a.out->done = done ? 1 : 2;
+        a.out->done = paused ? 0 : done ? 1 : 2;
+        a.out->omega = omega;
         a.out->l1 = it > 0 ? __ldcg(&a.st->slot[(it - 1) % kMaxIterSlots].l1) : 0.0;
         a.out->changed = it > 0 ? __ldcg(&a.st->slot[(it - 1) % kMaxIterSlots].changed) : 0;
         __threadfence_system();
@@ -994,7 +1006,9 @@ hc_status solve_begin(hc_graph *g, SweepArgs &a, SolveOut **out) {
     const size_t slots = std::min<size_t>((size_t)a.max_iters + 1, kMaxIterSlots);
     HC_CUDA_TRY(cudaMemsetAsync(a.st, 0, offsetof(IterState, slot) + sizeof(IterSlot) * slots, g->stream));
     HC_TRY(ctl_slot(g, 0, (void **)out, (void **)&a.out));
-    **out = SolveOut{0, 0, 0, 0, 0.0};
+    **out = SolveOut{0, 0, 0, 0, 0.0, 1.0};
+    a.first_iter = 0;
+    a.first_omega = 1.0;
     HC_CUDA_TRY(cudaEventRecord(g->ev_start, g->stream));
     return HC_OK;
 }
@@ -1020,8 +1034,13 @@ hc_status run_solve(hc_graph *g, SweepArgs a, const PrPlanDev &plan, SolveFn fn,
     a.final_x = final_x;
     SolveOut *out = nullptr;
     HC_TRY(solve_begin(g, a, &out));
-    HC_TRY(fn(g, a, plan, out));
-    return solve_end(g, out, res);
+    do {
+        HC_TRY(fn(g, a, plan, out));
+        HC_TRY(solve_end(g, out, res));
+        a.first_iter = out->iters;
+        a.first_omega = out->omega;
+    } while (!res->done);
+    return HC_OK;
 }
 
 // ------------------------------------------------- adjoint by conjugate gradients
@@ -1043,6 +1062,7 @@ struct CgArgs {
     const float *c;
     float *lam, *r, *p, *sp;
     float rel_tol;  // stop at |z|_1 < rel_tol * |c|_1
+    int first_iter;  // pr_cg: 0, or the iteration that this launch goes on with
 };
 
 __device__ __forceinline__ float row_weight(const float *rs, int32_t v) {
@@ -1106,7 +1126,7 @@ __device__ __forceinline__ double cg_tol(const SweepArgs &a, const CgArgs &q) {
 }
 
 // The whole solve in one cooperative launch, a grid barrier after each sweep and
-// each vector pass (three an iteration).
+// each vector pass (three an iteration).  Paused at the run limit as pr_solve.
 template <bool kEW>
 __global__ void __launch_bounds__(kPrThreads, kPrBlocks) pr_cg(SweepArgs a, PrPlanDev plan, CgArgs q) {
     __shared__ float s_acc[kPrThreads / 32][32];
@@ -1115,26 +1135,32 @@ __global__ void __launch_bounds__(kPrThreads, kPrBlocks) pr_cg(SweepArgs a, PrPl
     GridSync *const gs = &a.st->gs;
     float l1;
     int chg;
+    const unsigned long long t_start = globaltimer_ns();
     int iters = 0, converged = 0;
     double rz = 0.0, z1 = 0.0, c1 = 0.0, tol = 0.0;
-    // S x by the pull sweep with each row's own weights; its residual is p . q.
-    sweep_rows<kEW, false, false, false, true>(a, plan, SweepIter{q.lam, q.lam, q.sp, q.sp, 1.f}, s_acc, l1, chg);
-    bool ok = grid_barrier(gs);
-    if (ok) {
-        cg_start_rows(a, q, gtid, nthreads, rz, z1, c1);
-        add_dots(&a.st->slot[0], rz, z1);
-        __syncthreads();
-        c1 = block_sum(c1, s_c);
-        if (threadIdx.x == 0 && c1 != 0.0) atomicAdd(&a.st->slot[0].l1, c1);
+    bool ok = true, paused = false;
+    if (q.first_iter == 0) {
+        // S x by the pull sweep with each row's own weights; its residual is p . q.
+        sweep_rows<kEW, false, false, false, true>(a, plan, SweepIter{q.lam, q.lam, q.sp, q.sp, 1.f}, s_acc, l1, chg);
         ok = grid_barrier(gs);
+        if (ok) {
+            cg_start_rows(a, q, gtid, nthreads, rz, z1, c1);
+            add_dots(&a.st->slot[0], rz, z1);
+            __syncthreads();
+            c1 = block_sum(c1, s_c);
+            if (threadIdx.x == 0 && c1 != 0.0) atomicAdd(&a.st->slot[0].l1, c1);
+            ok = grid_barrier(gs);
+        }
+    } else {
+        iters = q.first_iter - 1;
     }
     if (ok) {
-        rz = __ldcg(&a.st->slot[0].rz);
-        z1 = __ldcg(&a.st->slot[0].z1);
+        rz = __ldcg(&a.st->slot[iters].rz);
+        z1 = __ldcg(&a.st->slot[iters].z1);
         tol = cg_tol(a, q);
-        converged = z1 < tol || rz <= 0.0;
+        converged = q.first_iter == 0 && (z1 < tol || rz <= 0.0);
     }
-    for (int it = 1; ok && !converged && it <= a.max_iters; it++) {
+    for (int it = iters + 1; ok && !converged && !paused && it <= a.max_iters; it++) {
         IterSlot *const slot = &a.st->slot[it];
         sweep_rows<kEW, false, false, false, true>(a, plan, SweepIter{q.p, q.p, q.sp, q.sp, 1.f}, s_acc, l1, chg);
         add_residual(slot, l1, 0);
@@ -1153,12 +1179,14 @@ __global__ void __launch_bounds__(kPrThreads, kPrBlocks) pr_cg(SweepArgs a, PrPl
         converged = z1 < tol;
         if (converged || it == a.max_iters) break;
         cg_direction_rows(a, q, gtid, nthreads, beta);  // the same thread's entries as above
+        if (gtid == 0 && globaltimer_ns() - t_start > c_limits.run_ns) slot->pause = 1;
         ok = grid_barrier(gs);
+        paused = ok && __ldcg(&slot->pause) != 0;
     }
     if (gtid == 0) {
         a.out->err = *(volatile int *)&gs->err;
         a.out->iters = iters;
-        a.out->done = converged;
+        a.out->done = paused ? 0 : converged ? 1 : 2;
         a.out->l1 = z1;
         a.out->changed = 0;
         __threadfence_system();
@@ -1257,7 +1285,7 @@ hc_status launch_cg(hc_graph *g, SweepArgs &a, const PrPlanDev &plan, CgArgs &q,
 hc_status run_cg(hc_graph *g, const PrPlanDev &plan, bool weighted, const float *c, float *lam, float d, float rel_tol,
                  int max_iters, float *work, float *partials, unsigned *hub_count, SolveResult *res) {
     const int64_t n = g->N;
-    CgArgs q{c, lam, work, work + n, work + 2 * n, rel_tol};
+    CgArgs q{c, lam, work, work + n, work + 2 * n, rel_tol, 0};
     SweepArgs a{};
     a.index = g->index.as<int64_t>();
     a.nbr = g->nbr.as<int32_t>();
@@ -1271,8 +1299,11 @@ hc_status run_cg(hc_graph *g, const PrPlanDev &plan, bool weighted, const float 
     a.n_active = g->n_active;
     SolveOut *out = nullptr;
     HC_TRY(solve_begin(g, a, &out));
-    HC_TRY(weighted ? launch_cg<true>(g, a, plan, q, out) : launch_cg<false>(g, a, plan, q, out));
-    HC_TRY(solve_end(g, out, res));
+    do {
+        HC_TRY(weighted ? launch_cg<true>(g, a, plan, q, out) : launch_cg<false>(g, a, plan, q, out));
+        HC_TRY(solve_end(g, out, res));
+        q.first_iter = out->iters + 1;
+    } while (!res->done);
     res->done = res->done == 1;
     return HC_OK;
 }

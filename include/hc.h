@@ -487,7 +487,9 @@ hc_status hc_profile_segments(hc_graph *g, hc_profile_algo algo, hc_variant vari
  * Every device-side wait here is bounded: a grid barrier gives up after
  * wait_ns (default 2 s), one persistent run after run_ns (20 s), one batched
  * group's epoch loop after loop_ns (60 s); each then ends its call with
- * HC_ERR_TIMEOUT and leaves the handle usable.  hc_set_time_limits replaces
+ * HC_ERR_TIMEOUT and leaves the handle usable.  (A PageRank solve ends such a
+ * launch after an iteration and goes on in another: its length is bounded by
+ * max_iters.)  hc_set_time_limits replaces
  * the three bounds on `device` for every later launch in this process
  * (0 = the default); it exists so that tests can make each wait run out. */
 hc_status hc_set_time_limits(int32_t device, uint64_t wait_ns, uint64_t run_ns, uint64_t loop_ns);

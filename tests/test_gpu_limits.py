@@ -79,3 +79,47 @@ def test_loop_limit_ends_batched_groups(graph, use_graph):
         s = src[i]
         assert np.array_equal(depth[i], oracle.bfs_depth(host.index, host.neighbors, s))
         assert np.array_equal(dist[i], oracle.sssp_dijkstra(host.index, host.neighbors, host.weights, s))
+
+
+@pytest.mark.parametrize("name", ["plain", "teleport", "chebyshev", "weighted", "adjoint", "adjoint_jacobi",
+                                  "adjoint_chebyshev", "ppr_tail"])
+def test_pagerank_goes_on_after_the_run_limit(graph, name):
+    """A solve's launch ends after an iteration once run_ns has passed, and another goes on: at 1 ns there is a launch
+    per iteration, and the result is that of one launch."""
+    host, g = graph
+    n = host.num_nodes
+    rng = np.random.default_rng(5)
+    t = rng.random(n).astype(np.float32)
+    t /= t.sum()
+    x = g.pagerank(tol_l1=1e-6, max_iters=200)[0]
+    c = rng.standard_normal(n).astype(np.float32)
+    opts = dict(tol_l1=1e-6, max_iters=200)
+    # Two more vertices, joined by an edge: a column with its seed there converges last, on the sweeps of one column.
+    slow = hc.Graph(np.append(host.index, host.num_edges + np.arange(1, 3)),
+                    np.append(host.neighbors, [n + 1, n]).astype(np.int32))
+    call = {
+        "plain": lambda **k: g.pagerank(**(opts | k)),
+        "teleport": lambda **k: g.pagerank(t, **(opts | k)),
+        "chebyshev": lambda **k: g.pagerank(accel=1, **(opts | k)),
+        "weighted": lambda **k: g.pagerank(weighted=True, **(opts | k)),
+        "adjoint": lambda **k: g.pagerank_backward(x, c, want_dw=False, **(opts | k))[::2],
+        "adjoint_jacobi": lambda **k: g.pagerank_backward(x, c, want_dw=False, accel=-1, **(opts | k))[::2],
+        "adjoint_chebyshev": lambda **k: g.pagerank_backward(x, c, want_dw=False, accel=2, **(opts | k))[::2],
+        "ppr_tail": lambda **k: slow.ppr_batched([0, 1, 2, 3, 4, 5], [0, 1, 2, 3, n], **(opts | k)),
+    }[name]
+    for extra in ({}, {"max_iters": 5}):
+        want, st = call(**extra)
+        before = hc.kernel_launches()
+        call(**extra)
+        whole = hc.kernel_launches() - before
+        hc.set_time_limits(0, run_ns=1)
+        before = hc.kernel_launches()
+        got, st1 = call(**extra)
+        launches = hc.kernel_launches() - before
+        hc.set_time_limits(0)
+        assert (st1.iterations, st1.converged) == (st.iterations, st.converged)
+        assert np.allclose(got, want, rtol=1e-5, atol=1e-9 if name != "adjoint" else 1e-5 * np.abs(want).max())
+        if name != "ppr_tail":
+            assert launches >= whole + st.iterations - 2
+        elif not extra:
+            assert launches >= whole + 20
