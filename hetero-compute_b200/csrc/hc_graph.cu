@@ -175,10 +175,19 @@ hc_status OutPipe::flush() {
     pending = false;
     const int s = pend_slot;
     HC_CUDA_TRY(cudaStreamWaitEvent(g->copy_stream, g->ev_ready[s], 0));
-    for (int j = 0; j < narr; j++)
-        if (pend_dst[j] && pend_rows > 0)
-            HC_CUDA_TRY(cudaMemcpy2DAsync(pend_dst[j], bytes, g->ws_stage[s][j].ptr, bytes, copy_bytes, pend_rows,
-                                          cudaMemcpyDefault, g->copy_stream));
+    // A 2-D copy takes pitches below 2^31 bytes only; a row may be longer.
+    const bool rows_apart = pend_rows == 1 || bytes > (size_t)INT32_MAX;
+    for (int j = 0; j < narr; j++) {
+        if (!pend_dst[j]) continue;
+        char *dst = static_cast<char *>(pend_dst[j]);
+        const char *src = g->ws_stage[s][j].as<char>();
+        for (int r = 0; rows_apart && r < pend_rows; r++)
+            HC_CUDA_TRY(cudaMemcpyAsync(dst + r * bytes, src + r * bytes, copy_bytes, cudaMemcpyDefault,
+                                        g->copy_stream));
+        if (!rows_apart && pend_rows > 0)
+            HC_CUDA_TRY(cudaMemcpy2DAsync(dst, bytes, src, bytes, copy_bytes, pend_rows, cudaMemcpyDefault,
+                                          g->copy_stream));
+    }
     HC_CUDA_TRY(cudaEventRecord(g->ev_done[s], g->copy_stream));
     return HC_OK;
 }
