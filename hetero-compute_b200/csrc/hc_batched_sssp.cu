@@ -1027,6 +1027,9 @@ extern "C" hc_status hc_sssp_batched(hc_graph *g, const int32_t *sources, int32_
         size_t free_b = 0, total_b = 0;
         HC_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
         free_b += g->ws_batch.bytes + g->ws_out0.bytes;  // workspaces are reused
+        free_b += g->ws_bfs.bytes + g->ws_sssp.bytes;    // released when they are in the way
+        for (auto &slot : g->ws_stage)
+            for (auto &b : slot) free_b += b.bytes;
         const double bytes = narrow_ok ? 2.0 : 4.0;
         group = narrow_ok ? 512 : 256;
         while (group > 32 && (double)g->N * group * bytes > 0.4 * (double)free_b) group /= 2;

@@ -977,11 +977,21 @@ extern "C" hc_status hc_bfs(hc_graph *g, const int32_t *sources, int32_t num_sou
         bfs_teams(g, resident, num_sources, (int)std::min<size_t>(std::max<size_t>(kBfsTeamBytes / each, 1), 1 << 20),
                   &team, &teams);
     }
-    hc_status reserved = reserve();
-    if (reserved == HC_ERR_OOM && teams > 1) {  // no room for several: one at a time
+    hc_status reserved;
+    {
+        ReclaimScope nothing(nullptr, 0u);
+        reserved = reserve();
+    }
+    if (reserved == HC_ERR_OOM) {  // no room: one source at a time, and what other calls left behind goes
         clear_error();
-        bfs_teams(g, resident, num_sources, 1, &team, &teams);
-        g->ws_bfs.release();
+        if (teams > 1) {
+            bfs_teams(g, resident, num_sources, 1, &team, &teams);
+            g->ws_bfs.release();
+            if (!depth_out) g->ws_out0.release();
+            if (!parent_out) g->ws_out1.release();
+            OutPipe::drop_staging(g);
+        }
+        ReclaimScope reclaim_scope(g, kKeepBfs);
         reserved = reserve();
     }
     HC_TRY(reserved);

@@ -50,10 +50,10 @@ bool reclaim(hc_graph *g, unsigned keep, const DevBuf *self) {
         drop(g->wf32);
     }
     if (!(keep & kKeepBatch)) drop(g->ws_batch);
-    // Workspaces of several sources at a time (hc_bfs itself opens no scope).
-    drop(g->ws_bfs);
-    if (!(keep & kKeepSssp)) {
-        drop(g->ws_sssp);
+    // Workspaces of several sources at a time, and their staging.
+    if (!(keep & kKeepBfs)) drop(g->ws_bfs);
+    if (!(keep & kKeepSssp)) drop(g->ws_sssp);
+    if (!(keep & (kKeepBfs | kKeepSssp))) {
         for (auto &slot : g->ws_stage)
             for (auto &b : slot) drop(b);
     }
@@ -69,6 +69,11 @@ ReclaimScope::ReclaimScope(hc_graph *g, unsigned keep) : prev_g(t_reclaim_g), pr
 ReclaimScope::~ReclaimScope() {
     t_reclaim_g = prev_g;
     t_reclaim_keep = prev_keep;
+}
+
+void OutPipe::drop_staging(hc_graph *g) {
+    for (auto &slot : g->ws_stage)
+        for (auto &b : slot) b.release();
 }
 
 hc_status DevBuf::ensure(size_t want) {

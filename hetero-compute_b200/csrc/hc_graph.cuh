@@ -178,6 +178,8 @@ struct OutPipe {
     // `rows` consecutive rows of each array.
     hc_status release(int i, void *const *dst, int rows = 1);
     hc_status flush();
+    // Releases the staging (no copy in flight).
+    static void drop_staging(hc_graph *g);
     hc_status finish();
 };
 
@@ -225,9 +227,12 @@ hc_status ctl_slot(hc_graph *g, int slot, void **host, void **dev);
 // Device memory pressure.  Derived arrays that can be built again (the
 // pull sweeps' pair array, the reference-order schedule, the weighted
 // PageRank arrays), the batched workspace and the BFS and SSSP workspaces and
-// staging are released, when an allocation fails, unless the running call needs them; the allocation is
-// then tried once more.  A call states what it needs for its lifetime.
-enum : unsigned { kKeepAdj = 1u, kKeepPrOrd = 2u, kKeepPrWeighted = 4u, kKeepBatch = 8u, kKeepSssp = 16u };
+// staging are released, when an allocation fails, unless the running call
+// needs them; the allocation is then tried once more.  A call states what it
+// needs for its lifetime.  Workspaces for several sources at a time are asked
+// for under a scope of no graph (nothing is released for them); when they
+// cannot be had, those of one source are, under the call's own scope.
+enum : unsigned { kKeepAdj = 1u, kKeepPrOrd = 2u, kKeepPrWeighted = 4u, kKeepBatch = 8u, kKeepSssp = 16u, kKeepBfs = 32u };
 struct ReclaimScope {
     ReclaimScope(hc_graph *g, unsigned keep);
     ~ReclaimScope();

@@ -42,3 +42,62 @@ def test_weighted_pagerank_reclaims_the_sssp_pair_array():
     for i, s in enumerate(src):
         assert np.array_equal(d1[i], oracle.sssp_dijkstra(host.index, host.neighbors, host.weights, s))
     g.close()
+
+
+@pytest.fixture(scope="module")
+def weighted20():
+    host = hc.gen_kronecker(20, 16, 7, wtype=hc.W_I32)
+    src = hc.pick_sources(host, 64)
+    ref = hc.Graph.from_host(host)
+    depth, dist = ref.bfs(src, want_parent=False)[0], ref.sssp(src)[0]
+    ref.close()
+    for i in (0, 63):
+        assert np.array_equal(depth[i], oracle.bfs_depth(host.index, host.neighbors, src[i]))
+        assert np.array_equal(dist[i], oracle.sssp_dijkstra(host.index, host.neighbors, host.weights, src[i]))
+    return host, src, depth, dist
+
+
+def _fill(torch, leave):
+    """Takes all but `leave` bytes of the device's free memory."""
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    free, _ = torch.cuda.mem_get_info()
+    return torch.empty(max(free - leave, 0), dtype=torch.uint8, device="cuda")
+
+
+@pytest.mark.parametrize("host_out", [False, True])
+def test_bfs_beside_the_sssp_workspace(weighted20, host_out):
+    """After hc_sssp with many sources, whose workspaces stay, hc_bfs fits where one source of each does."""
+    torch = pytest.importorskip("torch")
+    host, src, depth, _ = weighted20
+    g = hc.Graph.from_host(host)
+    out = torch.empty((64, host.num_nodes), dtype=torch.int32, device="cuda")
+    g.sssp(src, out)
+    got = np.empty((64, host.num_nodes), np.int32) if host_out else out
+    filler = _fill(torch, 12 << 20)  # a BFS workspace of one source takes more
+    try:
+        g.bfs(src, got, want_parent=False)
+    finally:
+        del filler
+        torch.cuda.empty_cache()
+    assert np.array_equal(got if host_out else got.cpu().numpy(), depth)
+    g.close()
+
+
+@pytest.mark.parametrize("room_mb", [60, 150, 400, 700])
+@pytest.mark.parametrize("op", ["bfs", "sssp"])
+def test_host_outputs_when_staging_does_not_fit(weighted20, op, room_mb):
+    """Workspaces and staging of several sources are given back when only a part of them can be had."""
+    torch = pytest.importorskip("torch")
+    host, src, depth, dist = weighted20
+    g = hc.Graph.from_host(host)
+    g.sssp(src[:1])
+    g.bfs(src[:1])
+    filler = _fill(torch, room_mb << 20)
+    try:
+        got = g.bfs(src, want_parent=False)[0] if op == "bfs" else g.sssp(src)[0]
+    finally:
+        del filler
+        torch.cuda.empty_cache()
+    assert np.array_equal(got, depth if op == "bfs" else dist)
+    g.close()
