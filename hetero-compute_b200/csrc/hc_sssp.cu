@@ -1358,7 +1358,7 @@ extern "C" hc_status hc_sssp(hc_graph *g, const int32_t *sources, int32_t num_so
                              int32_t *parent_out, const hc_sssp_opts *opts, hc_sssp_stats *stats) {
     clear_error();
     HC_TRY(activate(g));
-    ReclaimScope reclaim_scope(g, kKeepAdj | kKeepSssp);
+    ReclaimScope reclaim_scope(g, kKeepAdj);
     if (!sources || num_sources < 0) return fail(HC_ERR_INVALID_ARG, "hc_sssp: bad source list");
     if (g->wtype != HC_W_I32) return fail(HC_ERR_UNSUPPORTED, "hc_sssp: graph needs int32 edge weights");
     hc_sssp_opts o{};
@@ -1377,6 +1377,15 @@ extern "C" hc_status hc_sssp(hc_graph *g, const int32_t *sources, int32_t num_so
     HC_TRY(ensure_weight_stats(g));
     if (g->w_negative) return fail(HC_ERR_INVALID_ARG, "hc_sssp: negative edge weight");
     HC_TRY(ensure_base_plan(g));
+    // Zero fields: the handle's tuned values, else the defaults.
+    // The pull sweep reads w(u->v) from v's row: only valid when weights are symmetric.
+    if (o.pull_alpha == 0) o.pull_alpha = g->tune.sssp_pull_alpha;
+    if (o.delta == 0) o.delta = g->tune.sssp_delta;
+    const int pull_alpha =
+        !g->w_symmetric ? 0 : (o.pull_alpha == 0 ? kDefaultPullAlpha : std::max(o.pull_alpha, 0));
+    // Before the workspaces, which can do with one source's where the pair array
+    // cannot be had smaller.
+    if (pull_alpha > 0) HC_TRY(ensure_weight_order(g));
 
     const int64_t n = g->N;
     const int64_t W = (n + 31) / 32;
@@ -1412,11 +1421,20 @@ extern "C" hc_status hc_sssp(hc_graph *g, const int32_t *sources, int32_t num_so
         sssp_teams(g, resident, num_sources,
                    (int)std::min<size_t>(std::max<size_t>(kSsspTeamBytes / each, 1), 1 << 20), &team, &teams);
     }
-    hc_status reserved = reserve();
-    if (reserved == HC_ERR_OOM && teams > 1) {  // no room for several: one at a time
+    hc_status reserved;
+    {
+        ReclaimScope nothing(nullptr, 0u);
+        reserved = reserve();
+    }
+    if (reserved == HC_ERR_OOM) {  // no room: one source at a time, and what other calls left behind goes
         clear_error();
-        sssp_teams(g, resident, num_sources, 1, &team, &teams);
-        g->ws_sssp.release();
+        if (teams > 1) {
+            sssp_teams(g, resident, num_sources, 1, &team, &teams);
+            g->ws_sssp.release();
+            if (!dist_out) g->ws_out0.release();
+            OutPipe::drop_staging(g);
+        }
+        ReclaimScope own_scope(g, kKeepAdj | kKeepSssp);
         reserved = reserve();
     }
     HC_TRY(reserved);
@@ -1448,13 +1466,8 @@ extern "C" hc_status hc_sssp(hc_graph *g, const int32_t *sources, int32_t num_so
     a.team_stride = bytes;
     a.plan = g->base_view;
     a.max_epochs = o.max_epochs > 0 ? o.max_epochs : 0x7fffffff;
-    // The pull sweep reads w(u->v) from v's row: only valid when weights are symmetric.
-    // Zero fields: the handle's tuned values, else the defaults.
-    if (o.pull_alpha == 0) o.pull_alpha = g->tune.sssp_pull_alpha;
-    if (o.delta == 0) o.delta = g->tune.sssp_delta;
-    a.pull_alpha = !g->w_symmetric ? 0 : (o.pull_alpha == 0 ? kDefaultPullAlpha : std::max(o.pull_alpha, 0));
+    a.pull_alpha = pull_alpha;
     if (a.pull_alpha > 0) {
-        HC_TRY(ensure_weight_order(g));
         a.adj = g->sssp_adj.as<int2>();
         a.ws = weight_shift(g->w_max);
     }

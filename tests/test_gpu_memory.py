@@ -84,6 +84,25 @@ def test_bfs_beside_the_sssp_workspace(weighted20, host_out):
     g.close()
 
 
+@pytest.mark.parametrize("room", [1.15, 2.0, 3.5])
+def test_sssp_pair_array_before_many_workspaces(weighted20, room):
+    """The first call with pulls on a nearly full device: the pair array is built, and the workspaces of several
+    sources shrink to one where both do not fit."""
+    torch = pytest.importorskip("torch")
+    host, src, _, dist = weighted20
+    g = hc.Graph.from_host(host)
+    out = torch.empty((64, host.num_nodes), dtype=torch.int32, device="cuda")
+    g.sssp(src[:1], out[:1], pull_alpha=-1)  # weight statistics, row plan, one workspace
+    filler = _fill(torch, int(room * 8 * host.num_edges) + (8 << 20))
+    try:
+        g.sssp(src, out)
+    finally:
+        del filler
+        torch.cuda.empty_cache()
+    assert np.array_equal(out.cpu().numpy(), dist)
+    g.close()
+
+
 @pytest.mark.parametrize("room_mb", [60, 150, 400, 700])
 @pytest.mark.parametrize("op", ["bfs", "sssp"])
 def test_host_outputs_when_staging_does_not_fit(weighted20, op, room_mb):
