@@ -86,7 +86,7 @@ struct hc_graph {
     hc::DevBuf inv_wsum;       // f32[N]: 1/sum_k w_uk (weighted PageRank)
     hc::DevBuf wtn;            // f32[M]: slot (v,i) holds w_{u v}/sum_k w_uk, u = nbr[v][i]
     hc::DevBuf wf32;           // f32[M]: int32 weights as floats (weighted PageRank on int32 graphs)
-    hc::DevBuf pr_plan;        // row plan (device arrays)
+    hc::DevBuf pr_plan;        // row plan (device arrays; empty where base_plan is the same)
     hc::PrPlanDev pr_view{};   // host copy of its pointers and counts
     int32_t pr_partial_slots = 0;
     hc::DevBuf base_plan;      // the plan of 2048 edges (SSSP pull, adjoint)
@@ -203,10 +203,12 @@ hc_status edge_symmetry(hc_graph *g, const uint32_t *wbits, bool *structure, boo
 // The edge weights as fp32 for weighted PageRank: the weight array itself
 // (fp32 graphs) or its converted copy (int32 graphs, built by ensure_pr_derived).
 const float *pr_weights(const hc_graph *g);
-// Builds the PageRank row plan (g->pr_view, g->pr_partial_slots) or the plan of
-// 2048 edges (g->base_view, g->base_partial_slots) if missing.
-hc_status ensure_plan(hc_graph *g);
-hc_status ensure_base_plan(hc_graph *g);
+// Builds those of the row plans that are missing: PageRank's (g->pr_view,
+// g->pr_partial_slots), the plan of 2048 edges (g->base_view,
+// g->base_partial_slots), the multi-column one (g->spmm_view,
+// g->spmm_partial_slots).
+enum : unsigned { kPlanPr = 1u, kPlanBase = 2u, kPlanSpmm = 4u };
+hc_status ensure_plans(hc_graph *g, unsigned which);
 // Computes w_negative, w_max, w_mean and w_symmetric once (int32 weights).
 hc_status ensure_weight_stats(hc_graph *g);
 // Per-run control traffic kept off the copy engines.  A host-output call

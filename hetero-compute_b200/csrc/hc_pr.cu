@@ -19,6 +19,9 @@
 #include <algorithm>
 #include <cmath>
 #include <cstddef>
+#include <cstring>
+#include <memory>
+#include <new>
 #include <vector>
 
 #include "hc_graph.cuh"
@@ -768,119 +771,118 @@ int64_t plan_size(int64_t m, int64_t per) {
     return x;
 }
 
-hc_status build_plan(hc_graph *g, int64_t stream_edges, int64_t chunk, DevBuf *buf, PrPlanDev *view,
-                     int32_t *slots) {
-    const int32_t na = g->n_active;
-    std::vector<int64_t> idx((size_t)na + 1);
-    HC_CUDA_TRY(cudaMemcpy(idx.data(), g->index.as<int64_t>(), sizeof(int64_t) * ((size_t)na + 1),
-                           cudaMemcpyDeviceToHost));
-    std::vector<int32_t> stream, longrows;
+// A plan's device arrays go up in one copy.
+struct PlanPack {
+    std::vector<char> host;
+    template <class T>
+    size_t add(const std::vector<T> &v) {
+        const size_t at = host.size(), bytes = v.size() * sizeof(T);
+        host.resize(at + (bytes + 255) / 256 * 256);
+        if (bytes) std::memcpy(host.data() + at, v.data(), bytes);
+        return at;
+    }
+    hc_status upload(DevBuf *buf) const {
+        HC_TRY(buf->ensure(host.size() + 256));
+        if (!host.empty()) HC_CUDA_TRY(cudaMemcpy(buf->ptr, host.data(), host.size(), cudaMemcpyHostToDevice));
+        return HC_OK;
+    }
+};
+
+// Rows longer than `least` edges in chunks: (hub index, chunk) tasks and the hubs' partial sums.
+struct HubTasks {
     std::vector<int2> tasks;
     std::vector<HubInfo> hubs;
-    int32_t partial_slots = 0;
+    int32_t slots = 0;
+    void add(int32_t r, int64_t deg, int64_t chunk) {
+        HubInfo h{r, slots, (int32_t)((deg + chunk - 1) / chunk), 0};
+        for (int c = 0; c < h.nchunks; c++) tasks.push_back(make_int2((int)hubs.size(), c));
+        slots += h.nchunks;
+        hubs.push_back(h);
+    }
+};
+
+hc_status build_plan(const int64_t *idx, int32_t na, int64_t stream_edges, int64_t chunk, DevBuf *buf,
+                     PrPlanDev *view, int32_t *slots) {
+    std::vector<int32_t> stream, longrows;
+    HubTasks hub;
     const int32_t ngroups = (na + 31) / 32;
     for (int32_t gid = 0; gid < ngroups; gid++) {
         const int32_t r0 = gid * 32, r1 = std::min(r0 + 32, na);
-        const int64_t tot = idx[r1] - idx[r0];
-        if (tot <= stream_edges) {
+        if (idx[r1] - idx[r0] <= stream_edges) {
             stream.push_back(gid);
             continue;
         }
         for (int32_t r = r0; r < r1; r++) {
             const int64_t d = idx[r + 1] - idx[r];
-            if (d > 2 * chunk) {
-                HubInfo h{r, partial_slots, (int32_t)((d + chunk - 1) / chunk), 0};
-                for (int c = 0; c < h.nchunks; c++) tasks.push_back(make_int2((int)hubs.size(), c));
-                partial_slots += h.nchunks;
-                hubs.push_back(h);
-            } else {
-                longrows.push_back(r);
-            }
+            if (d > 2 * chunk) hub.add(r, d, chunk);
+            else longrows.push_back(r);
         }
     }
-    auto up = [](size_t b) { return (b + 255) / 256 * 256; };
-    const size_t b_stream = up(stream.size() * 4), b_long = up(longrows.size() * 4);
-    const size_t b_tasks = up(tasks.size() * sizeof(int2)), b_hubs = up(hubs.size() * sizeof(HubInfo));
-    HC_TRY(buf->ensure(b_stream + b_long + b_tasks + b_hubs + 256));
-    char *p = buf->as<char>();
-    PrPlanDev v{};
-    v.n_stream = (int)stream.size();
-    v.n_long = (int)longrows.size();
-    v.n_tasks = (int)tasks.size();
-    v.n_hub = (int)hubs.size();
-    v.chunk = (int)chunk;
-    v.stream = (const int32_t *)p;
-    if (!stream.empty()) HC_CUDA_TRY(cudaMemcpy(p, stream.data(), stream.size() * 4, cudaMemcpyHostToDevice));
-    p += b_stream;
-    v.longrows = (const int32_t *)p;
-    if (!longrows.empty()) HC_CUDA_TRY(cudaMemcpy(p, longrows.data(), longrows.size() * 4, cudaMemcpyHostToDevice));
-    p += b_long;
-    v.tasks = (const int2 *)p;
-    if (!tasks.empty()) HC_CUDA_TRY(cudaMemcpy(p, tasks.data(), tasks.size() * sizeof(int2), cudaMemcpyHostToDevice));
-    p += b_tasks;
-    v.hubs = (const HubInfo *)p;
-    if (!hubs.empty()) HC_CUDA_TRY(cudaMemcpy(p, hubs.data(), hubs.size() * sizeof(HubInfo), cudaMemcpyHostToDevice));
-    *view = v;
-    *slots = partial_slots;
+    PlanPack pack;
+    const size_t at_stream = pack.add(stream), at_long = pack.add(longrows);
+    const size_t at_tasks = pack.add(hub.tasks), at_hubs = pack.add(hub.hubs);
+    HC_TRY(pack.upload(buf));
+    const char *p = buf->as<char>();
+    *view = PrPlanDev{(const int32_t *)(p + at_stream), (const int32_t *)(p + at_long), (const int2 *)(p + at_tasks),
+                      (const HubInfo *)(p + at_hubs), (int)stream.size(), (int)longrows.size(),
+                      (int)hub.tasks.size(), (int)hub.hubs.size(), (int)chunk};
+    *slots = hub.slots;
+    return HC_OK;
+}
+
+// The multi-column sweeps' row plan.  A chunk is M / 65536 edges rounded down to
+// a power of two, in [512, 2048]: a chunk is a serial chain of its warp, and its
+// partial sums take a row of columns each.
+hc_status build_spmm_plan(hc_graph *g, const int64_t *idx) {
+    const int32_t na = g->n_active;
+    int64_t chunk = 512;
+    while (chunk < 2048 && chunk * 2 * 65536 <= g->M) chunk *= 2;
+    std::vector<int32_t> longs;
+    HubTasks hub;
+    for (int32_t r = 0; r < na; r++) {
+        const int64_t d = idx[r + 1] - idx[r];
+        if (d > chunk) hub.add(r, d, chunk);
+        else if (d > kSpmmLong) longs.push_back(r);
+        else if (g->degree_sorted) break;  // every later row is short too
+    }
+    PlanPack pack;
+    const size_t at_long = pack.add(longs), at_tasks = pack.add(hub.tasks), at_hubs = pack.add(hub.hubs);
+    HC_TRY(pack.upload(&g->spmm_plan));
+    const char *p = g->spmm_plan.as<char>();
+    g->spmm_view = SpmmPlanDev{(const int32_t *)(p + at_long), (const int2 *)(p + at_tasks),
+                               (const HubInfo *)(p + at_hubs), (int)longs.size(), (int)hub.tasks.size(),
+                               (int)hub.hubs.size(), (int)chunk};
+    g->spmm_partial_slots = hub.slots;
     return HC_OK;
 }
 }  // namespace
 
-hc_status ensure_plan(hc_graph *g) {
-    if (g->pr_plan.ptr) return HC_OK;
-    return build_plan(g, plan_size(g->M, 8192), plan_size(g->M, 4096), &g->pr_plan, &g->pr_view, &g->pr_partial_slots);
-}
-
-hc_status ensure_base_plan(hc_graph *g) {
-    if (g->base_plan.ptr) return HC_OK;
-    return build_plan(g, kMaxChunk, kMaxChunk, &g->base_plan, &g->base_view, &g->base_partial_slots);
-}
-
-// The multi-column sweeps' row plan, built on the first such call.  A chunk is M
-// / 65536 edges rounded down to a power of two, in [512, 2048]: a chunk is a
-// serial chain of its warp, and its partial sums take a row of columns each.
-hc_status ensure_spmm_plan(hc_graph *g) {
-    if (g->spmm_plan.ptr) return HC_OK;
+// One read of the offsets serves every plan that a call lacks.
+hc_status ensure_plans(hc_graph *g, unsigned which) {
+    const int64_t stream_edges = plan_size(g->M, 8192), chunk = plan_size(g->M, 4096);
+    // From 2^24 edges on the two plans are one.
+    const bool same = stream_edges == kMaxChunk && chunk == kMaxChunk;
+    if ((which & kPlanPr) && same) which = (which & ~kPlanPr) | kPlanBase;
+    if (g->pr_plan.ptr) which &= ~kPlanPr;
+    if (g->base_plan.ptr) which &= ~kPlanBase;
+    if (g->spmm_plan.ptr) which &= ~kPlanSpmm;
+    if (!which) return HC_OK;
     const int32_t na = g->n_active;
-    std::vector<int64_t> idx((size_t)na + 1);
-    HC_CUDA_TRY(cudaMemcpy(idx.data(), g->index.as<int64_t>(), sizeof(int64_t) * ((size_t)na + 1),
+    // Not a vector: clearing it first takes as long as the copy.
+    std::unique_ptr<int64_t[]> idx(new (std::nothrow) int64_t[(size_t)na + 1]);
+    if (!idx) return fail(HC_ERR_OOM, "row plans: no host memory for %d offsets", na + 1);
+    HC_CUDA_TRY(cudaMemcpy(idx.get(), g->index.as<int64_t>(), sizeof(int64_t) * ((size_t)na + 1),
                            cudaMemcpyDeviceToHost));
-    int64_t chunk = 512;
-    while (chunk < 2048 && chunk * 2 * 65536 <= g->M) chunk *= 2;
-    std::vector<int32_t> longs;
-    std::vector<int2> tasks;
-    std::vector<HubInfo> hubs;
-    int32_t slots = 0;
-    for (int32_t r = 0; r < na; r++) {
-        const int64_t d = idx[r + 1] - idx[r];
-        if (d > chunk) {
-            HubInfo h{r, slots, (int32_t)((d + chunk - 1) / chunk), 0};
-            for (int c = 0; c < h.nchunks; c++) tasks.push_back(make_int2((int)hubs.size(), c));
-            slots += h.nchunks;
-            hubs.push_back(h);
-        } else if (d > kSpmmLong) {
-            longs.push_back(r);
+    if (which & kPlanPr)
+        HC_TRY(build_plan(idx.get(), na, stream_edges, chunk, &g->pr_plan, &g->pr_view, &g->pr_partial_slots));
+    if (which & kPlanBase) {
+        HC_TRY(build_plan(idx.get(), na, kMaxChunk, kMaxChunk, &g->base_plan, &g->base_view, &g->base_partial_slots));
+        if (same) {
+            g->pr_view = g->base_view;
+            g->pr_partial_slots = g->base_partial_slots;
         }
     }
-    auto up = [](size_t b) { return (b + 255) / 256 * 256; };
-    const size_t b_long = up(longs.size() * 4), b_tasks = up(tasks.size() * sizeof(int2));
-    HC_TRY(g->spmm_plan.ensure(b_long + b_tasks + up(hubs.size() * sizeof(HubInfo)) + 256));
-    char *p = g->spmm_plan.as<char>();
-    SpmmPlanDev v{};
-    v.longs = (const int32_t *)p;
-    v.tasks = (const int2 *)(p + b_long);
-    v.hubs = (const HubInfo *)(p + b_long + b_tasks);
-    if (!longs.empty()) HC_CUDA_TRY(cudaMemcpy(p, longs.data(), longs.size() * 4, cudaMemcpyHostToDevice));
-    if (!tasks.empty()) {
-        HC_CUDA_TRY(cudaMemcpy(p + b_long, tasks.data(), tasks.size() * sizeof(int2), cudaMemcpyHostToDevice));
-        HC_CUDA_TRY(cudaMemcpy(p + b_long + b_tasks, hubs.data(), hubs.size() * sizeof(HubInfo), cudaMemcpyHostToDevice));
-    }
-    v.n_long = (int)longs.size();
-    v.n_tasks = (int)tasks.size();
-    v.n_hub = (int)hubs.size();
-    v.chunk = (int)chunk;
-    g->spmm_view = v;
-    g->spmm_partial_slots = slots;
+    if (which & kPlanSpmm) HC_TRY(build_spmm_plan(g, idx.get()));
     return HC_OK;
 }
 
@@ -902,11 +904,6 @@ void launch_spmm_cols(hc_graph *g, const SpmmArgs &a, const uint8_t *is_seed) {
 void launch_spmm(hc_graph *g, const SpmmArgs &a, const uint8_t *is_seed) {
     if (a.ew) launch_spmm_cols<true>(g, a, is_seed);
     else launch_spmm_cols<false>(g, a, is_seed);
-}
-
-PrPlanDev plan_view(hc_graph *g, int *partial_slots) {
-    *partial_slots = g->pr_partial_slots;
-    return g->pr_view;
 }
 
 // A cooperative launch of `fn` over the row plan's items: no more blocks than a
@@ -1338,9 +1335,11 @@ extern "C" hc_status hc_pr_forward(hc_graph *g, const float *teleport, int32_t n
     HC_TRY(after_default_stream(g));
     const bool weighted = o.weighted != 0;
     HC_TRY(ensure_pr_derived(g, weighted));
-    HC_TRY(ensure_plan(g));
-    int partial_slots = 0;
-    PrPlanDev plan = plan_view(g, &partial_slots);
+    // A single-column call builds the adjoint's plan too: a training step wants both,
+    // and the offsets are read once.
+    HC_TRY(ensure_plans(g, ncols > 1 ? kPlanSpmm : kPlanPr | kPlanBase));
+    const int partial_slots = g->pr_partial_slots;
+    const PrPlanDev plan = g->pr_view;
     const int64_t n = g->N;
     HC_TRY(g->ws_ctl.ensure(sizeof(IterState) + 4096));
 
@@ -1348,7 +1347,6 @@ extern "C" hc_status hc_pr_forward(hc_graph *g, const float *teleport, int32_t n
         // Dense multi-column form.
         const int K = ncols;
         if (K > 256) return fail(HC_ERR_UNSUPPORTED, "hc_pr_forward: at most 256 columns per call");
-        HC_TRY(ensure_spmm_plan(g));
         const int S = spmm_stride(K);
         const size_t nk = (size_t)n * S;
         const size_t slots = (size_t)g->spmm_partial_slots + 1;
@@ -1514,7 +1512,7 @@ extern "C" hc_status hc_pr_backward(hc_graph *g, const float *scores, const floa
     HC_TRY(after_default_stream(g));
     const bool weighted = o.weighted != 0;
     HC_TRY(ensure_pr_derived(g, weighted));
-    HC_TRY(ensure_base_plan(g));
+    HC_TRY(ensure_plans(g, kPlanBase));
     const int partial_slots = g->base_partial_slots;
     const PrPlanDev plan = g->base_view;
     const int64_t n = g->N;
@@ -1637,9 +1635,9 @@ extern "C" hc_status hc_ppr_batched(hc_graph *g, const int32_t *seed_offsets, co
     if (stats) std::memset(stats, 0, sizeof(*stats));
     const bool weighted = o.weighted != 0;
     HC_TRY(ensure_pr_derived(g, weighted));
-    HC_TRY(ensure_plan(g));
-    int partial_slots = 0;
-    PrPlanDev plan = plan_view(g, &partial_slots);
+    HC_TRY(ensure_plans(g, kPlanPr | kPlanSpmm));
+    const int partial_slots = g->pr_partial_slots;
+    const PrPlanDev plan = g->pr_view;
     std::vector<int32_t> off(ncols + 1);
     HC_CUDA_TRY(cudaMemcpy(off.data(), seed_offsets, sizeof(int32_t) * (ncols + 1), cudaMemcpyDefault));
     if (off[0] != 0) return fail(HC_ERR_INVALID_ARG, "hc_ppr_batched: seed_offsets[0] must be 0");
@@ -1652,7 +1650,6 @@ extern "C" hc_status hc_ppr_batched(hc_graph *g, const int32_t *seed_offsets, co
         if (s < 0 || s >= g->N) return fail(HC_ERR_INVALID_ARG, "hc_ppr_batched: seed %d out of range", s);
     const int K = ncols;
     const int64_t n = g->N;
-    HC_TRY(ensure_spmm_plan(g));
     const int S = spmm_stride(K);
     const size_t nk = (size_t)n * K, ns = (size_t)n * S;
     // One column's partial sums and counters (the tail's sweeps) fit these too.

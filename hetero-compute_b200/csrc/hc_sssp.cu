@@ -1376,7 +1376,7 @@ extern "C" hc_status hc_sssp(hc_graph *g, const int32_t *sources, int32_t num_so
     // Weights must be non-negative; the mean weight sets the default delta.
     HC_TRY(ensure_weight_stats(g));
     if (g->w_negative) return fail(HC_ERR_INVALID_ARG, "hc_sssp: negative edge weight");
-    HC_TRY(ensure_base_plan(g));
+    HC_TRY(ensure_plans(g, kPlanBase));
     // Zero fields: the handle's tuned values, else the defaults.
     // The pull sweep reads w(u->v) from v's row: only valid when weights are symmetric.
     if (o.pull_alpha == 0) o.pull_alpha = g->tune.sssp_pull_alpha;
