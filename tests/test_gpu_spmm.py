@@ -93,3 +93,31 @@ def test_single_column_against_two(kind, scale):
     capped, st = g.pagerank(None, tol_l1=TOL, max_iters=2)
     assert st.iterations == 2 and not st.converged
     g.close()
+
+
+@pytest.mark.parametrize("k", [2, 3, 4, 7, 33, 130, 255])
+def test_host_and_device_matrices(k):
+    """Teleport and scores in host or device memory, and one matrix for both: the same scores."""
+    import torch
+
+    import hc
+    h = hc.gen_kronecker(9, 16, 3)
+    g = hc.Graph.from_host(h)
+    t = np.random.default_rng(k).random((h.num_nodes, k)).astype(np.float32)
+    t /= t.sum(0)
+    opts = dict(tol_l1=1e-6, max_iters=100)
+    want, st = g.pagerank(t, **opts)
+    for tele_dev in (False, True):
+        for out_dev in (False, True):
+            tele = torch.from_numpy(t).cuda() if tele_dev else t
+            out = torch.full((h.num_nodes, k), 7.0, device="cuda") if out_dev else np.full_like(t, 7.0)
+            got, st1 = g.pagerank(tele, out, **opts)
+            got = got.cpu().numpy() if out_dev else got
+            assert st1.iterations == st.iterations and np.array_equal(got, want)
+    both = torch.from_numpy(t).cuda()
+    g.pagerank(both, both, **opts)
+    assert np.array_equal(both.cpu().numpy(), want)
+    both = t.copy()
+    g.pagerank(both, both, **opts)
+    assert np.array_equal(both, want)
+    g.close()
