@@ -43,14 +43,15 @@ struct PrPlanDev {
 // Row plan of the multi-column PageRank sweeps:
 //   tasks   chunks of rows longer than one chunk (hub index, chunk)
 //   longs   rows of more than kSpmmLong edges, a warp each
-//   the rest, kSpmmRows consecutive rows to a warp
+//   the rest, `rows` consecutive rows to a warp: as many as make about a warp's
+//   work of each (at most kSpmmRows)
 constexpr int kSpmmLong = 64;
 constexpr int kSpmmRows = 8;
 struct SpmmPlanDev {
     const int32_t *longs;
     const int2 *tasks;
     const HubInfo *hubs;
-    int n_long, n_tasks, n_hub, chunk;
+    int n_long, n_tasks, n_hub, chunk, rows;
 };
 }  // namespace hc
 

@@ -583,7 +583,7 @@ __global__ void __launch_bounds__(kPrThreads) spmm_sweep(SpmmArgs a, SpmmPlanDev
             }
         }
     };
-    const int total = plan.n_tasks + plan.n_long + (a.n_active + kSpmmRows - 1) / kSpmmRows;
+    const int total = plan.n_tasks + plan.n_long + (a.n_active + plan.rows - 1) / plan.rows;
     for (int item = gwarp; item < total; item += nwarps) {
         float4 acc[kVec];
         clear(acc);
@@ -629,8 +629,8 @@ __global__ void __launch_bounds__(kPrThreads) spmm_sweep(SpmmArgs a, SpmmPlanDev
             combine(acc);
             if (sub == 0) finish(r, acc);
         } else {
-            const int32_t r0 = (item - plan.n_tasks - plan.n_long) * kSpmmRows;
-            const int nr = min(kSpmmRows, a.n_active - r0);
+            const int32_t r0 = (item - plan.n_tasks - plan.n_long) * plan.rows;
+            const int nr = min(plan.rows, a.n_active - r0);
             const int64_t start = __ldg(a.index + r0 + min(lane, nr));
             const int64_t deg = __shfl_down_sync(kFull, start, 1) - start;
             if (!__any_sync(kFull, lane < nr && deg <= kSpmmLong)) continue;
@@ -862,13 +862,18 @@ hc_status build_spmm_plan(hc_graph *g, const int64_t *idx) {
         else if (d > kSpmmLong) longs.push_back(r);
         else if (g->degree_sorted) break;  // every later row is short too
     }
+    // Eight warps a block, eight blocks an SM (launch_spmm_cols).  On a small graph a
+    // sweep is the longest warp's chain, and eight rows one after the other are most
+    // of it (uniform, 2^11 vertices, three seeds a column: 200 columns 1350 us a solve, 410
+    // us so, 64 columns 493 and 356).
+    const int rows = (int)std::max<int64_t>(1, std::min<int64_t>(kSpmmRows, na / ((int64_t)g->sm_count * 64)));
     PlanPack pack;
     const size_t at_long = pack.add(longs), at_tasks = pack.add(hub.tasks), at_hubs = pack.add(hub.hubs);
     HC_TRY(pack.upload(&g->spmm_plan));
     const char *p = g->spmm_plan.as<char>();
     g->spmm_view = SpmmPlanDev{(const int32_t *)(p + at_long), (const int2 *)(p + at_tasks),
                                (const HubInfo *)(p + at_hubs), (int)longs.size(), (int)hub.tasks.size(),
-                               (int)hub.hubs.size(), (int)chunk};
+                               (int)hub.hubs.size(), (int)chunk, rows};
     g->spmm_partial_slots = hub.slots;
     return HC_OK;
 }

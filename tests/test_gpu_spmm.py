@@ -121,3 +121,25 @@ def test_host_and_device_matrices(k):
     g.pagerank(both, both, **opts)
     assert np.array_equal(both, want)
     g.close()
+
+
+@pytest.mark.parametrize("n", [9471, 18943, 18944, 28417, 47363, 66304, 75775, 75776])
+def test_rows_per_warp(n):
+    """Vertex counts at which a warp takes another number of short rows, against the single-column solve (bounds as
+    above)."""
+    import hc
+    rng = np.random.default_rng(n)
+    u, v = rng.integers(0, n, 4 * n), rng.integers(0, n, 4 * n)
+    key = np.unique(np.concatenate([u * n + v, v * n + u])[np.concatenate([u != v, u != v])])
+    index = np.zeros(n + 1, np.int64)
+    np.cumsum(np.bincount(key // n, minlength=n), out=index[1:])
+    g = hc.Graph(index, (key % n).astype(np.int32))
+    t = rng.random((n, 2)).astype(np.float32)
+    t /= t.sum(0)
+    opts = dict(tol_l1=TOL, max_iters=200)
+    one = [g.pagerank(np.ascontiguousarray(t[:, i]), **opts)[0] for i in (0, 1)]
+    for k in (2, 6, 19, 67, 140):
+        x = g.pagerank(np.ascontiguousarray(t[:, np.arange(k) % 2]), **opts)[0]
+        for c in {0, 1, k // 2, k - 1}:
+            assert np.abs(x[:, c] - one[c % 2]).sum() <= 2 * TOL * DAMPING / (1 - DAMPING) + 100 * 2.0 ** -23
+    g.close()
