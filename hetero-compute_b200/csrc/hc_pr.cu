@@ -39,12 +39,12 @@ constexpr int kMaxIterSlots = 4096;
 struct IterSlot {
     double l1;       // Jacobi: sum |change|; conjugate gradients: p . q
     double rz, z1;   // conjugate gradients: r . z, sum |z|
-    int changed;
-    int pause;       // the launch ends after this iteration (see pr_solve)
+    int changed, pad;
 };
 struct IterState {
     GridSync gs;
     int done, blocks_done;   // sweeps launched one by one
+    int pause_after, pad;    // 1 + the iteration after which the launch ends (see past_run_limit)
     IterSlot slot[kMaxIterSlots];
 };
 // What a solve reports, in mapped host memory.  done: 1 converged, 2 stopped, 0
@@ -247,6 +247,19 @@ __device__ __forceinline__ void sweep_rows(const SweepArgs &a, const PrPlanDev &
 
 }
 
+// Thread 0 of block 0, at the start of iteration `it`: once the launch has run for
+// the run limit, it ends after this iteration.  Every block reads pause_after
+// after the iteration's (first) barrier; by then block 0 may have moved on and
+// named a later iteration, so the number is compared.  In shared memory, and
+// before the sweep: the clock is slow to read, and a barrier's last arrival is
+// what everybody waits for.
+__device__ __forceinline__ void past_run_limit(IterState *st, int it, unsigned long long *s_start) {
+    if (blockIdx.x != 0 || threadIdx.x != 0) return;
+    const unsigned long long now = globaltimer_ns();
+    if (*s_start == 0ull) *s_start = now;
+    else if (now - *s_start > c_limits.run_ns) st->pause_after = it + 1;
+}
+
 // Adds the block's sums of l1 and chg to the iteration's slot (every thread calls it).
 __device__ __forceinline__ void add_residual(IterSlot *slot, float l1, int chg) {
     __shared__ double s_l1[kPrThreads / 32];
@@ -284,7 +297,9 @@ template <bool kEW, bool kRS, bool kPS, bool kBaseVec>
 __global__ void __launch_bounds__(kPrThreads, kPrBlocks) pr_solve(SweepArgs a, PrPlanDev plan) {
     __shared__ float s_acc[kPrThreads / 32][32];
     const double rho2 = (double)a.cheb_rho * a.cheb_rho;
-    const unsigned long long t_start = globaltimer_ns();
+    __shared__ unsigned long long s_start;
+    __shared__ bool s_done, s_paused;
+    if (threadIdx.x == 0) s_start = 0ull;
     double omega = a.first_omega;
     int it = a.first_iter, done = 0;
     bool ok = true, paused = false;
@@ -296,19 +311,24 @@ __global__ void __launch_bounds__(kPrThreads, kPrBlocks) pr_solve(SweepArgs a, P
                           (float)omega};
         float l1;
         int chg;
+        past_run_limit(a.st, it, &s_start);
         sweep_rows<kEW, kRS, kPS, kBaseVec>(a, plan, v, s_acc, l1, chg);
         IterSlot *const slot = &a.st->slot[it % kMaxIterSlots];
         add_residual(slot, l1, chg);
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
-            if (it + 2 >= kMaxIterSlots) a.st->slot[(it + 2) % kMaxIterSlots] = IterSlot{0.0, 0.0, 0.0, 0, 0};
-            if (globaltimer_ns() - t_start > c_limits.run_ns) slot->pause = 1;
-        }
+        if (it + 2 >= kMaxIterSlots && blockIdx.x == 0 && threadIdx.x == 0)
+            a.st->slot[(it + 2) % kMaxIterSlots] = IterSlot{0.0, 0.0, 0.0, 0, 0};
         if (!(ok = grid_barrier(&a.st->gs))) break;
-        // eps >= 3e38 marks the per-vertex rule as unused.
-        if ((a.tol_l1 > 0.f && __ldcg(&slot->l1) < (double)a.tol_l1) || (a.eps < 3e38f && __ldcg(&slot->changed) == 0))
-            done = 1;
-        paused = __ldcg(&slot->pause) != 0;
         it++;
+        if (threadIdx.x == 0) {  // one read a block: every warp's would queue at one L2 line
+            const double sum = __ldcg(&slot->l1);
+            const int moved = __ldcg(&slot->changed), pause_after = __ldcg(&a.st->pause_after);
+            // eps >= 3e38 marks the per-vertex rule as unused.
+            s_done = (a.tol_l1 > 0.f && sum < (double)a.tol_l1) || (a.eps < 3e38f && moved == 0);
+            s_paused = pause_after == it;
+        }
+        __syncthreads();
+        done = s_done;
+        paused = s_paused;
     }
     paused = paused && !done && it < a.max_iters;
     if (ok && !paused && a.final_x) {
@@ -1154,59 +1174,69 @@ __global__ void __launch_bounds__(kPrThreads, kPrBlocks) pr_cg(SweepArgs a, PrPl
     GridSync *const gs = &a.st->gs;
     float l1;
     int chg;
-    const unsigned long long t_start = globaltimer_ns();
+    __shared__ unsigned long long s_start;
+    if (threadIdx.x == 0) s_start = 0ull;
+    // The scalars of iteration it stay in slot it (as registers they would spill)
+    // and one thread a block reads them: every warp's reads would queue at one L2 line.
+    __shared__ float s_coef;  // alpha, then beta
+    __shared__ bool s_stop, s_paused;
     int iters = 0, converged = 0;
-    double rz = 0.0, z1 = 0.0, c1 = 0.0, tol = 0.0;
     bool ok = true, paused = false;
     if (q.first_iter == 0) {
         // S x by the pull sweep with each row's own weights; its residual is p . q.
         sweep_rows<kEW, false, false, false, true>(a, plan, SweepIter{q.lam, q.lam, q.sp, q.sp, 1.f}, s_acc, l1, chg);
         ok = grid_barrier(gs);
         if (ok) {
+            double rz = 0.0, z1 = 0.0, c1 = 0.0;
             cg_start_rows(a, q, gtid, nthreads, rz, z1, c1);
             add_dots(&a.st->slot[0], rz, z1);
             __syncthreads();
             c1 = block_sum(c1, s_c);
             if (threadIdx.x == 0 && c1 != 0.0) atomicAdd(&a.st->slot[0].l1, c1);
             ok = grid_barrier(gs);
+            converged = ok && (__ldcg(&a.st->slot[0].z1) < cg_tol(a, q) || __ldcg(&a.st->slot[0].rz) <= 0.0);
         }
     } else {
         iters = q.first_iter - 1;
     }
-    if (ok) {
-        rz = __ldcg(&a.st->slot[iters].rz);
-        z1 = __ldcg(&a.st->slot[iters].z1);
-        tol = cg_tol(a, q);
-        converged = q.first_iter == 0 && (z1 < tol || rz <= 0.0);
-    }
-    for (int it = iters + 1; ok && !converged && !paused && it <= a.max_iters; it++) {
-        IterSlot *const slot = &a.st->slot[it];
+    while (ok && !converged && !paused && iters < a.max_iters) {
+        IterSlot *const slot = &a.st->slot[iters + 1];
+        past_run_limit(a.st, iters + 1, &s_start);
         sweep_rows<kEW, false, false, false, true>(a, plan, SweepIter{q.p, q.p, q.sp, q.sp, 1.f}, s_acc, l1, chg);
         add_residual(slot, l1, 0);
         if (!(ok = grid_barrier(gs))) break;
-        const double pq = __ldcg(&slot->l1);
-        if (!(pq > 0.0)) break;  // p = 0 (already exact) or a breakdown: stop
+        if (threadIdx.x == 0) {
+            const double pq = __ldcg(&slot->l1), rz = __ldcg(&slot[-1].rz);
+            s_stop = !(pq > 0.0);  // p = 0 (already exact) or a breakdown
+            s_coef = (float)(rz / pq);
+        }
+        __syncthreads();
+        if (s_stop) break;
         double nrz = 0.0, nz1 = 0.0;
-        cg_update_rows(a, q, gtid, nthreads, (float)(rz / pq), nrz, nz1);
+        cg_update_rows(a, q, gtid, nthreads, s_coef, nrz, nz1);
         add_dots(slot, nrz, nz1);
         if (!(ok = grid_barrier(gs))) break;
-        nrz = __ldcg(&slot->rz);
-        z1 = __ldcg(&slot->z1);
-        const float beta = (float)(rz > 0.0 ? nrz / rz : 0.0);
-        rz = nrz;
         iters++;
-        converged = z1 < tol;
-        if (converged || it == a.max_iters) break;
-        cg_direction_rows(a, q, gtid, nthreads, beta);  // the same thread's entries as above
-        if (gtid == 0 && globaltimer_ns() - t_start > c_limits.run_ns) slot->pause = 1;
+        if (threadIdx.x == 0) {
+            const double rz = __ldcg(&slot[-1].rz), next = __ldcg(&slot->rz);
+            s_coef = (float)(rz > 0.0 ? next / rz : 0.0);
+            s_stop = __ldcg(&slot->z1) < cg_tol(a, q);
+            s_paused = __ldcg(&a.st->pause_after) == iters + 1;
+        }
+        __syncthreads();
+        converged = s_stop;
+        paused = s_paused;
+        if (converged || iters == a.max_iters) break;
+        // The same thread's entries as above.
+        cg_direction_rows(a, q, gtid, nthreads, s_coef);
         ok = grid_barrier(gs);
-        paused = ok && __ldcg(&slot->pause) != 0;
     }
+    paused = paused && !converged && iters < a.max_iters;
     if (gtid == 0) {
         a.out->err = *(volatile int *)&gs->err;
         a.out->iters = iters;
         a.out->done = paused ? 0 : converged ? 1 : 2;
-        a.out->l1 = z1;
+        a.out->l1 = __ldcg(&a.st->slot[iters].z1);
         a.out->changed = 0;
         __threadfence_system();
     }

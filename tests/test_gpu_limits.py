@@ -85,7 +85,7 @@ def test_loop_limit_ends_batched_groups(graph, use_graph):
                                   "adjoint_chebyshev", "ppr_tail"])
 def test_pagerank_goes_on_after_the_run_limit(graph, name):
     """A solve's launch ends after an iteration once run_ns has passed, and another goes on: at 1 ns there is a launch
-    per iteration, and the result is that of one launch."""
+    for every other iteration at least, and the result is that of one launch."""
     host, g = graph
     n = host.num_nodes
     rng = np.random.default_rng(5)
@@ -120,6 +120,6 @@ def test_pagerank_goes_on_after_the_run_limit(graph, name):
         assert (st1.iterations, st1.converged) == (st.iterations, st.converged)
         assert np.allclose(got, want, rtol=1e-5, atol=1e-9 if name != "adjoint" else 1e-5 * np.abs(want).max())
         if name != "ppr_tail":
-            assert launches >= whole + st.iterations - 2
+            assert launches >= whole + st.iterations // 2 - 1
         elif not extra:
-            assert launches >= whole + 20
+            assert launches >= whole + 10
