@@ -14,13 +14,22 @@ namespace hc {
 // no more than a few of those, they are short; on a large one they are long, as
 // a task ends with a fence and a counter and a warp per short row wastes lanes.
 //   chunk          M / 4096 edges rounded down to a power of two, in [256, 2048]
-//   stream group   at most M / 8192 edges, rounded likewise, in [256, 2048]
+//   stream group   at most M / 8192 edges, rounded likewise, in [256, 2048]; at
+//                  least 1024 when more than kMaxSingle1 rows in groups of up to
+//                  1024 edges would be single otherwise, and 2048 when more than
+//                  kMaxSingle2 in groups of 1024 to 2048 would: a warp a row of 16
+//                  to 64 edges is then many rounds of mostly idle lanes, where a
+//                  group is a few (uniform, ms a solve: 2^18 vertices, rows of 16,
+//                  0.57 with the limit at 512, 0.32 at 1024; rows of 48, 0.47 at
+//                  1024, 0.42 at 2048; 2^19, rows of 32, 0.69 and 0.65; but 2^14,
+//                  rows of 32, 0.10 at 256, 0.18 at 1024)
 // The SSSP pull (a lane per row) and the adjoint's conjugate gradients use the
 // plan of 2048 edges at every size.  The gradient of a weight is a difference of
 // two nearly equal numbers, so another order of the sums in the solve would show
 // in its last digits.
 constexpr int kMinChunk = 256;
 constexpr int kMaxChunk = 2048;
+constexpr int64_t kMaxSingle1 = 40000, kMaxSingle2 = 200000;
 // Batched SSSP keeps 16-bit distances when no weight exceeds this.
 constexpr int32_t kMsspNarrowMaxW = 0x0FFF;
 

@@ -843,6 +843,15 @@ hc_status build_plan(const int64_t *idx, int32_t na, int64_t stream_edges, int64
     std::vector<int32_t> stream, longrows;
     HubTasks hub;
     const int32_t ngroups = (na + 31) / 32;
+    // Rows that the limit would make single, in groups of up to 1024 and of up to 2048 edges.
+    int64_t rows1 = 0, rows2 = 0;
+    for (int32_t gid = 0; stream_edges < kMaxChunk && gid < ngroups; gid++) {
+        const int32_t r0 = gid * 32, r1 = std::min(r0 + 32, na);
+        const int64_t tot = idx[r1] - idx[r0];
+        if (tot > stream_edges && tot <= kMaxChunk) (tot <= kMaxChunk / 2 ? rows1 : rows2) += r1 - r0;
+    }
+    if (rows1 > kMaxSingle1) stream_edges = std::max<int64_t>(stream_edges, kMaxChunk / 2);
+    if (rows2 > kMaxSingle2) stream_edges = kMaxChunk;
     for (int32_t gid = 0; gid < ngroups; gid++) {
         const int32_t r0 = gid * 32, r1 = std::min(r0 + 32, na);
         if (idx[r1] - idx[r0] <= stream_edges) {
@@ -973,8 +982,13 @@ hc_status launch_solve(hc_graph *g, const void *fn, int *blocks_per_sm, SweepArg
 // edges without hub rows, whose sweeps miss L1 throughout (uniform, 33M edges: 1.19
 // ms so, 1.33 ms in one launch; at 8M edges both 0.48 ms).  With hubs one launch is
 // the faster at every size (Kronecker scale 22: 2.99 and 2.87 ms, scale 20: 0.94 and
-// 0.85 ms, scale 12: 0.35 and 0.09 ms).
-bool launched_sweeps(const hc_graph *g, const PrPlanDev &plan) { return plan.n_tasks == 0 && g->M >= (1ll << 24); }
+// 0.85 ms, scale 12: 0.35 and 0.09 ms).  Where nearly every
+// row is in a stream group, from 3 x 2^20 edges (uniform, 2^18 vertices, rows of 16:
+// 0.32 and 0.38 ms; 2^19: 0.47 and 0.55, rows of 32: 0.65 and 0.78; but 2^17, rows of
+// 16: 0.26 and 0.22, and 2^18, rows of 24, a quarter of them single: 0.38 and 0.35).
+bool launched_sweeps(const hc_graph *g, const PrPlanDev &plan) {
+    return plan.n_tasks == 0 && (g->M >= (1ll << 24) || (plan.n_long <= plan.n_stream && g->M >= (3ll << 20)));
+}
 
 using SolveFn = hc_status (*)(hc_graph *, SweepArgs &, const PrPlanDev &, volatile SolveOut *);
 
@@ -1096,6 +1110,12 @@ hc_status run_solve(hc_graph *g, SweepArgs a, const PrPlanDev &plan, SolveFn fn,
 // the loop around it (adjoint solve, Kronecker scale 20: 2.66 ms so, 3.09 ms in one
 // launch; scale 18: 1.18 and 1.00 ms).
 constexpr int64_t kCgLaunchEdges = 1ll << 23;
+// Without hub rows and with rows of up to 40 edges on average, from this many
+// (uniform, rows of 32: 2^16 vertices 0.56 ms so, 0.62 in one launch; 2^18 0.89 and
+// 1.02; rows of 16: 2^18 0.72 and 0.77, 2^17 0.58 and 0.56; but rows of 48: 2^17 0.62
+// and 0.55, 2^18 1.01 and 0.94).
+constexpr int64_t kCgFlatEdges = 2000000;
+constexpr int64_t kCgFlatRow = 40;
 
 struct CgArgs {
     const float *c;
@@ -1303,7 +1323,8 @@ __global__ void cg_direction(SweepArgs a, CgArgs q, int it) {
 
 template <bool kEW>
 hc_status launch_cg(hc_graph *g, SweepArgs &a, const PrPlanDev &plan, CgArgs &q, volatile SolveOut *out) {
-    if (g->M >= kCgLaunchEdges) {
+    const bool flat = plan.n_tasks == 0 && g->M >= kCgFlatEdges && g->M <= kCgFlatRow * g->n_active;
+    if (flat || g->M >= kCgLaunchEdges) {
         const int grid = g->sm_count * 4, sweep_grid = g->sm_count * kPrBlocks;
         auto sweep = [&](int it) { cg_sweep<kEW><<<sweep_grid, kPrThreads, 0, g->stream>>>(a, plan, q, it); ::hc::count_launch(); };
         auto direction = [&](int it) { cg_direction<<<grid, kPrThreads, 0, g->stream>>>(a, q, it); ::hc::count_launch(); };

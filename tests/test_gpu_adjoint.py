@@ -190,3 +190,47 @@ def test_adjoint_launch_forms(scale):
     _, _, st = g.pagerank_backward(x, c, dteleport=again, want_dw=False, tol_l1=1e-6, max_iters=3, weighted=True)
     assert st.iterations == 3 and not st.converged
     g.close()
+
+
+@pytest.mark.parametrize("kind,scale,degree", [("kronecker", 17, 16), ("kronecker", 19, 16), ("uniform", 15, 16),
+                                               ("uniform", 16, 16), ("uniform", 17, 24), ("uniform", 18, 8),
+                                               ("uniform", 18, 24)])
+@pytest.mark.parametrize("weighted", [True, False])
+def test_adjoint_per_vertex(kind, scale, degree, weighted):
+    """On both sides of the rules for one launch or one per phase, for one launch or one per sweep, and for rows by
+    the group or single: the forward and adjoint fixed-point equations per vertex in 64 bits, and the weight
+    gradients of every edge from the returned scores and teleport gradient."""
+    import torch
+
+    import hc
+    g = hc.Graph.generate(hc.GEN_KRONECKER if kind == "kronecker" else hc.GEN_UNIFORM, scale, degree, 1, hc.W_F32)
+    n, m = g.num_nodes, g.num_edges
+    index, nbr, w = (torch.from_numpy(a).cuda() for a in g.csr())
+    deg = index[1:] - index[:-1]
+    row, col = torch.repeat_interleave(torch.arange(n, device="cuda"), deg), nbr.long()
+    w = w.double() if weighted else torch.ones(m, dtype=torch.float64, device="cuda")
+    s = torch.zeros(n, dtype=torch.float64, device="cuda").index_add_(0, row, w)
+    linked = s > 0
+
+    def gather(y):  # sum over v's row of w y
+        return torch.zeros_like(s).index_add_(0, row, w * y[col])
+
+    c = torch.from_numpy(np.random.default_rng(scale).standard_normal(n).astype(np.float32)).cuda()
+    x, dt, dw = torch.empty(n, device="cuda"), torch.empty(n, device="cuda"), torch.empty(m, device="cuda")
+    o = dict(tol_l1=1e-6, max_iters=200, weighted=weighted)
+    _, st = g.pagerank(None, x, **o)
+    assert st.converged
+    x64, d, eps = x.double(), D, 2.0 ** -23
+    step = (1 - d) / n + d * gather(torch.where(linked, x64 / s, 0.0))
+    # A sweep's change is below the stop; a row's sum of fp32 terms adds its length in roundings at most.
+    assert float((step - x64)[linked].abs().sum()) <= 1e-6 + float((deg.clamp(max=2048) * eps * x64).sum())
+    _, _, st = g.pagerank_backward(x, c, dteleport=dt, dweights=dw, **o)
+    assert st.converged
+    lam, c64 = dt.double() / (1 - d), c.double()
+    z = torch.where(linked, c64 + d * gather(lam) / s.clamp(min=1e-30) - lam, c64 - lam)
+    assert float(z.abs().sum()) <= 1e-6 * float(c64.abs().sum()) + (st.iterations + 4) * 2 * eps * float(lam.abs().sum())
+    coef = torch.where(linked, x64 / s, 0.0)[row]
+    want = coef * (d * lam[col] - lam[row] + c64[row])
+    room = 4 * eps * coef * (d * lam[col].abs() + lam[row].abs() + c64[row].abs())
+    assert bool(((dw.double() - want).abs() <= room).all())
+    g.close()
