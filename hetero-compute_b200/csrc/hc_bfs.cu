@@ -408,11 +408,13 @@ union BfsShared {
 
 // kBlocks resident blocks per SM: two, or three for many sources at a time.  The
 // levels wait on dependent loads (issue slots 32 % used, DRAM 14 %), and with
-// enough teams to fill them a third block's warps are worth the spills they cost
-// (64 sources, Kronecker scale 22: 7.2 -> 6.0 ms, scale 16: 216 -> 205 us; but one
-// source at scale 22 253 -> 261 us, 64 at scale 10 90 -> 98 us).
-constexpr int kBfsWideSources = 4;
-constexpr int64_t kBfsWideEdges = 1ll << 20;
+// enough work to fill them a third block's warps are worth the spills they cost:
+// from kBfsWideWork edges times sources on, two sources at least.  Two / three
+// blocks in us: Kronecker scale 22, 1 source 273 / 283, 2 410 / 401, 16 2043 / 1606;
+// scale 20, 2 169 / 185, 4 220 / 214; scale 18, 8 160 / 166, 16 210 / 199; scale 16,
+// 16 123 / 130, 64 218 / 209; uniform 2^18 vertices, 4 194 / 197, 16 454 / 453; 2^16, 16
+// 134 / 136, 64 322 / 276.
+constexpr int64_t kBfsWideWork = 1ll << 26;
 template <bool kStats, int kBlocks>
 __global__ void __launch_bounds__(kBfsThreads, kBlocks) bfs_persistent(BfsArgs a) {
     __shared__ unsigned long long s_red[32];
@@ -955,7 +957,7 @@ extern "C" hc_status hc_bfs(hc_graph *g, const int32_t *sources, int32_t num_sou
                up(sizeof(int2) * (size_t)ntasks);
     }();
     int resident = 0;
-    const bool wide = !per_run && num_sources >= kBfsWideSources && g->M >= kBfsWideEdges;
+    const bool wide = !per_run && num_sources >= 2 && g->M * num_sources >= kBfsWideWork;
     HC_TRY((o.collect_stats ? bfs_resident<true, 2>(g, &resident)
             : wide          ? bfs_resident<false, 3>(g, &resident)
                             : bfs_resident<false, 2>(g, &resident)));

@@ -643,12 +643,16 @@ __device__ __forceinline__ void note_low(int32_t *p, int32_t x) {
 }
 
 // kBlocks resident blocks per SM: two, or three for many sources at a time on a
-// graph with hub rows, whose pulls wait on gathers (issue slots 32 % used, DRAM 20
-// %) and gain more from a third block's warps than its spills cost (16 sources,
-// Kronecker scale 22: 12.2 -> 10.7 ms, scale 20: 3.57 -> 3.28 ms; without hubs,
-// where the pushes' atomics are the work, 16 sources, uniform 2^18: 2.48 -> 2.98).
-constexpr int kSsspWideSources = 4;
-constexpr int64_t kSsspWideEdges = 1ll << 20;
+// large graph with hub rows, whose pulls wait on gathers (issue slots 32 % used,
+// DRAM 20 %) and gain more from a third block's warps than its spills cost: from
+// kSsspWideEdges edges and kSsspWideWork edges times sources on.  Two / three blocks
+// in ms: Kronecker scale 22, 2 sources 1.26 / 1.26, 8 4.98 / 4.54, 16 10.5 / 9.0; scale
+// 20, 4 0.90 / 0.93, 8 1.35 / 1.37, 16 2.73 / 2.66, 64 10.2 / 9.2; scale 19, 8 0.78 / 0.86,
+// 16 1.58 / 1.49; scale 18 (7.6M edges), 16 0.90 / 0.87, 64 2.62 / 2.75; scale 16, 16
+// 0.42 / 0.46; without hubs, where the pushes' atomics are the work, uniform 2^18, 16
+// sources 2.66 / 3.28.
+constexpr int64_t kSsspWideEdges = 1ll << 23;
+constexpr int64_t kSsspWideWork = 3ll << 26;
 template <bool kStats, int kBlocks>
 __global__ void __launch_bounds__(kSsspThreads, kBlocks) sssp_persistent(SsspArgs a) {
     __shared__ unsigned long long s_red[32];
@@ -1401,8 +1405,8 @@ extern "C" hc_status hc_sssp(hc_graph *g, const int32_t *sources, int32_t num_so
     // Parents and the range check read the distances after a launch: without
     // an output for them, one scratch row per source of a launch is kept.
     int resident = 0;
-    const bool wide = !per_run && num_sources >= kSsspWideSources && g->M >= kSsspWideEdges &&
-                      g->base_view.n_tasks > 0;
+    const bool wide = !per_run && num_sources >= 2 && g->M >= kSsspWideEdges &&
+                      g->M * num_sources >= kSsspWideWork && g->base_view.n_tasks > 0;
     HC_TRY((o.collect_stats ? sssp_resident<true, 2>(g, &resident)
             : wide          ? sssp_resident<false, 3>(g, &resident)
                             : sssp_resident<false, 2>(g, &resident)));

@@ -264,3 +264,36 @@ def test_bfs_scanned_edges(width, tail):
         _, _, st = g.bfs([src], stats=True)
         assert (st.vertices_scanned, st.edges_scanned) == scanned(index, nbr, g.info().num_active, src), src
     g.close()
+
+
+@pytest.mark.parametrize("kind,scale,counts", [("kronecker", 17, (17, 18, 19, 70)), ("uniform", 17, (15, 17, 33)),
+                                               ("kronecker", 19, (12, 13, 14, 33))])
+def test_many_sources_on_a_large_graph(kind, scale, counts):
+    """On both sides of the work from which three blocks an SM run: every source's rows equal those of its own call."""
+    import torch
+
+    import hc
+    g = hc.Graph.generate(hc.GEN_KRONECKER if kind == "kronecker" else hc.GEN_UNIFORM, scale, 16, 5, hc.W_I32)
+    n, m = g.num_nodes, g.num_edges
+    line = 1 << 26 if scale == 17 else 3 << 26
+    assert any(k * m < line for k in counts) and any(k * m >= line for k in counts)
+    src = g.pick_sources(max(counts))
+
+    def rows(k):
+        return [torch.full((k, n), 7, dtype=torch.int32, device="cuda") for _ in range(3)]
+
+    one = rows(len(src))
+    for i, s in enumerate(src):
+        g.bfs([s], one[0][i:i + 1], one[1][i:i + 1])
+        g.sssp([s], one[2][i:i + 1])
+    index, nbr, w = g.csr()
+    assert np.array_equal(one[0][0].cpu().numpy(), oracle.bfs_depth(index, nbr, src[0]))
+    assert np.array_equal(one[2][0].cpu().numpy(), oracle.sssp_dijkstra(index, nbr, w, src[0]))
+    for k in counts:
+        depth, parent, dist = rows(k)
+        g.bfs(src[:k], depth, parent)
+        g.sssp(src[:k], dist)
+        assert torch.equal(depth, one[0][:k]) and torch.equal(dist, one[2][:k])
+        for i in (0, k - 1):
+            assert oracle.verify_bfs_parents(index, nbr, depth[i].cpu().numpy(), parent[i].cpu().numpy(), src[i])[0] == 0
+    g.close()
