@@ -887,8 +887,7 @@ hc_status launch_bfs(hc_graph *g, BfsArgs &a, int teams) {
 }
 
 // Blocks per team and teams for k sources on a graph of m edges (at most `room`
-// teams), from sweeps of team
-// sizes on Kronecker and uniform graphs of 20k to 128M edges.  A team is no
+// teams), from sweeps of team sizes on Kronecker and uniform graphs of 20k to 128M edges.  A team is no
 // smaller than sqrt(m) / 300 blocks: below that the sources run at a time
 // outgrow the L2 (64 sources, 128M edges: 8 teams 7.6 ms, 12 teams 10.4 ms, 1
 // team 12.9 ms; 16 sources, 8M edges: 16 teams 0.41 ms, 1 team 1.45 ms).  It is
@@ -896,8 +895,8 @@ hc_status launch_bfs(hc_graph *g, BfsArgs &a, int teams) {
 // cost more than the blocks bring (one source, 20k edges: 8 blocks 79 us, 296
 // blocks 97 us; 8M edges: 148 blocks 108 us, 296 blocks 120 us).  Between the
 // two, as many teams as end the sources in the fewest rounds.
-void bfs_teams(const hc_graph *g, int resident, int k, int room, int *team, int *teams) {
-    const double root = std::sqrt((double)std::max<int64_t>(g->M, 1));
+void bfs_teams(int64_t m, int resident, int k, int room, int *team, int *teams) {
+    const double root = std::sqrt((double)std::max<int64_t>(m, 1));
     const int least = std::max(1, std::min(resident, (int)std::lround(root / 300.0)));
     const int most = std::max(1, std::min(resident, (int)std::lround(root / 19.0)));
     const int at_a_time = std::max(1, std::min({k, room, resident / least, kBfsLaunchSources}));
@@ -972,11 +971,13 @@ extern "C" hc_status hc_bfs(hc_graph *g, const int32_t *sources, int32_t num_sou
         if (host_depth || host_parent) HC_TRY(pipe.init(g, 2, 4 * n, teams));
         return HC_OK;
     };
-    if (!per_run) {
+    if (per_run) {
+        bfs_teams(g->M, resident, 1, 1, &team, &teams);
+    } else {
         // Bytes of one source at a time: workspace, staging (both arrays, two
         // slots), scratch rows of outputs nobody asked for.
         const size_t each = bytes + 4 * (size_t)n * ((host_depth || host_parent ? 4 : 0) + !depth_out + !parent_out);
-        bfs_teams(g, resident, num_sources, (int)std::min<size_t>(std::max<size_t>(kBfsTeamBytes / each, 1), 1 << 20),
+        bfs_teams(g->M, resident, num_sources, (int)std::min<size_t>(std::max<size_t>(kBfsTeamBytes / each, 1), 1 << 20),
                   &team, &teams);
     }
     hc_status reserved;
@@ -987,7 +988,7 @@ extern "C" hc_status hc_bfs(hc_graph *g, const int32_t *sources, int32_t num_sou
     if (reserved == HC_ERR_OOM) {  // no room: one source at a time, and what other calls left behind goes
         clear_error();
         if (teams > 1) {
-            bfs_teams(g, resident, num_sources, 1, &team, &teams);
+            bfs_teams(g->M, resident, num_sources, 1, &team, &teams);
             g->ws_bfs.release();
             if (!depth_out) g->ws_out0.release();
             if (!parent_out) g->ws_out1.release();
@@ -1282,7 +1283,10 @@ extern "C" hc_status hc_bfs_noalloc(const int64_t *index, const int32_t *neighbo
     a.parent = parent_out;
     a.nsrc = 1;
     a.src[0] = source;
-    a.team = sms * bps;
+    // The blocks that suit the graph's size: all that fit made every barrier dearer
+    // (Kronecker scale 16: 148 us with 296 blocks, 136 us so; scale 10: 110 and 91).
+    int teams = 1;
+    bfs_teams(num_edges, sms * bps, 1, 1, &a.team, &teams);
     a.alpha = 15;
     a.beta = 18;
     a.direction = 0;
@@ -1304,8 +1308,8 @@ extern "C" hc_status hc_bfs_noalloc(const int64_t *index, const int32_t *neighbo
     HC_CUDA_TRY(cudaMemsetAsync(a.fold, 0, sizeof(BfsFold), s));
     void *params[] = {&a};
     ::hc::count_launch();
-    HC_CUDA_TRY(cudaLaunchCooperativeKernel((void *)bfs_persistent<false, 2>, dim3(sms * bps), dim3(kBfsThreads), params,
-                                            0, s));
+    HC_CUDA_TRY(cudaLaunchCooperativeKernel((void *)bfs_persistent<false, 2>, dim3(a.team), dim3(kBfsThreads), params, 0,
+                                            s));
     int err = 0;
     HC_CUDA_TRY(cudaMemcpyAsync(&err, &a.ctl->gs.err, sizeof(int), cudaMemcpyDeviceToHost, s));
     HC_CUDA_TRY(cudaStreamSynchronize(s));
