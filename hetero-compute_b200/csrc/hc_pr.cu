@@ -985,9 +985,12 @@ hc_status launch_solve(hc_graph *g, const void *fn, int *blocks_per_sm, SweepArg
 // 0.85 ms, scale 12: 0.35 and 0.09 ms).  Where nearly every
 // row is in a stream group, from 3 x 2^20 edges (uniform, 2^18 vertices, rows of 16:
 // 0.32 and 0.38 ms; 2^19: 0.47 and 0.55, rows of 32: 0.65 and 0.78; but 2^17, rows of
-// 16: 0.26 and 0.22, and 2^18, rows of 24, a quarter of them single: 0.38 and 0.35).
+// 16: 0.26 and 0.22, and 2^18, rows of 24, a quarter of them single: 0.38 and 0.35);
+// from 2^18 vertices and 8 million edges whatever the rows (2^18, rows of 32: 0.42 and
+// 0.44 ms, Chebyshev weights 1.51 and 1.61; but 2^17, rows of 64: 0.31 and 0.27).
 bool launched_sweeps(const hc_graph *g, const PrPlanDev &plan) {
-    return plan.n_tasks == 0 && (g->M >= (1ll << 24) || (plan.n_long <= plan.n_stream && g->M >= (3ll << 20)));
+    return plan.n_tasks == 0 && (g->M >= (1ll << 24) || (plan.n_long <= plan.n_stream && g->M >= (3ll << 20)) ||
+                                 (g->n_active >= (1 << 18) && g->M >= 8000000));
 }
 
 using SolveFn = hc_status (*)(hc_graph *, SweepArgs &, const PrPlanDev &, volatile SolveOut *);
