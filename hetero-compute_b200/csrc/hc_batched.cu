@@ -598,9 +598,9 @@ hc_status run_msbfs(hc_graph *g, const MsPlan &plan, const int32_t *d_src, int n
     // building one takes 0.2 ms, more than the launches of a short loop
     // (Kronecker scale 12, 64 sources, 6 levels: 596 us with a graph, 389 us with
     // a look per level).
-    constexpr int kLaunchRound = 4, kLaunchLevels = 16;
+    constexpr int kLaunchRound = 4, kLaunchLevels = 12;
     bool ended = false;
-    if (o.use_graph != HC_GRAPH_ON && o.use_graph != HC_GRAPH_OFF && !trace) {
+    if (o.use_graph != HC_GRAPH_ON && o.use_graph != HC_GRAPH_OFF && !trace && !long_loop(g)) {
         for (int level = 0; !ended && level < kLaunchLevels; level += kLaunchRound) {
             for (int k = 0; k < kLaunchRound; k++) launch_level(g->stream, k & 1, 0, 0);
             ::hc::count_launch(kLaunchRound * per_level);
@@ -613,7 +613,7 @@ hc_status run_msbfs(hc_graph *g, const MsPlan &plan, const int32_t *d_src, int n
     if (ended) {
     } else if (o.use_graph != HC_GRAPH_OFF && !trace) {
         // The graph's body is two levels (parity 0 then 1).
-        const int done_levels = o.use_graph == HC_GRAPH_ON ? 0 : hctl->level;
+        const int done_levels = o.use_graph == HC_GRAPH_ON || long_loop(g) ? 0 : hctl->level;
         WhileGraph wg;
         auto body = [&](cudaStream_t cs, cudaGraphConditionalHandle cond) {
             launch_level(cs, 0, cond, 1);

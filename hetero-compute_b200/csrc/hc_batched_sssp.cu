@@ -186,6 +186,12 @@ __device__ __forceinline__ int ctl_queue(const MsspCtl *ctl, int c) { return ctl
 __device__ __forceinline__ bool ctl_pull(const MsspCtl *ctl, int c) {
     return ctl->pull_alpha > 0 && (double)ctl->qedges[c] * ctl->pull_alpha > (double)ctl->m;
 }
+// Whether the epoch notes the smallest distances it writes, for a pull after it:
+// not a push of few edges (on a grid graph every epoch is one), after which a
+// pull, should it come, takes 0 for them.
+__device__ __forceinline__ bool ctl_notes(const MsspCtl *ctl, int c) {
+    return ctl->pull_alpha > 0 && (double)ctl->qedges[c] * ctl->pull_alpha * 16.0 > (double)ctl->m;
+}
 
 // Folds a thread's running maximum of written halfwords into ctl->maxw (one
 // atomic per warp; every lane of the warp calls it).
@@ -428,6 +434,7 @@ __global__ void __launch_bounds__(256) mssp_epoch(const int64_t *index, const in
                                                   unsigned long long *relaxed, int32_t *low_parts) {
     const int nq = ctl_queue(ctl, c);
     if (nq == 0 || ctl_pull(ctl, c)) return;
+    const bool notes = ctl_notes(ctl, c);
     int *qnext_len = &ctl->qlen[c ^ 1];
     int *ntasks = &ctl->ntasks;
     const int lane = threadIdx.x & 31;
@@ -454,7 +461,7 @@ __global__ void __launch_bounds__(256) mssp_epoch(const int64_t *index, const in
         relax_range<D, SPL>(index, nbr, w, dist, m, du, b, e, act_next, qnext, qnext_len, rel, qe, wmax, mylow);
     }
     note_flush<D>(ctl, wmax);
-    low_flush<D, SPL>(low_parts, mylow);
+    if (notes) low_flush<D, SPL>(low_parts, mylow);
     rel = warp_sum(rel);
     qe = warp_sum(qe);
     if (lane == 0 && rel) atomicAdd(relaxed, rel);
@@ -468,6 +475,7 @@ __global__ void __launch_bounds__(256) mssp_tasks(const int64_t *index, const in
                                                   unsigned long long *relaxed, int32_t *low_parts) {
     const int nq = ctl_queue(ctl, c);
     if (nq == 0 || ctl_pull(ctl, c)) return;
+    const bool notes = ctl_notes(ctl, c);
     int *qnext_len = &ctl->qlen[c ^ 1];
     const int lane = threadIdx.x & 31;
     const int gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -489,7 +497,7 @@ __global__ void __launch_bounds__(256) mssp_tasks(const int64_t *index, const in
         relax_range<D, SPL>(index, nbr, w, dist, m, du, b, e, act_next, qnext, qnext_len, rel, qe, wmax, mylow);
     }
     note_flush<D>(ctl, wmax);
-    low_flush<D, SPL>(low_parts, mylow);
+    if (notes) low_flush<D, SPL>(low_parts, mylow);
     rel = warp_sum(rel);
     qe = warp_sum(qe);
     if (lane == 0 && rel) atomicAdd(relaxed, rel);
@@ -725,8 +733,14 @@ __global__ void mssp_clear(const int32_t *q, uint32_t *act, const MsspCtl *ctl, 
 // it sets the while node's condition.
 __global__ void mssp_end(MsspCtl *ctl, int c, int32_t *lows, int32_t *parts, int count, int32_t inf,
                          cudaGraphConditionalHandle cond, int use_cond) {
+    const bool notes = ctl_notes(ctl, c);
+    __syncthreads();  // thread 0 clears what that was read from
     if (threadIdx.x >= 32) {
         for (int i = threadIdx.x - 32; i < count; i += blockDim.x - 32) {
+            if (!notes) {
+                lows[i] = 0;
+                continue;
+            }
             int32_t m = inf;
 #pragma unroll
             for (int k = 0; k < kLowParts; k++) m = min(m, parts[k * count + i]);
@@ -888,10 +902,11 @@ hc_status run_group(hc_graph *g, const int32_t *h_src, int k, int32_t *dst, int 
     HC_CUDA_TRY(cudaGetLastError());
     const bool trace = std::getenv("HC_TRACE") != nullptr;
     // As the batched BFS's loop: plain launches in rounds first, a graph when
-    // kLaunchEpochs epochs have not ended it.
-    constexpr int kLaunchRound = 4, kLaunchEpochs = 40;
+    // kLaunchEpochs epochs have not ended it, or at once on a graph of short rows.
+    constexpr int kLaunchRound = 4, kLaunchEpochs = 32;
     bool ended = false;
-    if (use_graph != HC_GRAPH_ON && use_graph != HC_GRAPH_OFF && !trace && !eg.exec) {
+    if (use_graph != HC_GRAPH_ON && use_graph != HC_GRAPH_OFF && !trace && !eg.exec &&
+        !long_loop(g)) {
         for (int ep = 0; !ended && ep < kLaunchEpochs; ep += kLaunchRound) {
             for (int k = 0; k < kLaunchRound; k++) launch_epoch<D, SPL>(g, g->stream, b, k & 1, relaxed, 0, 0);
             ::hc::count_launch(kLaunchRound * kEpochLaunches);
@@ -906,7 +921,7 @@ hc_status run_group(hc_graph *g, const int32_t *h_src, int k, int32_t *dst, int 
     } else if (use_graph != HC_GRAPH_OFF && !trace) {
         // The graph's body is two epochs (parity 0 then 1); kernels of an
         // epoch whose queue is empty return at once.
-        const int before = use_graph == HC_GRAPH_ON || eg.exec ? 0 : hctl->epochs;
+        const int before = use_graph == HC_GRAPH_ON || eg.exec || long_loop(g) ? 0 : hctl->epochs;
         if (!eg.exec) {
             auto body = [&](cudaStream_t cs, cudaGraphConditionalHandle cond) {
                 launch_epoch<D, SPL>(g, cs, b, 0, relaxed, cond, 1);

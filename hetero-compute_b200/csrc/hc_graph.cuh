@@ -219,6 +219,11 @@ const float *pr_weights(const hc_graph *g);
 // g->spmm_partial_slots).
 enum : unsigned { kPlanPr = 1u, kPlanBase = 2u, kPlanSpmm = 4u };
 hc_status ensure_plans(hc_graph *g, unsigned which);
+// Whether a batched loop left to choose becomes a CUDA graph at once: on a graph of
+// at most 8 edges a row, road-like, it runs hundreds of epochs (33 sources on a 60 x
+// 70 grid: batched SSSP 3.0 ms with a graph, 3.6 with launches first, BFS 2.5 and
+// 2.6).
+inline bool long_loop(const hc_graph *g) { return g->M <= 8ll * g->n_active; }
 // Computes w_negative, w_max, w_mean and w_symmetric once (int32 weights).
 hc_status ensure_weight_stats(hc_graph *g);
 // Per-run control traffic kept off the copy engines.  A host-output call

@@ -297,3 +297,23 @@ def test_many_sources_on_a_large_graph(kind, scale, counts):
         for i in (0, k - 1):
             assert oracle.verify_bfs_parents(index, nbr, depth[i].cpu().numpy(), parent[i].cpu().numpy(), src[i])[0] == 0
     g.close()
+
+
+@pytest.mark.parametrize("rows,cols", [(3, 5), (40, 41)])
+@pytest.mark.parametrize("alpha", [0, -1, 3, 1 << 20])
+def test_batched_loops_on_short_rows(rows, cols, alpha):
+    """Road-like graphs: the batched loops are a graph from the start, most pushes note no minima, and a pull may
+    follow one that did not."""
+    import hc
+    h = hc.gen_grid(rows, cols, 3, wtype=hc.W_I32)
+    g = hc.Graph.from_host(h)
+    sources = np.random.default_rng(rows).integers(0, h.num_nodes, 70).astype(np.int32)
+    for bits in (0, 32):
+        for use_graph in (hc.GRAPH_AUTO, hc.GRAPH_OFF):
+            dist, _ = g.sssp_batched(sources, switch_alpha=alpha, dist_bits=bits, use_graph=use_graph)
+            for i in (0, 33, 69):
+                assert np.array_equal(dist[i], oracle.sssp_dijkstra(h.index, h.neighbors, h.weights, sources[i]))
+    depth, _ = g.bfs_batched(sources)
+    for i in (0, 33, 69):
+        assert np.array_equal(depth[i], oracle.bfs_depth(h.index, h.neighbors, sources[i]))
+    g.close()
