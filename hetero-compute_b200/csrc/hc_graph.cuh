@@ -164,11 +164,11 @@ hc_status activate(hc_graph *g);
 hc_status after_default_stream(hc_graph *g);
 // Builds inv_deg (and, for weighted graphs, inv_wsum / wtn) if missing.
 hc_status ensure_pr_derived(hc_graph *g, bool weighted);
-// Per-source outputs bound for host memory, double-buffered: source i writes
-// staging slot i & 1 on the compute stream, and its copy to the caller runs
-// on a copy stream while the next source computes (overlapped when the
-// destination is pinned).  Before a slot is written again the compute stream
-// waits for that slot's previous copy.
+// Outputs bound for host memory, double-buffered: launch i of a call writes the
+// rows of its sources to staging slot i & 1 on the compute stream, and their copy
+// to the caller runs on a copy stream while the next launch computes (overlapped
+// when the destination is pinned).  Before a slot is written again the compute
+// stream waits for that slot's previous copy.
 struct OutPipe {
     hc_graph *g = nullptr;
     int narr = 0;
@@ -180,12 +180,11 @@ struct OutPipe {
     void *pend_dst[2] = {nullptr, nullptr};
     // Staging and events for `arrays` outputs of up to `rows` rows of `each` bytes.
     hc_status init(hc_graph *graph, int arrays, size_t each, int rows = 1);
-    // Staging buffers of source i (after the wait for the slot's last copy).
+    // Staging buffers of launch i (after the wait for the slot's last copy).
     hc_status acquire(int i, int32_t **bufs);
-    // Source i's results are complete on the compute stream once what is
-    // queued there has run; copy them to dst[] (null entries are skipped).
-    // The copy is issued by the next acquire or by finish.
-    // `rows` consecutive rows of each array.
+    // Launch i's results are complete on the compute stream once what is queued
+    // there has run; copy `rows` consecutive rows of each array to dst[] (null
+    // entries are skipped).  The copy is issued by the next acquire or by finish.
     hc_status release(int i, void *const *dst, int rows = 1);
     hc_status flush();
     // Releases the staging (no copy in flight).

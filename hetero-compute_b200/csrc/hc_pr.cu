@@ -1381,6 +1381,35 @@ hc_status run_cg(hc_graph *g, const PrPlanDev &plan, bool weighted, const float 
     return HC_OK;
 }
 
+// A multi-column call whose workspace cannot be had (columns are padded to a
+// multiple of four, five matrices of them): its columns in two halves, each a call
+// of its own into a matrix on the device, from where they go to their places.
+template <class F>
+hc_status columns_in_halves(hc_graph *g, int K, float *scores, hc_pr_stats *stats, F solve) {
+    const int64_t n = g->N;
+    g->ws_pr.release();
+    hc_pr_stats all{};
+    all.converged = 1;
+    for (int c0 = 0, h = 0; h < 2; h++) {
+        const int k = h == 0 ? (K + 1) / 2 : K - c0;
+        DevBuf out;
+        HC_TRY(out.ensure((size_t)n * k * 4));
+        hc_pr_stats st{};
+        HC_TRY(solve(c0, k, out.as<float>(), &st));
+        HC_CUDA_TRY(cudaMemcpy2DAsync(scores + c0, (size_t)K * 4, out.ptr, (size_t)k * 4, (size_t)k * 4, n,
+                                      cudaMemcpyDefault, g->stream));
+        HC_CUDA_TRY(cudaStreamSynchronize(g->stream));
+        all.iterations = std::max(all.iterations, st.iterations);
+        all.converged = all.converged && st.converged;
+        all.residual_l1 = std::max(all.residual_l1, st.residual_l1);
+        all.ms += st.ms;
+        all.bytes_model += st.bytes_model;
+        c0 += k;
+    }
+    if (stats) *stats = all;
+    return HC_OK;
+}
+
 void fill_opts(const hc_pr_opts *opts, hc_pr_opts *o) {
     hc_pr_opts d{};
     if (opts) d = *opts;
@@ -1428,7 +1457,18 @@ extern "C" hc_status hc_pr_forward(hc_graph *g, const float *teleport, int32_t n
         const size_t slots = (size_t)g->spmm_partial_slots + 1;
         const size_t bytes = 5 * nk * sizeof(float) + slots * S * sizeof(float) +
                              (size_t)(g->spmm_view.n_hub + 1) * 4 + (size_t)S * 8 + 4096;
-        HC_TRY(g->ws_pr.ensure(bytes));
+        const hc_status room = g->ws_pr.ensure(bytes);
+        if (room == HC_ERR_OOM) {
+            clear_error();
+            return columns_in_halves(g, K, scores_out, stats, [&](int c0, int k, float *out, hc_pr_stats *st) {
+                DevBuf t;
+                HC_TRY(t.ensure((size_t)n * k * 4));
+                HC_CUDA_TRY(cudaMemcpy2DAsync(t.ptr, (size_t)k * 4, teleport + c0, (size_t)K * 4, (size_t)k * 4, n,
+                                              cudaMemcpyDefault, g->stream));
+                return hc_pr_forward(g, t.as<float>(), k, out, opts, st);
+            });
+        }
+        HC_TRY(room);
         char *p = g->ws_pr.as<char>();
         auto take = [&](size_t b) {
             char *r = p;
@@ -1736,7 +1776,30 @@ extern "C" hc_status hc_ppr_batched(hc_graph *g, const int32_t *seed_offsets, co
     const size_t slots = std::max((size_t)g->spmm_partial_slots * S, (size_t)partial_slots) + S;
     const size_t counters = (size_t)std::max(g->spmm_view.n_hub, plan.n_hub) + 1;
     const size_t bytes = 4 * ns * sizeof(float) + slots * 4 + counters * 4 + (size_t)S * 8 + (size_t)n + (size_t)(nseeds + ncols + 1) * 4 + 5 * (size_t)n * 4 + 16384;
-    HC_TRY(g->ws_pr.ensure(bytes));
+    const hc_status room = g->ws_pr.ensure(bytes);
+    if (room == HC_ERR_OOM && K == 1) {  // one column: the solve of one column takes less
+        clear_error();
+        DevBuf t, idx;
+        HC_TRY(t.ensure((size_t)n * 4));
+        HC_TRY(idx.ensure((size_t)nseeds * 4));
+        HC_CUDA_TRY(cudaMemsetAsync(t.ptr, 0, (size_t)n * 4, g->stream));
+        HC_CUDA_TRY(cudaMemcpyAsync(idx.ptr, sd.data(), (size_t)nseeds * 4, cudaMemcpyHostToDevice, g->stream));
+        { spmm_column_base<<<4, 256, 0, g->stream>>>(idx.as<int32_t>(), 0, nseeds, 1.0f, t.as<float>()); ::hc::count_launch(); }
+        HC_CUDA_TRY(cudaGetLastError());
+        hc_pr_opts one = o;
+        one.eps_vertex = 0.f;
+        one.accel = 0;
+        return hc_pr_forward(g, t.as<float>(), 1, scores_out, &one, stats);
+    }
+    if (room == HC_ERR_OOM) {
+        clear_error();
+        return columns_in_halves(g, K, scores_out, stats, [&](int c0, int k, float *out, hc_pr_stats *st) {
+            std::vector<int32_t> part(k + 1);
+            for (int c = 0; c <= k; c++) part[c] = off[c0 + c] - off[c0];
+            return hc_ppr_batched(g, part.data(), sd.data() + off[c0], k, out, opts, st);
+        });
+    }
+    HC_TRY(room);
     char *p = g->ws_pr.as<char>();
     auto take = [&](size_t b) {
         char *r = p;

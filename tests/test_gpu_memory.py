@@ -120,3 +120,48 @@ def test_host_outputs_when_staging_does_not_fit(weighted20, op, room_mb):
         torch.cuda.empty_cache()
     assert np.array_equal(got, depth if op == "bfs" else dist)
     g.close()
+
+
+@pytest.mark.parametrize("form,k", [("dense", 33), ("dense_host", 33), ("seeds", 33), ("seeds_weighted", 33),
+                                    ("seeds", 1)])
+def test_columns_when_the_workspace_does_not_fit(weighted20, form, k):
+    """Columns are padded to a multiple of four: a call whose padded matrices do not fit runs its columns in parts."""
+    torch = pytest.importorskip("torch")
+    host = weighted20[0]
+    n = host.num_nodes
+    g = hc.Graph.from_host(host)
+    opts = dict(tol_l1=1e-6, max_iters=100)
+    gen = torch.Generator("cuda").manual_seed(1)
+    if form.startswith("dense"):
+        t = torch.rand((n, k), generator=gen, device="cuda")
+        t /= t.sum(0)
+        out = torch.empty((n, k), device="cuda")
+        if form == "dense_host":
+            t, out = t.cpu().numpy(), np.empty((n, k), np.float32)
+
+        def call():
+            return g.pagerank(t, out, **opts)
+    else:
+        out = torch.empty((n, k), device="cuda")
+        seeds = weighted20[1][np.arange(3 * k) % 64].astype(np.int32)
+
+        def call():
+            return g.ppr_batched(np.arange(k + 1) * 3, seeds, out, weighted=form == "seeds_weighted", **opts)
+
+    want, st = call()
+    want = torch.as_tensor(want).clone().cpu()
+    assert st.converged
+    g.close()
+    g = hc.Graph.from_host(host)
+    g.pagerank(weighted=form == "seeds_weighted", max_iters=2)  # derived arrays
+    # All matrices of k columns but one (of half the columns they fit), or what one column's solve takes.
+    filler = _fill(torch, 4 * 4 * n * k if k > 1 else 4 * 13 * n)
+    try:
+        got, st = call()
+    finally:
+        del filler
+        torch.cuda.empty_cache()
+    assert st.converged
+    # Each run stops within tol d / (1 - d) of the fixed point in L1, per column.
+    assert float((torch.as_tensor(got).cpu() - want).abs().double().sum(0).max()) <= 2 * 1e-6 * 0.85 / 0.15 + 1e-5
+    g.close()
