@@ -727,10 +727,10 @@ __global__ void mssp_clear(const int32_t *q, uint32_t *act, const MsspCtl *ctl, 
 }
 
 // Closes epoch parity c (one block): all warps but the first fold the minima it
-// wrote into those that the next one reads; thread 0 counts it, resets its counters for reuse, and decides
-// whether another epoch runs (queue non-empty, under the epoch cap and the
-// time bound, and for narrow words inside the 16-bit range); inside a graph
-// it sets the while node's condition.
+// wrote into those that the next one reads; thread 0 counts it, resets its
+// counters for reuse, and decides whether another epoch runs (queue non-empty,
+// under the epoch cap and the time bound, and for narrow words inside the 16-bit
+// range); inside a graph it sets the while node's condition.
 __global__ void mssp_end(MsspCtl *ctl, int c, int32_t *lows, int32_t *parts, int count, int32_t inf,
                          cudaGraphConditionalHandle cond, int use_cond) {
     const bool notes = ctl_notes(ctl, c);

@@ -90,9 +90,12 @@ __device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long
 // one acquire follows the last: an acquire drops the SM's L1 lines, which the
 // SM's other blocks may still be gathering from.  Waiters poll back to back at
 // first, since a level of a sparse frontier ends within a few round trips, then
-// sleep between polls so that a long wait leaves the L2 slice alone.  They give up after the wait limit, setting *err.  Once *err is
-// set every later barrier returns at once, so a failed run drains in bounded
-// time.  Returns false when the run must stop.
+// sleep between polls so that a long wait leaves the L2 slice alone (against
+// acquire polls 32 ns apart: 20 sweeps of the reference-order PageRank, hundreds to
+// thousands of barriers each, Kronecker scale 10 8.9 -> 8.3 ms, scale 16 115.5 ->
+// 111.4, 300 x 300 grid 20.7 -> 18.4).  They give up after the wait limit, setting
+// *err.  Once *err is set every later barrier returns at once, so a failed run
+// drains in bounded time.  Returns false when the run must stop.
 struct GridSync {
     unsigned long long count;
     int err;
