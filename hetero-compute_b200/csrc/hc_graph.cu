@@ -180,7 +180,8 @@ hc_status OutPipe::flush() {
     pending = false;
     const int s = pend_slot;
     HC_CUDA_TRY(cudaStreamWaitEvent(g->copy_stream, g->ev_ready[s], 0));
-    // A 2-D copy takes pitches below 2^31 bytes only; a row may be longer.
+    // A 2-D copy's pitch is limited to 2^31 - 1 bytes, and a row may be longer (the
+    // present driver lets a single such row through; the limit is the documented one).
     const bool rows_apart = pend_rows == 1 || bytes > (size_t)INT32_MAX;
     for (int j = 0; j < narr; j++) {
         if (!pend_dst[j]) continue;
